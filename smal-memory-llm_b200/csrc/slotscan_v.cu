@@ -8,17 +8,28 @@
 //   dw = <v - V, dV'> + (1 - o) do',  dv = sum_n w dV',  dg = a . dw,  dz = a_s (g_h dw - a_s . g_h dw),  dwa = dz,
 //   dfr -= o . dz,  dV = (1 - w) dV' + dbuf,  do = (1 - w) do' - fr dz.
 //
-// One CTA per (sequence, head), values and occupancy resident in shared memory (the reference's shape is 48 x 16).
+// The address of a token depends on the occupancies alone, never on the values, and the values are linear in the known
+// addresses.  Only the occupancy recurrence is a chain over the tokens; everything that is wide is split off from it:
+//   forward   one warp per (sequence, head) runs the occupancies (rows in registers, 2 per lane at 64 rows) and hands the
+//             write weights over in chunks of tokens; eight warps of the same CTA apply them to the values, a chunk behind
+//   backward  the addresses again from the emitted occupancies, every block of G tokens at once (keyless_tables); the
+//             value gradients block by block (row_adjoint_kernel); then the chain of the occupancy gradient alone, one
+//             warp per (sequence, head) (keyless_bwd_chain)
+// Bound: the occupancy chain, one double-precision exp, sum over the rows and division per token.  B = 8, T = 512, H = 8,
+// 64 x 64, G = 4, forward + backward: 12.9 ms walking token by token in one CTA (2.35 + 10.4), 0.90 ms split (forward 0.43;
+// backward: tables 0.02, value gradients 0.31, chain 0.12).
 // The occupancies and the softmax run in double: with the penalty on o itself every rounding error of o comes back
-// multiplied by fr at every later token.  The emitted buffers (values, and occupancies as a second output) are the
-// backward's checkpoints: per block of G tokens it replays the forward into G state slots of scratch, then walks the
-// block in reverse.  Like the general keyed scan this mode is built for completeness of the reference's call surface
-// (no model of the reference run calls it) and is not tuned.
+// multiplied by fr at every later token.
+// More than 256 rows (the reference's shape is 48 x 16) keep the kernels below that hold everything in one CTA and walk
+// token by token.
 #include <math.h>
 #include <stdio.h>
 
+#include <algorithm>
+
 #include "slotscan_common.cuh"
 #include "slotscan_launch.h"
+#include "slotscan_rowadj.cuh"
 
 namespace slotscan {
 
@@ -264,6 +275,413 @@ __global__ void __launch_bounds__(256) keyless_finish_kernel(const float* __rest
     }
 }
 
+// ---- up to 256 rows: lane l of a warp holds rows l, l + 32, ... ----
+constexpr int KL_CT = 16;                                   // tokens per chunk handed from the chain to the value warps
+constexpr int KL_CW = 8;                                    // value warps
+
+// e[i] = exp(z_n - max z), returns the sum over the rows; am: the first row of the largest z.  zmax over finite and
+// infinite z alike; a NaN never wins, as in the token-by-token kernels.
+template <int R>
+__device__ __forceinline__ double kl_softmax(const float (&wa)[R], const double (&o)[R], int N, double fr, double (&e)[R],
+                                             int& am, bool soft = true) {
+    const int lane = threadIdx.x & 31;
+    double bz = -INFINITY;
+    int bi = BIGI;
+#pragma unroll
+    for (int i = 0; i < R; i++) {
+        const int n = lane + 32 * i;
+        e[i] = (double)wa[i] - fr * o[i];
+        if (n < N && e[i] > bz) { bz = e[i]; bi = n; }
+    }
+    // largest z through its order-preserving 64-bit key: two integer warp maxima instead of five 64-bit shuffle rounds
+    const long long zb = __double_as_longlong(bz + 0.0);    // -0 -> +0: equal values have one key
+    const unsigned long long key = (unsigned long long)(zb ^ ((zb >> 63) | (long long)0x8000000000000000ull));
+    const unsigned hi = (unsigned)(key >> 32), mhi = __reduce_max_sync(FULL, hi);
+    const unsigned mlo = __reduce_max_sync(FULL, hi == mhi ? (unsigned)key : 0u);
+    const bool mine = hi == mhi && (unsigned)key == mlo;
+    const unsigned long long mk = ((unsigned long long)mhi << 32) | mlo;
+    const double zmax = __longlong_as_double((mk >> 63) ? (long long)(mk ^ 0x8000000000000000ull) : (long long)~mk);
+    am = min((int)__reduce_min_sync(FULL, (unsigned)((bi != BIGI && mine) ? bi : BIGI)), N - 1);
+    if (!soft) return 1.0;                                  // the argmax is all that is asked for
+    double se = 0.0;
+#pragma unroll
+    for (int i = 0; i < R; i++) {
+        if (lane + 32 * i < N) { e[i] = exp(e[i] - zmax); se += e[i]; }
+    }
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) se += __shfl_xor_sync(FULL, se, off);
+    return se;
+}
+
+// 1 / s for a positive normal s: the hardware's approximation (about 20 bits) and one cubic Newton-Raphson step.
+__device__ __forceinline__ double kl_rcp(double s) {
+    double r;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(s));
+    const double t = fma(-s, r, 1.0);
+    return fma(r, fma(t, t, t), r);
+}
+
+// Warp 0: the chain.  Warp 1: what of a token's address does not depend on the occupancies -- exp(wa_n - max wa), a chunk
+// ahead -- so that the chain is exp(-fr o_n), one sum, one reciprocal and the blend.  Warps 2..9: the values, a chunk
+// behind.  The factors neither overflow nor vanish while |fr| <= 300 and the gates stay in [0, 1] (o in [0, 1]); anything
+// else takes the shifted softmax of kl_softmax.  hard: the chain needs the largest wa_n - fr o_n only.
+template <typename Tin, int R>
+__global__ void __launch_bounds__(32 * (2 + KL_CW), 2) keyless_fwd_chain_kernel(
+    const slotscan_v_params p, const Tin* __restrict__ v, const float* __restrict__ wa, const float* __restrict__ gate,
+    const float* __restrict__ fr_p, float* __restrict__ buf, float* __restrict__ obuf, int* __restrict__ addr) {
+    extern __shared__ __align__(16) float ksm[];
+    constexpr int NR = 32 * R;
+    const int N = p.N, T = p.T, H = p.H, DV = p.DV, G = p.G, NB = (T + G - 1) / G;
+    const int N4 = (N + 3) & ~3, NG = N4 / 4;
+    double* X = reinterpret_cast<double*>(ksm);             // [2][KL_CT][NR] exp(wa - max wa); hard: wa
+    float* gs = reinterpret_cast<float*>(X + 2 * KL_CT * NR);        // [2][KL_CT] gates
+    int* wild = reinterpret_cast<int*>(gs + 2 * KL_CT);     // [2] a gate of the chunk lies outside [0, 1]
+    float* wbuf = gs + 2 * KL_CT + 4;                       // [2][KL_CT][N4] write weights, 0 = row not written
+    float* V = wbuf + 2 * KL_CT * N4;                       // [N4][DV]
+    const int bh = blockIdx.x, b = bh / H, h = bh % H;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, ct = tid - 64;
+    const double fr = (double)fr_p[0];
+    const int NC = (T + KL_CT - 1) / KL_CT;
+    double o[R], e[R];
+#pragma unroll
+    for (int i = 0; i < R; i++) o[i] = 0.0;
+    bool slow = !(fabs(fr) <= 300.0);
+    int ph = 0, jb = 0;                                     // chain: token's place in its block, block
+    for (int i = ct; i < N4 * DV && ct >= 0; i += 32 * KL_CW) V[i] = 0.f;
+    // value threads: column and first group of four rows; with more columns than threads every thread walks all rows
+    const int per = DV <= 32 * KL_CW ? 32 * KL_CW / DV : 1;
+    const int dl = ct < 0 ? 0 : (DV <= 32 * KL_CW ? ct % DV : ct), gl = ct < 0 || DV > 32 * KL_CW ? 0 : ct / DV;
+    const int gstep = per, NGt = gl < per ? NG : 0;                // threads past the last whole set of columns idle
+    float xn[KL_CT];
+    auto fetch_v = [&](int t0) {
+#pragma unroll
+        for (int j = 0; j < KL_CT; j++) xn[j] = t0 + j < T ? ldv(v + (((size_t)b * T + t0 + j) * H + h) * DV + dl) : 0.f;
+    };
+    if (ct >= 0 && DV <= 32 * KL_CW) fetch_v(0);
+    for (int c = -1; c <= NC; c++) {
+        if (warp == 0) {
+            if (c >= 0 && c < NC) {
+                float* wr = wbuf + (c & 1) * KL_CT * N4;
+                const double* Xc = X + (c & 1) * KL_CT * NR + lane;
+                slow |= wild[c & 1] != 0;
+                const int cn = min(KL_CT, T - c * KL_CT);
+                for (int j = 0; j < cn; j++) {
+                    const size_t ix = ((size_t)b * T + c * KL_CT + j) * H + h;
+                    const float g = gs[(c & 1) * KL_CT + j];
+                    if (ph == 0) {
+                        const size_t so = ((size_t)b * NB + jb) * H + h;
+#pragma unroll
+                        for (int i = 0; i < R; i++) if (lane + 32 * i < N) obuf[so * N + lane + 32 * i] = (float)o[i];
+                    }
+                    if (++ph == G) { ph = 0; jb++; }
+                    int am = 0;
+                    double si;
+                    if (slow || p.hard) {
+                        float la[R];
+#pragma unroll
+                        for (int i = 0; i < R; i++) la[i] = lane + 32 * i < N ? (p.hard ? (float)Xc[j * NR + 32 * i] : wa[ix * N + lane + 32 * i]) : 0.f;
+                        si = 1.0 / kl_softmax<R>(la, o, N, fr, e, am, !p.hard);
+                    } else {
+                        double se = 0.0;
+#pragma unroll
+                        for (int i = 0; i < R; i++) {
+                            e[i] = Xc[j * NR + 32 * i] * exp(-fr * o[i]);          // rows past N: X = 0
+                            se += e[i];
+                        }
+#pragma unroll
+                        for (int off = 16; off > 0; off >>= 1) se += __shfl_xor_sync(FULL, se, off);
+                        si = kl_rcp(se);
+                    }
+#pragma unroll
+                    for (int i = 0; i < R; i++) {
+                        const int n = lane + 32 * i;
+                        const float a = p.hard ? (n == am ? 1.f : 0.f) : (float)(e[i] * si);
+                        const double w = (double)g * (double)a;
+                        if (a != 0.f) o[i] = (1.0 - w) * o[i] + w;
+                        if (n < N4) wr[j * N4 + n] = n < N ? g * a : 0.f;
+                    }
+                    if (addr != nullptr) {
+                        if (!p.hard && !slow) {                      // the argmax, for the caller's log only
+                            double be = -1.0;
+                            int bi = BIGI;
+#pragma unroll
+                            for (int i = 0; i < R; i++) if (lane + 32 * i < N && e[i] > be) { be = e[i]; bi = lane + 32 * i; }
+                            const unsigned hi = (unsigned)(__double_as_longlong(be) >> 32) ^ 0x80000000u, lo = (unsigned)__double_as_longlong(be);
+                            const unsigned mhi = __reduce_max_sync(FULL, hi), mlo = __reduce_max_sync(FULL, hi == mhi ? lo : 0u);
+                            am = min((int)__reduce_min_sync(FULL, (unsigned)(hi == mhi && lo == mlo ? bi : BIGI)), N - 1);
+                        }
+                        if (lane == 0) addr[ix] = am;
+                    }
+                }
+            }
+        } else if (warp == 1) {
+            if (c + 1 < NC) {
+                const int bf = (c + 1) & 1, t0 = (c + 1) * KL_CT;
+                double* Xc = X + bf * KL_CT * NR + lane;
+                if (lane < KL_CT) {
+                    const float g = t0 + lane < T ? gate_eff(gate[((size_t)b * T + t0 + lane) * H + h], p.hard_gate) : 0.f;
+                    gs[bf * KL_CT + lane] = g;
+                    const unsigned any = __ballot_sync(0xffffu, !(g >= 0.f && g <= 1.f));
+                    if (lane == 0) wild[bf] = any != 0u;
+                }
+                for (int j = 0; j < KL_CT; j += 4) {                 // four tokens' loads in flight
+                    float la[4][R];
+#pragma unroll
+                    for (int u = 0; u < 4; u++)
+#pragma unroll
+                        for (int i = 0; i < R; i++)
+                            la[u][i] = (t0 + j + u < T && lane + 32 * i < N) ? wa[(((size_t)b * T + t0 + j + u) * H + h) * N + lane + 32 * i] : -INFINITY;
+#pragma unroll
+                    for (int u = 0; u < 4; u++) {
+                        float m = -INFINITY;
+#pragma unroll
+                        for (int i = 0; i < R; i++) m = fmaxf(m, la[u][i]);
+#pragma unroll
+                        for (int off = 16; off > 0; off >>= 1) m = fmaxf(m, __shfl_xor_sync(FULL, m, off));
+#pragma unroll
+                        for (int i = 0; i < R; i++)
+                            Xc[(j + u) * NR + 32 * i] = p.hard ? (double)la[u][i] : (lane + 32 * i < N ? exp((double)la[u][i] - (double)m) : 0.0);
+                    }
+                }
+            }
+        } else if (c > 0) {
+            const int t0 = (c - 1) * KL_CT, cn = min(KL_CT, T - t0), ph0 = t0 % G, jb0 = t0 / G;
+            const float* wr = wbuf + ((c - 1) & 1) * KL_CT * N4;
+            // a thread keeps its column, so that a token's value is loaded once for all its rows, a chunk ahead of its use;
+            // 4 rows at a time
+            for (int d = dl; d < DV; d += 32 * KL_CW) {
+                float xv[KL_CT];
+                bool odd = p.hard != 0;                            // a row a token does not write must not see it: only an
+#pragma unroll
+                for (int j = 0; j < KL_CT; j++) {                  // infinite or NaN value would tell
+                    xv[j] = DV <= 32 * KL_CW ? xn[j] : (j < cn ? ldv(v + (((size_t)b * T + t0 + j) * H + h) * DV + d) : 0.f);
+                    odd |= !(fabsf(xv[j]) <= 3e38f);
+                }
+                if (DV <= 32 * KL_CW) fetch_v(t0 + KL_CT);
+                for (int ng = gl; ng < NGt; ng += gstep) {
+                    const int n0 = ng * 4;
+                    float s[4];
+#pragma unroll
+                    for (int i = 0; i < 4; i++) s[i] = V[(n0 + i) * DV + d];
+                    int q = ph0, k = jb0;
+#pragma unroll
+                    for (int j = 0; j < KL_CT; j++) {
+                        if (j < cn) {
+                            if (q == 0) {                          // the pre-write state, every G tokens
+                                float* out = buf + ((((size_t)b * NB + k) * H + h) * N + n0) * DV + d;
+#pragma unroll
+                                for (int i = 0; i < 4; i++) if (n0 + i < N) out[(size_t)i * DV] = s[i];
+                            }
+                            if (++q == G) { q = 0; k++; }
+                            const float4 w = ld4(wr + j * N4 + n0);
+                            const float wv[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+                            for (int i = 0; i < 4; i++) {
+                                const float t = fmaf(wv[i], xv[j], (1.f - wv[i]) * s[i]);
+                                s[i] = odd && wv[i] == 0.f ? s[i] : t;
+                            }
+                        }
+                    }
+#pragma unroll
+                    for (int i = 0; i < 4; i++) V[(n0 + i) * DV + d] = s[i];
+                }
+            }
+        }
+        __syncthreads();
+    }
+}
+
+// The backward's tables: a warp per (sequence, block) runs the block's tokens from the emitted occupancies.
+template <int R>
+__global__ void __launch_bounds__(128) keyless_tables_kernel(const slotscan_v_params p, const float* __restrict__ wa,
+                                                             const float* __restrict__ gate, const float* __restrict__ fr_p,
+                                                             const float* __restrict__ obuf, int bh0, int nbh,
+                                                             float* __restrict__ as, float* __restrict__ ot, int* __restrict__ am) {
+    const int N = p.N, T = p.T, H = p.H, G = p.G, NB = (T + G - 1) / G, lane = threadIdx.x & 31;
+    const size_t wid = (size_t)blockIdx.x * 4 + (threadIdx.x >> 5);
+    if (wid >= (size_t)nbh * NB) return;
+    const int lb = (int)(wid / NB), jb = (int)(wid % NB), bh = bh0 + lb, b = bh / H, h = bh % H;
+    const int t0 = jb * G, t1 = min(T, t0 + G);
+    const double fr = (double)fr_p[0];
+    const size_t so = ((size_t)b * NB + jb) * H + h;
+    double o[R], e[R];
+    float cur[R];
+#pragma unroll
+    for (int i = 0; i < R; i++) {
+        const int n = lane + 32 * i;
+        o[i] = n < N ? (double)obuf[so * N + n] : 0.0;
+        cur[i] = n < N ? wa[(((size_t)b * T + t0) * H + h) * N + n] : 0.f;
+    }
+    for (int t = t0; t < t1; t++) {
+        const size_t ix = ((size_t)b * T + t) * H + h;
+        float la[R];
+#pragma unroll
+        for (int i = 0; i < R; i++) {
+            const int n = lane + 32 * i;
+            la[i] = cur[i];
+            cur[i] = (t + 1 < t1 && n < N) ? wa[(ix + H) * N + n] : 0.f;
+        }
+        int m;
+        const double si = 1.0 / kl_softmax<R>(la, o, N, fr, e, m);
+        const float g = gate_eff(gate[ix], p.hard_gate);
+#pragma unroll
+        for (int i = 0; i < R; i++) {
+            const int n = lane + 32 * i;
+            if (n < N) {
+                const float s = (float)(e[i] * si), a = p.hard ? (n == m ? 1.f : 0.f) : s;
+                as[((size_t)lb * T + t) * N + n] = s;
+                ot[((size_t)lb * T + t) * N + n] = (float)o[i];
+                const double w = (double)g * (double)a;
+                if (a != 0.f) o[i] = (1.0 - w) * o[i] + w;
+            }
+        }
+        if (lane == 0) am[(size_t)lb * T + t] = m;
+    }
+}
+
+// The chain of the backward: the occupancy gradient, token by token in reverse.  D: <v_t - V_n(t), dV_n> per token and row.
+template <int R>
+__global__ void __launch_bounds__(32) keyless_bwd_chain_kernel(const slotscan_v_params p, const float* __restrict__ gate,
+                                                               const float* __restrict__ fr_p, const float* __restrict__ as,
+                                                               const float* __restrict__ ot, const int* __restrict__ am,
+                                                               const float* __restrict__ D, int bh0,
+                                                               float* __restrict__ dwa, float* __restrict__ dgate,
+                                                               float* __restrict__ part) {
+    constexpr int PF = R <= 2 ? 8 : (R == 4 ? 4 : 2);       // tokens in flight
+    const int N = p.N, T = p.T, H = p.H, lane = threadIdx.x;
+    const int lb = blockIdx.x, bh = bh0 + lb, b = bh / H, h = bh % H;
+    const float fr = fr_p[0];
+    const bool hard = p.hard != 0;
+    const size_t tab = (size_t)lb * T * N + lane;
+    as += tab; ot += tab; D += tab;
+    dwa += ((size_t)b * T * H + h) * N + lane;
+    gate += (size_t)b * T * H + h;
+    dgate += (size_t)b * T * H + h;
+    am += (size_t)lb * T;
+    float dO[R], ca[PF][R], co[PF][R], cd[PF][R];
+    double f1 = 0.0;
+#pragma unroll
+    for (int i = 0; i < R; i++) dO[i] = 0.f;
+    auto fetch = [&](int u, int t) {
+        const size_t at = (size_t)t * N;
+#pragma unroll
+        for (int i = 0; i < R; i++) {
+            const bool in = t >= 0 && lane + 32 * i < N;    // rows past N: all zero, they add nothing below
+            ca[u][i] = in ? as[at + 32 * i] : 0.f;
+            co[u][i] = in ? ot[at + 32 * i] : 0.f;
+            cd[u][i] = in ? D[at + 32 * i] : 0.f;
+        }
+    };
+#pragma unroll
+    for (int u = 0; u < PF; u++) fetch(u, T - 1 - u);
+    for (int tw = T - 1; tw >= 0; tw -= 32) {               // gates and addresses of 32 tokens, one per lane
+        const float gl = tw - lane >= 0 ? gate_eff(gate[(size_t)(tw - lane) * H], p.hard_gate) : 0.f;
+        const int ml = (hard && tw - lane >= 0) ? am[tw - lane] : 0;
+        float dgl = 0.f;
+        for (int tb = 0; tb < 32 && tb <= tw; tb += PF) {
+#pragma unroll
+            for (int u = 0; u < PF; u++) {
+                const int t = tw - tb - u;
+                const float g = __shfl_sync(FULL, gl, tb + u);
+                const int m = hard ? __shfl_sync(FULL, ml, tb + u) : 0;
+                float dw[R], a[R], dg = 0.f, sa = 0.f;
+#pragma unroll
+                for (int i = 0; i < R; i++) {
+                    dw[i] = fmaf(1.f - co[u][i], dO[i], cd[u][i]);
+                    a[i] = hard ? (lane + 32 * i == m ? 1.f : 0.f) : ca[u][i];
+                    dg = fmaf(a[i], dw[i], dg);
+                    sa = fmaf(ca[u][i], g * dw[i], sa);
+                }
+                dg = warp_sum(dg);
+                sa = hard ? warp_sum(sa) : g * dg;
+#pragma unroll
+                for (int i = 0; i < R; i++) {
+                    const float z = ca[u][i] * (g * dw[i] - sa);
+                    if (t >= 0 && lane + 32 * i < N) dwa[(size_t)t * H * N + 32 * i] = z;
+                    f1 -= (double)co[u][i] * (double)z;
+                    dO[i] = fmaf(1.f - g * a[i], dO[i], -fr * z);
+                }
+                if (lane == tb + u) dgl = dg;
+                fetch(u, t - PF);
+            }
+        }
+        if (tw - lane >= 0) dgate[(size_t)(tw - lane) * H] = dgl;
+    }
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) f1 += __shfl_xor_sync(FULL, f1, off);
+    if (lane == 0) part[bh] = (float)f1;
+}
+
+// scratch of the split backward: the tables of `nbh` sequences at a time (as many as 2 GiB hold), then the sums
+struct KeylessScratch { size_t as, ot, am, dp, part, bytes; int nbh, nsl; };
+inline KeylessScratch keyless_scratch(const slotscan_v_params& p) {
+    KeylessScratch s;
+    const size_t BH = (size_t)p.B * p.H, tn = (size_t)p.T * p.N;
+    s.nsl = row_adjoint_slices(p.N, p.DV);
+    const size_t per = 4 * (tn * (2 + s.nsl) + p.T);
+    s.nbh = (int)std::min(std::min(BH, (size_t)65535), std::max((size_t)1, ((size_t)2 << 30) / per));
+    auto up = [](size_t x) { return (x + 255) & ~(size_t)255; };
+    s.as = 0;
+    s.ot = up(4 * tn * s.nbh);
+    s.dp = 2 * s.ot;
+    s.am = s.dp + up(4 * tn * s.nbh * s.nsl);
+    s.part = s.am + up(4 * (size_t)p.T * s.nbh);
+    s.bytes = s.part + 4 * BH;
+    return s;
+}
+inline size_t keyless_chain_smem(int N, int DV) {
+    const size_t n4 = (N + 3) & ~3, nr = N <= 32 ? 32 : (N <= 64 ? 64 : (N <= 128 ? 128 : 256));
+    return 8 * (2 * KL_CT * nr) + 4 * (2 * KL_CT + 4 + 2 * KL_CT * n4 + n4 * DV);
+}
+// the split kernels: rows in one warp's registers, and the forward's chunk of weights beside the values
+inline bool keyless_split(const slotscan_v_params& p) {
+    return p.N <= 256 && keyless_chain_smem(p.N, p.DV) <= 227 * 1024 && row_adjoint_slices(p.N, p.DV) <= 64;
+}
+#define KEYLESS_ROWS(N_, ...)                                \
+    if ((N_) <= 32) { constexpr int R = 1; __VA_ARGS__; }           \
+    else if ((N_) <= 64) { constexpr int R = 2; __VA_ARGS__; }      \
+    else if ((N_) <= 128) { constexpr int R = 4; __VA_ARGS__; }     \
+    else { constexpr int R = 8; __VA_ARGS__; }
+
+template <typename Tin>
+cudaError_t run_keyless_fwd(const slotscan_v_params& p, const Tin* v, const float* wa, const float* gate, const float* fr,
+                            float* buf, float* obuf, int* addr, cudaStream_t st) {
+    const size_t sm = keyless_chain_smem(p.N, p.DV);
+    cudaError_t e = cudaSuccess;
+    KEYLESS_ROWS(p.N, {
+        auto kern = keyless_fwd_chain_kernel<Tin, R>;
+        if ((e = opt_in_smem(kern, sm)) != cudaSuccess) return e;
+        kern<<<p.B * p.H, 32 * (2 + KL_CW), sm, st>>>(p, v, wa, gate, fr, buf, obuf, addr);
+    });
+    return cudaGetLastError();
+}
+
+template <typename Tin>
+cudaError_t run_keyless_bwd(const slotscan_v_params& p, const Tin* v, const float* wa, const float* gate, const float* fr,
+                            const float* buf, const float* obuf, const float* dbuf, char* scratch, Tin* dv, float* dwa,
+                            float* dgate, cudaStream_t st) {
+    const KeylessScratch s = keyless_scratch(p);
+    float *as = (float*)(scratch + s.as), *ot = (float*)(scratch + s.ot), *dp = (float*)(scratch + s.dp);
+    int* am = (int*)(scratch + s.am);
+    float* part = (float*)(scratch + s.part);
+    const int BH = p.B * p.H, NB = (p.T + p.G - 1) / p.G;
+    cudaError_t e;
+    for (int bh0 = 0; bh0 < BH; bh0 += s.nbh) {
+        const int nbh = std::min(s.nbh, BH - bh0);
+        const size_t warps = (size_t)nbh * NB, tn = (size_t)nbh * p.T * p.N;
+        KEYLESS_ROWS(p.N, (keyless_tables_kernel<R><<<(unsigned)((warps + 3) / 4), 128, 0, st>>>(p, wa, gate, fr, obuf, bh0, nbh,
+                                                                                                as, ot, am)));
+        if ((e = cudaGetLastError()) != cudaSuccess) return e;
+        RowAdjArgs A = {p.N, p.T, p.H, p.G, p.hard, p.hard_gate, as, am, nullptr, gate, dp, bh0, nbh, s.nsl,
+                        {v, buf, dbuf, dv, p.DV}, {nullptr, nullptr, nullptr, nullptr, 0}};
+        if ((e = run_row_adjoint(A, p.in_dtype, st)) != cudaSuccess) return e;
+        if ((e = run_row_dsum(dp, tn, s.nsl, st)) != cudaSuccess) return e;
+        KEYLESS_ROWS(p.N, (keyless_bwd_chain_kernel<R><<<nbh, 32, 0, st>>>(p, gate, fr, as, ot, am, dp, bh0, dwa, dgate, part)));
+        if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    }
+    return cudaSuccess;
+}
+
 }  // namespace slotscan
 
 using namespace slotscan;
@@ -283,6 +701,10 @@ extern "C" int slotscan_v_fwd(const slotscan_v_params* p, const void* v, const f
     if (rc) return rc;
     if (!v || !wa || !gate || !fr || !buf || !obuf) return SLOTSCAN_E_NULL;
     cudaStream_t st = (cudaStream_t)stream;
+    if (keyless_split(*p))
+        return (int)(p->in_dtype == SLOTSCAN_F32
+                         ? run_keyless_fwd<float>(*p, (const float*)v, wa, gate, fr, buf, obuf, addr, st)
+                         : run_keyless_fwd<__nv_bfloat16>(*p, (const __nv_bfloat16*)v, wa, gate, fr, buf, obuf, addr, st));
     const size_t sm = sizeof(float) * keyless_fwd_smem_floats(p->N, p->DV);
     cudaError_t e;
     if (p->in_dtype == SLOTSCAN_F32) {
@@ -299,6 +721,7 @@ extern "C" int slotscan_v_fwd(const slotscan_v_params* p, const void* v, const f
 
 extern "C" size_t slotscan_v_bwd_scratch_bytes(const slotscan_v_params* p) {
     if (slotscan_v_check(p)) return 0;
+    if (keyless_split(*p)) return keyless_scratch(*p).bytes;
     size_t o = sizeof(float) * (size_t)p->B * p->H * p->G * keyless_state_floats(p->N, p->DV);
     o = (o + 255) & ~(size_t)255;
     return o + sizeof(float) * (size_t)p->B * p->H;
@@ -312,6 +735,15 @@ extern "C" int slotscan_v_bwd(const slotscan_v_params* p, const void* v, const f
     if (!v || !wa || !gate || !fr || !buf || !obuf || !scratch || !dv || !dwa || !dgate || !dfr) return SLOTSCAN_E_NULL;
     if (scratch_bytes < slotscan_v_bwd_scratch_bytes(p)) return SLOTSCAN_E_SHAPE;
     cudaStream_t st = (cudaStream_t)stream;
+    if (keyless_split(*p)) {
+        const cudaError_t e = p->in_dtype == SLOTSCAN_F32
+            ? run_keyless_bwd<float>(*p, (const float*)v, wa, gate, fr, buf, obuf, dbuf, (char*)scratch, (float*)dv, dwa, dgate, st)
+            : run_keyless_bwd<__nv_bfloat16>(*p, (const __nv_bfloat16*)v, wa, gate, fr, buf, obuf, dbuf, (char*)scratch,
+                                             (__nv_bfloat16*)dv, dwa, dgate, st);
+        if (e != cudaSuccess) return (int)e;
+        keyless_finish_kernel<<<1, 256, 0, st>>>((const float*)((char*)scratch + keyless_scratch(*p).part), p->B * p->H, dfr);
+        return (int)cudaGetLastError();
+    }
     const size_t sm = sizeof(float) * keyless_bwd_smem_floats(p->N, p->DV);
     const size_t seg_bytes = (sizeof(float) * (size_t)p->B * p->H * p->G * keyless_state_floats(p->N, p->DV) + 255) & ~(size_t)255;
     float* seg = (float*)scratch;

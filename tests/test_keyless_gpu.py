@@ -81,3 +81,29 @@ def test_keyless_contract():
     assert b16.dtype == torch.bfloat16 and b16.shape == (B, 23, H, N, DV) and torch.equal(b16, b32.to(torch.bfloat16))
     with pytest.raises(RuntimeError):
         S.slot_scan_v(v.cpu(), wa.cpu(), gate.cpu(), fr.cpu(), N)
+
+
+@pytest.mark.parametrize("case", [(1, 1, 1, 1, 1, 1, False, False), (2, 33, 2, 31, 5, 16, False, False), (1, 50, 3, 33, 33, 17, True, False),
+                                  (1, 70, 2, 65, 64, 40, False, True), (2, 40, 1, 129, 36, 4, False, False),
+                                  (1, 37, 2, 256, 32, 1, True, True), (1, 21, 2, 257, 8, 8, False, False)],
+                         ids=lambda c: "B%d_T%d_H%d_N%d_D%d_G%d%s" % (c[:6] + ("_hard" if c[6] else "",)))
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16], ids=["f32", "bf16"])
+def test_keyless_edges(case, dtype):
+    """Row counts around a warp's multiples, one row, strides beyond a step of 16 tokens, widths that are no multiple of
+    4 or of a column slice, and the first row count that takes the one-CTA kernels.  bf16 values: the oracle runs on the
+    rounded values; a bf16 gradient is within its own rounding (2^-8 of itself) of the oracle's."""
+    B, T, H, N, DV, G, hard, hard_gate = case
+    gen = torch.Generator().manual_seed(77)
+    v = torch.randn(B, T, H, DV, generator=gen).to(dtype).float()
+    wa = 1.5 * torch.randn(B, T, H, N, generator=gen)
+    gate = torch.sigmoid(torch.randn(B, T, H, generator=gen))
+    fr = torch.tensor([3.0])
+    ref = O.scan_v_fwd(v, wa, gate, fr, N, G=G, hard=hard, hard_gate=hard_gate)
+    w = torch.randn(ref["buf"].shape, generator=gen).numpy()
+    gr = O.scan_v_bwd(v, wa, gate, fr, N, w, G=G, hard=hard, hard_gate=hard_gate)
+    buf, grads = run(v.numpy(), wa.numpy(), gate.numpy(), fr.numpy(), N, G, hard, hard_gate, w, dtype=dtype)
+    okc, worst = allclose_report(buf, ref["buf"], 1e-5, 1e-5)
+    assert okc, worst
+    for g, n in zip(grads, ("dv", "dwa", "dgate", "dfr")):
+        band = 2.0 ** -8 if n == "dv" and dtype == torch.bfloat16 else 1e-4
+        assert rel_to_max(g.reshape(gr[n].shape), gr[n]) < band or np.abs(gr[n]).max() < 1e-12, n
