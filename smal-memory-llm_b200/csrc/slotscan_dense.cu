@@ -3,6 +3,13 @@
 // attached to the stored keys.  [reference: forward gqa25/slotkern_kvt.py:43-119, step adjoint :157-171 and
 // gqa25/slotkern_kvg.py:163-200 (stride-G replay backward); definition gqa25/slotkern_kv.py:66-123]
 //
+// Up to 256 rows: the forward and, for a soft detached address, the backward with the token chain reduced to scalars
+// (slotscan_dense_chain.cuh) and the row gradients block by block (slotscan_rowadj.cuh).  B = 4, T = 512, H = 12,
+// 192 x (64 + 64), G = 16, soft, detached, forward + backward: 35.2 ms token by token (5.9 + 29.9), 2.66 ms so (forward 1.15;
+// backward: tables 0.48, row gradients 0.60, query gradient 0.34, softmax adjoint 0.04).
+// The token-by-token kernels below take the rest: more rows than 256, or more shared memory than a CTA has beside the
+// chain's token buffers; and the backward of an attached address, where the gradient of the score of every token enters
+// the row gradients that the token before it needs, so that they are no longer linear in known factors.
 // One CTA per (sequence, head).  Forward: keys, values and occupancy resident in shared memory as float32
 // (N x (dk + dv) + N floats: 197 KB at 192 x (128 + 128)), four phases per token -- token vectors in, scores (a warp
 // per row), address (one warp: mask, argmax, softmax), write (all threads).  The pre-write state goes out every G
@@ -14,22 +21,22 @@
 // Rows are occupied in index order and occupancy never decreases, so the candidates of a token are exactly rows
 // 0 .. first-empty; everything above is zero and is not visited.
 //
-// These modes are not the training path of the reference run; they are built for completeness of the call signature
-// and checked against the same oracle and golden vectors, not tuned.
+// The training path of the reference run is the hard, detached address (csrc/slotscan_hard.cu).
 #include <math.h>
 #include <stdio.h>
 
+#include <algorithm>
+
 #include "slotscan_common.cuh"
+#include "slotscan_dense_chain.cuh"
 #include "slotscan_launch.h"
+#include "slotscan_rowadj.cuh"
 
 namespace slotscan {
 
 constexpr int DN_THREADS = 256, DN_WARPS = DN_THREADS / 32;
 
-__device__ __forceinline__ float ldtok(const float* p) { return *p; }
-__device__ __forceinline__ float ldtok(const __nv_bfloat16* p) { return __bfloat162float(*p); }
-__device__ __forceinline__ void sttok(float* p, float v) { *p = v; }
-__device__ __forceinline__ void sttok(__nv_bfloat16* p, float v) { *p = __float2bfloat16_rn(v); }
+
 
 // The address of one token from the scores s[0..lim] and occupancies o[0..lim] (rows 0..lim are the candidates: the
 // occupied rows and the first empty one).  Writes afwd[n] (the address the forward uses) and asoft[n] (its softmax);
@@ -37,11 +44,6 @@ __device__ __forceinline__ void sttok(__nv_bfloat16* p, float v) { *p = __float2
 // The scores arrive in double and the softmax runs in double: a soft address feeds every rounding error of a score
 // back into every row of the state, token after token, and float32 scores alone put the snapshots several 1e-5 away
 // from the float64 definition after a few dozen tokens (the reference's own float32 path shows the same drift).
-__device__ __forceinline__ double warp_sum_d(double v) {
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(FULL, v, off);
-    return v;
-}
 template <typename TO>
 __device__ __forceinline__ int dense_address(double* s, const TO* o, int lim, float fr_t, float eps, int occ_bin,
                                              int hard, float* asoft, float* afwd, float* occ_out) {
@@ -475,18 +477,18 @@ __global__ void __launch_bounds__(DN_THREADS) dense_bwd_kernel(
     }
 }
 
-__global__ void __launch_bounds__(256) dense_finish_kernel(const float* __restrict__ part, int n, int fr_per_token,
+__global__ void __launch_bounds__(256) dense_finish_kernel(const float* __restrict__ part, size_t n, int fr_per_token,
                                                            float* dtemp, float* dfr) {
-    __shared__ float s_a[256], s_c[256];
-    float a = 0.f, c = 0.f;
-    for (int i = threadIdx.x; i < n; i += 256) { a += part[i]; c += part[n + i]; }
+    __shared__ double s_a[256], s_c[256];
+    double a = 0.0, c = 0.0;
+    for (size_t i = threadIdx.x; i < n; i += 256) { a += (double)part[i]; c += (double)part[n + i]; }
     s_a[threadIdx.x] = a; s_c[threadIdx.x] = c;
     __syncthreads();
     if (threadIdx.x == 0) {
-        a = 0.f; c = 0.f;
+        a = 0.0; c = 0.0;
         for (int i = 0; i < 256; i++) { a += s_a[i]; c += s_c[i]; }      // fixed order: bitwise repeatable
-        dtemp[0] = a;
-        if (!fr_per_token) dfr[0] = c;
+        dtemp[0] = (float)a;
+        if (!fr_per_token) dfr[0] = (float)c;
     }
 }
 template <typename Tin>
@@ -496,6 +498,86 @@ __global__ void dense_add_into_kernel(Tin* __restrict__ dst, const Tin* __restri
 }
 
 constexpr size_t DENSE_SMEM_CAP = 227 * 1024;
+
+// tokens per chunk of the chain kernels: 8 where the token buffers fit beside the rows, 4 where only those do, 0: neither
+inline int dense_chunk(int N, int DK, int DV, bool values) {
+    if (N > DC_NMAX) return 0;
+    return dc_smem(8, N, DK, DV, values) <= DENSE_SMEM_CAP ? 8 : (dc_smem(4, N, DK, DV, values) <= DENSE_SMEM_CAP ? 4 : 0);
+}
+// the split backward: a soft detached address whose shapes the chain, the row gradients and the query gradient all take
+inline bool dense_split_bwd(const slotscan_dense_params& d) {
+    const slotscan_params& b = d.base;
+    return !d.hard && d.detach_addr && dense_chunk(b.N, b.DK, b.DV, false) && dense_dq_smem(b.N, b.DK) <= DENSE_SMEM_CAP &&
+           (long long)b.B * b.H * ((b.T + b.G - 1) / b.G) <= 2147483647LL;
+}
+// its scratch: the tables of `nbh` sequences at a time (as many as 2 GiB hold), then the partial sums of all
+struct DenseScratch { size_t as, sf, ki, ot, dp, lim, part, bytes; int nbh, nsl, chunk; size_t part_n; };
+inline DenseScratch dense_scratch(const slotscan_params& p) {
+    DenseScratch s;
+    auto up = [](size_t x) { return (x + 255) & ~(size_t)255; };
+    const size_t BH = (size_t)p.B * p.H, tn = (size_t)p.T * p.N, NB = (p.T + p.G - 1) / p.G;
+    s.nsl = row_adjoint_slices(p.N, p.DK) + row_adjoint_slices(p.N, p.DV);
+    s.nbh = (int)std::min(std::min(BH, (size_t)65535), std::max((size_t)1, ((size_t)2 << 30) / (4 * tn * (4 + s.nsl))));
+    s.chunk = p.occ_bin ? 32 : p.T;
+    s.part_n = BH * ((p.T + s.chunk - 1) / s.chunk);
+    const size_t one = up(4 * tn * s.nbh);
+    s.as = 0; s.sf = one; s.ki = 2 * one; s.ot = 3 * one; s.dp = 4 * one;
+    s.lim = s.dp + up(4 * tn * s.nbh * s.nsl);
+    s.part = s.lim + up(4 * NB * s.nbh);
+    s.bytes = s.part + 8 * s.part_n;
+    return s;
+}
+
+template <typename Tin, bool TABLES>
+cudaError_t run_dense_chain(const DenseChainArgs& A, int grid, cudaStream_t st) {
+    const slotscan_params& p = A.p;
+    const int C = dense_chunk(p.N, p.DK, p.DV, !TABLES);
+    const size_t sm = dc_smem(C, p.N, p.DK, p.DV, !TABLES);
+    auto go = [&](auto kern) {
+        const cudaError_t e = opt_in_smem(kern, sm);
+        if (e != cudaSuccess) return e;
+        kern<<<grid, ((p.N + 31) & ~31) + DC_HELP, sm, st>>>(A);
+        return cudaGetLastError();
+    };
+    return C == 8 ? go(dense_chain_kernel<Tin, 8, TABLES>) : go(dense_chain_kernel<Tin, 4, TABLES>);
+}
+
+template <typename Tin>
+cudaError_t run_dense_split_bwd(const slotscan_params& p, const void* k, const void* q, const void* v, const float* gate,
+                                const float* fr, const float* temp, const float* kbuf, const float* vbuf, const float* obuf,
+                                const float* dkbuf, const float* dvbuf, char* scratch, void* dk, void* dq, void* dv,
+                                float* dgate, float* dfr, cudaStream_t st) {
+    const DenseScratch s = dense_scratch(p);
+    float *as = (float*)(scratch + s.as), *sf = (float*)(scratch + s.sf), *ki = (float*)(scratch + s.ki);
+    float *ot = (float*)(scratch + s.ot), *dp = (float*)(scratch + s.dp), *part = (float*)(scratch + s.part);
+    int* lim = (int*)(scratch + s.lim);
+    const int BH = p.B * p.H, NB = (p.T + p.G - 1) / p.G, NC = (p.T + s.chunk - 1) / s.chunk;
+    cudaError_t e;
+    for (int bh0 = 0; bh0 < BH; bh0 += s.nbh) {
+        const int nbh = std::min(s.nbh, BH - bh0);
+        DenseChainArgs C = {p, 0, k, q, v, gate, fr, temp, const_cast<float*>(kbuf), nullptr, const_cast<float*>(obuf), nullptr,
+                            nullptr, nullptr, nullptr, as, sf, ki, ot, lim, bh0};
+        if ((e = run_dense_chain<Tin, true>(C, nbh * NB, st)) != cudaSuccess) return e;
+        RowAdjArgs R = {p.N, p.T, p.H, p.G, 0, p.hard_gate, as, nullptr, lim, gate, dp, bh0, nbh, row_adjoint_slices(p.N, p.DK),
+                        {k, kbuf, dkbuf, dk, p.DK}, {v, vbuf, dvbuf, dv, p.DV}};
+        if ((e = run_row_adjoint(R, p.in_dtype, st)) != cudaSuccess) return e;
+        const size_t tn = (size_t)nbh * p.T * p.N;
+        if ((e = run_row_dsum(dp, tn, s.nsl, st)) != cudaSuccess) return e;
+        const size_t warps = (size_t)nbh * NC;
+        auto dz = [&](auto kern) {
+            kern<<<(unsigned)((warps + 3) / 4), 128, 0, st>>>(p, s.chunk, gate, fr, temp, as, sf, ki, ot, lim, dp, bh0, nbh, dgate,
+                                                            dfr, part, s.part_n);
+            return cudaGetLastError();
+        };
+        e = p.N <= 64 ? dz(dense_dz_kernel<2>) : (p.N <= 128 ? dz(dense_dz_kernel<4>) : (p.N <= 192 ? dz(dense_dz_kernel<6>) : dz(dense_dz_kernel<8>)));
+        if (e != cudaSuccess) return e;
+        const size_t sm = dense_dq_smem(p.N, p.DK);
+        if ((e = opt_in_smem(dense_dq_kernel<Tin>, sm)) != cudaSuccess) return e;
+        dense_dq_kernel<Tin><<<nbh * NB, DQ_T, sm, st>>>(p, (const Tin*)k, (const Tin*)q, gate, kbuf, as, dp, bh0, (Tin*)dq);
+        if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    }
+    return cudaSuccess;
+}
 
 }  // namespace slotscan
 
@@ -521,6 +603,12 @@ extern "C" int slotscan_dense_fwd(const slotscan_dense_params* p, const void* k,
     if (!k || !v || !gate || !fr || !temp || !kbuf || !vbuf || !obuf) return SLOTSCAN_E_NULL;
     const slotscan_params& b = p->base;
     cudaStream_t st = (cudaStream_t)stream;
+    if (dense_chunk(b.N, b.DK, b.DV, true)) {
+        const DenseChainArgs C = {b, p->hard, k, q ? q : k, v, gate, fr, temp, kbuf, vbuf, obuf, addr, kfin, vfin, ofin,
+                                  nullptr, nullptr, nullptr, nullptr, nullptr, 0};
+        return (int)(b.in_dtype == SLOTSCAN_F32 ? run_dense_chain<float, false>(C, b.B * b.H, st)
+                                                : run_dense_chain<__nv_bfloat16, false>(C, b.B * b.H, st));
+    }
     const size_t sm = sizeof(float) * dense_fwd_smem_floats(b.N, b.DK, b.DV);
     cudaError_t e;
     if (b.in_dtype == SLOTSCAN_F32) {
@@ -541,9 +629,36 @@ extern "C" int slotscan_dense_fwd(const slotscan_dense_params* p, const void* k,
 extern "C" size_t slotscan_dense_bwd_scratch_bytes(const slotscan_dense_params* p) {
     if (slotscan_dense_check(p)) return 0;
     const slotscan_params& b = p->base;
+    if (dense_split_bwd(*p)) return dense_scratch(b).bytes;
     size_t o = sizeof(float) * (size_t)b.B * b.H * b.G * dense_state_floats(b.N, b.DK, b.DV);
     o = (o + 255) & ~(size_t)255;
     return o + sizeof(float) * 2 * (size_t)b.B * b.H;
+}
+
+// the token-by-token backward
+static cudaError_t run_dense_bwd(const slotscan_dense_params& d, const void* k, const void* q, const void* v, const float* gate,
+                                 const float* fr, const float* temp, const float* kbuf, const float* vbuf, const float* obuf,
+                                 const float* dkbuf, const float* dvbuf, float* seg, void* dk, void* dq, void* dv, float* dgate,
+                                 float* dfr, float* part, cudaStream_t st) {
+    const slotscan_dense_params* p = &d;
+    const slotscan_params& b = d.base;
+    const size_t sm = sizeof(float) * dense_bwd_smem_floats(b.N, b.DK, b.DV);
+    cudaError_t e;
+    if (b.in_dtype == SLOTSCAN_F32) {
+        auto kern = dense_bwd_kernel<float>;
+        if ((e = opt_in_smem(kern, sm)) != cudaSuccess) return e;
+        kern<<<b.B * b.H, DN_THREADS, sm, st>>>(b, p->hard, p->detach_addr, (const float*)k, (const float*)(q ? q : k),
+                                                (const float*)v, gate, fr, temp, kbuf, vbuf, obuf, dkbuf, dvbuf, seg,
+                                                (float*)dk, (float*)dq, (float*)dv, dgate, dfr, part);
+    } else {
+        typedef __nv_bfloat16 bf;
+        auto kern = dense_bwd_kernel<bf>;
+        if ((e = opt_in_smem(kern, sm)) != cudaSuccess) return e;
+        kern<<<b.B * b.H, DN_THREADS, sm, st>>>(b, p->hard, p->detach_addr, (const bf*)k, (const bf*)(q ? q : k), (const bf*)v,
+                                                gate, fr, temp, kbuf, vbuf, obuf, dkbuf, dvbuf, seg, (bf*)dk, (bf*)dq, (bf*)dv,
+                                                dgate, dfr, part);
+    }
+    return cudaGetLastError();
 }
 
 extern "C" int slotscan_dense_bwd(const slotscan_dense_params* p, const void* k, const void* q, const void* v,
@@ -559,27 +674,24 @@ extern "C" int slotscan_dense_bwd(const slotscan_dense_params* p, const void* k,
     if (scratch_bytes < slotscan_dense_bwd_scratch_bytes(p)) return SLOTSCAN_E_SHAPE;
     const slotscan_params& b = p->base;
     cudaStream_t st = (cudaStream_t)stream;
-    const size_t sm = sizeof(float) * dense_bwd_smem_floats(b.N, b.DK, b.DV);
+    const bool split = dense_split_bwd(*p);
     const size_t seg_bytes = (sizeof(float) * (size_t)b.B * b.H * b.G * dense_state_floats(b.N, b.DK, b.DV) + 255) & ~(size_t)255;
     float* seg = (float*)scratch;
-    float* part = (float*)((char*)scratch + seg_bytes);
+    float* part = (float*)((char*)scratch + (split ? dense_scratch(b).part : seg_bytes));
+    const size_t npart = split ? dense_scratch(b).part_n : (size_t)b.B * b.H;
     cudaError_t e;
-    if (b.in_dtype == SLOTSCAN_F32) {
-        auto kern = dense_bwd_kernel<float>;
-        if ((e = opt_in_smem(kern, sm)) != cudaSuccess) return (int)e;
-        kern<<<b.B * b.H, DN_THREADS, sm, st>>>(b, p->hard, p->detach_addr, (const float*)k, (const float*)(q ? q : k),
-                                                (const float*)v, gate, fr, temp, kbuf, vbuf, obuf, dkbuf, dvbuf, seg,
-                                                (float*)dk, (float*)dq, (float*)dv, dgate, dfr, part);
-    } else {
-        typedef __nv_bfloat16 bf;
-        auto kern = dense_bwd_kernel<bf>;
-        if ((e = opt_in_smem(kern, sm)) != cudaSuccess) return (int)e;
-        kern<<<b.B * b.H, DN_THREADS, sm, st>>>(b, p->hard, p->detach_addr, (const bf*)k, (const bf*)(q ? q : k), (const bf*)v,
-                                                gate, fr, temp, kbuf, vbuf, obuf, dkbuf, dvbuf, seg, (bf*)dk, (bf*)dq, (bf*)dv,
-                                                dgate, dfr, part);
+    if (split) {
+        const void* q_ = q ? q : k;
+        e = b.in_dtype == SLOTSCAN_F32
+                ? run_dense_split_bwd<float>(b, k, q_, v, gate, fr, temp, kbuf, vbuf, obuf, dkbuf, dvbuf, (char*)scratch, dk, dq, dv, dgate, dfr, st)
+                : run_dense_split_bwd<__nv_bfloat16>(b, k, q_, v, gate, fr, temp, kbuf, vbuf, obuf, dkbuf, dvbuf, (char*)scratch, dk, dq, dv,
+                                                     dgate, dfr, st);
+        if (e != cudaSuccess) return (int)e;
+    } else if ((e = run_dense_bwd(*p, k, q, v, gate, fr, temp, kbuf, vbuf, obuf, dkbuf, dvbuf, seg, dk, dq, dv, dgate, dfr, part, st)) !=
+               cudaSuccess) {
+        return (int)e;
     }
-    if ((e = cudaGetLastError()) != cudaSuccess) return (int)e;
-    dense_finish_kernel<<<1, 256, 0, st>>>(part, b.B * b.H, b.fr_per_token, dtemp, dfr);
+    dense_finish_kernel<<<1, 256, 0, st>>>(part, npart, b.fr_per_token, dtemp, dfr);
     if ((e = cudaGetLastError()) != cudaSuccess) return (int)e;
     if (q == nullptr) {           // the search query is the stored key: both gradient paths land in dk
         const size_t n = (size_t)b.B * b.T * b.H * b.DK;

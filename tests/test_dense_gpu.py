@@ -124,3 +124,37 @@ def test_general_scan_contract():
     with pytest.raises(ValueError):                                        # 256 rows of 128 + 128 do not fit one CTA
         S.kv_scan_g(torch.zeros(1, 8, 1, 128, device=DEV), torch.zeros(1, 8, 1, 128, device=DEV),
                     torch.zeros(1, 8, 1, device=DEV), 1.0, 256, 16.0, G=8)
+
+
+@pytest.mark.parametrize("case", [  # B, T, H, N, DK, DV, G, temp, hard, occ_bin, hard_gate, frtok, sepq
+    (1, 1, 1, 1, 1, 1, 1, 16.0, False, True, False, True, True), (2, 40, 2, 31, 24, 40, 7, 16.0, False, False, False, True, False),
+    (1, 50, 2, 33, 64, 64, 1, 16.0, False, True, False, False, True), (1, 90, 1, 65, 128, 16, 40, 16.0, False, True, True, True, True),
+    (1, 45, 2, 129, 16, 128, 8, 400.0, False, False, False, True, True), (1, 60, 2, 192, 128, 128, 16, 16.0, False, False, False, True, True),
+    (1, 40, 1, 256, 8, 8, 17, 16.0, False, True, False, True, True), (1, 30, 1, 257, 8, 8, 4, 16.0, False, True, False, True, True),
+    (1, 70, 2, 65, 36, 64, 9, 16.0, True, False, False, True, True)],
+    ids=lambda c: "N%d_K%d_V%d_G%d_temp%g%s" % (c[3], c[4], c[5], c[6], c[7], "_hard" if c[8] else ""))
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16], ids=["f32", "bf16"])
+def test_general_scan_edges(case, dtype):
+    """One row, row counts around a warp's multiples, widths that are no multiple of a slice or of 4, strides around and
+    beyond the chain's chunks, a sharpness whose softmax needs its maximum, and the first row count past the chain kernels
+    (whose bounds are the tolerances of the tests above).  The address detached, as the split backward takes it; hard:
+    attached, or the call would take the specialised kernels.  bf16 streams: the oracle runs on the rounded values; a bf16
+    gradient is within its rounding (2^-8 of itself)."""
+    B, T, H, N, DK, DV, G, temp, hard, occ_bin, hard_gate, frtok, sepq = case
+    inp = make_inputs("clustered" if temp > 100 else "fill", B, T, H, DK, DV, seed=900 + N, frtok=frtok, sepq=sepq)
+    inp["temp"] = temp
+    for n in ("k", "q", "v"):
+        inp[n] = None if inp[n] is None else inp[n].to(dtype).float()
+    kw = dict(N=N, temp=temp, G=G, hard=hard, hard_gate=hard_gate, q=inp["q"], occ_bin=occ_bin)
+    ref = O.scan_fwd(inp["k"], inp["v"], inp["gate"], inp["fr"], dtype=np.float64, **kw)
+    gen = torch.Generator().manual_seed(8)
+    wk, wv = (torch.randn(ref[n].shape, generator=gen).numpy() for n in ("kbuf", "vbuf"))
+    out = run(inp, N, G, hard, hard_gate, occ_bin, not hard, wk, wv, dtype=dtype)
+    for n in ("kbuf", "vbuf"):
+        okc, worst = allclose_report(out[n], ref[n], 1e-5, 1e-5)
+        assert okc, (n, worst)
+    gr = O.scan_bwd(inp["k"], inp["v"], inp["gate"], inp["fr"], dkbuf=wk, dvbuf=wv, detach_addr=not hard, dtype=np.float64, **kw)
+    for n in ["dk", "dv", "dgate", "dtemp", "dfr"] + (["dq"] if sepq else []):
+        # q = None, bf16: dk is the sum of two bf16-rounded parts, three roundings in all
+        band = (3 * 2.0 ** -8 if not sepq else 2.0 ** -8) if dtype == torch.bfloat16 and n in ("dk", "dq", "dv") else 1e-4
+        assert rel_to_max(out[n].reshape(gr[n].shape), gr[n]) < band or np.abs(gr[n]).max() < 1e-9, n
