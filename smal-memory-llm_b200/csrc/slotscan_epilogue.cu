@@ -10,38 +10,19 @@
 // group / 8 neighbouring lanes (absmax by shuffles); groups of 4 are two per lane.  Grid: a multiple of the SM
 // count, grid-stride over rows.  HBM-bound: (e_in + e_out) * D bytes per row plus 5 bytes for kinv and valid.
 #include <cuda_bf16.h>
-#include <cuda_fp8.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
 #include <stdio.h>
 
 #include "slotscan.h"
 #include "slotscan_common.cuh"
+#include "slotscan_fq.cuh"
 #include "slotscan_launch.h"
 
 namespace slotscan {
 
 constexpr int EP_THREADS = 256;
 
-__device__ __forceinline__ float round_to(float v, float) { return v; }
-__device__ __forceinline__ float round_to(float v, __nv_bfloat16) { return __bfloat162float(__float2bfloat16_rn(v)); }
-
-// fq of one group member, in the arithmetic of the reference: s = max(a / half, 1e-30),
-// q = (clamp(floor(x / s), -half, half - 1) + 0.5) * s, zero for an all-zero group, returned in the straight-through
-// form x + (q - x) evaluated in the input dtype (memlm_sh.py:229).
-// The IEEE division x / s is what costs: it is replaced by x * (1 / s) wherever that provably has the same floor (the
-// product is off by a few ulp of a quotient that is at most 128 in size, so any result further than 1e-3 from an
-// integer floors alike), by the known answer for the group's own extreme (x = +-a gives exactly +-half), and kept for
-// the rare rest.  s, 1 / s are per group.
-struct FqScale { float a, half, s, rs; bool plain; };
-__device__ __forceinline__ FqScale fq_scale(float a, float half) {
-    FqScale g;
-    g.a = a; g.half = half;
-    g.s = fmaxf(__fdiv_rn(a, half), 1e-30f);
-    g.rs = __frcp_rn(g.s);
-    g.plain = a > 1e-20f;                    // s = a / half exactly: not clamped, not denormal
-    return g;
-}
 // The same for the packed bf16 path: a * (1 / half) is the same float as a / half (half is a power of two), and 1 / s
 // only has to place k within one of the quotient, so the approximate reciprocal will do; a group that is not `plain`
 // goes through fq_one and gets the exact one.
@@ -54,20 +35,6 @@ __device__ __forceinline__ FqScale fq_scale_packed(float a, float half, float in
     else g.rs = __frcp_rn(g.s);
     return g;
 }
-template <typename Tin>
-__device__ __forceinline__ float fq_one(float x, const FqScale& g) {
-    float f;
-    const float qt = x * g.rs, fl = floorf(qt), fr = qt - fl;
-    if (g.plain && fabsf(x) == g.a) f = x > 0.f ? g.half : -g.half;
-    else if (g.plain && fr > 1e-3f && fr < 0.999f) f = fl;
-    else f = floorf(__fdiv_rn(x, g.s));
-    f = fminf(fmaxf(f, -g.half), g.half - 1.f);
-    const float q = (g.a > 0.f) ? __fmul_rn(__fadd_rn(f, 0.5f), g.s) : 0.f;
-    const float qd = round_to(q, Tin());
-    const float diff = round_to(__fsub_rn(qd, x), Tin());
-    return round_to(__fadd_rn(x, diff), Tin());
-}
-
 // bf16 input, two elements at a time, in packed bf16 arithmetic wherever that is exact.  The group's extreme a is a
 // bf16 value, so s = a / half (half a power of two) is a bf16 value too.  With k = rint(x * (1 / s)) (|k| <= 128, a
 // bf16 value; one fused multiply-add against 1.5 * 2^23 rounds it)
@@ -186,13 +153,9 @@ __global__ void __launch_bounds__(EP_THREADS, PACKED ? 6 : 1) writer_epilogue_ke
 #pragma unroll
             for (int j = 0; j < 8; j++) a = fmaxf(a, fabsf(v[j]));
             for (int off = 1; off < LPR; off <<= 1) a = fmaxf(a, __shfl_xor_sync(FULL, a, off));
-            const float sc = fmaxf(__fdiv_rn(a, 448.f), 1e-30f);
+            const float sc = e4m3_scale(a);
 #pragma unroll
-            for (int j = 0; j < 8; j++) {
-                const __nv_fp8_storage_t b = __nv_cvt_float_to_fp8(__fdiv_rn(v[j], sc), __NV_SATFINITE, __NV_E4M3);
-                const float f = __half2float(__half(__nv_cvt_fp8_to_halfraw(b, __NV_E4M3)));
-                v[j] = a > 0.f ? __fmul_rn(f, sc) : 0.f;
-            }
+            for (int j = 0; j < 8; j++) v[j] = e4m3_one(v[j], a, sc);
         } else if (bits) {
             if (group >= 8) {
                 float a = 0.f;

@@ -32,7 +32,8 @@ struct RowsBwdLayout {                         // byte offsets into dynamic shar
     static constexpr int off_am = off_g + 3 * RC * 4, off_bar = off_am + 3 * RC * 4, total = off_bar + 16;
 };
 
-template <int D, typename Tin, typename Tsn, bool DKINV>
+// DKINV: 0 no kinv gradient, 1 of the float32 row, 2 of the row behind the storage quantiser
+template <int D, typename Tin, typename Tsn, int DKINV>
 __global__ void __launch_bounds__(ROW_THREADS, 3) rows_bwd2_kernel(
     const slotscan_params p, const RowsBwdArgs<Tin, Tsn> a0, const RowsBwdArgs<Tin, Tsn> a1,
     const float* __restrict__ gate, const int* __restrict__ am, const int* __restrict__ tfirst, const int ntens) {
@@ -140,16 +141,18 @@ __global__ void __launch_bounds__(ROW_THREADS, 3) rows_bwd2_kernel(
     // gradient itself and, through kinv = rsqrt(max(|X|^2, 1e-12)), -kinv^3 dkinv X.  All lanes of the warp call.
 #define RB_ADD_SNAPSHOT(ON)                                                                 \
     {                                                                                       \
-        float w_ = 0.f;                                                                     \
+        float w_ = 0.f, Y_[8];                                                              \
+        _Pragma("unroll") for (int j = 0; j < 8; j++) Y_[j] = X[j];                         \
         if (DKINV && dki0 != nullptr) {                                                     \
             float nsq_ = 0.f;                                                               \
-            _Pragma("unroll") for (int j = 0; j < 8; j++) nsq_ = fmaf(X[j], X[j], nsq_);    \
+            if (DKINV == 2) quantise_lanes<LPR, 1>(Y_, X, A.bits, A.group, FULL);           \
+            _Pragma("unroll") for (int j = 0; j < 8; j++) nsq_ = fmaf(Y_[j], Y_[j], nsq_);  \
             nsq_ = group_sum<LPR>(nsq_);                                                    \
             const float ki_ = rsqrtf(fmaxf(nsq_, 1e-12f));                                  \
             w_ = nsq_ > 1e-12f ? -(ki_ * ki_ * ki_) * nxt_w : 0.f;                          \
         }                                                                                   \
         if (ON) {                                                                           \
-            _Pragma("unroll") for (int j = 0; j < 8; j++) dX[j] += nxt[j] + w_ * X[j];      \
+            _Pragma("unroll") for (int j = 0; j < 8; j++) dX[j] += nxt[j] + w_ * Y_[j];     \
             RB_PXD()                                                                        \
         }                                                                                   \
     }
@@ -339,7 +342,7 @@ struct RowsBwd3Layout {
     static constexpr int off_bar = off_ts + RPB * 4, total = off_bar + 32;
 };
 
-template <int D, int GG, typename Tin, typename Tsn, bool DKINV>
+template <int D, int GG, typename Tin, typename Tsn, int DKINV>
 __global__ void __launch_bounds__(ROW_THREADS, (sizeof(Tin) == 2 ? 3 : 2)) rows_bwd3_kernel(
     const slotscan_params p, const RowsBwdArgs<Tin, Tsn> a0, const RowsBwdArgs<Tin, Tsn> a1,
     const float* __restrict__ gate, const int* __restrict__ am, const int* __restrict__ tfirst, const int ntens) {
@@ -551,17 +554,20 @@ __global__ void __launch_bounds__(ROW_THREADS, (sizeof(Tin) == 2 ? 3 : 2)) rows_
                     if (jb * G >= tstop) {
                         float nx[8];
                         slot.get(nx);
-                        float w_ = 0.f;
+                        float w_ = 0.f, Y_[8];
+#pragma unroll
+                        for (int j = 0; j < 8; j++) Y_[j] = X[j];
                         if (DKINV && dki0 != nullptr) {
                             float nsq_ = 0.f;
+                            if (DKINV == 2) quantise_lanes<LPR, 1>(Y_, X, A.bits, A.group, gmask);
 #pragma unroll
-                            for (int j = 0; j < 8; j++) nsq_ = fmaf(X[j], X[j], nsq_);
+                            for (int j = 0; j < 8; j++) nsq_ = fmaf(Y_[j], Y_[j], nsq_);
                             nsq_ = rsum(nsq_);
                             const float ki_ = rsqrtf(fmaxf(nsq_, 1e-12f));
                             w_ = nsq_ > 1e-12f ? -(ki_ * ki_ * ki_) * slotw : 0.f;
                         }
 #pragma unroll
-                        for (int j = 0; j < 8; j++) dX[j] += nx[j] + w_ * X[j];
+                        for (int j = 0; j < 8; j++) dX[j] += nx[j] + w_ * Y_[j];
                     }
                     fetch(jb - 2, slot, slotw);
                 }

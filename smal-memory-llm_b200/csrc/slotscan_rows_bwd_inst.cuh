@@ -19,10 +19,10 @@ static cudaError_t rows_bwd_one(const slotscan_params& p, int ntensors, const Ro
     // first, keys and values side by side
     dim3 grid((unsigned)((size_t)p.B * p.H * ((p.N + RPB - 1) / RPB) * ntensors));
     constexpr size_t sm = RowsBwdLayout<D, Tin>::total;
-    const RowsBwdArgs<Tin, Tsn> b0{(const Tin*)a0.x, a0.xold, a0.xfin, (const Tsn*)a0.dxbuf, (Tin*)a0.dx, a0.Dn, a0.dkinv};
-    const RowsBwdArgs<Tin, Tsn> b1{(const Tin*)a1.x, a1.xold, a1.xfin, (const Tsn*)a1.dxbuf, (Tin*)a1.dx, a1.Dn, a1.dkinv};
+    const RowsBwdArgs<Tin, Tsn> b0{(const Tin*)a0.x, a0.xold, a0.xfin, (const Tsn*)a0.dxbuf, (Tin*)a0.dx, a0.Dn, a0.dkinv, a0.bits, a0.group};
+    const RowsBwdArgs<Tin, Tsn> b1{(const Tin*)a1.x, a1.xold, a1.xfin, (const Tsn*)a1.dxbuf, (Tin*)a1.dx, a1.Dn, a1.dkinv, a1.bits, a1.group};
     cudaError_t e;
-    const bool dkinv = a0.dkinv != nullptr || a1.dkinv != nullptr;
+    const bool dkinv = a0.dkinv != nullptr || a1.dkinv != nullptr, quant = dkinv && a0.bits != 0;
     // the event-walk form: snapshot stride 8 or 16 (2 or 4 blocks per chunk) and D >= 64
     if constexpr (D >= 64) {
         constexpr size_t sm3 = RowsBwd3Layout<D, Tin>::total;
@@ -33,19 +33,13 @@ static cudaError_t rows_bwd_one(const slotscan_params& p, int ntensors, const Ro
             kern<<<grid, ROW_THREADS, sm3, st>>>(p, b0, b1, gate, am, tfirst, ntensors);     \
             return cudaGetLastError();                                                       \
         }
-        if (p.G == 8) { if (dkinv) RB3_LAUNCH(8, true) else RB3_LAUNCH(8, false) }
-        if (p.G == 16) { if (dkinv) RB3_LAUNCH(16, true) else RB3_LAUNCH(16, false) }
+        if (p.G == 8) { if (quant) RB3_LAUNCH(8, 2) else if (dkinv) RB3_LAUNCH(8, 1) else RB3_LAUNCH(8, 0) }
+        if (p.G == 16) { if (quant) RB3_LAUNCH(16, 2) else if (dkinv) RB3_LAUNCH(16, 1) else RB3_LAUNCH(16, 0) }
 #undef RB3_LAUNCH
     }
-    if (dkinv) {
-        auto kern = rows_bwd2_kernel<D, Tin, Tsn, true>;
-        if ((e = opt_in_smem(kern, sm)) != cudaSuccess) return e;
-        kern<<<grid, ROW_THREADS, sm, st>>>(p, b0, b1, gate, am, tfirst, ntensors);
-    } else {
-        auto kern = rows_bwd2_kernel<D, Tin, Tsn, false>;
-        if ((e = opt_in_smem(kern, sm)) != cudaSuccess) return e;
-        kern<<<grid, ROW_THREADS, sm, st>>>(p, b0, b1, gate, am, tfirst, ntensors);
-    }
+    auto kern = quant ? rows_bwd2_kernel<D, Tin, Tsn, 2> : (dkinv ? rows_bwd2_kernel<D, Tin, Tsn, 1> : rows_bwd2_kernel<D, Tin, Tsn, 0>);
+    if ((e = opt_in_smem(kern, sm)) != cudaSuccess) return e;
+    kern<<<grid, ROW_THREADS, sm, st>>>(p, b0, b1, gate, am, tfirst, ntensors);
     return cudaGetLastError();
 }
 
@@ -65,8 +59,8 @@ cudaError_t SS_CAT(run_rows_bwd_, SLOTSCAN_SUFFIX)(const slotscan_params& p, int
 }
 
 void SS_CAT(attrs_rows_bwd_, SLOTSCAN_SUFFIX)(slotscan_kernel_attr* out, int cap, int& n) {
-    fill_attr(out, cap, n, "rows_bwd<128,snap=in>", rows_bwd3_kernel<128, 8, Tin, Tin, false>);
-    fill_attr(out, cap, n, "rows_bwd_lockstep<128,snap=in>", rows_bwd2_kernel<128, Tin, Tin, false>);
+    fill_attr(out, cap, n, "rows_bwd<128,snap=in>", rows_bwd3_kernel<128, 8, Tin, Tin, 0>);
+    fill_attr(out, cap, n, "rows_bwd_lockstep<128,snap=in>", rows_bwd2_kernel<128, Tin, Tin, 0>);
 }
 
 // 1 when a bounded wait of this translation unit's kernels gave up since the last call (clears the flag)

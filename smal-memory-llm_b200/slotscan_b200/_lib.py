@@ -41,6 +41,11 @@ class FwdExtra(ctypes.Structure):
                [("no_undo_log", ctypes.c_int32)]
 
 
+class Storage(ctypes.Structure):
+    """slotscan_storage of include/slotscan.h."""
+    _fields_ = [("bits", ctypes.c_int32), ("group", ctypes.c_int32)]
+
+
 class EpilogueParams(ctypes.Structure):
     """slotscan_epilogue_params of include/slotscan.h."""
     _fields_ = [("rows", ctypes.c_int64), ("D", ctypes.c_int32), ("in_dtype", ctypes.c_int32),
@@ -82,6 +87,11 @@ def lib():
         L.slotscan_hard_fwd_ex.restype = ci
         L.slotscan_hard_bwd_ex.argtypes = [PP, vp, vp, vp, vp, vp, vp, LP, vp, vp, vp, vp, sz, vp, vp, vp, vp, vp, vp, vp]
         L.slotscan_hard_bwd_ex.restype = ci
+        SP = ctypes.POINTER(Storage)
+        L.slotscan_hard_fwd_q.argtypes = [PP, vp, vp, vp, vp, vp, vp, vp, vp, LP, ctypes.POINTER(FwdExtra), SP, vp]
+        L.slotscan_hard_fwd_q.restype = ci
+        L.slotscan_hard_bwd_q.argtypes = [PP] + [vp] * 6 + [LP, vp, vp, vp, SP, vp, sz] + [vp] * 7
+        L.slotscan_hard_bwd_q.restype = ci
         DP = ctypes.POINTER(DenseParams)
         L.slotscan_dense_check.argtypes = [DP]
         L.slotscan_dense_check.restype = ci

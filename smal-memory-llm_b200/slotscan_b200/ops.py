@@ -60,11 +60,12 @@ def _fwd_shapes(k, v, N, G, snap_bf16, want_norm, undo_log, new):
 def hard_fwd(k: torch.Tensor, q: Optional[torch.Tensor], v: torch.Tensor, gate: torch.Tensor, fr: torch.Tensor,
              temp: torch.Tensor, K0: Optional[torch.Tensor], V0: Optional[torch.Tensor], o0: Optional[torch.Tensor],
              nsq0: Optional[torch.Tensor], N: int, G: int, hard_gate: bool, eps: float, occ_bin: bool,
-             snap_bf16: bool, want_norm: bool, undo_log: bool
+             snap_bf16: bool, want_norm: bool, undo_log: bool, qbits: int = 0, qgroup: int = 16
              ) -> Tuple[torch.Tensor, torch.Tensor, torch.Tensor, torch.Tensor, torch.Tensor, torch.Tensor, torch.Tensor,
                         torch.Tensor, torch.Tensor, torch.Tensor, torch.Tensor, torch.Tensor, torch.Tensor, torch.Tensor]:
     """k, q, v: contiguous f32 or bf16 (same dtype); gate, fr, temp: contiguous f32.  K0, V0, o0 (f32), nsq0 (f64):
-    the state carried in from the preceding chunk, or None.  Returns, in the order of `OUT`: kbuf, vbuf, the log
+    the state carried in from the preceding chunk, or None.  qbits, qgroup: the storage quantiser of the emitted
+    snapshots (codes of slotscan_epilogue_params, 0: none); kinv and valid are then the quantised rows'.  Returns, in the order of `OUT`: kbuf, vbuf, the log
     (addr, oold, kold, vold, kfin, vfin, ofin, tfirst, kiold; include/slotscan.h), nsqfin, kinv, valid."""
     _require_cuda(k, q, v, gate, fr, temp, K0, V0, o0, nsq0)
     dev = k.device
@@ -77,14 +78,16 @@ def hard_fwd(k: torch.Tensor, q: Optional[torch.Tensor], v: torch.Tensor, gate: 
     ex = _lib.FwdExtra(_addr(K0), _addr(V0), _addr(o0), _addr(nsq0), _addr(nsqfin), _addr(kinv), _addr(valid),
                        0 if undo_log else 1)
     with torch.cuda.device(dev):
-        rc = _lib.lib().slotscan_hard_fwd_ex(ctypes.byref(p), _ptr(k), _ptr(q), _ptr(v), _ptr(gate), _ptr(fr), _ptr(temp),
-                                             _ptr(kbuf), _ptr(vbuf), ctypes.byref(log), ctypes.byref(ex), _stream(dev))
-    _lib.check(rc, "slotscan_hard_fwd_ex")
+        rc = _lib.lib().slotscan_hard_fwd_q(ctypes.byref(p), _ptr(k), _ptr(q), _ptr(v), _ptr(gate), _ptr(fr), _ptr(temp),
+                                            _ptr(kbuf), _ptr(vbuf), ctypes.byref(log), ctypes.byref(ex),
+                                            ctypes.byref(_lib.Storage(qbits, qgroup)), _stream(dev))
+    _lib.check(rc, "slotscan_hard_fwd_q")
     return out
 
 
 @hard_fwd.register_fake
-def _(k, q, v, gate, fr, temp, K0, V0, o0, nsq0, N, G, hard_gate, eps, occ_bin, snap_bf16, want_norm, undo_log):
+def _(k, q, v, gate, fr, temp, K0, V0, o0, nsq0, N, G, hard_gate, eps, occ_bin, snap_bf16, want_norm, undo_log, qbits=0,
+      qgroup=16):
     return _fwd_shapes(k, v, N, G, snap_bf16, want_norm, undo_log, lambda s, dt: k.new_empty(s, dtype=dt))
 
 
@@ -93,7 +96,7 @@ def hard_bwd(k: torch.Tensor, q: Optional[torch.Tensor], v: torch.Tensor, gate: 
              temp: torch.Tensor, addr: torch.Tensor, oold: torch.Tensor, kold: torch.Tensor, vold: torch.Tensor,
              kfin: torch.Tensor, vfin: torch.Tensor, ofin: torch.Tensor, tfirst: torch.Tensor, kiold: torch.Tensor,
              dkbuf: Optional[torch.Tensor], dvbuf: Optional[torch.Tensor], dkinv: Optional[torch.Tensor], N: int, G: int,
-             hard_gate: bool, eps: float, occ_bin: bool, snap_bf16: bool
+             hard_gate: bool, eps: float, occ_bin: bool, snap_bf16: bool, qbits: int = 0, qgroup: int = 16
              ) -> Tuple[torch.Tensor, torch.Tensor, torch.Tensor, torch.Tensor, torch.Tensor, torch.Tensor]:
     """Returns dk, dq, dv (dtype of k), dgate (B,T,H) f32, dfr (shape of fr) f32, dtemp (1,) f32.
     With q None, dq holds the search-path part, which the kernel has already added into dk.
@@ -113,38 +116,39 @@ def hard_bwd(k: torch.Tensor, q: Optional[torch.Tensor], v: torch.Tensor, gate: 
     dtemp = torch.empty(1, device=dev, dtype=torch.float32)
     log = _lib.Log(*(t.data_ptr() for t in (addr, oold, kold, vold, kfin, vfin, ofin, tfirst, kiold)))
     with torch.cuda.device(dev):
-        rc = L.slotscan_hard_bwd_ex(ctypes.byref(p), _ptr(k), _ptr(q), _ptr(v), _ptr(gate), _ptr(fr), _ptr(temp),
-                                    ctypes.byref(log), _ptr(dkbuf), _ptr(dvbuf), _ptr(dkinv), _ptr(scratch), nbytes,
-                                    _ptr(dk), _ptr(dq), _ptr(dv), _ptr(dgate), _ptr(dfr), _ptr(dtemp), _stream(dev))
-    _lib.check(rc, "slotscan_hard_bwd_ex")
+        rc = L.slotscan_hard_bwd_q(ctypes.byref(p), _ptr(k), _ptr(q), _ptr(v), _ptr(gate), _ptr(fr), _ptr(temp),
+                                   ctypes.byref(log), _ptr(dkbuf), _ptr(dvbuf), _ptr(dkinv),
+                                   ctypes.byref(_lib.Storage(qbits, qgroup)), _ptr(scratch), nbytes, _ptr(dk), _ptr(dq),
+                                   _ptr(dv), _ptr(dgate), _ptr(dfr), _ptr(dtemp), _stream(dev))
+    _lib.check(rc, "slotscan_hard_bwd_q")
     return dk, dq, dv, dgate, dfr, dtemp
 
 
 @hard_bwd.register_fake
 def _(k, q, v, gate, fr, temp, addr, oold, kold, vold, kfin, vfin, ofin, tfirst, kiold, dkbuf, dvbuf, dkinv, N, G,
-      hard_gate, eps, occ_bin, snap_bf16):
+      hard_gate, eps, occ_bin, snap_bf16, qbits=0, qgroup=16):
     f = lambda t: t.new_empty(t.shape, dtype=torch.float32)
     return torch.empty_like(k), torch.empty_like(k), torch.empty_like(v), f(gate), f(fr), gate.new_empty(1)
 
 
 def _setup(ctx, inputs, output):
-    k, q, v, gate, fr, temp, K0, V0, o0, nsq0, N, G, hard_gate, eps, occ_bin, snap_bf16, want_norm, undo_log = inputs
+    k, q, v, gate, fr, temp, K0, V0, o0, nsq0, N, G, hard_gate, eps, occ_bin, snap_bf16, want_norm, undo_log, qbits, qgroup = inputs
     ctx.save_for_backward(k, q, v, gate, fr, temp, *output[2:11])
-    ctx.meta = (N, G, hard_gate, eps, occ_bin, snap_bf16)
+    ctx.meta = (N, G, hard_gate, eps, occ_bin, snap_bf16, qbits, qgroup)
     ctx.set_materialize_grads(False)
 
 
 def _backward(ctx, *grads):
     dkbuf, dvbuf, dkinv = grads[0], grads[1], grads[12]
     k, q, v, gate, fr, temp, addr, oold, kold, vold, kfin, vfin, ofin, tfirst, kiold = ctx.saved_tensors
-    N, G, hard_gate, eps, occ_bin, snap_bf16 = ctx.meta
+    N, G, hard_gate, eps, occ_bin, snap_bf16, qbits, qgroup = ctx.meta
     sdt = torch.bfloat16 if snap_bf16 else torch.float32
     c = lambda g, dt: None if g is None else g.contiguous().to(dt)
     dk, dq, dv, dgate, dfr, dtemp = hard_bwd(k, q, v, gate, fr, temp, addr, oold, kold, vold, kfin, vfin, ofin, tfirst,
                                              kiold, c(dkbuf, sdt), c(dvbuf, sdt), c(dkinv, torch.float32), N, G, hard_gate,
-                                             eps, occ_bin, snap_bf16)
+                                             eps, occ_bin, snap_bf16, qbits, qgroup)
     # no gradient for the carried-in state (K0, V0, o0, nsq0) nor for the integer / flag arguments
-    return (dk, (None if q is None else dq), dv, dgate, dfr, dtemp) + (None,) * 12
+    return (dk, (None if q is None else dq), dv, dgate, dfr, dtemp) + (None,) * 14
 
 
 hard_fwd.register_autograd(_backward, setup_context=_setup)

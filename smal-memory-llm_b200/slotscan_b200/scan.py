@@ -23,6 +23,7 @@ There is no Triton path, no dispatch and no CPU fallback: CPU tensors and unimpl
 import torch
 
 from . import ops
+from .epilogue import _bits
 
 
 def _as_f32(x):
@@ -90,6 +91,12 @@ def scan_with_log(k, v, gate, fr, N, temp, G=16, hard_gate=False, eps=1e-4, q=No
     state: (K0, V0, o0) or (K0, V0, o0, nsq0) -- kfin, vfin, ofin[, nsqfin] of the call that scanned the preceding
     tokens; snapshot 0 is then that state.  undo_log=False skips the rows-before-each-write log (kold, vold come back
     empty): less memory and traffic for inference."""
+    return _scan_with_log(k, v, gate, fr, N, temp, G, hard_gate, eps, q, occ_bin, out_dtype, state, want_norm, undo_log)
+
+
+def _scan_with_log(k, v, gate, fr, N, temp, G, hard_gate, eps, q, occ_bin, out_dtype, state, want_norm, undo_log, qbits=0,
+                   qgroup=16):
+    """scan_with_log, with the storage quantiser of the emitted snapshots."""
     if not k.is_cuda:
         raise RuntimeError("slotscan_b200.scan_with_log: CUDA tensors only (no CPU path in this package)")
     k_, v_, q_ = _token_streams(k, v, q)
@@ -98,7 +105,7 @@ def scan_with_log(k, v, gate, fr, N, temp, G=16, hard_gate=False, eps=1e-4, q=No
     with torch.no_grad():
         out = ops.hard_fwd(k_, q_, v_, _as_f32(gate), fr_, temp_, st[0], st[1], st[2], st[3], int(N), int(G),
                            bool(hard_gate), float(eps), bool(occ_bin), out_dtype == torch.bfloat16, bool(want_norm),
-                           bool(undo_log))
+                           bool(undo_log), qbits, int(qgroup))
     d = dict(zip(ops.OUT, out))
     if want_norm:
         d["valid"] = d["valid"].bool()
@@ -112,23 +119,19 @@ def write_memory(k, v, gate, fr, N, temp, G=16, hard_gate=False, eps=1e-4, q=Non
     """What a writer layer hands to its readers, in one call: `(kbuf', buf', kinv, valid)`  [memlm_sh.py:454-475: the
     scan, then nsq / kinv / valid from the float32 keys, the cast to the model dtype, and `_quantize_mem` when the
     storage is quantised].  Hard address, address gradient detached (the reference's training mode).
-    qbits = 0: the scan kernels emit the snapshots in `out_dtype` and kinv / valid from the float32 state while each
-    key row is in registers -- no pass over the snapshots at all; in the backward the kinv gradient enters the key rows
-    inside the reverse row scan.  qbits in {2,3,4,8}: float32 snapshots, then one quantiser pass (`writer_epilogue`).
+    The scan kernels emit the snapshots in `out_dtype` and kinv / valid from the float32 state while each key row is in
+    registers -- no pass over the snapshots at all; in the backward the kinv gradient enters the key rows inside the
+    reverse row scan.  qbits in {2,3,4,8} or "e4m3": the rows go through the storage quantiser of `writer_epilogue` there,
+    and kinv / valid are the quantised rows'.
     Differentiable in k, q, v, gate, fr, temp."""
     if not k.is_cuda:
         raise RuntimeError("slotscan_b200.write_memory: CUDA tensors only (no CPU path in this package)")
     if out_dtype not in (torch.float32, torch.bfloat16):
         raise ValueError("out_dtype must be float32 or bfloat16")
-    if qbits:
-        from .epilogue import writer_epilogue
-        kb, vb = kv_scan_g(k, v, gate, fr, N, temp, G=G, hard=True, hard_gate=hard_gate, eps=eps, detach_addr=True, q=q,
-                           occ_bin=occ_bin, out_dtype=torch.float32)
-        return writer_epilogue(kb, vb, out_dtype, qbits=qbits, qgroup=qgroup)
     k_, v_, q_ = _token_streams(k, v, q)
     fr_, temp_ = _scalars(fr, temp, k.device)
     out = ops.hard_fwd(k_, q_, v_, _as_f32(gate), fr_, temp_, None, None, None, None, int(N), int(G), bool(hard_gate),
-                       float(eps), bool(occ_bin), out_dtype == torch.bfloat16, True, True)
+                       float(eps), bool(occ_bin), out_dtype == torch.bfloat16, True, True, _bits(qbits), int(qgroup))
     return out[0], out[1], out[12], out[13].bool()
 
 
@@ -149,12 +152,10 @@ class StreamingScan:
     def push(self, k, v, gate, fr, q=None):
         if self.tokens % self.G:
             raise ValueError("StreamingScan: only the last chunk may have a length that is not a multiple of G")
-        emit = torch.float32 if self.qbits else self.out_dtype
-        lg = scan_with_log(k, v, gate, fr, q=q, out_dtype=emit, state=self.state, want_norm=not self.qbits,
-                           undo_log=False, **self.kw)
+        if self.qbits and self.out_dtype not in (torch.float32, torch.bfloat16):
+            raise TypeError("out_dtype must be float32 or bfloat16")
+        lg = _scan_with_log(k, v, gate, fr, q=q, out_dtype=self.out_dtype, state=self.state, want_norm=True, undo_log=False,
+                            qbits=_bits(self.qbits), qgroup=self.qgroup, **self.kw)
         self.state = (lg["kfin"], lg["vfin"], lg["ofin"], lg["nsqfin"])
         self.tokens += k.shape[1]
-        if self.qbits:
-            from .epilogue import writer_epilogue
-            return writer_epilogue(lg["kbuf"], lg["vbuf"], self.out_dtype, qbits=self.qbits, qgroup=self.qgroup)
         return lg["kbuf"], lg["vbuf"], lg["kinv"], lg["valid"]

@@ -221,3 +221,42 @@ def test_config3_fp8_e4m3_storage_streamed():
         # beyond that only the few elements that landed on the neighbouring code differ
         assert (d > np.abs(want) * 1e-6 + 1e-12).mean() < 2e-3
     assert np.array_equal(valid.numpy(), O.epilogue(want_k.astype(np.float64))[1])
+
+
+@pytest.mark.parametrize("case", [(64, 64, 8, 3, 16, "fill"), (128, 128, 8, "e4m3", 16, "fill"), (128, 128, 16, 8, 128, "clustered"),
+                                  (128, 128, 5, 2, 4, "clustered"), (16, 32, 8, 4, 8, "fill"), (8, 8, 16, 3, 4, "bench"),
+                                  (64, 64, 16, "e4m3", 16, "clustered")], ids=lambda c: "K%d_V%d_G%d_%s_%d" % c[:5])
+@pytest.mark.parametrize("dtypes", [("f32", "f32"), ("bf16", "bf16"), ("bf16", "f32")], ids="_".join)
+def test_quantised_write_equals_scan_then_quantiser(case, dtypes):
+    """write_memory with a quantiser against the float32 scan followed by writer_epilogue: the emitted rows come from the
+    same float32 state through the same arithmetic, so they are bit-identical; kinv sums its squares in another order
+    (128 float32 terms: 1e-5 of itself is far above it), and the gradients differ by the order of two float32 additions,
+    the bound of the other gradient tests), with bf16 streams by their rounding (2^-8 of the largest) where that tips."""
+    S = _S()
+    DK, DV, G, bits, group, dist = case
+    din, dout = (dict(f32=torch.float32, bf16=torch.bfloat16)[x] for x in dtypes)
+    B, T, H, N = 2, 131, 2, 48
+    inp = make_inputs(dist, B, T, H, DK, DV, seed=41)
+    gen = torch.Generator(device=DEV).manual_seed(3)
+    NB = (T + G - 1) // G
+    ups = [torch.randn(B, NB, H, N, d, device=DEV, generator=gen).to(dout) for d in (DK, DV)]
+    ups.append(0.1 * torch.randn(B, NB, H, N, device=DEV, generator=gen))
+
+    def go(fused):
+        x = [inp[n].to(DEV, din if n in "kqv" else torch.float32).requires_grad_() for n in ("k", "q", "v", "gate", "fr")]
+        k, q, v, g, fr = x
+        x.append(torch.tensor(16.0, device=DEV, requires_grad=True))
+        if fused:
+            out = S.write_memory(k, v, g, fr, N, x[5], G=G, q=q, occ_bin=True, out_dtype=dout, qbits=bits, qgroup=group)
+        else:
+            kb, vb = S.kv_scan_g(k, v, g, fr, N, x[5], G=G, hard=True, detach_addr=True, q=q, occ_bin=True)
+            out = S.writer_epilogue(kb, vb, dout, qbits=bits, qgroup=group)
+        return out, torch.autograd.grad(out[:3], x, ups)
+    (a, ga), (b, gb) = go(True), go(False)
+    assert torch.equal(a[0], b[0]) and torch.equal(a[1], b[1]) and torch.equal(a[3], b[3])
+    assert ((a[2] - b[2]).abs() <= 1e-5 * b[2]).all()
+    for n, x, y in zip(("dk", "dq", "dv", "dgate", "dfr", "dtemp"), ga, gb):
+        band = 2.0 ** -8 if x.dtype == torch.bfloat16 else 1e-4
+        assert (x.float() - y.float()).abs().max() <= band * y.float().abs().max(), n
+    from slotscan_b200 import _lib
+    assert _lib.device_status() == 0
