@@ -135,14 +135,34 @@ int slotscan_hard_bwd_ex(const slotscan_params* p, const void* k, const void* q,
                          const void* dvbuf, const float* dkinv, void* scratch, size_t scratch_bytes, void* dk, void* dq,
                          void* dv, float* dgate, float* dfr, float* dtemp, void* stream);
 
+/* The two calls with the storage quantiser of slotscan_writer_epilogue inside: the emitted snapshots are the quantised rows
+ * (in snap_dtype), taken from the float32 state while a row is in registers, and kinv / valid are the quantised key row's
+ * -- what memlm_sh.py:464-475 hands over when the storage is quantised, without float32 snapshots and without a pass over
+ * them.  The state itself and the log are not quantised.  The backward treats the quantiser as the identity
+ * (straight-through, memlm_sh.py:229): dkbuf, dvbuf are the gradients of the quantised snapshots, and dkinv enters as
+ * -kinv^3 dkinv fq(K_n).  bits, group: as in slotscan_epilogue_params, for both widths; NULL or bits = 0: the _ex call. */
+typedef struct {
+    int32_t bits, group;
+} slotscan_storage;
+int slotscan_hard_fwd_q(const slotscan_params* p, const void* k, const void* q, const void* v, const float* gate,
+                        const float* fr, const float* temp, void* kbuf, void* vbuf, const slotscan_log* log,
+                        const slotscan_fwd_extra* ex, const slotscan_storage* storage, void* stream);
+int slotscan_hard_bwd_q(const slotscan_params* p, const void* k, const void* q, const void* v, const float* gate,
+                        const float* fr, const float* temp, const slotscan_log* log, const void* dkbuf,
+                        const void* dvbuf, const float* dkinv, const slotscan_storage* storage, void* scratch,
+                        size_t scratch_bytes, void* dk, void* dq, void* dv, float* dgate, float* dfr, float* dtemp,
+                        void* stream);
+
 /* The same backward for callers that cannot supply scratch memory.  [No counterpart in the reference: its host side
  * always allocates through torch.]  Meant for hosts whose device memory is already fully assigned (a server that
  * handed everything to its own arena, a binding with no device allocator) or that must not make a synchronising
  * allocation on this path.  The table D[t,n] and the partial sums live in ONE fixed array of
  * SLOTSCAN_NOALLOC_SCRATCH_BYTES inside the library (each GPU that loads the library holds that much until the process
  * exits).  Arguments and results are those of slotscan_hard_bwd without `scratch`; results are bit-identical to it.
- *   - Limit: slotscan_hard_bwd_scratch_bytes(p) must not exceed the capacity, i.e. roughly B*H*T*N <= 1 M table
- *     entries; beyond that the call returns SLOTSCAN_E_TOO_LARGE and launches nothing.
+ *   - Limit: the two D tables, the partial sums and a 32-row next-write table must fit the capacity, i.e. roughly
+ *     B*H*T*N <= 1 M table entries; beyond that the call returns SLOTSCAN_E_TOO_LARGE and launches nothing.  (For the last
+ *     2 % below the limit the next-write table of all rows has no room: sequences with more than 32 rows in use then take
+ *     another kernel than slotscan_hard_bwd's, with the sums in another order.)
  *   - The call itself allocates no device memory and frees none.
  *   - On EVERY call the current device (cudaGetDevice) must be the one that owns `stream` and all the pointers: the
  *     array used is the current device's copy.  Inputs found on another device are refused with SLOTSCAN_E_MODE.

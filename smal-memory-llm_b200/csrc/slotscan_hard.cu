@@ -93,7 +93,7 @@ static cudaStream_t side_stream(cudaStream_t caller) {
 
 static cudaError_t fwd_run(const slotscan_params& p, const void* k, const void* q, const void* v, const float* gate,
                            const float* fr, const float* temp, void* kbuf, void* vbuf, const slotscan_log& L,
-                           const slotscan_fwd_extra& ex, cudaStream_t st) {
+                           const slotscan_fwd_extra& ex, const slotscan_storage& qs, cudaStream_t st) {
     cudaError_t e;
     // While the address scan runs (sequential, almost no memory traffic; on a second stream, see below) every snapshot
     // row above the first row tile is zero-filled: rows are taken in index order, so a tile that never becomes a
@@ -122,8 +122,8 @@ static cudaError_t fwd_run(const slotscan_params& p, const void* k, const void* 
         return (p.in_dtype == SLOTSCAN_F32) ? run_addr_fwd_f32(p, q ? q : k, k, gate, fr, temp, L, S0, s)
                                             : run_addr_fwd_bf16(p, q ? q : k, k, gate, fr, temp, L, S0, s);
     };
-    const ReplayPtrs rk{k, ex.K0, kbuf, ex.no_undo_log ? nullptr : L.kold, L.kfin, ex.kinv, ex.valid, zk};
-    const ReplayPtrs rv{v, ex.V0, vbuf, ex.no_undo_log ? nullptr : L.vold, L.vfin, nullptr, nullptr, zv};
+    const ReplayPtrs rk{k, ex.K0, kbuf, ex.no_undo_log ? nullptr : L.kold, L.kfin, ex.kinv, ex.valid, zk, qs.bits, qs.group};
+    const ReplayPtrs rv{v, ex.V0, vbuf, ex.no_undo_log ? nullptr : L.vold, L.vfin, nullptr, nullptr, zv, qs.bits, qs.group};
     if (joined != nullptr) {
         // The zero-fill goes on the caller's stream and the SCAN on the second stream, behind `fork`: the fill's CTAs (one
         // per SM) are then placed first, on an idle machine, evenly, and three CTAs of the scan still fit beside each.
@@ -187,7 +187,7 @@ static cudaError_t fwd_run(const slotscan_params& p, const void* k, const void* 
 
 static cudaError_t bwd_run(const slotscan_params& p, const void* k, const void* q, const void* v, const float* gate,
                            const float* fr, const float* temp, const slotscan_log& L, const void* dkbuf, const void* dvbuf,
-                           const float* dkinv, float* Dn, float* part, int* vend, void* dk, void* dq, void* dv,
+                           const float* dkinv, const slotscan_storage& qs, float* Dn, float* part, int* vend, int* vend_all, void* dk, void* dq, void* dv,
                            float* dgate, float* dfr, float* dtemp, cudaStream_t st) {
     cudaError_t e;
     // partial sums of dtemp / scalar dfr: one slot per (sequence, 32-token chunk) + one per sequence; slots that no
@@ -204,7 +204,7 @@ static cudaError_t bwd_run(const slotscan_params& p, const void* k, const void* 
         if (side != nullptr && cudaEventCreateWithFlags(&fork, cudaEventDisableTiming) == cudaSuccess &&
             cudaEventCreateWithFlags(&joined, cudaEventDisableTiming) == cudaSuccess) {
             if (cudaEventRecord(fork, st) == cudaSuccess && cudaStreamWaitEvent(side, fork, 0) == cudaSuccess) {
-                vend_ready = run_next_write(p, L, vend, side) == cudaSuccess && cudaEventRecord(joined, side) == cudaSuccess;
+                vend_ready = run_next_write(p, L, vend, vend_all, side) == cudaSuccess && cudaEventRecord(joined, side) == cudaSuccess;
                 // error path: nothing of this call stays in flight on the second stream; the table is then filled on the caller's
                 if (!vend_ready) cudaStreamSynchronize(side);
             }
@@ -216,8 +216,8 @@ static cudaError_t bwd_run(const slotscan_params& p, const void* k, const void* 
     if ((e = cudaMemsetAsync(part, 0, 2 * part_n * sizeof(float), st)) != cudaSuccess) return e;
     // keys and values are independent given the log: one launch (blockIdx.z) when dk == dv, each into its own D table
     float* DnV = Dn + (size_t)p.B * p.H * p.T * p.N;
-    const RowsBwdPtrs ak{k, L.kold, L.kfin, dkbuf, dk, Dn, dkinv};
-    const RowsBwdPtrs av{v, L.vold, L.vfin, dvbuf, dv, DnV, nullptr};
+    const RowsBwdPtrs ak{k, L.kold, L.kfin, dkbuf, dk, Dn, dkinv, qs.bits, qs.group};
+    const RowsBwdPtrs av{v, L.vold, L.vfin, dvbuf, dv, DnV, nullptr, 0, 0};
     if (p.DK == p.DV) {
         ProfScope ps(K_ROWS_BWD_K, st);
         e = run_rows_bwd(p, p.DK, 2, ak, av, gate, L.addr, L.tfirst, st);
@@ -235,8 +235,8 @@ static cudaError_t bwd_run(const slotscan_params& p, const void* k, const void* 
     {
         ProfScope ps(K_ADDR_BWD, st);
         e = (p.in_dtype == SLOTSCAN_F32)
-                ? run_addr_bwd_f32(p, q ? q : k, k, gate, fr, temp, L, Dn, dq, dgate, dfr, part, vend, part_stride, vend_ready, st)
-                : run_addr_bwd_bf16(p, q ? q : k, k, gate, fr, temp, L, Dn, dq, dgate, dfr, part, vend, part_stride, vend_ready, st);
+                ? run_addr_bwd_f32(p, q ? q : k, k, gate, fr, temp, L, Dn, dq, dgate, dfr, part, vend, vend_all, part_stride, vend_ready, st)
+                : run_addr_bwd_bf16(p, q ? q : k, k, gate, fr, temp, L, Dn, dq, dgate, dfr, part, vend, vend_all, part_stride, vend_ready, st);
     }
     if (e != cudaSuccess) return e;
     ProfScope ps(K_FINISH, st);
@@ -282,11 +282,30 @@ extern "C" int slotscan_check(const slotscan_params* p) {
     return SLOTSCAN_OK;
 }
 
+// the quantiser's arguments for both widths: those of the writer epilogue
+static int check_storage(const slotscan_params* p, const slotscan_storage* s) {
+    if (s == nullptr || s->bits == 0) return SLOTSCAN_OK;
+    for (int D : {p->DK, p->DV}) {
+        const slotscan_epilogue_params e = {0, D, p->snap_dtype, p->snap_dtype, s->bits, s->group};
+        const int rc = slotscan_epilogue_check(&e);
+        if (rc) return rc;
+    }
+    return SLOTSCAN_OK;
+}
+
 extern "C" int slotscan_hard_fwd_ex(const slotscan_params* p, const void* k, const void* q, const void* v,
                                     const float* gate, const float* fr, const float* temp, void* kbuf, void* vbuf,
-                                    const slotscan_log* log, const slotscan_fwd_extra* ex_, void* stream) {
+                                    const slotscan_log* log, const slotscan_fwd_extra* ex, void* stream) {
+    return slotscan_hard_fwd_q(p, k, q, v, gate, fr, temp, kbuf, vbuf, log, ex, nullptr, stream);
+}
+
+extern "C" int slotscan_hard_fwd_q(const slotscan_params* p, const void* k, const void* q, const void* v,
+                                   const float* gate, const float* fr, const float* temp, void* kbuf, void* vbuf,
+                                   const slotscan_log* log, const slotscan_fwd_extra* ex_, const slotscan_storage* storage,
+                                   void* stream) {
     int rc = slotscan_check(p);
     if (rc) return rc;
+    if ((rc = check_storage(p, storage)) != SLOTSCAN_OK) return rc;
     slotscan_fwd_extra ex = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, 0};
     if (ex_) ex = *ex_;
     if (!k || !v || !gate || !fr || !temp || !kbuf || !vbuf || !log) return SLOTSCAN_E_NULL;
@@ -300,7 +319,7 @@ extern "C" int slotscan_hard_fwd_ex(const slotscan_params* p, const void* k, con
         misaligned(log->vold) || misaligned(log->kfin) || misaligned(log->vfin) || misaligned(ex.K0) || misaligned(ex.V0))
         return SLOTSCAN_E_ALIGN;
     cudaStream_t st = (cudaStream_t)stream;
-    const cudaError_t e = fwd_run(*p, k, q, v, gate, fr, temp, kbuf, vbuf, *log, ex, st);
+    const cudaError_t e = fwd_run(*p, k, q, v, gate, fr, temp, kbuf, vbuf, *log, ex, storage ? *storage : slotscan_storage{0, 0}, st);
     return (int)e;
 }
 
@@ -311,7 +330,8 @@ extern "C" int slotscan_hard_fwd(const slotscan_params* p, const void* k, const 
 }
 
 // scratch layout: [D table keys | D table values] [partial sums 2 x B*H x (chunks + 1) f32] [next-write table B*H x chunks x 32 i32]
-static void bwd_scratch_layout(const slotscan_params* p, size_t* off_part, size_t* off_vend, size_t* total) {
+// and, where the call takes it and there is room, [next-write table of all rows B*H x chunks x N i32]; least: without that
+static void bwd_scratch_layout(const slotscan_params* p, size_t* off_part, size_t* off_vend, size_t* least, size_t* total) {
     const size_t BH = (size_t)p->B * p->H, nc = ((size_t)p->T + GATHER_CHUNK - 1) / GATHER_CHUNK;
     size_t o = 2 * sizeof(float) * BH * p->T * p->N;       // one D table for the keys, one for the values
     o = (o + 255) & ~(size_t)255;
@@ -320,13 +340,15 @@ static void bwd_scratch_layout(const slotscan_params* p, size_t* off_part, size_
     o = (o + 255) & ~(size_t)255;
     *off_vend = o;
     o += sizeof(int) * BH * nc * GATHER_ROWS_MAX;
+    *least = o;
+    if (next_write_used(*p) && p->N > GATHER_ROWS_MAX) o = ((o + 255) & ~(size_t)255) + sizeof(int) * BH * nc * p->N;
     *total = o;
 }
 
 extern "C" size_t slotscan_hard_bwd_scratch_bytes(const slotscan_params* p) {
     if (slotscan_check(p)) return 0;
-    size_t a, b, t;
-    bwd_scratch_layout(p, &a, &b, &t);
+    size_t a, b, l, t;
+    bwd_scratch_layout(p, &a, &b, &l, &t);
     return t;
 }
 
@@ -343,25 +365,37 @@ extern "C" int slotscan_hard_bwd_ex(const slotscan_params* p, const void* k, con
                                     const void* dkbuf, const void* dvbuf, const float* dkinv, void* scratch,
                                     size_t scratch_bytes, void* dk, void* dq, void* dv, float* dgate, float* dfr,
                                     float* dtemp, void* stream) {
+    return slotscan_hard_bwd_q(p, k, q, v, gate, fr, temp, log, dkbuf, dvbuf, dkinv, nullptr, scratch, scratch_bytes, dk, dq, dv,
+                               dgate, dfr, dtemp, stream);
+}
+
+extern "C" int slotscan_hard_bwd_q(const slotscan_params* p, const void* k, const void* q, const void* v,
+                                   const float* gate, const float* fr, const float* temp, const slotscan_log* log,
+                                   const void* dkbuf, const void* dvbuf, const float* dkinv, const slotscan_storage* storage,
+                                   void* scratch, size_t scratch_bytes, void* dk, void* dq, void* dv, float* dgate,
+                                   float* dfr, float* dtemp, void* stream) {
     int rc = slotscan_check(p);
     if (rc) return rc;
+    if ((rc = check_storage(p, storage)) != SLOTSCAN_OK) return rc;
     if (!k || !v || !gate || !fr || !temp || !log || !scratch || !dk || !dq || !dv || !dgate || !dfr || !dtemp)
         return SLOTSCAN_E_NULL;
     if (!log->addr || !log->oold || !log->kold || !log->vold || !log->kfin || !log->vfin || !log->ofin || !log->tfirst ||
         !log->kiold)
         return SLOTSCAN_E_NULL;
-    if (scratch_bytes < slotscan_hard_bwd_scratch_bytes(p)) return SLOTSCAN_E_SHAPE;
+    size_t off_part, off_vend, least, total;
+    bwd_scratch_layout(p, &off_part, &off_vend, &least, &total);
+    if (scratch_bytes < least) return SLOTSCAN_E_SHAPE;
     if (misaligned(k) || misaligned(q) || misaligned(v) || misaligned(dkbuf) || misaligned(dvbuf) || misaligned(dk) ||
         misaligned(dq) || misaligned(dv) || misaligned(scratch) || misaligned(log->kold) || misaligned(log->vold) ||
         misaligned(log->kfin) || misaligned(log->vfin))
         return SLOTSCAN_E_ALIGN;
-    size_t off_part, off_vend, total;
-    bwd_scratch_layout(p, &off_part, &off_vend, &total);
     float* Dn = (float*)scratch;
     float* part = (float*)((char*)scratch + off_part);
     int* vend = (int*)((char*)scratch + off_vend);
+    int* vend_all = total > least && scratch_bytes >= total ? (int*)((char*)scratch + ((least + 255) & ~(size_t)255)) : nullptr;
     cudaStream_t st = (cudaStream_t)stream;
-    const cudaError_t e = bwd_run(*p, k, q, v, gate, fr, temp, *log, dkbuf, dvbuf, dkinv, Dn, part, vend, dk, dq, dv, dgate,
+    const cudaError_t e = bwd_run(*p, k, q, v, gate, fr, temp, *log, dkbuf, dvbuf, dkinv,
+                                  storage ? *storage : slotscan_storage{0, 0}, Dn, part, vend, vend_all, dk, dq, dv, dgate,
                                   dfr, dtemp, st);
     return (int)e;
 }
@@ -433,7 +467,9 @@ extern "C" int slotscan_hard_bwd_noalloc(const slotscan_params* p, const void* k
                                          float* dfr, float* dtemp, void* stream) {
     int rc = slotscan_check(p);
     if (rc) return rc;
-    if (slotscan_hard_bwd_scratch_bytes(p) > (size_t)SLOTSCAN_NOALLOC_SCRATCH_BYTES) return SLOTSCAN_E_TOO_LARGE;
+    size_t off_part, off_vend, least, total;
+    bwd_scratch_layout(p, &off_part, &off_vend, &least, &total);
+    if (least > (size_t)SLOTSCAN_NOALLOC_SCRATCH_BYTES) return SLOTSCAN_E_TOO_LARGE;
     int dev = -1;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return (int)e;

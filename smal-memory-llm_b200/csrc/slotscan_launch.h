@@ -24,24 +24,26 @@ cudaError_t run_addr_fwd_f32(const slotscan_params& p, const void* q, const void
                              const float* temp, const slotscan_log& L, const AddrFwdState& S0, cudaStream_t st);
 cudaError_t run_addr_fwd_bf16(const slotscan_params& p, const void* q, const void* k, const float* gate, const float* fr,
                               const float* temp, const slotscan_log& L, const AddrFwdState& S0, cudaStream_t st);
-// vend_ready: the next-write table (run_next_write) has been filled already, on a stream this one is ordered after
+// vend_ready: the next-write tables (run_next_write) have been filled already, on a stream this one is ordered after;
+// vend_all: the table of all rows, NULL where the scratch has no room for it (the chunked kernel then takes its sequences)
 cudaError_t run_addr_bwd_f32(const slotscan_params& p, const void* q, const void* k, const float* gate, const float* fr,
                              const float* temp, const slotscan_log& L, const float* Dn, void* dq, float* dgate, float* dfr,
-                             float* part, int* vend, int part_stride, bool vend_ready, cudaStream_t st);
+                             float* part, int* vend, int* vend_all, int part_stride, bool vend_ready, cudaStream_t st);
 cudaError_t run_addr_bwd_bf16(const slotscan_params& p, const void* q, const void* k, const float* gate, const float* fr,
                               const float* temp, const slotscan_log& L, const float* Dn, void* dq, float* dgate, float* dfr,
-                              float* part, int* vend, int part_stride, bool vend_ready, cudaStream_t st);
+                              float* part, int* vend, int* vend_all, int part_stride, bool vend_ready, cudaStream_t st);
 // the next-write table of the token-parallel address backward: it depends on the forward's log only, so it can run
 // beside the reverse row scan; true when the address backward of this shape uses it
 bool next_write_used(const slotscan_params& p);
-cudaError_t run_next_write(const slotscan_params& p, const slotscan_log& L, int* vend, cudaStream_t st);
+cudaError_t run_next_write(const slotscan_params& p, const slotscan_log& L, int* vend, int* vend_all, cudaStream_t st);
 // tokens per CTA of the token-parallel address backward: the partial-sum table has one slot per such chunk (+ 1)
 constexpr int GATHER_CHUNK = 32;
 constexpr int GATHER_ROWS_MAX = 32;
 // One tensor (keys: D = DK, values: D = DV) of the forward row replay.  x0: the rows the replay starts from (NULL =
 // zeros); xold NULL: no undo log; kinv / valid: per emitted row, from the float32 state (keys only, or NULL);
 // zero_from: rows >= zero_from were zero-filled ahead by run_zero_rows (N = none).
-struct ReplayPtrs { const void* x; const float* x0; void* xbuf; float* xold; float* xfin; float* kinv; uint8_t* valid; int zero_from; };
+// bits, group: storage quantiser of the emitted rows (bits 0: none), the same for both tensors
+struct ReplayPtrs { const void* x; const float* x0; void* xbuf; float* xold; float* xfin; float* kinv; uint8_t* valid; int zero_from; int bits, group; };
 // ntensors = 2 runs keys and values in one launch (needs DK == DV), 1 runs r0 only
 // row tiles [tile_lo, tile_hi) of replay_tile_rows(D) rows each; tile_hi < 0: up to the last one
 cudaError_t run_replay(const slotscan_params& p, int D, int ntensors, const ReplayPtrs& r0, const ReplayPtrs& r1,
@@ -53,7 +55,8 @@ cudaError_t run_zero_rows(const slotscan_params& p, void* kbuf, int zk, void* vb
                           cudaStream_t st);
 // reverse row scan; ntensors = 2 runs keys and values in one launch (needs DK == DV), 1 runs the first set only
 // dkinv: upstream gradient of the kinv output (keys only, NULL otherwise)
-struct RowsBwdPtrs { const void* x; const float* xold; const float* xfin; const void* dxbuf; void* dx; float* Dn; const float* dkinv; };
+// bits, group: the storage quantiser that output was taken behind (bits 0: none)
+struct RowsBwdPtrs { const void* x; const float* xold; const float* xfin; const void* dxbuf; void* dx; float* Dn; const float* dkinv; int bits, group; };
 cudaError_t run_rows_bwd_f32(const slotscan_params& p, int D, int ntensors, const RowsBwdPtrs& a0, const RowsBwdPtrs& a1,
                              const float* gate, const int* am, const int* tfirst, cudaStream_t st);
 cudaError_t run_rows_bwd_bf16(const slotscan_params& p, int D, int ntensors, const RowsBwdPtrs& a0, const RowsBwdPtrs& a1,

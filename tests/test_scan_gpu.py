@@ -260,3 +260,33 @@ def test_full_size_properties():
     assert torch.equal(lg2["vbuf"], 2 * vb[:8]) and torch.equal(lg2["addr"], addr[:8])
     del lg, lg2, sub, kb, vb, changed, hit
     torch.cuda.empty_cache()
+
+
+@pytest.mark.parametrize("N,T,DK,DV,G,frtok,sepq", [(33, 97, 32, 32, 8, True, True), (64, 128, 64, 64, 16, True, False),
+                                                    (65, 140, 128, 128, 8, False, True), (97, 129, 32, 64, 8, True, True),
+                                                    (160, 300, 64, 64, 8, True, True), (192, 420, 128, 128, 16, True, True)])
+def test_address_backward_many_rows(N, T, DK, DV, G, frtok, sepq):
+    """The token-parallel address backward of sequences with more than 32 rows in use: row counts around its groups of 32
+    slots, a last chunk of one token and of 32, each width it is built for; a batch in which some sequences use few rows
+    (the gather kernel's) and some many, so that its work list has gaps.  Gradients within 1e-4 of their largest, as the
+    other float32 cases of this file."""
+    import slotscan_b200 as S
+    few, many = (make_inputs(d, 2, T, 3, DK, DV, seed=61, frtok=frtok, sepq=sepq) for d in ("bench", "fill"))
+    inp = {n: (torch.cat([few[n][:1], many[n], few[n][1:]]) if torch.is_tensor(few[n]) and few[n].dim() > 1 else many[n])
+           for n in many}
+    kw = dict(N=N, temp=16.0, G=G, hard=True, q=inp["q"], occ_bin=True)
+    ref = O.scan_fwd(inp["k"], inp["v"], inp["gate"], inp["fr"], dtype=np.float64, **kw)
+    assert ref["margin"].min() > 1e-5, "pick another seed: a near-tie flips everything after it"
+    gen = torch.Generator().manual_seed(9)
+    wk, wv = (torch.randn(ref[n].shape, generator=gen) for n in ("kbuf", "vbuf"))
+    x = [None if inp[n] is None else inp[n].to("cuda").requires_grad_() for n in ("k", "q", "v", "gate", "fr")]
+    tp = torch.tensor(16.0, device="cuda", requires_grad=True)
+    kb, vb = S.kv_scan_c(x[0], x[2], x[3], x[4], N, tp, G=G, hard=True, detach_addr=True, q=x[1], occ_bin=True)
+    torch.autograd.backward([kb, vb], [wk.cuda(), wv.cuda()])
+    gr = O.scan_bwd(inp["k"], inp["v"], inp["gate"], inp["fr"], dkbuf=wk.numpy(), dvbuf=wv.numpy(), detach_addr=True,
+                    dtype=np.float64, **kw)
+    for n, t in (("dk", x[0]), ("dq", x[1]), ("dv", x[2]), ("dgate", x[3]), ("dfr", x[4]), ("dtemp", tp)):
+        if t is not None:
+            assert rel_to_max(t.grad.cpu().numpy().reshape(gr[n].shape), gr[n]) < 1e-4, n
+    from slotscan_b200 import _lib
+    assert _lib.device_status() == 0
