@@ -3,6 +3,7 @@
 #include <stdio.h>
 
 #include "slotscan_addr_fwd.cuh"
+#include "slotscan_addr_wide.cuh"
 #include "slotscan_launch.h"
 
 namespace slotscan {
@@ -31,13 +32,31 @@ static cudaError_t launch_one(const slotscan_params& p, const void* q, const voi
     return cudaGetLastError();
 }
 
+template <int DK, int RPL>
+static cudaError_t launch_wide(const slotscan_params& p, const void* q, const void* k, const float* gate, const float* fr,
+                               const float* temp, const slotscan_log& L, const AddrFwdState& S0, cudaStream_t st) {
+    const size_t sm = sizeof(float) * (size_t)addr_wide_layout(RPL, DK).total;
+    cudaError_t e = cudaSuccess;
+    auto go = [&](auto kern) {
+        if ((e = opt_in_smem(kern, sm)) != cudaSuccess) return e;
+        kern<<<p.B * p.H, aw_threads(RPL), sm, st>>>(p, (const Tin*)q, (const Tin*)k, gate, fr, temp, L.addr, L.oold, L.kiold, L.ofin,
+                                                     L.tfirst, S0.K0, S0.o0, S0.nsq0, S0.nsqfin);
+        return cudaGetLastError();
+    };
+    const bool carry = S0.K0 != nullptr;
+    if (p.occ_bin) return carry ? go(addr_fwd_wide_kernel<DK, RPL, true, true, Tin>) : go(addr_fwd_wide_kernel<DK, RPL, true, false, Tin>);
+    return carry ? go(addr_fwd_wide_kernel<DK, RPL, false, true, Tin>) : go(addr_fwd_wide_kernel<DK, RPL, false, false, Tin>);
+}
 template <int DK>
 static cudaError_t launch_dk(const slotscan_params& p, const void* q, const void* k, const float* gate, const float* fr,
                              const float* temp, const slotscan_log& L, const AddrFwdState& S0, cudaStream_t st) {
     if (p.N <= AF_NCAP1) return launch_one<DK, 2>(p, q, k, gate, fr, temp, L, S0, p.N, 0, st);
     cudaError_t e = launch_one<DK, 2>(p, q, k, gate, fr, temp, L, S0, AF_NCAP1, 0, st);
     if (e != cudaSuccess) return e;
-    return launch_one<DK, 6>(p, q, k, gate, fr, temp, L, S0, p.N, 1, st);       // N <= 192
+    if constexpr (DK >= 64) {
+        if (p.N <= 128) return launch_wide<DK, 4>(p, q, k, gate, fr, temp, L, S0, st);
+        return launch_wide<DK, 6>(p, q, k, gate, fr, temp, L, S0, st);           // N <= 192
+    } else return launch_one<DK, 6>(p, q, k, gate, fr, temp, L, S0, p.N, 1, st);  // N <= 192
 }
 
 cudaError_t SS_CAT(run_addr_fwd_, SLOTSCAN_SUFFIX)(const slotscan_params& p, const void* q, const void* k, const float* gate,
@@ -50,7 +69,7 @@ cudaError_t SS_CAT(run_addr_fwd_, SLOTSCAN_SUFFIX)(const slotscan_params& p, con
 
 void SS_CAT(attrs_addr_fwd_, SLOTSCAN_SUFFIX)(slotscan_kernel_attr* out, int cap, int& n) {
     fill_attr(out, cap, n, "addr_fwd<128,rows<=64>", addr_fwd_direct_kernel<128, 2, true, false, Tin>);
-    fill_attr(out, cap, n, "addr_fwd<128,rows<=192>", addr_fwd_direct_kernel<128, 6, true, false, Tin>);
+    fill_attr(out, cap, n, "addr_fwd_wide<128,rows<=192>", addr_fwd_wide_kernel<128, 6, true, false, Tin>);
 }
 
 }  // namespace slotscan

@@ -13,7 +13,7 @@
 // Bound: 2 x (32 + rows) x DK multiply-adds per token on the CUDA cores (float32: the tensor cores' bf16 or tf32 operands
 // would lose bits); the chunked resident-state kernel (slotscan_addr_bwd.cuh) walks 8-token chunks of a sequence one after
 // another with five barriers each.  B = 32, T = 1024, H = 6, 192 rows x 128 all in use, bf16: 2.07 ms chunked, 1.44 ms here;
-// B = 4, T = 1000, H = 12, ~60 rows x 64, float32 (48 sequences, so that the chunked kernel had 48 CTAs): 1.29 -> 0.30 ms.
+// B = 4, T = 1000, H = 12, ~60 rows x 64, float32 (48 sequences, so that the chunked kernel had 48 CTAs): 1.29 -> 0.20 ms.
 // Persistent: the CTAs share the items of the sequences that need this kernel, which they find from the forward's tfirst
 // table (a launch whose sequences all use few rows returns after that look).
 #pragma once
@@ -65,34 +65,47 @@ template <int DK, int NS>
 __device__ __forceinline__ void tiles_scores(const float* rows, const float* sq, float* St) {
     constexpr int RS = TilesLayout<DK>::RS;
     const int lane = threadIdx.x & 31, rg = (threadIdx.x >> 5) * 4 + (lane >> 3), tq = lane & 7;
-    float acc[NS][4];
+    float tot[NS][4];
 #pragma unroll
     for (int i = 0; i < NS; i++)
 #pragma unroll
-        for (int k = 0; k < 4; k++) acc[i][k] = 0.f;
+        for (int k = 0; k < 4; k++) tot[i][k] = 0.f;
+    // a quarter of the columns at a time: four short chains instead of one of DK, whose rounding showed in the gradients
+#pragma unroll 1
+    for (int d0 = 0; d0 < DK; d0 += DK / 4) {
+        float acc[NS][4];
+#pragma unroll
+        for (int i = 0; i < NS; i++)
+#pragma unroll
+            for (int k = 0; k < 4; k++) acc[i][k] = 0.f;
 #pragma unroll 2
-    for (int d = 0; d < DK; d += 4) {
-        float4 q[4];
+        for (int d = d0; d < d0 + DK / 4; d += 4) {
+            float4 q[4];
 #pragma unroll
-        for (int k = 0; k < 4; k++) q[k] = ld4(sq + (tq + 8 * k) * RS + d);
+            for (int k = 0; k < 4; k++) q[k] = ld4(sq + (tq + 8 * k) * RS + d);
 #pragma unroll
-        for (int i = 0; i < NS; i++) {
-            const float4 r = ld4(rows + (rg + 32 * i) * RS + d);
+            for (int i = 0; i < NS; i++) {
+                const float4 r = ld4(rows + (rg + 32 * i) * RS + d);
 #pragma unroll
-            for (int k = 0; k < 4; k++) {
-                acc[i][k] = fmaf(r.x, q[k].x, acc[i][k]);
-                acc[i][k] = fmaf(r.y, q[k].y, acc[i][k]);
-                acc[i][k] = fmaf(r.z, q[k].z, acc[i][k]);
-                acc[i][k] = fmaf(r.w, q[k].w, acc[i][k]);
+                for (int k = 0; k < 4; k++) {
+                    acc[i][k] = fmaf(r.x, q[k].x, acc[i][k]);
+                    acc[i][k] = fmaf(r.y, q[k].y, acc[i][k]);
+                    acc[i][k] = fmaf(r.z, q[k].z, acc[i][k]);
+                    acc[i][k] = fmaf(r.w, q[k].w, acc[i][k]);
+                }
             }
         }
+#pragma unroll
+        for (int i = 0; i < NS; i++)
+#pragma unroll
+            for (int k = 0; k < 4; k++) tot[i][k] += acc[i][k];
     }
 #pragma unroll
     for (int i = 0; i < NS; i++)
 #pragma unroll
         for (int k = 0; k < 4; k++) {
             const int s = rg + 32 * i, j = tq + 8 * k;
-            St[s * 32 + ((((j >> 2) ^ (s & 7)) << 2) | (j & 3))] = acc[i][k];
+            St[s * 32 + ((((j >> 2) ^ (s & 7)) << 2) | (j & 3))] = tot[i][k];
         }
 }
 // place of (slot, token) in St / C: quads of tokens swapped around by slot, so that 8 neighbouring slots of one token (step
@@ -359,32 +372,45 @@ __global__ void __launch_bounds__(TL_THREADS) addr_bwd_tiles_kernel(
             {
                 const int tg = (warp & 3) * 8, half = warp >> 2, cq = lane % CQ, sub = lane / CQ;
                 const int sh = NS * 16, s_lo = half * sh + sub, s_hi = half * sh + sh;
-                float acc[8][4];
+                float tot[8][4];
 #pragma unroll
                 for (int j = 0; j < 8; j++)
 #pragma unroll
-                    for (int k = 0; k < 4; k++) acc[j][k] = 0.f;
+                    for (int k = 0; k < 4; k++) tot[j][k] = 0.f;
                 const bool bad = *s_bad != 0;
+#pragma unroll 1
+                for (int sb = s_lo; sb < s_hi; sb += 16) {               // 16 slots at a time: short chains
+                    float acc[8][4];
+#pragma unroll
+                    for (int j = 0; j < 8; j++)
+#pragma unroll
+                        for (int k = 0; k < 4; k++) acc[j][k] = 0.f;
 #pragma unroll 2
-                for (int s = s_lo; s < s_hi; s += SUB) {
-                    const float4 r = ld4(rows + s * RS + cq * 4);
-                    const float4 c0 = ld4(St + tiles_at(s, tg)), c1 = ld4(St + tiles_at(s, tg + 4));
-                    const float cv[8] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w};
-                    if (!bad) {
+                    for (int s = sb; s < sb + 16; s += SUB) {            // half * sh is a multiple of 16
+                        const float4 r = ld4(rows + s * RS + cq * 4);
+                        const float4 c0 = ld4(St + tiles_at(s, tg)), c1 = ld4(St + tiles_at(s, tg + 4));
+                        const float cv[8] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w};
+                        if (!bad) {
 #pragma unroll
-                        for (int j = 0; j < 8; j++) {
-                            acc[j][0] = fmaf(cv[j], r.x, acc[j][0]);
-                            acc[j][1] = fmaf(cv[j], r.y, acc[j][1]);
-                            acc[j][2] = fmaf(cv[j], r.z, acc[j][2]);
-                            acc[j][3] = fmaf(cv[j], r.w, acc[j][3]);
-                        }
-                    } else {                                             // a version a token does not see stays out of its sum
+                            for (int j = 0; j < 8; j++) {
+                                acc[j][0] = fmaf(cv[j], r.x, acc[j][0]);
+                                acc[j][1] = fmaf(cv[j], r.y, acc[j][1]);
+                                acc[j][2] = fmaf(cv[j], r.z, acc[j][2]);
+                                acc[j][3] = fmaf(cv[j], r.w, acc[j][3]);
+                            }
+                        } else {                                         // a version a token does not see stays out of its sum
 #pragma unroll
-                        for (int j = 0; j < 8; j++) {
-                            if (cv[j] != 0.f) { acc[j][0] += cv[j] * r.x; acc[j][1] += cv[j] * r.y; acc[j][2] += cv[j] * r.z; acc[j][3] += cv[j] * r.w; }
+                            for (int j = 0; j < 8; j++) {
+                                if (cv[j] != 0.f) { acc[j][0] += cv[j] * r.x; acc[j][1] += cv[j] * r.y; acc[j][2] += cv[j] * r.z; acc[j][3] += cv[j] * r.w; }
+                            }
                         }
                     }
+#pragma unroll
+                    for (int j = 0; j < 8; j++)
+#pragma unroll
+                        for (int k = 0; k < 4; k++) tot[j][k] += acc[j][k];
                 }
+                float (&acc)[8][4] = tot;
 #pragma unroll
                 for (int j = 0; j < 8; j++)
 #pragma unroll

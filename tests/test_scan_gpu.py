@@ -290,3 +290,31 @@ def test_address_backward_many_rows(N, T, DK, DV, G, frtok, sepq):
             assert rel_to_max(t.grad.cpu().numpy().reshape(gr[n].shape), gr[n]) < 1e-4, n
     from slotscan_b200 import _lib
     assert _lib.device_status() == 0
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("N,dtype,occ_bin", [(65, torch.float32, True), (128, torch.bfloat16, False), (129, torch.float32, True),
+                                             (192, torch.bfloat16, True)], ids=lambda x: str(x).split(".")[-1])
+def test_wide_address_scan_equals_direct_bitwise(N, D, dtype, occ_bin):
+    """The second pass (rows in registers) against the first (rows in shared memory): the whole sequence uses more than 64
+    rows and takes the second, its first tokens alone stay in the first.  Same sums in the same order, so the log of those
+    tokens is the same bit for bit -- from the empty memory, and with the state carried in (so that more than 32 rows are
+    candidates from the first token on); a length of one staging ring and less, and one that is no multiple of it."""
+    import slotscan_b200 as S
+    B, H, G, T = 3, 2, 8, 211
+    inp = make_inputs("fill", B, T, H, D, D, seed=17)
+    k, q, v = (inp[n].to("cuda", dtype) for n in ("k", "q", "v"))
+    g, fr = inp["gate"].cuda(), inp["fr"].cuda() * (1.0 if occ_bin else 8.0)     # the penalty on o itself is the weaker one
+    kw = dict(G=G, occ_bin=occ_bin)
+    for t0, state in ((0, None), (40, "carry")):
+        if state is not None:
+            lg = S.scan_with_log(k[:, :t0], v[:, :t0], g[:, :t0], fr[:, :t0], N, 16.0, q=q[:, :t0], **kw)
+            state = tuple(lg[n] for n in ("kfin", "vfin", "ofin", "nsqfin"))
+        cut = lambda x, t1: x[:, t0:t1].contiguous()
+        a = S.scan_with_log(*(cut(x, T) for x in (k, v, g, fr)), N, 16.0, q=cut(q, T), state=state, **kw)
+        assert (a["tfirst"][:, 64] < T - t0).all()                     # the whole: second pass
+        for t1 in (t0 + 1, t0 + 9, t0 + 15):
+            b = S.scan_with_log(*(cut(x, t1) for x in (k, v, g, fr)), N, 16.0, q=cut(q, t1), state=state, **kw)
+            assert (b["tfirst"][:, 64] == t1 - t0).all()               # the start of it: first pass
+            for n in ("addr", "oold", "kiold", "kold"):
+                assert torch.equal(a[n][:, :t1 - t0], b[n]), (n, t1)
