@@ -15,8 +15,9 @@
 // Snapshot and gradient tiles arrive by cp.async, issued half a block ahead.
 // Bound: the double-precision dots (N * DS * (G + 1) per block and slice) and, for few rows, the latency of one block's
 // phases -- hence 16-wide slices (half the dot's chain, twice the CTAs) up to 64 rows.  64 sequences, 64 x 64, 128 blocks of
-// 4 tokens: 0.31 ms (0.54 with loads that waited for one another before the weighted sum, 1.23 with 32-wide slices and 16
-// tokens a step); 48 sequences, 192 x (64 + 64), 32 blocks of 16: 0.60 ms.
+// 4 tokens: 0.29 ms (0.54 with loads that waited for one another before the weighted sum, 1.23 with 32-wide slices and 16
+// tokens a step); 48 sequences, 192 x (64 + 64), 32 blocks of 16: 0.42 ms
+// (0.60 with more than 168 registers a thread: 192 CTAs then run in two rounds).
 #include <algorithm>
 
 #include "slotscan_common.cuh"
@@ -43,7 +44,7 @@ struct RowAdjShape {
 };
 
 template <typename Tin, int CT, int DS, bool HARD>
-__global__ void __launch_bounds__(RA_NMAX) row_adjoint_kernel(const RowAdjArgs A) {
+__global__ void __maxnreg__(DS == 32 ? 168 : 255) row_adjoint_kernel(const RowAdjArgs A) {
     constexpr int FS = RowAdjShape<CT, DS>::FS, SS = RowAdjShape<CT, DS>::SS;
     constexpr int XP = (CT * DS + 31) / 32;                          // token elements per thread at 32 threads
     constexpr int NQ = DS / 4, PER = CT / 4 * NQ, NSUB = 32 / PER;   // weighted sum: lanes per row, rows side by side

@@ -16,8 +16,8 @@
 //             value gradients block by block (row_adjoint_kernel); then the chain of the occupancy gradient alone, one
 //             warp per (sequence, head) (keyless_bwd_chain)
 // Bound: the occupancy chain, one double-precision exp, sum over the rows and division per token.  B = 8, T = 512, H = 8,
-// 64 x 64, G = 4, forward + backward: 12.9 ms walking token by token in one CTA (2.35 + 10.4), 0.90 ms split (forward 0.43;
-// backward: tables 0.02, value gradients 0.31, chain 0.12).
+// 64 x 64, G = 4, forward + backward: 12.9 ms walking token by token in one CTA (2.35 + 10.4), 0.85 ms split (forward 0.39;
+// backward: tables 0.02, value gradients 0.29, chain 0.12).
 // The occupancies and the softmax run in double: with the penalty on o itself every rounding error of o comes back
 // multiplied by fr at every later token.
 // More than 256 rows (the reference's shape is 48 x 16) keep the kernels below that hold everything in one CTA and walk
@@ -325,8 +325,8 @@ __device__ __forceinline__ double kl_rcp(double s) {
 // ahead -- so that the chain is exp(-fr o_n), one sum, one reciprocal and the blend.  Warps 2..9: the values, a chunk
 // behind.  The factors neither overflow nor vanish while |fr| <= 300 and the gates stay in [0, 1] (o in [0, 1]); anything
 // else takes the shifted softmax of kl_softmax.  hard: the chain needs the largest wa_n - fr o_n only.
-template <typename Tin, int R>
-__global__ void __launch_bounds__(32 * (2 + KL_CW), 2) keyless_fwd_chain_kernel(
+template <typename Tin, int R, int MINB>
+__global__ void __launch_bounds__(32 * (2 + KL_CW), MINB) keyless_fwd_chain_kernel(
     const slotscan_v_params p, const Tin* __restrict__ v, const float* __restrict__ wa, const float* __restrict__ gate,
     const float* __restrict__ fr_p, float* __restrict__ buf, float* __restrict__ obuf, int* __restrict__ addr) {
     extern __shared__ __align__(16) float ksm[];
@@ -336,6 +336,7 @@ __global__ void __launch_bounds__(32 * (2 + KL_CW), 2) keyless_fwd_chain_kernel(
     double* X = reinterpret_cast<double*>(ksm);             // [2][KL_CT][NR] exp(wa - max wa); hard: wa
     float* gs = reinterpret_cast<float*>(X + 2 * KL_CT * NR);        // [2][KL_CT] gates
     int* wild = reinterpret_cast<int*>(gs + 2 * KL_CT);     // [2] a gate of the chunk lies outside [0, 1]
+    int* soft_chunk = wild + 2;                             // [2] the chunk's factors are in X
     float* wbuf = gs + 2 * KL_CT + 4;                       // [2][KL_CT][N4] write weights, 0 = row not written
     float* V = wbuf + 2 * KL_CT * N4;                       // [N4][DV]
     const int bh = blockIdx.x, b = bh / H, h = bh % H;
@@ -363,6 +364,7 @@ __global__ void __launch_bounds__(32 * (2 + KL_CW), 2) keyless_fwd_chain_kernel(
             if (c >= 0 && c < NC) {
                 float* wr = wbuf + (c & 1) * KL_CT * N4;
                 const double* Xc = X + (c & 1) * KL_CT * NR + lane;
+                double* Xw = X + (c & 1) * KL_CT * NR + lane;
                 slow |= wild[c & 1] != 0;
                 const int cn = min(KL_CT, T - c * KL_CT);
                 for (int j = 0; j < cn; j++) {
@@ -400,21 +402,31 @@ __global__ void __launch_bounds__(32 * (2 + KL_CW), 2) keyless_fwd_chain_kernel(
                         if (a != 0.f) o[i] = (1.0 - w) * o[i] + w;
                         if (n < N4) wr[j * N4 + n] = n < N ? g * a : 0.f;
                     }
-                    if (addr != nullptr) {
-                        if (!p.hard && !slow) {                      // the argmax, for the caller's log only
-                            double be = -1.0;
-                            int bi = BIGI;
+                    if (p.hard || slow) {
+                        if (lane == 0 && addr != nullptr) addr[ix] = am;
+                    } else {                                         // the factors, for warp 1 to find the largest of
 #pragma unroll
-                            for (int i = 0; i < R; i++) if (lane + 32 * i < N && e[i] > be) { be = e[i]; bi = lane + 32 * i; }
-                            const unsigned hi = (unsigned)(__double_as_longlong(be) >> 32) ^ 0x80000000u, lo = (unsigned)__double_as_longlong(be);
-                            const unsigned mhi = __reduce_max_sync(FULL, hi), mlo = __reduce_max_sync(FULL, hi == mhi ? lo : 0u);
-                            am = min((int)__reduce_min_sync(FULL, (unsigned)(hi == mhi && lo == mlo ? bi : BIGI)), N - 1);
-                        }
-                        if (lane == 0) addr[ix] = am;
+                        for (int i = 0; i < R; i++) Xw[j * NR + 32 * i] = e[i];
                     }
                 }
+                if (lane == 0) soft_chunk[c & 1] = !(p.hard || slow);
             }
         } else if (warp == 1) {
+            if (c >= 1 && addr != nullptr && soft_chunk[(c - 1) & 1]) {      // the address of the chunk before, for the caller's log
+                const int cn = min(KL_CT, T - (c - 1) * KL_CT);
+                for (int j = 0; j < cn; j++) {
+                    const double* E = X + ((c - 1) & 1) * KL_CT * NR + j * NR + lane;
+                    double be = -1.0;
+                    int bi = BIGI;
+#pragma unroll
+                    for (int i = 0; i < R; i++) if (lane + 32 * i < N && E[32 * i] > be) { be = E[32 * i]; bi = lane + 32 * i; }
+                    const unsigned hi = (unsigned)(__double_as_longlong(be) >> 32) ^ 0x80000000u, lo = (unsigned)__double_as_longlong(be);
+                    const unsigned mhi = __reduce_max_sync(FULL, hi), mlo = __reduce_max_sync(FULL, hi == mhi ? lo : 0u);
+                    const int am = min((int)__reduce_min_sync(FULL, (unsigned)(hi == mhi && lo == mlo ? bi : BIGI)), N - 1);
+                    if (lane == 0) addr[((size_t)b * T + (c - 1) * KL_CT + j) * H + h] = am;
+                }
+                __syncwarp();
+            }
             if (c + 1 < NC) {
                 const int bf = (c + 1) & 1, t0 = (c + 1) * KL_CT;
                 double* Xc = X + bf * KL_CT * NR + lane;
@@ -648,8 +660,13 @@ cudaError_t run_keyless_fwd(const slotscan_v_params& p, const Tin* v, const floa
                             float* buf, float* obuf, int* addr, cudaStream_t st) {
     const size_t sm = keyless_chain_smem(p.N, p.DV);
     cudaError_t e = cudaSuccess;
+    // one CTA per SM at most: registers for the value warps' loads ahead (0.43 ms where the form for two has 0.50)
+    int dev = 0, sms = 148;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const bool alone = (long long)p.B * p.H <= sms;
     KEYLESS_ROWS(p.N, {
-        auto kern = keyless_fwd_chain_kernel<Tin, R>;
+        auto kern = alone ? keyless_fwd_chain_kernel<Tin, R, 1> : keyless_fwd_chain_kernel<Tin, R, 2>;
         if ((e = opt_in_smem(kern, sm)) != cudaSuccess) return e;
         kern<<<p.B * p.H, 32 * (2 + KL_CW), sm, st>>>(p, v, wa, gate, fr, buf, obuf, addr);
     });
