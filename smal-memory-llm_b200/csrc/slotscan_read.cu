@@ -18,6 +18,8 @@
 #include <stdint.h>
 #include <stdio.h>
 
+#include <algorithm>
+
 #include "slotscan.h"
 #include "slotscan_common.cuh"
 #include "slotscan_launch.h"
@@ -31,26 +33,64 @@ __device__ __forceinline__ float ldf(const __nv_bfloat16* p) { return __bfloat16
 __device__ __forceinline__ void stf(float* p, float v) { *p = v; }
 __device__ __forceinline__ void stf(__nv_bfloat16* p, float v) { *p = __float2bfloat16_rn(v); }
 
-template <typename Tq, typename Tsn>
-__global__ void __launch_bounds__(RD_THREADS) read_fwd_kernel(const slotscan_read_params p, const Tq* __restrict__ qr,
+// Highest valid row + 1 of a snapshot; warp-collective.
+__device__ __forceinline__ int read_rows_in_use(const uint8_t* v, int N) {
+    const int lane = threadIdx.x & 31;
+    int hv = 0;
+    for (int base = 0; base < N; base += 32) {
+        const unsigned bal = __ballot_sync(FULL, base + lane < N && v[base + lane] != 0);
+        if (bal) hv = base + 32 - __clz(bal);
+    }
+    return hv;
+}
+// Which snapshots a CTA of the two kernels below works on.  On its own: one, blockIdx.x.  Beside the tensor-core kernel
+// (SPARSE: the snapshots with at most `rows` rows in use) most are not its own, and a launch of a CTA per snapshot to
+// find that out took longer than the work (B = 32, T = 1024, every slot in use: 0.11 ms forward, 0.16 ms backward; now
+// 0.08, most of it the 4 % of snapshots that are its own, and 0.04): a grid that fits the machine looks the snapshots over, one per warp at a time.
+template <bool SPARSE, typename F>
+__device__ __forceinline__ void read_each_snapshot(const uint8_t* valid, int N, long long total, int rows, F work) {
+    if constexpr (!SPARSE) {
+        work((int)blockIdx.x);
+        return;
+    }
+    __shared__ int s_todo[RD_WARPS];
+    // the four of a look a grid apart: the heads of a block, next to one another, are alike, and must not end up in one CTA
+    const int warp = threadIdx.x >> 5;
+    const long long grid = gridDim.x;
+    for (long long so0 = blockIdx.x; so0 < total; so0 += grid * RD_WARPS) {
+        const long long mine = so0 + warp * grid;
+        const bool todo = mine < total && read_rows_in_use(valid + (size_t)mine * N, N) <= rows;
+        if ((threadIdx.x & 31) == 0) s_todo[warp] = todo;
+        __syncthreads();
+        for (int u = 0; u < RD_WARPS; u++) {
+            if (s_todo[u]) {                                    // uniform
+                work((int)(so0 + u * grid));
+                __syncthreads();                                // its shared memory is free again
+            }
+        }
+        __syncthreads();
+    }
+}
+
+template <typename Tq, typename Tsn, bool SPARSE>
+__global__ void __launch_bounds__(RD_THREADS, SPARSE ? 8 : 0) read_fwd_kernel(const slotscan_read_params p, const Tq* __restrict__ qr,
                                                              const float* __restrict__ sharp,
                                                              const Tsn* __restrict__ kbuf, const Tsn* __restrict__ vbuf,
                                                              const float* __restrict__ kinv,
-                                                             const uint8_t* __restrict__ valid, Tq* __restrict__ rd,
-                                                             const int sparse_only) {
+                                                             const uint8_t* __restrict__ valid, Tq* __restrict__ rd) {
     extern __shared__ __align__(16) float rsm[];
     const int N = p.N, T = p.T, H = p.H, NQ = p.NQ, DK = p.DK, DV = p.DV, G = p.G;
     const int NB = (T + G - 1) / G;
     int* s_rows = reinterpret_cast<int*>(rsm);                 // [N] indices of the valid rows
     float* s_ki = rsm + N;                                     // [N] their kinv
     float* s_sc = rsm + ((2 * N + 3) & ~3);                    // [warps][N][4] logits, then attention weights (16-byte aligned)
-    __shared__ int s_nv, s_hv;
-    const int so = blockIdx.x;                                 // (b * NB + nb) * H + h
+    __shared__ int s_nv;
+    read_each_snapshot<SPARSE>(valid, N, (long long)p.B * NB * H, RM_SPARSE_ROWS, [&](const int so) {   // (b * NB + nb) * H + h
     const int h = so % H, nb = (so / H) % NB, b = so / (H * NB);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
 
     if (warp == 0) {
-        int nv = 0, hv = 0;
+        int nv = 0;
         for (int base = 0; base < N; base += 32) {
             const int n = base + lane;
             const bool v = n < N && valid[(size_t)so * N + n] != 0;
@@ -61,13 +101,11 @@ __global__ void __launch_bounds__(RD_THREADS) read_fwd_kernel(const slotscan_rea
                 s_ki[pos] = kinv[(size_t)so * N + n];
             }
             nv += __popc(bal);
-            if (bal) hv = base + 32 - __clz(bal);              // highest valid row + 1
         }
-        if (lane == 0) { s_nv = nv; s_hv = hv; }
+        if (lane == 0) s_nv = nv;
     }
     __syncthreads();
     const int nv = s_nv;
-    if (sparse_only && s_hv > RM_SPARSE_ROWS) return;          // the tensor-core kernel reads this snapshot
     const int t0 = nb * G, tc = min(G, T - t0), M = tc * NQ;   // queries that read this snapshot
     float* sc = s_sc + (size_t)warp * N * RD_QPW;
     const Tsn* Kb = kbuf + (size_t)so * N * DK;
@@ -156,6 +194,18 @@ __global__ void __launch_bounds__(RD_THREADS) read_fwd_kernel(const slotscan_rea
         }
         __syncwarp();
     }
+    });
+}
+
+// a CTA per snapshot, or (sparse_only) what fits the machine beside `smem` bytes and 64 registers a thread each: one wave, or
+// the snapshots would be dealt to CTAs that start when the others have finished theirs
+static unsigned read_grid(int snapshots, size_t smem, int sparse_only) {
+    if (!sparse_only) return (unsigned)snapshots;
+    int dev = 0, sms = 148;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const long long fit = (long long)sms * std::min<long long>(8, std::max<long long>(1, (long long)(227 * 1024 / (smem + 1024))));
+    return (unsigned)std::min<long long>(snapshots, fit);
 }
 
 template <typename Tq, typename Tsn>
@@ -164,13 +214,13 @@ static cudaError_t launch_read(const slotscan_read_params& p, const void* qr, co
                                int sparse_only = 0) {
     const int NB = (p.T + p.G - 1) / p.G;
     const size_t sm = sizeof(float) * ((size_t)((2 * p.N + 3) & ~3) + (size_t)p.N * RD_WARPS * RD_QPW);
-    auto kern = read_fwd_kernel<Tq, Tsn>;
+    auto kern = sparse_only ? read_fwd_kernel<Tq, Tsn, true> : read_fwd_kernel<Tq, Tsn, false>;
     if (sm > 48 * 1024) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
         if (e != cudaSuccess) return e;
     }
-    kern<<<p.B * NB * p.H, RD_THREADS, sm, st>>>(p, (const Tq*)qr, sharp, (const Tsn*)kbuf, (const Tsn*)vbuf, kinv, valid,
-                                                  (Tq*)rd, sparse_only);
+    kern<<<read_grid(p.B * NB * p.H, sm, sparse_only), RD_THREADS, sm, st>>>(p, (const Tq*)qr, sharp, (const Tsn*)kbuf, (const Tsn*)vbuf,
+                                                                            kinv, valid, (Tq*)rd);
     return cudaGetLastError();
 }
 
@@ -250,12 +300,12 @@ __host__ __device__ inline ReadBwdSmem read_bwd_layout(int N, int M) {
     return L;
 }
 
-template <typename Tq, typename Tsn>
-__global__ void __launch_bounds__(RD_THREADS) read_bwd_kernel(
+template <typename Tq, typename Tsn, bool SPARSE>
+__global__ void __launch_bounds__(RD_THREADS, SPARSE ? 4 : 0) read_bwd_kernel(
     const slotscan_read_params p, const Tq* __restrict__ qr, const float* __restrict__ sharp, const Tsn* __restrict__ kbuf,
     const Tsn* __restrict__ vbuf, const float* __restrict__ kinv, const uint8_t* __restrict__ valid,
     const Tq* __restrict__ drd, Tq* __restrict__ dqr, float* __restrict__ dsharp, Tsn* __restrict__ dkbuf,
-    Tsn* __restrict__ dvbuf, float* __restrict__ dkinv, const int sparse_only) {
+    Tsn* __restrict__ dvbuf, float* __restrict__ dkinv) {
     extern __shared__ __align__(16) float rsm[];
     const int N = p.N, T = p.T, H = p.H, NQ = p.NQ, DK = p.DK, DV = p.DV, G = p.G;
     const int NB = (T + G - 1) / G, N4 = (N + 3) & ~3;
@@ -265,13 +315,13 @@ __global__ void __launch_bounds__(RD_THREADS) read_bwd_kernel(
     float* s_qinv = rsm + L.qinv;
     float* s_att = rsm + L.att;
     float* s_cf = rsm + L.cf;
-    __shared__ int s_nv, s_hvb;
-    const int so = blockIdx.x;
+    __shared__ int s_nv;
+    read_each_snapshot<SPARSE>(valid, N, (long long)p.B * NB * H, RB_SPARSE_ROWS, [&](const int so) {
     const int h = so % H, nb = (so / H) % NB, b = so / (H * NB);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
 
     if (warp == 0) {
-        int nv = 0, hv = 0;
+        int nv = 0;
         for (int base = 0; base < N; base += 32) {
             const int n = base + lane;
             const bool v = n < N && valid[(size_t)so * N + n] != 0;
@@ -282,13 +332,11 @@ __global__ void __launch_bounds__(RD_THREADS) read_bwd_kernel(
                 s_ki[pos] = kinv[(size_t)so * N + n];
             }
             nv += __popc(bal);
-            if (bal) hv = base + 32 - __clz(bal);              // highest valid row + 1
         }
-        if (lane == 0) { s_nv = nv; s_hvb = hv; }
+        if (lane == 0) s_nv = nv;
     }
     __syncthreads();
     const int nv = s_nv;
-    if (sparse_only && s_hvb > RB_SPARSE_ROWS) return;            // the tensor-core kernel takes this snapshot (uniform per CTA)
     // zero the whole block of snapshot gradients first; the valid rows are overwritten after the barrier below
     zero_fill(dkbuf + (size_t)so * N * DK, (size_t)N * DK, tid);
     zero_fill(dvbuf + (size_t)so * N * DV, (size_t)N * DV, tid);
@@ -447,6 +495,7 @@ __global__ void __launch_bounds__(RD_THREADS) read_bwd_kernel(
             dkinv[(size_t)so * N + n] = s;
         }
     }
+    });
 }
 
 template <typename Tq, typename Tsn>
@@ -455,13 +504,14 @@ static cudaError_t launch_read_bwd(const slotscan_read_params& p, const void* qr
                                    float* dsharp, void* dkbuf, void* dvbuf, float* dkinv, int sparse_only, cudaStream_t st) {
     const int NB = (p.T + p.G - 1) / p.G;
     const size_t sm = sizeof(float) * (size_t)read_bwd_layout(p.N, p.G * p.NQ).total;
-    auto kern = read_bwd_kernel<Tq, Tsn>;
+    auto kern = sparse_only ? read_bwd_kernel<Tq, Tsn, true> : read_bwd_kernel<Tq, Tsn, false>;
     if (sm > 48 * 1024) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
         if (e != cudaSuccess) return e;
     }
-    kern<<<p.B * NB * p.H, RD_THREADS, sm, st>>>(p, (const Tq*)qr, sharp, (const Tsn*)kbuf, (const Tsn*)vbuf, kinv, valid,
-                                                  (const Tq*)drd, (Tq*)dqr, dsharp, (Tsn*)dkbuf, (Tsn*)dvbuf, dkinv, sparse_only);
+    kern<<<read_grid(p.B * NB * p.H, sm, sparse_only), RD_THREADS, sm, st>>>(p, (const Tq*)qr, sharp, (const Tsn*)kbuf, (const Tsn*)vbuf,
+                                                                            kinv, valid, (const Tq*)drd, (Tq*)dqr, dsharp, (Tsn*)dkbuf,
+                                                                            (Tsn*)dvbuf, dkinv);
     return cudaGetLastError();
 }
 
