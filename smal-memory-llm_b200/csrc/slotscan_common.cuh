@@ -68,6 +68,48 @@ __device__ __forceinline__ float group_sum(float v) {
 }
 __device__ __forceinline__ float dot4(float4 a, float4 b) { return a.x * b.x + a.y * b.y + a.z * b.z + a.w * b.w; }
 
+// ---- two float32 multiply-adds in one instruction (sm_100), each rounded as its own: half the instructions where a warp's
+// instruction stream is what bounds (the pipe's rate per operation is about the same) ----
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pack2(float x, float y) {
+    f32x2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
+    return r;
+}
+__device__ __forceinline__ float2 unpack2(f32x2 a) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(a));
+    return r;
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+    f32x2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+struct f32x4 { f32x2 a, b; };                             // x, y | z, w of a float4
+__device__ __forceinline__ f32x4 ld4x2(const float* p) {
+    const ulonglong2 u = *reinterpret_cast<const ulonglong2*>(p);
+    return {u.x, u.y};
+}
+__device__ __forceinline__ f32x4 pack4(float4 v) { return {pack2(v.x, v.y), pack2(v.z, v.w)}; }
+__device__ __forceinline__ f32x4 ld4x2(const __nv_bfloat16* p) { return pack4(ld4(p)); }
+__device__ __forceinline__ void fma4(f32x4& c, const f32x4& a, const f32x4& b) { c.a = fma2(a.a, b.a, c.a); c.b = fma2(a.b, b.b, c.b); }
+// (x + y) + (z + w)
+__device__ __forceinline__ float sum4(const f32x4& v) {
+    const float2 p = unpack2(v.a), q = unpack2(v.b);
+    return (p.x + p.y) + (q.x + q.y);
+}
+
 // The one write rule of the scan, state <- (1-g) state + g x, spelled identically in every kernel so that a row
 // replayed by another kernel is bit-identical to the row the address kernel held.
 __device__ __forceinline__ float blend(float old, float x, float g, float omw) {

@@ -28,7 +28,7 @@ __host__ __device__ inline size_t dc_tok_bytes(int C, int DK) {
 __host__ __device__ inline size_t dc_smem(int C, int N, int DK, int DV, bool values) {
     const int kp = dc_kpad(DK);
     const size_t n4 = (N + 3) & ~3;
-    return 2 * dc_tok_bytes(C, DK) + 8 * 128 + 4 * ((size_t)N * (kp + 4) + (values ? n4 * DV : 0) + 2 * C * n4 + 16);
+    return 2 * dc_tok_bytes(C, DK) + 8 * 128 + 8 * (size_t)2 * C * 8 + 4 * ((size_t)N * (kp + 4) + (values ? n4 * DV : 0) + 2 * C * n4 + 16);
 }
 
 __device__ __forceinline__ double dc_rcp(double s) {         // hardware approximation + one cubic Newton-Raphson step
@@ -51,6 +51,20 @@ __device__ __forceinline__ double warp_sum_d(double v) {
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(FULL, v, off);
     return v;
+}
+
+// N rows of DK floats into rows of stride kpad + 4 (the padding zero), 16 bytes at a time and several in flight where the
+// rows allow it
+__device__ __forceinline__ void dense_load_rows(float* K, const float* src, int N, int DK, int tid, int nt) {
+    const int kp = dc_kpad(DK), KS = kp + 4;
+    if (DK % 4 == 0 && (reinterpret_cast<size_t>(src) & 15) == 0) {
+        const int q = DK / 4, n = N * q;
+#pragma unroll 8
+        for (int i = tid; i < n; i += nt) { const int r = i / q, c = (i - r * q) * 4; st4(K + r * KS + c, __ldg(reinterpret_cast<const float4*>(src) + i)); }
+        for (int r = tid; r < N; r += nt) st4(K + r * KS + kp, make_float4(0.f, 0.f, 0.f, 0.f));
+    } else {
+        for (int i = tid; i < N * KS; i += nt) { const int r = i / KS, d = i % KS; K[i] = d < DK ? src[(size_t)r * DK + d] : 0.f; }
+    }
 }
 
 struct DenseChainArgs {
@@ -78,7 +92,8 @@ __global__ void __launch_bounds__(DC_NMAX + DC_HELP) dense_chain_kernel(const De
     const int kp = dc_kpad(DK), KS = kp + 4, QS = kp + 2, N4 = (N + 3) & ~3;
     const size_t tokb = dc_tok_bytes(C, DK);
     double* ex = reinterpret_cast<double*>(dc_sm + 2 * tokb);        // [2][64] exchange of the row warps
-    float* K = reinterpret_cast<float*>(ex + 128);                   // [N][KS]
+    int2* s_arg = reinterpret_cast<int2*>(ex + 128);                 // [2][C][8] a row warp's largest address (float bits) and its row
+    float* K = reinterpret_cast<float*>(s_arg + 2 * C * 8);          // [N][KS]
     float* wbuf = K + (size_t)N * KS;                                // [2][C][N4]
     float* V = wbuf + 2 * C * N4;                                    // [N4][DV] (forward)
     auto tq = [&](int b) { return reinterpret_cast<double*>(dc_sm + b * tokb); };            // [C][QS] q
@@ -140,40 +155,66 @@ __global__ void __launch_bounds__(DC_NMAX + DC_HELP) dense_chain_kernel(const De
             else tqi(bf)[t] = 1.0 / fmax(sqrt(s), 1e-6);
         }
     };
-    // helper: the values of chunk [t0, t0 + cn), first token at place ph of block jb
-    auto values = [&](const float* wr, int t0, int cn, int ph, int jb) {
-        const int NU = (N4 / 4) * DV;
-        for (int u = ht; u < NU; u += DC_HELP) {
-            const int n0 = (u / DV) * 4, d = u % DV;
-            float xv[C], s[4];
+    // helper: a thread keeps its column (DV <= 128 of 256 threads; `hper` threads share one), so that a token's value is loaded
+    // once for all its rows, a chunk ahead; 4 rows at a time, two to an instruction
+    const int hper = DC_HELP / DV, hd = row ? 0 : ht % DV, hg = row ? 0 : ht / DV;
+    float xn[C];
+    auto fetch_v = [&](int t0, int cn) {
 #pragma unroll
-            for (int j = 0; j < C; j++) xv[j] = j < cn ? ldtok(vg + (((size_t)b * T + t0 + j) * H + h) * DV + d) : 0.f;
+        for (int j = 0; j < C; j++) xn[j] = j < cn ? ldtok(vg + (((size_t)b * T + t0 + j) * H + h) * DV + hd) : 0.f;
+    };
+    // the values of a chunk whose tokens fetch_v has loaded, first token at place ph of block jb; and its addresses
+    auto values = [&](int bf, int t0, int cn, int ph, int jb) {
+        const float* wr = wbuf + bf * C * N4;
+        if (!A.hard && A.addr != nullptr && ht < cn) {
+            int2 m = s_arg[(bf * C + ht) * 8];
+            for (int w = 1; w < RW; w++) { const int2 x = s_arg[(bf * C + ht) * 8 + w]; if ((unsigned)x.x > (unsigned)m.x) m = x; }
+            A.addr[((size_t)b * T + t0 + ht) * H + h] = m.y;
+        }
+        if (hg >= hper) return;
+        bool odd = A.hard != 0;                              // a row a token does not write must not see it: only an infinite
 #pragma unroll
-            for (int i = 0; i < 4; i++) s[i] = V[(n0 + i) * DV + d];
+        for (int j = 0; j < C; j++) odd |= !(fabsf(xn[j]) <= 3e38f);     // or NaN value would tell
+        const f32x2 one = pack2(1.f, 1.f), minus = pack2(-1.f, -1.f);
+        for (int n0 = hg * 4; n0 < N4; n0 += hper * 4) {
+            float s[4];
+#pragma unroll
+            for (int i = 0; i < 4; i++) s[i] = V[(n0 + i) * DV + hd];
             if (ph == 0) {
-                float* out = A.vbuf + (snap(jb) * N + n0) * DV + d;
+                float* out = A.vbuf + (snap(jb) * N + n0) * DV + hd;
 #pragma unroll
                 for (int i = 0; i < 4; i++) if (n0 + i < N) out[(size_t)i * DV] = s[i];
             }
+            if (!odd) {
+                f32x2 s0 = pack2(s[0], s[1]), s1 = pack2(s[2], s[3]);
 #pragma unroll
-            for (int j = 0; j < C; j++) {
-                const float4 w = ld4(wr + j * N4 + n0);             // tokens past cn: 0
-                const float wv[4] = {w.x, w.y, w.z, w.w};
+                for (int j = 0; j < C; j++) {                        // tokens past cn: weight 0
+                    const f32x4 w = ld4x2(wr + j * N4 + n0);
+                    const f32x2 x = pack2(xn[j], xn[j]);
+                    s0 = fma2(w.a, x, mul2(fma2(w.a, minus, one), s0));
+                    s1 = fma2(w.b, x, mul2(fma2(w.b, minus, one), s1));
+                }
+                const float2 p0 = unpack2(s0), p1 = unpack2(s1);
+                s[0] = p0.x; s[1] = p0.y; s[2] = p1.x; s[3] = p1.y;
+            } else {
 #pragma unroll
-                for (int i = 0; i < 4; i++) s[i] = wv[i] != 0.f ? (1.f - wv[i]) * s[i] + wv[i] * xv[j] : s[i];
+                for (int j = 0; j < C; j++) {
+                    const float4 w = ld4(wr + j * N4 + n0);
+                    const float wv[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+                    for (int i = 0; i < 4; i++) s[i] = wv[i] != 0.f ? (1.f - wv[i]) * s[i] + wv[i] * xn[j] : s[i];
+                }
             }
 #pragma unroll
-            for (int i = 0; i < 4; i++) V[(n0 + i) * DV + d] = s[i];
+            for (int i = 0; i < 4; i++) V[(n0 + i) * DV + hd] = s[i];
         }
     };
 
     // ---- initial state ----
     double o = 0.0;
     int fe = 0;                                              // first empty row; candidates: rows 0 .. min(fe, N - 1)
-    for (int i = tid; i < N * KS; i += NT) {
-        const int r = i / KS, d = i % KS;
-        K[i] = (TABLES && d < DK) ? A.kbuf[(snap(jb0) * N + r) * DK + d] : 0.f;
-    }
+    if (TABLES) dense_load_rows(K, A.kbuf + snap(jb0) * N * DK, N, DK, tid, NT);
+    else for (int i = tid; i < N * KS; i += NT) K[i] = 0.f;
     for (int i = tid; i < 2 * C * N4; i += NT) wbuf[i] = 0.f;
     if (!TABLES) for (int i = tid; i < N4 * DV; i += NT) V[i] = 0.f;
     if (TABLES && live) o = (double)A.obuf[snap(jb0) * N + n];
@@ -191,6 +232,9 @@ __global__ void __launch_bounds__(DC_NMAX + DC_HELP) dense_chain_kernel(const De
         if (tid == 0) A.lim[(size_t)lb * NB + jb0] = min(fe, N - 1);
     }
     __syncthreads();                                         // the exchange slots are used again below
+    for (int i = tid; row && i < 128; i += rows_t) ex[i] = 0.0;     // row warps that are not there: no weight, no key
+    if (row) dc_bar_rows(rows_t);
+    if (!TABLES && !row) fetch_v(0, min(C, min(G, T)));
 
     bool wild = false;                                       // a gate outside [0, 1] so far: occupancies are not bounded by 1
     int par = 0, c = 0, pt0 = 0, pcn = 0, pph = 0, pjb = 0;  // parity of the exchange, chunk, the chunk before
@@ -261,7 +305,7 @@ __global__ void __launch_bounds__(DC_NMAX + DC_HELP) dense_chain_kernel(const De
                             for (int off = 16; off > 0; off >>= 1) se += __shfl_xor_sync(FULL, se, off);
                             if (lane == 0) xs[warp] = se;
                         }
-                        if (!TABLES) {                       // the address: first row of the largest z
+                        if (!TABLES && A.hard) {             // the address: first row of the largest z
                             const unsigned long long key = (cand && z > -INFINITY) ? dc_key(z) : 0ull;
                             const unsigned hi = (unsigned)(key >> 32), mh = __reduce_max_sync(FULL, hi);
                             const unsigned ml = __reduce_max_sync(FULL, hi == mh ? (unsigned)key : 0u);
@@ -274,18 +318,20 @@ __global__ void __launch_bounds__(DC_NMAX + DC_HELP) dense_chain_kernel(const De
                         if (n == fe && live) { xs[32] = E; xs[33] = o; }
                         dc_bar_rows(rows_t);
                         int am = 0;
-                        if (!TABLES && (A.hard || tid == 0)) {
+                        if (!TABLES && A.hard) {
                             const unsigned long long* ks = reinterpret_cast<const unsigned long long*>(xs) + 16;
                             unsigned long long bk = ks[0];
                             int bw = 0;
-                            for (int i = 1; i < RW; i++) if (ks[i] > bk) { bk = ks[i]; bw = i; }
+#pragma unroll
+                            for (int i = 1; i < 8; i++) if (ks[i] > bk) { bk = ks[i]; bw = i; }
                             am = bk == 0ull ? min(fe, N - 1) : reinterpret_cast<const int*>(xs + 24)[bw];   // all NaN: the last candidate
                             if (tid == 0 && A.addr != nullptr) A.addr[((size_t)b * T + t0 + j) * H + h] = am;
                         }
                         double si = 0.0;
                         if (soft) {
-                            double se = xs[0];
-                            for (int i = 1; i < RW; i++) se += xs[i];
+                            const double2 e0 = *reinterpret_cast<const double2*>(xs), e1 = *reinterpret_cast<const double2*>(xs + 2);
+                            const double2 e2 = *reinterpret_cast<const double2*>(xs + 4), e3 = *reinterpret_cast<const double2*>(xs + 6);
+                            const double se = ((e0.x + e0.y) + (e1.x + e1.y)) + ((e2.x + e2.y) + (e3.x + e3.y));
                             si = bounded ? dc_rcp(se) : 1.0 / se;
                         }
                         const float as = (float)(E * si);
@@ -305,6 +351,11 @@ __global__ void __launch_bounds__(DC_NMAX + DC_HELP) dense_chain_kernel(const De
                             const double wf = (double)g * (double)af, of = xs[33];
                             if ((af != 0.f ? (1.0 - wf) * of + wf : of) >= (double)eps) fe++;
                         }
+                        if (!TABLES && !A.hard && A.addr != nullptr) {       // soft: the argmax of the address, for the log
+                            const unsigned ak = a > 0.f ? __float_as_uint(a) : 0u, mk = __reduce_max_sync(FULL, ak);
+                            const unsigned who = __ballot_sync(FULL, ak == mk);
+                            if (lane == 0) s_arg[(bf * C + j) * 8 + warp] = make_int2((int)mk, warp * 32 + __ffs((int)who) - 1);
+                        }
                         if (a != 0.f) o = (1.0 - wd0) * o + wd0;
                         w[j] = g * a;
                         if (live) wr[j * N4 + n] = w[j];
@@ -322,14 +373,22 @@ __global__ void __launch_bounds__(DC_NMAX + DC_HELP) dense_chain_kernel(const De
             } else {
                 if (!TABLES && s0 == 0) {                    // the pre-write keys, every G tokens
                     float* out = A.kbuf + snap(jb) * N * DK;
-                    for (int i = ht; i < N * DK; i += DC_HELP) out[i] = K[(i / DK) * KS + i % DK];
+                    if (DK % 4 == 0 && DC_HELP % (DK / 4) == 0 && (reinterpret_cast<size_t>(A.kbuf) & 15) == 0) {
+                        const int q4 = DK / 4, cc = (ht % q4) * 4;
+                        for (int r = ht / q4; r < N; r += DC_HELP / q4) st4(out + r * DK + cc, ld4(K + r * KS + cc));
+                    } else {
+                        for (int i = ht; i < N * DK; i += DC_HELP) out[i] = K[(i / DK) * KS + i % DK];
+                    }
                 }
                 const bool more = s0 + C < bn;
                 if (more || jb + 1 < jb1) {
                     const int nt0 = more ? t0 + C : tb + G;
                     prep(bf ^ 1, nt0, min(C, more ? bn - s0 - C : min(G, T - nt0)));
                 }
-                if (!TABLES && c > 0) values(wbuf + (bf ^ 1) * C * N4, pt0, pcn, pph, pjb);
+                if (!TABLES && c > 0) {
+                    values(bf ^ 1, pt0, pcn, pph, pjb);
+                    fetch_v(t0, cn);
+                }
             }
             pt0 = t0; pcn = cn; pph = s0; pjb = jb;
             __syncthreads();
@@ -367,7 +426,7 @@ __global__ void __launch_bounds__(DC_NMAX + DC_HELP) dense_chain_kernel(const De
         }
     }
     if (TABLES) return;
-    if (!row) values(wbuf + ((c - 1) & 1) * C * N4, pt0, pcn, pph, pjb);
+    if (!row) values((c - 1) & 1, pt0, pcn, pph, pjb);
     __syncthreads();
     const size_t f0 = (size_t)bh * N;
     if (A.kfin != nullptr) for (int i = tid; i < N * DK; i += NT) A.kfin[f0 * DK + i] = K[(i / DK) * KS + i % DK];
@@ -470,20 +529,25 @@ __global__ void __launch_bounds__(DQ_T) dense_dq_kernel(const slotscan_params p,
     float* kt = zs + DQ_C * N;                               // [DQ_C][kp]
     float* gq = kt + DQ_C * kp;                              // [DQ_C][kp] raw query gradient
     float* red = gq + DQ_C * kp;                             // [RG][DQ_C][kp]
+    __shared__ float gs[DQ_C];
     const int lb = blockIdx.x / NB, jb = blockIdx.x % NB, bh = bh0 + lb, b = bh / H, h = bh % H;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int cg = tid % CG, rg = tid / CG;
     const bool act = rg < RG;
     const size_t so = ((size_t)b * NB + jb) * H + h;
-    for (int i = tid; i < N * kp; i += DQ_T) { const int r = i / kp, d = i % kp; K[r * KS + d] = d < DK ? kbuf[(so * N + r) * DK + d] : 0.f; }
+    dense_load_rows(K, kbuf + so * N * DK, N, DK, tid, DQ_T);
     const int tb = jb * G, te = min(T, tb + G);
     for (int t0 = tb; t0 < te; t0 += DQ_C) {
         const int cn = min(DQ_C, te - t0);
-        for (int i = tid; i < DQ_C * N; i += DQ_T) {
-            const int j = i / N, n = i % N;
-            const size_t at = ((size_t)lb * T + t0 + j) * N + n;
-            ws[i] = j < cn ? gate_eff(gate[((size_t)b * T + t0 + j) * H + h], p.hard_gate) * as[at] : 0.f;
-            zs[i] = j < cn ? cz[at] : 0.f;
+        if (tid < DQ_C) gs[tid] = tid < cn ? gate_eff(gate[((size_t)b * T + t0 + tid) * H + h], p.hard_gate) : 0.f;
+        __syncthreads();
+#pragma unroll 6
+        for (int i = tid; i < DQ_C * N; i += DQ_T) {         // tokens t0 .. are rows of the tables: one run of memory
+            const size_t at = ((size_t)lb * T + t0) * N + i;
+            const bool in = i < cn * N;
+            const float a = in ? as[at] : 0.f, z = in ? cz[at] : 0.f;
+            ws[i] = gs[i / N] * a;
+            zs[i] = z;
         }
         for (int i = tid; i < DQ_C * kp; i += DQ_T) {
             const int j = i / kp, d = i % kp;
