@@ -61,7 +61,7 @@ def kv_scan_g(k, v, gate, fr, N, temp, G=16, hard=False, hard_gate=False, eps=1e
                             bool(detach_addr), bool(occ_bin))
         return out[0].to(out_dtype), out[1].to(out_dtype)
     out = ops.hard_fwd(k_, q_, v_, g_, fr_, temp_, None, None, None, None, int(N), int(G), bool(hard_gate), float(eps),
-                       bool(occ_bin), out_dtype == torch.bfloat16, False, True)
+                       bool(occ_bin), out_dtype == torch.bfloat16, False, True, 0, 16)
     return out[0], out[1]
 
 
@@ -91,16 +91,16 @@ def scan_with_log(k, v, gate, fr, N, temp, G=16, hard_gate=False, eps=1e-4, q=No
     state: (K0, V0, o0) or (K0, V0, o0, nsq0) -- kfin, vfin, ofin[, nsqfin] of the call that scanned the preceding
     tokens; snapshot 0 is then that state.  undo_log=False skips the rows-before-each-write log (kold, vold come back
     empty): less memory and traffic for inference."""
-    return _scan_with_log(k, v, gate, fr, N, temp, G, hard_gate, eps, q, occ_bin, out_dtype, state, want_norm, undo_log)
-
-
-def _scan_with_log(k, v, gate, fr, N, temp, G, hard_gate, eps, q, occ_bin, out_dtype, state, want_norm, undo_log, qbits=0,
-                   qgroup=16):
-    """scan_with_log, with the storage quantiser of the emitted snapshots."""
     if not k.is_cuda:
         raise RuntimeError("slotscan_b200.scan_with_log: CUDA tensors only (no CPU path in this package)")
-    k_, v_, q_ = _token_streams(k, v, q)
-    fr_, temp_ = _scalars(fr, temp, k.device)
+    return _scan_streams(*_token_streams(k, v, q), gate, fr, N, temp, G, hard_gate, eps, occ_bin, out_dtype, state, want_norm,
+                         undo_log)
+
+
+def _scan_streams(k_, v_, q_, gate, fr, N, temp, G, hard_gate, eps, occ_bin, out_dtype, state, want_norm, undo_log, qbits=0,
+                  qgroup=16):
+    """scan_with_log on streams in the kernels' dtype, with the storage quantiser of the emitted snapshots."""
+    fr_, temp_ = _scalars(fr, temp, k_.device)
     st = (None, None, None, None) if state is None else (tuple(state) + (None,))[:4]
     with torch.no_grad():
         out = ops.hard_fwd(k_, q_, v_, _as_f32(gate), fr_, temp_, st[0], st[1], st[2], st[3], int(N), int(G),
@@ -114,6 +114,18 @@ def _scan_with_log(k, v, gate, fr, N, temp, G, hard_gate, eps, q, occ_bin, out_d
     return d
 
 
+# The storage quantiser inside the row replay saves the float32 snapshots and the passes over them, but lengthens the
+# replay's walk of a busy row.  With few snapshots the walk is what takes the time: 2.29 ms with the quantiser as a pass of
+# its own against 2.73 inside for 4 chunks of 6 sequences whose float32 snapshots are 71 MB each, 1.1 against 1.3 ms for a
+# training step with 62 MB; at 1.2 GB it is 6.7 against 3.3 and 4.8 against 2.0 ms.
+_QUANT_INSIDE_BYTES = 192 << 20
+
+
+def _quant_inside(k_, v_, N, G, qbits):
+    B, T, H, DK = k_.shape
+    return bool(qbits) and 4 * B * ((T + G - 1) // G) * H * N * (DK + v_.shape[-1]) >= _QUANT_INSIDE_BYTES
+
+
 def write_memory(k, v, gate, fr, N, temp, G=16, hard_gate=False, eps=1e-4, q=None, occ_bin=False,
                  out_dtype=torch.bfloat16, qbits=0, qgroup=16):
     """What a writer layer hands to its readers, in one call: `(kbuf', buf', kinv, valid)`  [memlm_sh.py:454-475: the
@@ -122,12 +134,17 @@ def write_memory(k, v, gate, fr, N, temp, G=16, hard_gate=False, eps=1e-4, q=Non
     The scan kernels emit the snapshots in `out_dtype` and kinv / valid from the float32 state while each key row is in
     registers -- no pass over the snapshots at all; in the backward the kinv gradient enters the key rows inside the
     reverse row scan.  qbits in {2,3,4,8} or "e4m3": the rows go through the storage quantiser of `writer_epilogue` there,
-    and kinv / valid are the quantised rows'.
+    and kinv / valid are the quantised rows' (with few snapshots: float32 snapshots, then that pass over them).
     Differentiable in k, q, v, gate, fr, temp."""
     if not k.is_cuda:
         raise RuntimeError("slotscan_b200.write_memory: CUDA tensors only (no CPU path in this package)")
     if out_dtype not in (torch.float32, torch.bfloat16):
         raise ValueError("out_dtype must be float32 or bfloat16")
+    if qbits and not _quant_inside(k, v, int(N), int(G), qbits):
+        from .epilogue import writer_epilogue
+        kb, vb = kv_scan_g(k, v, gate, fr, N, temp, G=G, hard=True, hard_gate=hard_gate, eps=eps, detach_addr=True, q=q,
+                           occ_bin=occ_bin, out_dtype=torch.float32)
+        return writer_epilogue(kb, vb, out_dtype, qbits=qbits, qgroup=qgroup)
     k_, v_, q_ = _token_streams(k, v, q)
     fr_, temp_ = _scalars(fr, temp, k.device)
     out = ops.hard_fwd(k_, q_, v_, _as_f32(gate), fr_, temp_, None, None, None, None, int(N), int(G), bool(hard_gate),
@@ -154,8 +171,16 @@ class StreamingScan:
             raise ValueError("StreamingScan: only the last chunk may have a length that is not a multiple of G")
         if self.qbits and self.out_dtype not in (torch.float32, torch.bfloat16):
             raise TypeError("out_dtype must be float32 or bfloat16")
-        lg = _scan_with_log(k, v, gate, fr, q=q, out_dtype=self.out_dtype, state=self.state, want_norm=True, undo_log=False,
-                            qbits=_bits(self.qbits), qgroup=self.qgroup, **self.kw)
+        if not k.is_cuda:
+            raise RuntimeError("slotscan_b200.StreamingScan: CUDA tensors only (no CPU path in this package)")
+        k_, v_, q_ = _token_streams(k, v, q)
+        inside = not self.qbits or _quant_inside(k_, v_, int(self.kw["N"]), int(self.G), self.qbits)
+        lg = _scan_streams(k_, v_, q_, gate, fr, out_dtype=self.out_dtype if inside else torch.float32, state=self.state,
+                           want_norm=inside, undo_log=False, qbits=_bits(self.qbits) if inside else 0, qgroup=self.qgroup,
+                           **self.kw)
         self.state = (lg["kfin"], lg["vfin"], lg["ofin"], lg["nsqfin"])
         self.tokens += k.shape[1]
+        if not inside:
+            from .epilogue import writer_epilogue
+            return writer_epilogue(lg["kbuf"], lg["vbuf"], self.out_dtype, qbits=self.qbits, qgroup=self.qgroup)
         return lg["kbuf"], lg["vbuf"], lg["kinv"], lg["valid"]
