@@ -13,7 +13,7 @@ from typing import Optional, Tuple
 import torch
 
 from . import _lib
-from .ops import _ptr, _require_cuda, _stream
+from .ops import _Here, _ptr, _require_cuda, _stream, plain_call, wants_grad
 
 _DT = {torch.float32: _lib.F32, torch.bfloat16: _lib.BF16}
 
@@ -23,8 +23,7 @@ def _params(v, wa, G, hard, hard_gate):
     return _lib.KeylessParams(B, T, H, wa.shape[-1], DV, G, int(hard), int(hard_gate), _DT[v.dtype])
 
 
-@torch.library.custom_op("slotscan::keyless_fwd", mutates_args=())
-def keyless_fwd(v: torch.Tensor, wa: torch.Tensor, gate: torch.Tensor, fr: torch.Tensor, G: int, hard: bool,
+def _keyless_fwd(v: torch.Tensor, wa: torch.Tensor, gate: torch.Tensor, fr: torch.Tensor, G: int, hard: bool,
                 hard_gate: bool) -> Tuple[torch.Tensor, torch.Tensor, torch.Tensor]:
     """Returns buf (B,NB,H,N,DV) f32, obuf (B,NB,H,N) f32, addr (B,T,H) int32."""
     _require_cuda(v, wa, gate, fr)
@@ -36,11 +35,14 @@ def keyless_fwd(v: torch.Tensor, wa: torch.Tensor, gate: torch.Tensor, fr: torch
     addr = torch.empty(B, T, H, device=v.device, dtype=torch.int32)
     p = _params(v, wa, G, hard, hard_gate)
     _lib.check(_lib.lib().slotscan_v_check(ctypes.byref(p)), "slotscan_v_check")
-    with torch.cuda.device(v.device):
+    with _Here(v.device):
         rc = _lib.lib().slotscan_v_fwd(ctypes.byref(p), _ptr(v), _ptr(wa), _ptr(gate), _ptr(fr), _ptr(buf), _ptr(obuf),
                                        _ptr(addr), _stream(v.device))
     _lib.check(rc, "slotscan_v_fwd")
     return buf, obuf, addr
+
+
+keyless_fwd = torch.library.custom_op("slotscan::keyless_fwd", mutates_args=())(_keyless_fwd)
 
 
 @keyless_fwd.register_fake
@@ -52,8 +54,7 @@ def _(v, wa, gate, fr, G, hard, hard_gate):
             v.new_empty((B, T, H), dtype=torch.int32))
 
 
-@torch.library.custom_op("slotscan::keyless_bwd", mutates_args=())
-def keyless_bwd(v: torch.Tensor, wa: torch.Tensor, gate: torch.Tensor, fr: torch.Tensor, buf: torch.Tensor,
+def _keyless_bwd(v: torch.Tensor, wa: torch.Tensor, gate: torch.Tensor, fr: torch.Tensor, buf: torch.Tensor,
                 obuf: torch.Tensor, dbuf: Optional[torch.Tensor], G: int, hard: bool, hard_gate: bool
                 ) -> Tuple[torch.Tensor, torch.Tensor, torch.Tensor, torch.Tensor]:
     """dv (dtype of v), dwa, dgate, dfr (1,)."""
@@ -66,11 +67,14 @@ def keyless_bwd(v: torch.Tensor, wa: torch.Tensor, gate: torch.Tensor, fr: torch
     dv, dwa = torch.empty_like(v), torch.empty_like(wa)
     dgate = torch.empty(gate.shape, device=dev, dtype=torch.float32)
     dfr = torch.empty(1, device=dev, dtype=torch.float32)
-    with torch.cuda.device(dev):
+    with _Here(dev):
         rc = L.slotscan_v_bwd(ctypes.byref(p), _ptr(v), _ptr(wa), _ptr(gate), _ptr(fr), _ptr(buf), _ptr(obuf), _ptr(dbuf),
                               _ptr(scratch), nbytes, _ptr(dv), _ptr(dwa), _ptr(dgate), _ptr(dfr), _stream(dev))
     _lib.check(rc, "slotscan_v_bwd")
     return dv, dwa, dgate, dfr
+
+
+keyless_bwd = torch.library.custom_op("slotscan::keyless_bwd", mutates_args=())(_keyless_bwd)
 
 
 @keyless_bwd.register_fake
@@ -85,14 +89,29 @@ def _setup(ctx, inputs, output):
     ctx.set_materialize_grads(False)
 
 
-def _backward(ctx, dbuf, *unused):
+def _backward(ctx, dbuf, *unused, bwd=None):
     v, wa, gate, fr, buf, obuf = ctx.saved_tensors
     d = None if dbuf is None else dbuf.contiguous().to(torch.float32)
-    dv, dwa, dgate, dfr = keyless_bwd(v, wa, gate, fr, buf, obuf, d, *ctx.meta)
+    dv, dwa, dgate, dfr = (bwd or keyless_bwd)(v, wa, gate, fr, buf, obuf, d, *ctx.meta)
     return dv, dwa, dgate, dfr, None, None, None
 
 
 keyless_fwd.register_autograd(_backward, setup_context=_setup)
+
+
+class _Keyless(torch.autograd.Function):
+    """keyless_fwd and its backward for a plain_call."""
+
+    @staticmethod
+    def forward(ctx, *inputs):
+        out = _keyless_fwd(*inputs)
+        _setup(ctx, inputs, out)
+        return out
+
+    @staticmethod
+    @torch.autograd.function.once_differentiable
+    def backward(ctx, *grads):
+        return _backward(ctx, *grads, bwd=_keyless_bwd if plain_call(*grads) else None)
 
 
 def slot_scan_v(v, wa, gate, fr, N, C=256, G=1, buf_dtype=torch.float32, hard=False, hard_gate=False):
@@ -103,5 +122,9 @@ def slot_scan_v(v, wa, gate, fr, N, C=256, G=1, buf_dtype=torch.float32, hard=Fa
     v_ = v.contiguous() if v.dtype == torch.bfloat16 else v.contiguous().to(torch.float32)
     f = lambda x: x.contiguous().to(torch.float32)
     fr_ = torch.as_tensor(fr, dtype=torch.float32, device=v.device).reshape(1)     # slotkern_v.py:239
-    buf = keyless_fwd(v_, f(wa), f(gate), fr_, int(G), bool(hard), bool(hard_gate))[0]
+    args = (v_, f(wa), f(gate), fr_, int(G), bool(hard), bool(hard_gate))
+    if not plain_call(*args[:4]):
+        buf = keyless_fwd(*args)[0]
+    else:
+        buf = (_Keyless.apply(*args) if wants_grad(*args[:4]) else _keyless_fwd(*args))[0]
     return buf.to(buf_dtype)

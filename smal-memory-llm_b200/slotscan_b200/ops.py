@@ -21,7 +21,50 @@ def _ptr(t):
 
 
 def _stream(dev):
-    return ctypes.c_void_p(torch.cuda.current_stream(dev).cuda_stream)
+    """The current stream of `dev`, whose index the tensors carry."""
+    return ctypes.c_void_p(torch._C._cuda_getCurrentRawStream(dev.index))
+
+
+class _Here:
+    """`with torch.cuda.device(dev)`, free of charge where that device is the current one already."""
+    __slots__ = ("dev", "guard")
+
+    def __init__(self, dev):
+        self.dev = dev
+
+    def __enter__(self):
+        self.guard = None
+        if torch._C._cuda_getDevice() != self.dev.index:
+            self.guard = torch.cuda.device(self.dev)
+            self.guard.__enter__()
+
+    def __exit__(self, *a):
+        if self.guard is not None:
+            self.guard.__exit__(*a)
+
+
+def plain_call(*ts):
+    """True when nothing looks over this call's shoulder: ordinary tensors, no tracing, compiling, fake or functional mode.
+    The custom op's own wrapping costs about 80 us of host time per call and direction, as much as the kernels of a small
+    call take; such a call goes to the same implementation without it, and through an autograd.Function with the same
+    backward when a gradient is wanted.  Everything else takes the registered op."""
+    if torch.compiler.is_compiling() or torch.jit.is_tracing() or torch._C._len_torch_dispatch_stack() > 0 or \
+            torch._C._functorch.peek_interpreter_stack() is not None:
+        return False
+    for t in ts:
+        if t is not None and type(t) is not torch.Tensor and type(t) is not torch.nn.Parameter:
+            return False
+    return True
+
+
+def wants_grad(*ts):
+    return torch.is_grad_enabled() and any(t is not None and t.requires_grad for t in ts)
+
+
+def as_flag_bytes(valid):
+    """A bool or byte tensor as contiguous bytes; a bool tensor's storage holds them already."""
+    valid = valid.contiguous()
+    return valid.view(torch.uint8) if valid.dtype == torch.bool else valid.to(torch.uint8)
 
 
 def _params(k, v, gate, fr, N, G, hard_gate, eps, occ_bin, snap_dtype):
@@ -56,8 +99,7 @@ def _fwd_shapes(k, v, N, G, snap_bf16, want_norm, undo_log, new):
             new((B, NB, H, N) if want_norm else (0,), f32), new((B, NB, H, N) if want_norm else (0,), torch.uint8))
 
 
-@torch.library.custom_op("slotscan::hard_fwd", mutates_args=())
-def hard_fwd(k: torch.Tensor, q: Optional[torch.Tensor], v: torch.Tensor, gate: torch.Tensor, fr: torch.Tensor,
+def _hard_fwd(k: torch.Tensor, q: Optional[torch.Tensor], v: torch.Tensor, gate: torch.Tensor, fr: torch.Tensor,
              temp: torch.Tensor, K0: Optional[torch.Tensor], V0: Optional[torch.Tensor], o0: Optional[torch.Tensor],
              nsq0: Optional[torch.Tensor], N: int, G: int, hard_gate: bool, eps: float, occ_bin: bool,
              snap_bf16: bool, want_norm: bool, undo_log: bool, qbits: int = 0, qgroup: int = 16
@@ -77,12 +119,15 @@ def hard_fwd(k: torch.Tensor, q: Optional[torch.Tensor], v: torch.Tensor, gate: 
     K0, V0, o0, nsq0 = c(K0, torch.float32), c(V0, torch.float32), c(o0, torch.float32), c(nsq0, torch.float64)
     ex = _lib.FwdExtra(_addr(K0), _addr(V0), _addr(o0), _addr(nsq0), _addr(nsqfin), _addr(kinv), _addr(valid),
                        0 if undo_log else 1)
-    with torch.cuda.device(dev):
+    with _Here(dev):
         rc = _lib.lib().slotscan_hard_fwd_q(ctypes.byref(p), _ptr(k), _ptr(q), _ptr(v), _ptr(gate), _ptr(fr), _ptr(temp),
                                             _ptr(kbuf), _ptr(vbuf), ctypes.byref(log), ctypes.byref(ex),
                                             ctypes.byref(_lib.Storage(qbits, qgroup)), _stream(dev))
     _lib.check(rc, "slotscan_hard_fwd_q")
     return out
+
+
+hard_fwd = torch.library.custom_op("slotscan::hard_fwd", mutates_args=())(_hard_fwd)
 
 
 @hard_fwd.register_fake
@@ -91,8 +136,7 @@ def _(k, q, v, gate, fr, temp, K0, V0, o0, nsq0, N, G, hard_gate, eps, occ_bin, 
     return _fwd_shapes(k, v, N, G, snap_bf16, want_norm, undo_log, lambda s, dt: k.new_empty(s, dtype=dt))
 
 
-@torch.library.custom_op("slotscan::hard_bwd", mutates_args=())
-def hard_bwd(k: torch.Tensor, q: Optional[torch.Tensor], v: torch.Tensor, gate: torch.Tensor, fr: torch.Tensor,
+def _hard_bwd(k: torch.Tensor, q: Optional[torch.Tensor], v: torch.Tensor, gate: torch.Tensor, fr: torch.Tensor,
              temp: torch.Tensor, addr: torch.Tensor, oold: torch.Tensor, kold: torch.Tensor, vold: torch.Tensor,
              kfin: torch.Tensor, vfin: torch.Tensor, ofin: torch.Tensor, tfirst: torch.Tensor, kiold: torch.Tensor,
              dkbuf: Optional[torch.Tensor], dvbuf: Optional[torch.Tensor], dkinv: Optional[torch.Tensor], N: int, G: int,
@@ -115,13 +159,16 @@ def hard_bwd(k: torch.Tensor, q: Optional[torch.Tensor], v: torch.Tensor, gate: 
     dfr = torch.empty(fr.shape, device=dev, dtype=torch.float32)
     dtemp = torch.empty(1, device=dev, dtype=torch.float32)
     log = _lib.Log(*(t.data_ptr() for t in (addr, oold, kold, vold, kfin, vfin, ofin, tfirst, kiold)))
-    with torch.cuda.device(dev):
+    with _Here(dev):
         rc = L.slotscan_hard_bwd_q(ctypes.byref(p), _ptr(k), _ptr(q), _ptr(v), _ptr(gate), _ptr(fr), _ptr(temp),
                                    ctypes.byref(log), _ptr(dkbuf), _ptr(dvbuf), _ptr(dkinv),
                                    ctypes.byref(_lib.Storage(qbits, qgroup)), _ptr(scratch), nbytes, _ptr(dk), _ptr(dq),
                                    _ptr(dv), _ptr(dgate), _ptr(dfr), _ptr(dtemp), _stream(dev))
     _lib.check(rc, "slotscan_hard_bwd_q")
     return dk, dq, dv, dgate, dfr, dtemp
+
+
+hard_bwd = torch.library.custom_op("slotscan::hard_bwd", mutates_args=())(_hard_bwd)
 
 
 @hard_bwd.register_fake
@@ -138,13 +185,13 @@ def _setup(ctx, inputs, output):
     ctx.set_materialize_grads(False)
 
 
-def _backward(ctx, *grads):
+def _backward(ctx, *grads, bwd=None):
     dkbuf, dvbuf, dkinv = grads[0], grads[1], grads[12]
     k, q, v, gate, fr, temp, addr, oold, kold, vold, kfin, vfin, ofin, tfirst, kiold = ctx.saved_tensors
     N, G, hard_gate, eps, occ_bin, snap_bf16, qbits, qgroup = ctx.meta
     sdt = torch.bfloat16 if snap_bf16 else torch.float32
     c = lambda g, dt: None if g is None else g.contiguous().to(dt)
-    dk, dq, dv, dgate, dfr, dtemp = hard_bwd(k, q, v, gate, fr, temp, addr, oold, kold, vold, kfin, vfin, ofin, tfirst,
+    dk, dq, dv, dgate, dfr, dtemp = (bwd or hard_bwd)(k, q, v, gate, fr, temp, addr, oold, kold, vold, kfin, vfin, ofin, tfirst,
                                              kiold, c(dkbuf, sdt), c(dvbuf, sdt), c(dkinv, torch.float32), N, G, hard_gate,
                                              eps, occ_bin, snap_bf16, qbits, qgroup)
     # no gradient for the carried-in state (K0, V0, o0, nsq0) nor for the integer / flag arguments
@@ -154,6 +201,29 @@ def _backward(ctx, *grads):
 hard_fwd.register_autograd(_backward, setup_context=_setup)
 
 
+class _HardScan(torch.autograd.Function):
+    """hard_fwd and its backward for a plain_call."""
+
+    @staticmethod
+    def forward(ctx, *inputs):
+        out = _hard_fwd(*inputs)
+        _setup(ctx, inputs, out)
+        return out
+
+    @staticmethod
+    @torch.autograd.function.once_differentiable
+    def backward(ctx, *grads):
+        return _backward(ctx, *grads, bwd=_hard_bwd if plain_call(*grads) else None)
+
+
+def run_hard_fwd(*args):
+    """hard_fwd with every argument given, by the shorter way where that is the same thing."""
+    ts = args[:10]
+    if not plain_call(*ts):
+        return hard_fwd(*args)
+    return _HardScan.apply(*args) if wants_grad(*ts) else _hard_fwd(*args)
+
+
 # ------------------------------------------------------------------------------------------------------------------
 # The general scan (soft address, attached address gradient): slotscan_dense_fwd / slotscan_dense_bwd.
 def _dense_params(k, v, gate, fr, N, G, hard, hard_gate, eps, detach_addr, occ_bin):
@@ -161,8 +231,7 @@ def _dense_params(k, v, gate, fr, N, G, hard, hard_gate, eps, detach_addr, occ_b
     return _lib.DenseParams(base, int(hard), int(detach_addr))
 
 
-@torch.library.custom_op("slotscan::dense_fwd", mutates_args=())
-def dense_fwd(k: torch.Tensor, q: Optional[torch.Tensor], v: torch.Tensor, gate: torch.Tensor, fr: torch.Tensor,
+def _dense_fwd(k: torch.Tensor, q: Optional[torch.Tensor], v: torch.Tensor, gate: torch.Tensor, fr: torch.Tensor,
               temp: torch.Tensor, N: int, G: int, hard: bool, hard_gate: bool, eps: float, detach_addr: bool,
               occ_bin: bool) -> Tuple[torch.Tensor, torch.Tensor, torch.Tensor, torch.Tensor, torch.Tensor, torch.Tensor,
                                       torch.Tensor]:
@@ -178,12 +247,15 @@ def dense_fwd(k: torch.Tensor, q: Optional[torch.Tensor], v: torch.Tensor, gate:
     kfin, vfin, ofin = e(B * H, N, DK), e(B * H, N, DV), e(B * H, N)
     p = _dense_params(k, v, gate, fr, N, G, hard, hard_gate, eps, detach_addr, occ_bin)
     _lib.check(_lib.lib().slotscan_dense_check(ctypes.byref(p)), "slotscan_dense_check")
-    with torch.cuda.device(dev):
+    with _Here(dev):
         rc = _lib.lib().slotscan_dense_fwd(ctypes.byref(p), _ptr(k), _ptr(q), _ptr(v), _ptr(gate), _ptr(fr), _ptr(temp),
                                            _ptr(kbuf), _ptr(vbuf), _ptr(obuf), _ptr(addr), _ptr(kfin), _ptr(vfin),
                                            _ptr(ofin), _stream(dev))
     _lib.check(rc, "slotscan_dense_fwd")
     return kbuf, vbuf, obuf, addr, kfin, vfin, ofin
+
+
+dense_fwd = torch.library.custom_op("slotscan::dense_fwd", mutates_args=())(_dense_fwd)
 
 
 @dense_fwd.register_fake
@@ -196,8 +268,7 @@ def _(k, q, v, gate, fr, temp, N, G, hard, hard_gate, eps, detach_addr, occ_bin)
             e(B * H, N, DV), e(B * H, N))
 
 
-@torch.library.custom_op("slotscan::dense_bwd", mutates_args=())
-def dense_bwd(k: torch.Tensor, q: Optional[torch.Tensor], v: torch.Tensor, gate: torch.Tensor, fr: torch.Tensor,
+def _dense_bwd(k: torch.Tensor, q: Optional[torch.Tensor], v: torch.Tensor, gate: torch.Tensor, fr: torch.Tensor,
               temp: torch.Tensor, kbuf: torch.Tensor, vbuf: torch.Tensor, obuf: torch.Tensor,
               dkbuf: Optional[torch.Tensor], dvbuf: Optional[torch.Tensor], N: int, G: int, hard: bool, hard_gate: bool,
               eps: float, detach_addr: bool, occ_bin: bool
@@ -214,12 +285,15 @@ def dense_bwd(k: torch.Tensor, q: Optional[torch.Tensor], v: torch.Tensor, gate:
     dgate = torch.empty(gate.shape, device=dev, dtype=torch.float32)
     dfr = torch.empty(fr.shape, device=dev, dtype=torch.float32)
     dtemp = torch.empty(1, device=dev, dtype=torch.float32)
-    with torch.cuda.device(dev):
+    with _Here(dev):
         rc = L.slotscan_dense_bwd(ctypes.byref(p), _ptr(k), _ptr(q), _ptr(v), _ptr(gate), _ptr(fr), _ptr(temp), _ptr(kbuf),
                                   _ptr(vbuf), _ptr(obuf), _ptr(dkbuf), _ptr(dvbuf), _ptr(scratch), nbytes, _ptr(dk),
                                   _ptr(dq), _ptr(dv), _ptr(dgate), _ptr(dfr), _ptr(dtemp), _stream(dev))
     _lib.check(rc, "slotscan_dense_bwd")
     return dk, dq, dv, dgate, dfr, dtemp
+
+
+dense_bwd = torch.library.custom_op("slotscan::dense_bwd", mutates_args=())(_dense_bwd)
 
 
 @dense_bwd.register_fake
@@ -235,11 +309,34 @@ def _dense_setup(ctx, inputs, output):
     ctx.set_materialize_grads(False)
 
 
-def _dense_backward(ctx, dkbuf, dvbuf, *unused):
+def _dense_backward(ctx, dkbuf, dvbuf, *unused, bwd=None):
     k, q, v, gate, fr, temp, kbuf, vbuf, obuf = ctx.saved_tensors
     c = lambda g: None if g is None else g.contiguous().to(torch.float32)
-    dk, dq, dv, dgate, dfr, dtemp = dense_bwd(k, q, v, gate, fr, temp, kbuf, vbuf, obuf, c(dkbuf), c(dvbuf), *ctx.meta)
+    dk, dq, dv, dgate, dfr, dtemp = (bwd or dense_bwd)(k, q, v, gate, fr, temp, kbuf, vbuf, obuf, c(dkbuf), c(dvbuf), *ctx.meta)
     return (dk, (None if q is None else dq), dv, dgate, dfr, dtemp) + (None,) * 7
 
 
 dense_fwd.register_autograd(_dense_backward, setup_context=_dense_setup)
+
+
+class _DenseScan(torch.autograd.Function):
+    """dense_fwd and its backward for a plain_call."""
+
+    @staticmethod
+    def forward(ctx, *inputs):
+        out = _dense_fwd(*inputs)
+        _dense_setup(ctx, inputs, out)
+        return out
+
+    @staticmethod
+    @torch.autograd.function.once_differentiable
+    def backward(ctx, *grads):
+        return _dense_backward(ctx, *grads, bwd=_dense_bwd if plain_call(*grads) else None)
+
+
+def run_dense_fwd(*args):
+    """dense_fwd by the shorter way where that is the same thing."""
+    ts = args[:6]
+    if not plain_call(*ts):
+        return dense_fwd(*args)
+    return _DenseScan.apply(*args) if wants_grad(*ts) else _dense_fwd(*args)

@@ -57,10 +57,10 @@ def kv_scan_g(k, v, gate, fr, N, temp, G=16, hard=False, hard_gate=False, eps=1e
     if not (hard and detach_addr):
         # soft address and / or address gradient attached to the stored keys: the general kernels (float32 snapshots,
         # which are also the checkpoints of their backward; a bf16 hand-over is a cast of the result)
-        out = ops.dense_fwd(k_, q_, v_, g_, fr_, temp_, int(N), int(G), bool(hard), bool(hard_gate), float(eps),
+        out = ops.run_dense_fwd(k_, q_, v_, g_, fr_, temp_, int(N), int(G), bool(hard), bool(hard_gate), float(eps),
                             bool(detach_addr), bool(occ_bin))
         return out[0].to(out_dtype), out[1].to(out_dtype)
-    out = ops.hard_fwd(k_, q_, v_, g_, fr_, temp_, None, None, None, None, int(N), int(G), bool(hard_gate), float(eps),
+    out = ops.run_hard_fwd(k_, q_, v_, g_, fr_, temp_, None, None, None, None, int(N), int(G), bool(hard_gate), float(eps),
                        bool(occ_bin), out_dtype == torch.bfloat16, False, True, 0, 16)
     return out[0], out[1]
 
@@ -103,12 +103,12 @@ def _scan_streams(k_, v_, q_, gate, fr, N, temp, G, hard_gate, eps, occ_bin, out
     fr_, temp_ = _scalars(fr, temp, k_.device)
     st = (None, None, None, None) if state is None else (tuple(state) + (None,))[:4]
     with torch.no_grad():
-        out = ops.hard_fwd(k_, q_, v_, _as_f32(gate), fr_, temp_, st[0], st[1], st[2], st[3], int(N), int(G),
+        out = ops.run_hard_fwd(k_, q_, v_, _as_f32(gate), fr_, temp_, st[0], st[1], st[2], st[3], int(N), int(G),
                            bool(hard_gate), float(eps), bool(occ_bin), out_dtype == torch.bfloat16, bool(want_norm),
                            bool(undo_log), qbits, int(qgroup))
     d = dict(zip(ops.OUT, out))
     if want_norm:
-        d["valid"] = d["valid"].bool()
+        d["valid"] = d["valid"].view(torch.bool)          # 0 / 1 bytes are a bool tensor's storage
     else:
         del d["kinv"], d["valid"]
     return d
@@ -147,9 +147,9 @@ def write_memory(k, v, gate, fr, N, temp, G=16, hard_gate=False, eps=1e-4, q=Non
         return writer_epilogue(kb, vb, out_dtype, qbits=qbits, qgroup=qgroup)
     k_, v_, q_ = _token_streams(k, v, q)
     fr_, temp_ = _scalars(fr, temp, k.device)
-    out = ops.hard_fwd(k_, q_, v_, _as_f32(gate), fr_, temp_, None, None, None, None, int(N), int(G), bool(hard_gate),
+    out = ops.run_hard_fwd(k_, q_, v_, _as_f32(gate), fr_, temp_, None, None, None, None, int(N), int(G), bool(hard_gate),
                        float(eps), bool(occ_bin), out_dtype == torch.bfloat16, True, True, _bits(qbits), int(qgroup))
-    return out[0], out[1], out[12], out[13].bool()
+    return out[0], out[1], out[12], out[13].view(torch.bool)
 
 
 class StreamingScan:

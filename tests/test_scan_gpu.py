@@ -318,3 +318,44 @@ def test_wide_address_scan_equals_direct_bitwise(N, D, dtype, occ_bin):
             assert (b["tfirst"][:, 64] == t1 - t0).all()               # the start of it: first pass
             for n in ("addr", "oold", "kiold", "kold"):
                 assert torch.equal(a[n][:, :t1 - t0], b[n]), (n, t1)
+
+
+@pytest.mark.parametrize("mode", ["hard", "soft", "keyless", "read"])
+def test_plain_calls_equal_registered_ops(mode, monkeypatch):
+    """Ordinary eager calls go round the custom ops' wrapping; the same call through the ops gives the same bits, values and
+    gradients, saved-tensor hooks see the saved tensors on both ways, and under a fake mode the ops' fake kernels answer."""
+    import slotscan_b200 as S
+    from slotscan_b200 import keyless, ops, read
+    B, T, H, N, D, G = 2, 40, 2, 24, 64, 8
+    inp = make_inputs("clustered", B, T, H, D, D, seed=3)
+    base = [inp[n].cuda() for n in ("k", "q", "v", "gate", "fr")]
+    gen = torch.Generator(device="cuda").manual_seed(4)
+    wa, qr = (torch.randn(B, T, H, n, device="cuda", generator=gen) for n in (N, D))
+
+    def call(x):
+        k, q, v, g, fr = x
+        if mode == "keyless":
+            return [S.slot_scan_v(v, wa, g, 2.0, N, G=G)]
+        if mode == "read":
+            kb, vb, kinv, valid = S.write_memory(k, v, g, fr, N, 16.0, G=G, q=q, occ_bin=True, out_dtype=torch.float32)
+            return [S.read_snapshots(qr.unsqueeze(3), g.unsqueeze(3) + 1, kb, vb, kinv, valid, G)]
+        return list(S.kv_scan_g(k, v, g, fr, N, 16.0, G=G, hard=mode == "hard", detach_addr=True, q=q, occ_bin=True))
+
+    def once():
+        x = [t.clone().requires_grad_() for t in base]
+        packed = []
+        with torch.autograd.graph.saved_tensors_hooks(lambda t: (packed.append(t), t)[1], lambda t: t):
+            out = call(x)
+        g = torch.autograd.grad(out, x, [torch.ones_like(o) for o in out], allow_unused=True)
+        assert packed
+        return out + [t for t in g if t is not None]
+    plain = once()
+    for m in (ops, read, keyless):
+        monkeypatch.setattr(m, "plain_call", lambda *ts: False)
+    for a, b in zip(plain, once()):
+        assert torch.equal(a, b)
+    monkeypatch.undo()
+    from torch._subclasses.fake_tensor import FakeTensorMode
+    with FakeTensorMode(allow_non_fake_inputs=True) as fm:
+        fake = call([fm.from_tensor(t) for t in base])
+    assert all(f.shape == p.shape and f.dtype == p.dtype for f, p in zip(fake, plain))
