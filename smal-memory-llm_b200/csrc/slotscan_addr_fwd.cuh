@@ -247,24 +247,21 @@ __global__ void __launch_bounds__(AF_THREADS, (RPL <= 2 ? 3 : 1)) addr_fwd_direc
     //                 registers), compute its per-token constants and write the previous chunk's log out.
 #define AF_DOTS(NS, SL, BUF)                                                                                   \
     {                                                                                                          \
-        float4 q4[NF], k4[NF];                                                                                 \
+        f32x4 q4[NF], k4[NF];                                                                                  \
         _Pragma("unroll") for (int i = 0; i < NF; i++) {                                                       \
-            q4[i] = ld4(Qs + (SL) * DK + c0 + 4 * i);                                                          \
-            k4[i] = ld4(Ks + (SL) * DK + c0 + 4 * i);                                                          \
+            q4[i] = ld4x2(Qs + (SL) * DK + c0 + 4 * i);                                                        \
+            k4[i] = ld4x2(Ks + (SL) * DK + c0 + 4 * i);                                                        \
         }                                                                                                      \
         _Pragma("unroll") for (int s = 0; s < (NS); s++) {                                                     \
             const int n = min(lane + 32 * s, ncap - 1);                                                        \
             const float* Kr = K + (size_t)n * KS + c0;                                                         \
-            float4 aS = zero4, aR = zero4;      /* 8 independent FMA chains; summed once at the end */          \
+            f32x4 aS = {0ull, 0ull}, aR = aS;   /* 8 independent FMA chains, two to an instruction; summed once at the end */ \
             _Pragma("unroll") for (int i = 0; i < NF; i++) {                                                   \
-                const float4 K4 = ld4(Kr + 4 * i);                                                             \
-                aS.x = fmaf(K4.x, q4[i].x, aS.x); aS.y = fmaf(K4.y, q4[i].y, aS.y);                            \
-                aS.z = fmaf(K4.z, q4[i].z, aS.z); aS.w = fmaf(K4.w, q4[i].w, aS.w);                            \
-                aR.x = fmaf(K4.x, k4[i].x, aR.x); aR.y = fmaf(K4.y, k4[i].y, aR.y);                            \
-                aR.z = fmaf(K4.z, k4[i].z, aR.z); aR.w = fmaf(K4.w, k4[i].w, aR.w);                            \
+                const f32x4 K4 = ld4x2(Kr + 4 * i);                                                            \
+                fma4(aS, K4, q4[i]);                                                                           \
+                fma4(aR, K4, k4[i]);                                                                           \
             }                                                                                                  \
-            part[(((BUF) * RPL + s) * AF_CWARPS + cw) * 32 + lane] =                                           \
-                make_float2((aS.x + aS.y) + (aS.z + aS.w), (aR.x + aR.y) + (aR.z + aR.w));                     \
+            part[(((BUF) * RPL + s) * AF_CWARPS + cw) * 32 + lane] = make_float2(sum4(aS), sum4(aR));          \
         }                                                                                                      \
     }
     // Few live rows (< 32 / F): a lane takes row lane % (32 / F) and the F-th part lane / (32 / F) of the warp's columns,
@@ -274,21 +271,19 @@ __global__ void __launch_bounds__(AF_THREADS, (RPL <= 2 ? 3 : 1)) addr_fwd_direc
     {                                                                                                          \
         constexpr int FF = (NF >= (F)) ? (F) : 1, R_ = 32 / FF, NFS = NF / FF;                                 \
         const int cb = c0 + (lane / R_) * (CW / FF);                                                           \
-        float4 q4[NFS], k4[NFS];                                                                               \
+        f32x4 q4[NFS], k4[NFS];                                                                                \
         _Pragma("unroll") for (int i = 0; i < NFS; i++) {                                                      \
-            q4[i] = ld4(Qs + (SL) * DK + cb + 4 * i);                                                          \
-            k4[i] = ld4(Ks + (SL) * DK + cb + 4 * i);                                                          \
+            q4[i] = ld4x2(Qs + (SL) * DK + cb + 4 * i);                                                        \
+            k4[i] = ld4x2(Ks + (SL) * DK + cb + 4 * i);                                                        \
         }                                                                                                      \
         const float* Kr = K + (size_t)min(lane & (R_ - 1), ncap - 1) * KS + cb;                                \
-        float4 aS = zero4, aR = zero4;                                                                         \
+        f32x4 aS = {0ull, 0ull}, aR = aS;                                                                      \
         _Pragma("unroll") for (int i = 0; i < NFS; i++) {                                                      \
-            const float4 K4 = ld4(Kr + 4 * i);                                                                 \
-            aS.x = fmaf(K4.x, q4[i].x, aS.x); aS.y = fmaf(K4.y, q4[i].y, aS.y);                                \
-            aS.z = fmaf(K4.z, q4[i].z, aS.z); aS.w = fmaf(K4.w, q4[i].w, aS.w);                                \
-            aR.x = fmaf(K4.x, k4[i].x, aR.x); aR.y = fmaf(K4.y, k4[i].y, aR.y);                                \
-            aR.z = fmaf(K4.z, k4[i].z, aR.z); aR.w = fmaf(K4.w, k4[i].w, aR.w);                                \
+            const f32x4 K4 = ld4x2(Kr + 4 * i);                                                                \
+            fma4(aS, K4, q4[i]);                                                                               \
+            fma4(aR, K4, k4[i]);                                                                               \
         }                                                                                                      \
-        float sS = (aS.x + aS.y) + (aS.z + aS.w), sR = (aR.x + aR.y) + (aR.z + aR.w);                          \
+        float sS = sum4(aS), sR = sum4(aR);                                                                    \
         _Pragma("unroll") for (int off = 16; off >= R_; off >>= 1) {                                           \
             sS += __shfl_xor_sync(FULL, sS, off);                                                              \
             sR += __shfl_xor_sync(FULL, sR, off);                                                              \

@@ -12,8 +12,9 @@
 // [reference addr_bwd, slotkern_cuda.py:264-443]
 // Bound: 2 x (32 + rows) x DK multiply-adds per token on the CUDA cores (float32: the tensor cores' bf16 or tf32 operands
 // would lose bits); the chunked resident-state kernel (slotscan_addr_bwd.cuh) walks 8-token chunks of a sequence one after
-// another with five barriers each.  B = 32, T = 1024, H = 6, 192 rows x 128 all in use, bf16: 2.07 ms chunked, 1.44 ms here;
-// B = 4, T = 1000, H = 12, ~60 rows x 64, float32 (48 sequences, so that the chunked kernel had 48 CTAs): 1.29 -> 0.20 ms.
+// another with five barriers each.  B = 32, T = 1024, H = 6, 192 rows x 128 all in use, bf16: 2.07 ms chunked, 1.33 ms here
+// (1.44 with scalar multiply-adds);
+// B = 4, T = 1000, H = 12, ~60 rows x 64, float32 (48 sequences, so that the chunked kernel had 48 CTAs): 1.29 -> 0.27 ms.
 // Persistent: the CTAs share the items of the sequences that need this kernel, which they find from the forward's tfirst
 // table (a launch whose sequences all use few rows returns after that look).
 #pragma once
@@ -73,32 +74,30 @@ __device__ __forceinline__ void tiles_scores(const float* rows, const float* sq,
     // a quarter of the columns at a time: four short chains instead of one of DK, whose rounding showed in the gradients
 #pragma unroll 1
     for (int d0 = 0; d0 < DK; d0 += DK / 4) {
-        float acc[NS][4];
+        f32x2 acc[NS][4];                                    // even and odd columns
 #pragma unroll
         for (int i = 0; i < NS; i++)
 #pragma unroll
-            for (int k = 0; k < 4; k++) acc[i][k] = 0.f;
+            for (int k = 0; k < 4; k++) acc[i][k] = 0ull;
 #pragma unroll 2
         for (int d = d0; d < d0 + DK / 4; d += 4) {
-            float4 q[4];
+            f32x4 q[4];
 #pragma unroll
-            for (int k = 0; k < 4; k++) q[k] = ld4(sq + (tq + 8 * k) * RS + d);
+            for (int k = 0; k < 4; k++) q[k] = ld4x2(sq + (tq + 8 * k) * RS + d);
 #pragma unroll
             for (int i = 0; i < NS; i++) {
-                const float4 r = ld4(rows + (rg + 32 * i) * RS + d);
+                const f32x4 r = ld4x2(rows + (rg + 32 * i) * RS + d);
 #pragma unroll
                 for (int k = 0; k < 4; k++) {
-                    acc[i][k] = fmaf(r.x, q[k].x, acc[i][k]);
-                    acc[i][k] = fmaf(r.y, q[k].y, acc[i][k]);
-                    acc[i][k] = fmaf(r.z, q[k].z, acc[i][k]);
-                    acc[i][k] = fmaf(r.w, q[k].w, acc[i][k]);
+                    acc[i][k] = fma2(r.a, q[k].a, acc[i][k]);
+                    acc[i][k] = fma2(r.b, q[k].b, acc[i][k]);
                 }
             }
         }
 #pragma unroll
         for (int i = 0; i < NS; i++)
 #pragma unroll
-            for (int k = 0; k < 4; k++) tot[i][k] += acc[i][k];
+            for (int k = 0; k < 4; k++) { const float2 v = unpack2(acc[i][k]); tot[i][k] += v.x + v.y; }
     }
 #pragma unroll
     for (int i = 0; i < NS; i++)
@@ -293,7 +292,7 @@ __global__ void __launch_bounds__(TL_THREADS) addr_bwd_tiles_kernel(
                 }
 #pragma unroll
                 for (int i = 0; i < NR; i++) dwv[i] += zv[i];            // key part + value part
-                float zmax = -INFINITY;
+                float zmax = -INFINITY, smax = -INFINITY;
 #pragma unroll
                 for (int i = 0; i < NR; i++) {
                     const int n = r8 + 8 * i;
@@ -302,7 +301,9 @@ __global__ void __launch_bounds__(TL_THREADS) addr_bwd_tiles_kernel(
                         const int s = s_slot[j * NP + n];
                         const float oc = s_oc[s];
                         const bool occ = oc >= eps;
-                        zv[i] = tqi * (s_ki[s] * St[tiles_at(s, j)]) - (occ ? frv : 0.f);
+                        const float sc = tqi * (s_ki[s] * St[tiles_at(s, j)]);
+                        zv[i] = sc - (occ ? frv : 0.f);
+                        smax = fmaxf(smax, sc);
                         if (occ) { okm |= 1u << i; zmax = fmaxf(zmax, zv[i]); }
                         else if (oc < eps && n < ei) ei = n;
                     }
@@ -313,7 +314,10 @@ __global__ void __launch_bounds__(TL_THREADS) addr_bwd_tiles_kernel(
                 for (int i = 0; i < NR; i++)
                     if (r8 + 8 * i == ei) { okm |= 1u << i; zmax = fmaxf(zmax, zv[i]); }
 #pragma unroll
-                for (int off = 4; off < 32; off <<= 1) zmax = fmaxf(zmax, __shfl_xor_sync(FULL, zmax, off));
+                for (int off = 4; off < 32; off <<= 1) {
+                    zmax = fmaxf(zmax, __shfl_xor_sync(FULL, zmax, off));
+                    smax = fmaxf(smax, __shfl_xor_sync(FULL, smax, off));
+                }
                 float se = 0.f, sd = 0.f;
 #pragma unroll
                 for (int i = 0; i < NR; i++) {
@@ -341,7 +345,8 @@ __global__ void __launch_bounds__(TL_THREADS) addr_bwd_tiles_kernel(
                         const int s = s_slot[j * NP + n];
                         const float dz = (okm >> i) & 1u ? (zv[i] * inv) * (g * dwv[i] - sa) : 0.f;
                         const float ki = s_ki[s];
-                        f2 += dz * (tqi * (ki * St[tiles_at(s, j)]));
+                        // (the dz of a token add up to zero: against the largest score instead of zero the products cancel less)
+                        f2 += (okm >> i) & 1u ? dz * (tqi * (ki * St[tiles_at(s, j)]) - smax) : 0.f;
                         if (s_oc[s] >= eps) f1 -= dz;
                         cv[i] = dz * temp * ki;
                         if (n == a) dg[ix] = dwv[i];
@@ -372,52 +377,42 @@ __global__ void __launch_bounds__(TL_THREADS) addr_bwd_tiles_kernel(
             {
                 const int tg = (warp & 3) * 8, half = warp >> 2, cq = lane % CQ, sub = lane / CQ;
                 const int sh = NS * 16, s_lo = half * sh + sub, s_hi = half * sh + sh;
-                float tot[8][4];
+                f32x2 tot[8][2];
 #pragma unroll
-                for (int j = 0; j < 8; j++)
-#pragma unroll
-                    for (int k = 0; k < 4; k++) tot[j][k] = 0.f;
+                for (int j = 0; j < 8; j++) tot[j][0] = tot[j][1] = 0ull;
                 const bool bad = *s_bad != 0;
 #pragma unroll 1
                 for (int sb = s_lo; sb < s_hi; sb += 16) {               // 16 slots at a time: short chains
-                    float acc[8][4];
+                    f32x2 part2[8][2];
 #pragma unroll
-                    for (int j = 0; j < 8; j++)
-#pragma unroll
-                        for (int k = 0; k < 4; k++) acc[j][k] = 0.f;
+                    for (int j = 0; j < 8; j++) part2[j][0] = part2[j][1] = 0ull;
 #pragma unroll 2
                     for (int s = sb; s < sb + 16; s += SUB) {            // half * sh is a multiple of 16
-                        const float4 r = ld4(rows + s * RS + cq * 4);
+                        const f32x4 r = ld4x2(rows + s * RS + cq * 4);
                         const float4 c0 = ld4(St + tiles_at(s, tg)), c1 = ld4(St + tiles_at(s, tg + 4));
                         const float cv[8] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w};
-                        if (!bad) {
 #pragma unroll
-                            for (int j = 0; j < 8; j++) {
-                                acc[j][0] = fmaf(cv[j], r.x, acc[j][0]);
-                                acc[j][1] = fmaf(cv[j], r.y, acc[j][1]);
-                                acc[j][2] = fmaf(cv[j], r.z, acc[j][2]);
-                                acc[j][3] = fmaf(cv[j], r.w, acc[j][3]);
-                            }
-                        } else {                                         // a version a token does not see stays out of its sum
-#pragma unroll
-                            for (int j = 0; j < 8; j++) {
-                                if (cv[j] != 0.f) { acc[j][0] += cv[j] * r.x; acc[j][1] += cv[j] * r.y; acc[j][2] += cv[j] * r.z; acc[j][3] += cv[j] * r.w; }
-                            }
+                        for (int j = 0; j < 8; j++) {
+                            if (bad && cv[j] == 0.f) continue;           // a version a token does not see stays out of its sum
+                            const f32x2 c2 = pack2(cv[j], cv[j]);
+                            part2[j][0] = fma2(c2, r.a, part2[j][0]);
+                            part2[j][1] = fma2(c2, r.b, part2[j][1]);
                         }
                     }
 #pragma unroll
-                    for (int j = 0; j < 8; j++)
-#pragma unroll
-                        for (int k = 0; k < 4; k++) tot[j][k] += acc[j][k];
+                    for (int j = 0; j < 8; j++) { tot[j][0] = add2(tot[j][0], part2[j][0]); tot[j][1] = add2(tot[j][1], part2[j][1]); }
                 }
-                float (&acc)[8][4] = tot;
+                float acc[8][4];
 #pragma unroll
-                for (int j = 0; j < 8; j++)
+                for (int j = 0; j < 8; j++) {
+                    const float2 lo = unpack2(tot[j][0]), hi = unpack2(tot[j][1]);
+                    acc[j][0] = lo.x; acc[j][1] = lo.y; acc[j][2] = hi.x; acc[j][3] = hi.y;
 #pragma unroll
                     for (int k = 0; k < 4; k++) {
 #pragma unroll
                         for (int off = 16; off >= CQ; off >>= 1) acc[j][k] += __shfl_xor_sync(FULL, acc[j][k], off);
                     }
+                }
                 __syncthreads();                                         // rows are free: the halves meet there
                 if (half == 1 && sub == 0) {
 #pragma unroll

@@ -13,8 +13,8 @@
 // The roles run one token apart as in the direct kernel (see its schedule comment), one barrier per token.  Every warp issues an instruction about every five cycles, so what counts is the longest role's
 // instructions per token.  One CTA fills an SM, as the direct kernel's 192 rows did; it is the second pass, of sequences that
 // use more than AF_NCAP1 rows: with few rows the direct kernel's split of a row over lanes is shorter.  B200, second
-// pass alone: 192 sequences x 1024 tokens, 192 rows x 128 all in use, bf16: 2.27 -> 1.77 ms (two CTAs' worth of rounds on 148 SMs;
-// column warps of three slots: 2.02); 48 x 1000, ~60 rows x 64, float32: 0.81 -> 0.60; 24 x 8 carried-in tokens: 31 -> 17 us.
+// pass alone: 192 sequences x 1024 tokens, 192 rows x 128 all in use, bf16: 2.27 -> 1.74 ms (two CTAs' worth of rounds on 148 SMs;
+// column warps of three slots: 2.02); 48 x 1000, ~60 rows x 64, float32: 0.81 -> 0.56; 24 x 8 carried-in tokens: 31 -> 17 us.
 #pragma once
 #include "slotscan_addr_fwd.cuh"
 
@@ -45,18 +45,12 @@ __host__ __device__ inline AddrWideSmem addr_wide_layout(int RPL, int DK) {
 // a partial dot from the four chains of each of F pieces of a quarter, the pieces paired as the direct kernel's shuffles pair
 // the lanes that share a row
 template <int F>
-__device__ __forceinline__ float aw_sum(const float4 (&a)[F]) {
-    float s[F];
-#pragma unroll
-    for (int f = 0; f < F; f++) s[f] = (a[f].x + a[f].y) + (a[f].z + a[f].w);
-    if constexpr (F == 4) return (s[0] + s[2]) + (s[1] + s[3]);
-    else if constexpr (F == 2) return s[0] + s[1];
-    else return s[0];
+__device__ __forceinline__ float aw_sum(const f32x4 (&a)[F]) {
+    if constexpr (F == 4) return (sum4(a[0]) + sum4(a[2])) + (sum4(a[1]) + sum4(a[3]));
+    else if constexpr (F == 2) return sum4(a[0]) + sum4(a[1]);
+    else return sum4(a[0]);
 }
-__device__ __forceinline__ float4 aw_mul(float4 a, float4 b) { return make_float4(a.x * b.x, a.y * b.y, a.z * b.z, a.w * b.w); }
-__device__ __forceinline__ void aw_fma(float4& c, float4 a, float4 b) {
-    c.x = fmaf(a.x, b.x, c.x); c.y = fmaf(a.y, b.y, c.y); c.z = fmaf(a.z, b.z, c.z); c.w = fmaf(a.w, b.w, c.w);
-}
+__device__ __forceinline__ f32x4 aw_mul(const f32x4& a, const f32x4& b) { return {mul2(a.a, b.a), mul2(a.b, b.b)}; }
 
 template <int DK, int RPL, bool OCCB, bool CARRY, typename Tin>
 __global__ void __launch_bounds__(aw_threads(RPL), 1) addr_fwd_wide_kernel(
@@ -133,14 +127,14 @@ __global__ void __launch_bounds__(aw_threads(RPL), 1) addr_fwd_wide_kernel(
     if (warp < AW_COL) {
         // ------------------------------------------------------------------ column warps
         const int cw = warp & 3, s_base = (warp >> 2) * SPG, c0 = cw * CW;
-        float4 K[SPG][NF];
+        f32x4 K[SPG][NF];
 #pragma unroll
         for (int s = 0; s < SPG; s++) {
             const int n = (s_base + s) * 32 + lane;
 #pragma unroll
             for (int i = 0; i < NF; i++) {
-                K[s][i] = make_float4(0.f, 0.f, 0.f, 0.f);
-                if (CARRY && n < N) K[s][i] = ld4(K0 + ((size_t)bh * N + n) * DK + c0 + 4 * i);
+                K[s][i] = {0ull, 0ull};
+                if (CARRY && n < N) K[s][i] = ld4x2(K0 + ((size_t)bh * N + n) * DK + c0 + 4 * i);
             }
         }
         auto dots = [&](int limd, int sl, int buf) {
@@ -149,14 +143,14 @@ __global__ void __launch_bounds__(aw_threads(RPL), 1) addr_fwd_wide_kernel(
             float2* out = part + ((buf * RPL + s_base) * 4 + cw) * 32 + lane;
             auto few = [&](auto fc) {                                 // fewer than 16 rows: slot 0 only, in pieces
                 constexpr int F = decltype(fc)::value, NFS = NF / F;
-                float4 aS[F], aR[F];
+                f32x4 aS[F], aR[F];
 #pragma unroll
                 for (int f = 0; f < F; f++) {
 #pragma unroll
                     for (int i = 0; i < NFS; i++) {
-                        const float4 q4 = ld4(qr + 4 * (f * NFS + i)), k4 = ld4(kr + 4 * (f * NFS + i));
+                        const f32x4 q4 = ld4x2(qr + 4 * (f * NFS + i)), k4 = ld4x2(kr + 4 * (f * NFS + i));
                         if (i == 0) { aS[f] = aw_mul(K[0][f * NFS], q4); aR[f] = aw_mul(K[0][f * NFS], k4); }
-                        else { aw_fma(aS[f], K[0][f * NFS + i], q4); aw_fma(aR[f], K[0][f * NFS + i], k4); }
+                        else { fma4(aS[f], K[0][f * NFS + i], q4); fma4(aR[f], K[0][f * NFS + i], k4); }
                     }
                 }
                 out[0] = make_float2(aw_sum<F>(aS), aw_sum<F>(aR));
@@ -167,19 +161,19 @@ __global__ void __launch_bounds__(aw_threads(RPL), 1) addr_fwd_wide_kernel(
 #pragma unroll
                 for (int pass = 0; pass < 2; pass++) {                // queries, then keys: half the sums in registers
                     const float* r = pass ? kr : qr;
-                    float4 a[NS];
+                    f32x4 a[NS];
 #pragma unroll
                     for (int i = 0; i < NF; i++) {
-                        const float4 r4 = ld4(r + 4 * i);
+                        const f32x4 r4 = ld4x2(r + 4 * i);
 #pragma unroll
                         for (int s = 0; s < NS; s++) {
                             if (i == 0) a[s] = aw_mul(K[s][0], r4);
-                            else aw_fma(a[s], K[s][i], r4);
+                            else fma4(a[s], K[s][i], r4);
                         }
                     }
 #pragma unroll
                     for (int s = 0; s < NS; s++) {
-                        const float v = (a[s].x + a[s].y) + (a[s].z + a[s].w);
+                        const float v = sum4(a[s]);
                         if (pass == 0) sS[s] = v;
                         else out[s * 4 * 32] = make_float2(sS[s], v);
                     }
@@ -207,16 +201,17 @@ __global__ void __launch_bounds__(aw_threads(RPL), 1) addr_fwd_wide_kernel(
                 lim = max(lim, min(a + 1, N - 1));
                 if (sa >= 0 && sa < SPG) {
                     const int sl = (t - 1) & (AW_RING - 1);
-                    const float g = s_tok[AW_TOK * sl + 2], omw = 1.f - g;
+                    const float g = s_tok[AW_TOK * sl + 2];
+                    const f32x2 g2 = pack2(g, g), om2 = pack2(1.f - g, 1.f - g);
                     const float* kr = Ks + sl * DK + c0;
 #pragma unroll
                     for (int s = 0; s < SPG; s++) {
                         if (s == sa && lane == (a & 31)) {
 #pragma unroll
                             for (int i = 0; i < NF; i++) {
-                                const float4 k4 = ld4(kr + 4 * i);
-                                K[s][i].x = blend(K[s][i].x, k4.x, g, omw); K[s][i].y = blend(K[s][i].y, k4.y, g, omw);
-                                K[s][i].z = blend(K[s][i].z, k4.z, g, omw); K[s][i].w = blend(K[s][i].w, k4.w, g, omw);
+                                const f32x4 k4 = ld4x2(kr + 4 * i);
+                                K[s][i].a = fma2(g2, k4.a, mul2(om2, K[s][i].a));      // blend, two columns at a time
+                                K[s][i].b = fma2(g2, k4.b, mul2(om2, K[s][i].b));
                             }
                         }
                     }

@@ -22,19 +22,23 @@
 namespace slotscan {
 
 // fixed-order sum of the partial sums (per sequence and token chunk) -> dtemp, scalar dfr: each thread adds a strided
-// subset in index order, then the 256 subtotals are added in order, so the result is bitwise repeatable
+// subset in index order, then the subtotals are added in a fixed order, so the result is bitwise repeatable
+// (in double: the sums cancel, and the order of float additions showed in the sixth digit of dtemp)
 __global__ void __launch_bounds__(256) finish_scalars_kernel(const float* __restrict__ part, int n, int fr_per_token,
                                                              float* dtemp, float* dfr) {
-    __shared__ float s_a[256], s_c[256];
-    float a = 0.f, c = 0.f;
-    for (int i = threadIdx.x; i < n; i += 256) { a += part[i]; c += part[n + i]; }
-    s_a[threadIdx.x] = a; s_c[threadIdx.x] = c;
+    __shared__ double s_a[8], s_c[8];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    double a = 0.0, c = 0.0;
+    for (int i = threadIdx.x; i < n; i += 256) { a += (double)part[i]; c += (double)part[n + i]; }
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) { a += __shfl_xor_sync(FULL, a, off); c += __shfl_xor_sync(FULL, c, off); }
+    if (lane == 0) { s_a[warp] = a; s_c[warp] = c; }
     __syncthreads();
     if (threadIdx.x == 0) {
-        a = 0.f; c = 0.f;
-        for (int i = 0; i < 256; i++) { a += s_a[i]; c += s_c[i]; }
-        dtemp[0] = a;
-        if (!fr_per_token) dfr[0] = c;
+        a = 0.0; c = 0.0;
+        for (int i = 0; i < 8; i++) { a += s_a[i]; c += s_c[i]; }
+        dtemp[0] = (float)a;
+        if (!fr_per_token) dfr[0] = (float)c;
     }
 }
 template <typename Tin>

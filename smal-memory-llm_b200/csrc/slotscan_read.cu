@@ -46,7 +46,8 @@ __device__ __forceinline__ int read_rows_in_use(const uint8_t* v, int N) {
 // Which snapshots a CTA of the two kernels below works on.  On its own: one, blockIdx.x.  Beside the tensor-core kernel
 // (SPARSE: the snapshots with at most `rows` rows in use) most are not its own, and a launch of a CTA per snapshot to
 // find that out took longer than the work (B = 32, T = 1024, every slot in use: 0.11 ms forward, 0.16 ms backward; now
-// 0.08, most of it the 4 % of snapshots that are its own, and 0.04): a grid that fits the machine looks the snapshots over, one per warp at a time.
+// 0.08, most of it the 4 % of snapshots that are its own, and 0.04): a grid that fits the machine looks the snapshots
+// over, one per warp at a time.
 template <bool SPARSE, typename F>
 __device__ __forceinline__ void read_each_snapshot(const uint8_t* valid, int N, long long total, int rows, F work) {
     if constexpr (!SPARSE) {

@@ -326,6 +326,14 @@ __device__ __forceinline__ void row8(float* f, const __nv_bfloat16* p) {
     for (int i = 0; i < 4; i++) { f[2 * i] = __uint_as_float(w[i] << 16); f[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u); }
 }
 
+__device__ __forceinline__ void row8x2(f32x4& a, f32x4& b, const float* p) { a = ld4x2(p); b = ld4x2(p + 4); }
+__device__ __forceinline__ void row8x2(f32x4& a, f32x4& b, const __nv_bfloat16* p) {
+    float f[8];
+    row8(f, p);
+    a = pack4(make_float4(f[0], f[1], f[2], f[3]));
+    b = pack4(make_float4(f[4], f[5], f[6], f[7]));
+}
+
 template <int D, typename Tin>
 struct RowsBwd3Layout {
     static constexpr int RPB = ROW_THREADS / (D / 8);
@@ -580,21 +588,18 @@ __global__ void __launch_bounds__(ROW_THREADS, (sizeof(Tin) == 2 ? 3 : 2)) rows_
             const int t = t0 + lane, sg = lane / G;
             const Tin* xr = reinterpret_cast<const Tin*>(dsm + LY::off_x + st * LY::x_bytes + lane * LY::XRS);
             // one row: 128-long dot of the token vector with the row's S of this token's block
+            // (chains as four sums of every fourth product, two to an instruction)
             auto one_row = [&](int rr) {
                 const float* Sr = s_S + (size_t)sg * LY::SBS + rr * D;
-                float a0_ = 0.f, a1_ = 0.f, a2_ = 0.f, a3_ = 0.f;
+                f32x4 a = {0ull, 0ull};
 #pragma unroll 4
                 for (int d = 0; d < D; d += 8) {
-                    float xv[8];
-                    row8(xv, xr + d);
-                    const float4 s0 = ld4(Sr + d / 2), s1 = ld4(Sr + D / 2 + d / 2);      // elements d .. d+3 and d+4 .. d+7
-                    a0_ = fmaf(xv[0], s0.x, a0_); a1_ = fmaf(xv[1], s0.y, a1_);
-                    a2_ = fmaf(xv[2], s0.z, a2_); a3_ = fmaf(xv[3], s0.w, a3_);
-                    a0_ = fmaf(xv[4], s1.x, a0_); a1_ = fmaf(xv[5], s1.y, a1_);
-                    a2_ = fmaf(xv[6], s1.z, a2_); a3_ = fmaf(xv[7], s1.w, a3_);
+                    f32x4 x0, x1;
+                    row8x2(x0, x1, xr + d);
+                    fma4(a, x0, ld4x2(Sr + d / 2));                          // elements d .. d+3 and d+4 .. d+7
+                    fma4(a, x1, ld4x2(Sr + D / 2 + d / 2));
                 }
-                const float dot = (a0_ + a1_) + (a2_ + a3_);
-                Dn[((size_t)bh * T + t) * N + row0 + rr] = fmaf(s_c[rr * RC + lane], dot, -s_xdx[rr * RC + lane]);
+                Dn[((size_t)bh * T + t) * N + row0 + rr] = fmaf(s_c[rr * RC + lane], sum4(a), -s_xdx[rr * RC + lane]);
             };
             constexpr int NW = ROW_THREADS / 32;
             for (int rr = warp; rr < RPB; rr += 2 * NW) {                  // rows rr and rr + NW of this warp
@@ -603,23 +608,17 @@ __global__ void __launch_bounds__(ROW_THREADS, (sizeof(Tin) == 2 ? 3 : 2)) rows_
                 if (okA && okB) {                                          // both: the token vector is unpacked once
                     const float* SA = s_S + (size_t)sg * LY::SBS + rr * D;
                     const float* SB = s_S + (size_t)sg * LY::SBS + rb * D;
-                    float a0_ = 0.f, a1_ = 0.f, a2_ = 0.f, a3_ = 0.f, b0_ = 0.f, b1_ = 0.f, b2_ = 0.f, b3_ = 0.f;
+                    f32x4 a = {0ull, 0ull}, b_ = a;
 #pragma unroll 4
                     for (int d = 0; d < D; d += 8) {
-                        float xv[8];
-                        row8(xv, xr + d);
-                        const float4 s0 = ld4(SA + d / 2), s1 = ld4(SA + D / 2 + d / 2);
-                        const float4 u0 = ld4(SB + d / 2), u1 = ld4(SB + D / 2 + d / 2);
-                        a0_ = fmaf(xv[0], s0.x, a0_); a1_ = fmaf(xv[1], s0.y, a1_);
-                        a2_ = fmaf(xv[2], s0.z, a2_); a3_ = fmaf(xv[3], s0.w, a3_);
-                        b0_ = fmaf(xv[0], u0.x, b0_); b1_ = fmaf(xv[1], u0.y, b1_);
-                        b2_ = fmaf(xv[2], u0.z, b2_); b3_ = fmaf(xv[3], u0.w, b3_);
-                        a0_ = fmaf(xv[4], s1.x, a0_); a1_ = fmaf(xv[5], s1.y, a1_);
-                        a2_ = fmaf(xv[6], s1.z, a2_); a3_ = fmaf(xv[7], s1.w, a3_);
-                        b0_ = fmaf(xv[4], u1.x, b0_); b1_ = fmaf(xv[5], u1.y, b1_);
-                        b2_ = fmaf(xv[6], u1.z, b2_); b3_ = fmaf(xv[7], u1.w, b3_);
+                        f32x4 x0, x1;
+                        row8x2(x0, x1, xr + d);
+                        fma4(a, x0, ld4x2(SA + d / 2));
+                        fma4(b_, x0, ld4x2(SB + d / 2));
+                        fma4(a, x1, ld4x2(SA + D / 2 + d / 2));
+                        fma4(b_, x1, ld4x2(SB + D / 2 + d / 2));
                     }
-                    const float dotA = (a0_ + a1_) + (a2_ + a3_), dotB = (b0_ + b1_) + (b2_ + b3_);
+                    const float dotA = sum4(a), dotB = sum4(b_);
                     Dn[((size_t)bh * T + t) * N + row0 + rr] = fmaf(s_c[rr * RC + lane], dotA, -s_xdx[rr * RC + lane]);
                     Dn[((size_t)bh * T + t) * N + row0 + rb] = fmaf(s_c[rb * RC + lane], dotB, -s_xdx[rb * RC + lane]);
                 } else if (okA) {
