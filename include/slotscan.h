@@ -183,14 +183,15 @@ int slotscan_hard_bwd_noalloc(const slotscan_params* p, const void* k, const voi
  * [replaces the Triton kernels _kvfwd (gqa25/slotkern_kvt.py:43-119) and _kvbwd_g (gqa25/slotkern_kvg.py:41-205), which
  * the reference falls back to for everything but its hard + detached training mode (slotkern_cuda.py:540-542).]
  * The hard + detached mode has its own, much faster kernels (slotscan_hard_*); this entry point exists so that no
- * argument combination of the reference call is without a CUDA implementation.  One CTA per (sequence, head).
+ * argument combination of the reference call is without a CUDA implementation.
  *   base.snap_dtype must be SLOTSCAN_F32: kbuf, vbuf and obuf (B,NB,H,N) are float32 -- they are the checkpoints the
  *   backward replays from.  Any 1 <= DK, DV <= 128; N * (DK + DV + 8) floats must fit one CTA's shared memory
  *   (N <= 192 at 128 + 128).
  * slotscan_dense_fwd: addr (B,T,H) int32 = argmax of each token's address, kfin / vfin / ofin = the final state; each
  * of the four may be NULL.
- * slotscan_dense_bwd: needs the forward's kbuf, vbuf, obuf and scratch of slotscan_dense_bwd_scratch_bytes (G states
- * per (sequence, head)); dkbuf / dvbuf float32, either may be NULL.  Outputs as slotscan_hard_bwd. */
+ * slotscan_dense_bwd: needs the forward's kbuf, vbuf, obuf and scratch of slotscan_dense_bwd_scratch_bytes (soft,
+ * detached, N <= 256: per-token tables of as many sequences as 2 GiB hold, more sequences go through in turns; else G
+ * states per (sequence, head)); dkbuf / dvbuf float32, either may be NULL.  Outputs as slotscan_hard_bwd. */
 typedef struct {
     slotscan_params base;
     int32_t hard;           /* forward address: 1 = one-hot argmax, 0 = the softmax over the candidate rows */
