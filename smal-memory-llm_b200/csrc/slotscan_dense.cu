@@ -3,13 +3,14 @@
 // attached to the stored keys.  [reference: forward gqa25/slotkern_kvt.py:43-119, step adjoint :157-171 and
 // gqa25/slotkern_kvg.py:163-200 (stride-G replay backward); definition gqa25/slotkern_kv.py:66-123]
 //
-// Up to 256 rows: the forward and, for a soft detached address, the backward with the token chain reduced to scalars
+// Soft address, up to 256 rows: the forward and, where it is detached, the backward with the token chain reduced to scalars
 // (slotscan_dense_chain.cuh) and the row gradients block by block (slotscan_rowadj.cuh).  B = 4, T = 512, H = 12,
 // 192 x (64 + 64), G = 16, soft, detached, forward + backward: 35.2 ms token by token (5.9 + 29.9), 2.00 ms so (forward 0.92;
 // backward: tables 0.34, row gradients 0.42, query gradient 0.22, softmax adjoint 0.04).
-// The token-by-token kernels below take the rest: more rows than 256, or more shared memory than a CTA has beside the
-// chain's token buffers; and the backward of an attached address, where the gradient of the score of every token enters
-// the row gradients that the token before it needs, so that they are no longer linear in known factors.
+// The token-by-token kernels below take the rest: a hard address, whose backward has to find the forward's addresses again;
+// more rows than 256, or more shared memory than a CTA has beside the chain's token buffers; and the backward of an
+// attached address, where the gradient of the score of every token enters the row gradients that the token before it
+// needs, so that they are no longer linear in known factors.
 // One CTA per (sequence, head).  Forward: keys, values and occupancy resident in shared memory as float32
 // (N x (dk + dv) + N floats: 197 KB at 192 x (128 + 128)), four phases per token -- token vectors in, scores (a warp
 // per row), address (one warp: mask, argmax, softmax), write (all threads).  The pre-write state goes out every G
@@ -555,7 +556,7 @@ cudaError_t run_dense_split_bwd(const slotscan_params& p, const void* k, const v
     cudaError_t e;
     for (int bh0 = 0; bh0 < BH; bh0 += s.nbh) {
         const int nbh = std::min(s.nbh, BH - bh0);
-        DenseChainArgs C = {p, 0, k, q, v, gate, fr, temp, const_cast<float*>(kbuf), nullptr, const_cast<float*>(obuf), nullptr,
+        DenseChainArgs C = {p, k, q, v, gate, fr, temp, const_cast<float*>(kbuf), nullptr, const_cast<float*>(obuf), nullptr,
                             nullptr, nullptr, nullptr, as, sf, ki, ot, lim, bh0};
         if ((e = run_dense_chain<Tin, true>(C, nbh * NB, st)) != cudaSuccess) return e;
         RowAdjArgs R = {p.N, p.T, p.H, p.G, 0, p.hard_gate, as, nullptr, lim, gate, dp, bh0, nbh, row_adjoint_slices(p.N, p.DK),
@@ -603,8 +604,11 @@ extern "C" int slotscan_dense_fwd(const slotscan_dense_params* p, const void* k,
     if (!k || !v || !gate || !fr || !temp || !kbuf || !vbuf || !obuf) return SLOTSCAN_E_NULL;
     const slotscan_params& b = p->base;
     cudaStream_t st = (cudaStream_t)stream;
-    if (dense_chunk(b.N, b.DK, b.DV, true)) {
-        const DenseChainArgs C = {b, p->hard, k, q ? q : k, v, gate, fr, temp, kbuf, vbuf, obuf, addr, kfin, vfin, ofin,
+    // A hard address stays with the kernel whose arithmetic the backward repeats: dense_bwd_kernel finds the addresses again
+    // from rows it replays token by token, and the chain's recurrences and once-a-chunk rows resolve a tie between rows of
+    // one content (a key that recurs) otherwise, in the snapshots and, against the forward, in the gradients.
+    if (!p->hard && dense_chunk(b.N, b.DK, b.DV, true)) {
+        const DenseChainArgs C = {b, k, q ? q : k, v, gate, fr, temp, kbuf, vbuf, obuf, addr, kfin, vfin, ofin,
                                   nullptr, nullptr, nullptr, nullptr, nullptr, 0};
         return (int)(b.in_dtype == SLOTSCAN_F32 ? run_dense_chain<float, false>(C, b.B * b.H, st)
                                                 : run_dense_chain<__nv_bfloat16, false>(C, b.B * b.H, st));

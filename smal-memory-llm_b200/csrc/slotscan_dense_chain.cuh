@@ -1,4 +1,4 @@
-// The general scan with its token chain reduced to scalars.
+// The general scan under a soft address with its token chain reduced to scalars.
 //
 // Within a chunk of C tokens every score is a linear recurrence of dot products that are known at its start: with
 // u_n(j) = <K_n, q_j>, e_n(j) = <K_n, k_j> and s_n = |K_n|^2 of the row as it stands, a write of token t with weight w does
@@ -39,10 +39,6 @@ __device__ __forceinline__ double dc_rcp(double s) {         // hardware approxi
 }
 __device__ __forceinline__ void dc_bar_rows(int threads) { asm volatile("bar.sync 1, %0;" ::"r"(threads) : "memory"); }
 __device__ __forceinline__ void dc_bar_help() { asm volatile("bar.sync 2, %0;" ::"n"(DC_HELP) : "memory"); }
-__device__ __forceinline__ unsigned long long dc_key(double z) {       // order-preserving, -0 = +0
-    const long long b = __double_as_longlong(z + 0.0);
-    return (unsigned long long)(b ^ ((b >> 63) | (long long)0x8000000000000000ull));
-}
 __device__ __forceinline__ float ldtok(const float* p) { return *p; }
 __device__ __forceinline__ float ldtok(const __nv_bfloat16* p) { return __bfloat162float(*p); }
 __device__ __forceinline__ void sttok(float* p, float v) { *p = v; }
@@ -69,7 +65,6 @@ __device__ __forceinline__ void dense_load_rows(float* K, const float* src, int 
 
 struct DenseChainArgs {
     slotscan_params p;
-    int hard;
     const void *k, *q, *v;
     const float *gate, *fr, *temp;
     // forward: snapshots, log and final state out.  tables: kbuf / obuf in
@@ -166,13 +161,13 @@ __global__ void __launch_bounds__(DC_NMAX + DC_HELP) dense_chain_kernel(const De
     // the values of a chunk whose tokens fetch_v has loaded, first token at place ph of block jb; and its addresses
     auto values = [&](int bf, int t0, int cn, int ph, int jb) {
         const float* wr = wbuf + bf * C * N4;
-        if (!A.hard && A.addr != nullptr && ht < cn) {
+        if (A.addr != nullptr && ht < cn) {
             int2 m = s_arg[(bf * C + ht) * 8];
             for (int w = 1; w < RW; w++) { const int2 x = s_arg[(bf * C + ht) * 8 + w]; if ((unsigned)x.x > (unsigned)m.x) m = x; }
             A.addr[((size_t)b * T + t0 + ht) * H + h] = m.y;
         }
         if (hg >= hper) return;
-        bool odd = A.hard != 0;                              // a row a token does not write must not see it: only an infinite
+        bool odd = false;                                    // a row a token does not write must not see it: only an infinite
 #pragma unroll
         for (int j = 0; j < C; j++) odd |= !(fabsf(xn[j]) <= 3e38f);     // or NaN value would tell
         const f32x2 one = pack2(1.f, 1.f), minus = pack2(-1.f, -1.f);
@@ -282,14 +277,12 @@ __global__ void __launch_bounds__(DC_NMAX + DC_HELP) dense_chain_kernel(const De
                         const double kinv = ns > 1e-12 ? rsqrt(ns) : 1e6;
                         const double s = (u[j] * kinv * qi[j]) * temp;
                         const double z = s - fr * (p.occ_bin ? (o >= (double)eps ? 1.0 : 0.0) : o);
-                        double* xs = ex + par * 64;          // [0..7] sums, [8..15] maxima, [16..23] argmax keys, [24..31] their rows, [32] e, [33] o of row fe
+                        double* xs = ex + par * 64;          // [0..7] sums, [8..15] maxima, [16] e, [17] o of row fe
                         par ^= 1;
-                        double E = 0.0;
                         // the softmax's shift: a bound of every z where that cannot under- or overflow, the maximum else
                         double shift = fabs(temp) + fmax(0.0, -fr);
-                        const bool soft = TABLES || !A.hard;
                         const bool bounded = 2.0 * fabs(temp) + fabs(fr) < 600.0 && (p.occ_bin || !wild);
-                        if (soft && !bounded) {
+                        if (!bounded) {
                             double m = cand ? z : -INFINITY;
 #pragma unroll
                             for (int off = 16; off > 0; off >>= 1) m = fmax(m, __shfl_xor_sync(FULL, m, off));
@@ -298,60 +291,34 @@ __global__ void __launch_bounds__(DC_NMAX + DC_HELP) dense_chain_kernel(const De
                             shift = xs[8];
                             for (int i = 1; i < RW; i++) shift = fmax(shift, xs[8 + i]);
                         }
-                        if (soft) {
-                            E = cand ? exp(z - shift) : 0.0;
-                            double se = E;
+                        const double E = cand ? exp(z - shift) : 0.0;
+                        double sw = E;
 #pragma unroll
-                            for (int off = 16; off > 0; off >>= 1) se += __shfl_xor_sync(FULL, se, off);
-                            if (lane == 0) xs[warp] = se;
-                        }
-                        if (!TABLES && A.hard) {             // the address: first row of the largest z
-                            const unsigned long long key = (cand && z > -INFINITY) ? dc_key(z) : 0ull;
-                            const unsigned hi = (unsigned)(key >> 32), mh = __reduce_max_sync(FULL, hi);
-                            const unsigned ml = __reduce_max_sync(FULL, hi == mh ? (unsigned)key : 0u);
-                            const unsigned who = __ballot_sync(FULL, hi == mh && (unsigned)key == ml);
-                            if (lane == 0) {
-                                reinterpret_cast<unsigned long long*>(xs)[16 + warp] = ((unsigned long long)mh << 32) | ml;
-                                reinterpret_cast<int*>(xs + 24)[warp] = warp * 32 + __ffs(who) - 1;
-                            }
-                        }
-                        if (n == fe && live) { xs[32] = E; xs[33] = o; }
+                        for (int off = 16; off > 0; off >>= 1) sw += __shfl_xor_sync(FULL, sw, off);
+                        if (lane == 0) xs[warp] = sw;
+                        if (n == fe && live) { xs[16] = E; xs[17] = o; }
                         dc_bar_rows(rows_t);
-                        int am = 0;
-                        if (!TABLES && A.hard) {
-                            const unsigned long long* ks = reinterpret_cast<const unsigned long long*>(xs) + 16;
-                            unsigned long long bk = ks[0];
-                            int bw = 0;
-#pragma unroll
-                            for (int i = 1; i < 8; i++) if (ks[i] > bk) { bk = ks[i]; bw = i; }
-                            am = bk == 0ull ? min(fe, N - 1) : reinterpret_cast<const int*>(xs + 24)[bw];   // all NaN: the last candidate
-                            if (tid == 0 && A.addr != nullptr) A.addr[((size_t)b * T + t0 + j) * H + h] = am;
-                        }
-                        double si = 0.0;
-                        if (soft) {
-                            const double2 e0 = *reinterpret_cast<const double2*>(xs), e1 = *reinterpret_cast<const double2*>(xs + 2);
-                            const double2 e2 = *reinterpret_cast<const double2*>(xs + 4), e3 = *reinterpret_cast<const double2*>(xs + 6);
-                            const double se = ((e0.x + e0.y) + (e1.x + e1.y)) + ((e2.x + e2.y) + (e3.x + e3.y));
-                            si = bounded ? dc_rcp(se) : 1.0 / se;
-                        }
-                        const float as = (float)(E * si);
+                        const double2 e0 = *reinterpret_cast<const double2*>(xs), e1 = *reinterpret_cast<const double2*>(xs + 2);
+                        const double2 e2 = *reinterpret_cast<const double2*>(xs + 4), e3 = *reinterpret_cast<const double2*>(xs + 6);
+                        const double se = ((e0.x + e0.y) + (e1.x + e1.y)) + ((e2.x + e2.y) + (e3.x + e3.y));
+                        const double si = bounded ? dc_rcp(se) : 1.0 / se;
+                        const float a = (float)(E * si);
                         if (TABLES) {
                             if (live) {
                                 const size_t at = ((size_t)lb * T + t0 + j) * N + n;
-                                A.as[at] = as;
+                                A.as[at] = a;
                                 A.sf[at] = cand ? (float)s : 0.f;
                                 A.ki[at] = (float)kinv;
                                 A.ot[at] = (float)o;
                             }
                         }
-                        const float a = A.hard ? (cand && n == am ? 1.f : 0.f) : as;
                         const double wd0 = (double)g * (double)a;
                         if (fe < N) {                        // only the first empty row can become occupied
-                            const float af = A.hard ? (fe == am ? 1.f : 0.f) : (float)(xs[32] * si);
-                            const double wf = (double)g * (double)af, of = xs[33];
+                            const float af = (float)(xs[16] * si);
+                            const double wf = (double)g * (double)af, of = xs[17];
                             if ((af != 0.f ? (1.0 - wf) * of + wf : of) >= (double)eps) fe++;
                         }
-                        if (!TABLES && !A.hard && A.addr != nullptr) {       // soft: the argmax of the address, for the log
+                        if (!TABLES && A.addr != nullptr) {      // the argmax of the address, for the log
                             const unsigned ak = a > 0.f ? __float_as_uint(a) : 0u, mk = __reduce_max_sync(FULL, ak);
                             const unsigned who = __ballot_sync(FULL, ak == mk);
                             if (lane == 0) s_arg[(bf * C + j) * 8 + warp] = make_int2((int)mk, warp * 32 + __ffs((int)who) - 1);

@@ -158,3 +158,40 @@ def test_general_scan_edges(case, dtype):
         # q = None, bf16: dk is the sum of two bf16-rounded parts, three roundings in all
         band = (3 * 2.0 ** -8 if not sepq else 2.0 ** -8) if dtype == torch.bfloat16 and n in ("dk", "dq", "dv") else 1e-4
         assert rel_to_max(out[n].reshape(gr[n].shape), gr[n]) < band or np.abs(gr[n]).max() < 1e-9, n
+
+
+@pytest.mark.parametrize("gates", ["ones", "01", "sigmoid"])
+@pytest.mark.parametrize("N,D,G", [(32, 64, 16), (70, 64, 5), (24, 32, 8)])
+def test_hard_attached_recurring_keys(N, D, G, gates):
+    """A hard address over keys that recur, as text has them: rows of one content tie.  The backward finds the addresses again
+    from the snapshots, so it must land on the forward's: the values' gradient is a linear function of the addresses, here
+    those that the forward returned, in 64 bits (float32 sums of at most T terms: 1e-5 of the largest is far above them).
+    With gates of 0 and 1 a row holds a key exactly, ties are exact, and the first of the rows is taken."""
+    from slotscan_b200 import ops
+    B, T, H = 8, 64, 2
+    gen = torch.Generator().manual_seed(5)
+    words = torch.randn(12, H, D, generator=gen)
+    k = words[torch.randint(0, 12, (B, T), generator=gen)]
+    gate = dict(ones=torch.ones(B, T, H), sigmoid=torch.sigmoid(torch.randn(B, T, H, generator=gen)))
+    gate["01"] = (torch.rand(B, T, H, generator=gen) < 0.85).float()
+    gate, v = gate[gates], torch.randn(B, T, H, D, generator=gen)
+    fr = 24.0 * torch.rand(B, T, H, generator=gen)          # up to 1.5 times the sharpness: a free row often wins over a match
+    x = [t.to(DEV) for t in (k, v, gate, fr)]
+    x[1].requires_grad_()
+    out = ops.run_dense_fwd(x[0], None, x[1], x[2], x[3], torch.full((1,), 16.0, device=DEV), N, G, True, False, 1e-4, False, True)
+    wv = torch.randn(out[1].shape, generator=gen).to(DEV)
+    dv, = torch.autograd.grad([out[1]], [x[1]], [wv])
+    a = torch.nn.functional.one_hot(out[3].long(), N).double()
+    v64, V, snaps = x[1].detach().double().requires_grad_(), torch.zeros(B, H, N, D, device=DEV, dtype=torch.float64), []
+    for t in range(T):
+        if t % G == 0:
+            snaps.append(V)
+        w = (x[2].double()[:, t].unsqueeze(-1) * a[:, t]).unsqueeze(-1)
+        V = (1 - w) * V + w * v64[:, t].unsqueeze(2)
+    snaps = torch.stack(snaps, 1)
+    assert (out[1] - snaps).abs().max() < 1e-5
+    want, = torch.autograd.grad([snaps], [v64], [wv.double()])
+    assert rel_to_max(dv.cpu().numpy(), want.cpu().numpy()) < 1e-5
+    if gates != "sigmoid":
+        ref = O.scan_fwd(k, v, gate, fr, N=N, temp=16.0, G=G, hard=True, occ_bin=True)
+        assert np.array_equal(out[3].cpu().numpy(), ref["addr"])
