@@ -8,6 +8,7 @@ import ctypes
 from typing import Optional, Tuple
 
 import torch
+from torch.utils._device import DeviceContext
 
 from . import _lib
 
@@ -43,16 +44,29 @@ class _Here:
             self.guard.__exit__(*a)
 
 
+_is_batched = torch._C._functorch.is_legacy_batchedtensor
+
+
+def _watched():
+    """A mode, tracer or profiler that has to see the call.  The mode of `torch.device` and `torch.set_default_device` concerns
+    factory functions alone."""
+    if torch.compiler.is_compiling() or torch.jit.is_tracing() or torch._C._len_torch_dispatch_stack() > 0 or \
+            torch._C._functorch.peek_interpreter_stack() is not None or torch._C._autograd._profiler_enabled():
+        return True
+    modes = torch._C._len_torch_function_stack()
+    return modes > 0 and any(type(torch._C._get_function_stack_at(i)) is not DeviceContext for i in range(modes))
+
+
 def plain_call(*ts):
-    """True when nothing looks over this call's shoulder: ordinary tensors, no tracing, compiling, fake or functional mode.
+    """True when nothing looks over this call's shoulder (`_watched`) and its tensors are ordinary ones: of no other class, not
+    batched by the older vmap (`is_grads_batched`, `jacobian(vectorize=True)`), not a lazy negation.
     The custom op's own wrapping costs about 80 us of host time per call and direction, as much as the kernels of a small
     call take; such a call goes to the same implementation without it, and through an autograd.Function with the same
     backward when a gradient is wanted.  Everything else takes the registered op."""
-    if torch.compiler.is_compiling() or torch.jit.is_tracing() or torch._C._len_torch_dispatch_stack() > 0 or \
-            torch._C._functorch.peek_interpreter_stack() is not None:
+    if _watched():
         return False
     for t in ts:
-        if t is not None and type(t) is not torch.Tensor and type(t) is not torch.nn.Parameter:
+        if t is not None and (type(t) is not torch.Tensor and type(t) is not torch.nn.Parameter or _is_batched(t) or t.is_neg()):
             return False
     return True
 
