@@ -274,7 +274,7 @@ __global__ void __launch_bounds__(DC_NMAX + DC_HELP) dense_chain_kernel(const De
                         const double fr = (double)frf;
                         wild |= !(g >= 0.f && g <= 1.f);
                         const bool cand = live && n <= fe;
-                        const double kinv = ns > 1e-12 ? rsqrt(ns) : 1e6;
+                        const double kinv = ns <= 1e-12 ? 1e6 : rsqrt(ns);     // NaN stays NaN
                         const double s = (u[j] * kinv * qi[j]) * temp;
                         const double z = s - fr * (p.occ_bin ? (o >= (double)eps ? 1.0 : 0.0) : o);
                         double* xs = ex + par * 64;          // [0..7] sums, [8..15] maxima, [16] e, [17] o of row fe
@@ -302,7 +302,7 @@ __global__ void __launch_bounds__(DC_NMAX + DC_HELP) dense_chain_kernel(const De
                         const double2 e2 = *reinterpret_cast<const double2*>(xs + 4), e3 = *reinterpret_cast<const double2*>(xs + 6);
                         const double se = ((e0.x + e0.y) + (e1.x + e1.y)) + ((e2.x + e2.y) + (e3.x + e3.y));
                         const double si = bounded ? dc_rcp(se) : 1.0 / se;
-                        const float a = (float)(E * si);
+                        const float a = cand ? (float)(E * si) : 0.f;        // also where the sum is not finite
                         if (TABLES) {
                             if (live) {
                                 const size_t at = ((size_t)lb * T + t0 + j) * N + n;
@@ -326,12 +326,14 @@ __global__ void __launch_bounds__(DC_NMAX + DC_HELP) dense_chain_kernel(const De
                         if (a != 0.f) o = (1.0 - wd0) * o + wd0;
                         w[j] = g * a;
                         if (live) wr[j * N4 + n] = w[j];
-                        const double wd = (double)w[j], om = 1.0 - wd;
-                        ns = fma(om * om, ns, fma(2.0 * wd * om, e[j], wd * wd * Cm[j * C + j]));
+                        if (w[j] != 0.f) {                   // a row that token j does not write never sees its key, finite or not
+                            const double wd = (double)w[j], om = 1.0 - wd;
+                            ns = fma(om * om, ns, fma(2.0 * wd * om, e[j], wd * wd * Cm[j * C + j]));
 #pragma unroll
-                        for (int i = j + 1; i < C; i++) {
-                            u[i] = fma(wd, Bm[j * C + i] - u[i], u[i]);
-                            e[i] = fma(wd, Cm[j * C + i] - e[i], e[i]);
+                            for (int i = j + 1; i < C; i++) {
+                                u[i] = fma(wd, Bm[j * C + i] - u[i], u[i]);
+                                e[i] = fma(wd, Cm[j * C + i] - e[i], e[i]);
+                            }
                         }
                     } else if (live) {
                         wr[j * N4 + n] = 0.f;

@@ -195,3 +195,41 @@ def test_hard_attached_recurring_keys(N, D, G, gates):
     if gates != "sigmoid":
         ref = O.scan_fwd(k, v, gate, fr, N=N, temp=16.0, G=G, hard=True, occ_bin=True)
         assert np.array_equal(out[3].cpu().numpy(), ref["addr"])
+
+
+def test_soft_scan_isolates_rows_a_token_does_not_write():
+    """An infinite key reaches the rows its token writes and no others.  With gate 0 it writes none: the scan is the one of a
+    finite key, bit for bit, wherever in a chunk the token lies.  With an open gate the candidate rows are lost, and the rows
+    above them stay empty, as in the token-by-token kernel (which takes more than 256 rows)."""
+    from slotscan_b200 import ops
+    B, T, H, D, G = 2, 21, 2, 32, 16
+    inp = make_inputs("fill", B, T, H, D, D, seed=11)
+    temp = torch.full((1,), 16.0, device=DEV)
+
+    def go(k, gate, N):
+        x = [t.to(DEV) for t in (k, inp["q"], inp["v"], gate, inp["fr"])]
+        return ops.run_dense_fwd(*x, temp, N, G, False, False, 1e-4, True, True)
+    for t in (0, 3, 7, 9):
+        gate, bad = inp["gate"].clone(), inp["k"].clone()
+        gate[:, t], bad[:, t, :, 3] = 0.0, float("inf")
+        for a, b in zip(go(bad, gate, 40), go(inp["k"], gate, 40)):
+            assert torch.isfinite(a).all() and torch.equal(a, b), t
+        few, many = go(bad, inp["gate"], 40), go(bad, inp["gate"], 257)
+        for i in (0, 1):                                     # snapshots of keys and values
+            assert torch.equal(torch.isfinite(few[i]).all(-1), torch.isfinite(many[i][:, :, :, :40]).all(-1)), t
+        assert not torch.isfinite(few[4]).all() and (few[4][:, T:] == 0).all()
+
+
+def test_hard_scan_isolates_rows_a_token_does_not_write():
+    """The same for a hard address, attached: only the row that took the infinite key is lost, and the tokens after it find
+    their addresses among the others, as the oracle does."""
+    from slotscan_b200 import ops
+    B, T, H, N, D, G = 2, 24, 2, 20, 32, 16
+    inp = make_inputs("fill", B, T, H, D, D, seed=11)
+    bad = inp["k"].clone()
+    bad[0, 9, 0, 3] = float("inf")
+    x = [t.to(DEV) for t in (bad, inp["q"], inp["v"], inp["gate"], inp["fr"])]
+    out = ops.run_dense_fwd(*x, torch.full((1,), 16.0, device=DEV), N, G, True, False, 1e-4, False, True)
+    ref = O.scan_fwd(bad, inp["v"], inp["gate"], inp["fr"], N=N, temp=16.0, G=G, hard=True, q=inp["q"], occ_bin=True)
+    assert np.array_equal(out[3].cpu().numpy(), ref["addr"])
+    assert np.array_equal(np.isfinite(out[4].cpu().numpy().reshape(ref["kfin"].shape)), np.isfinite(ref["kfin"]))
