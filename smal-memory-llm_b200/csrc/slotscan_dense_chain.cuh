@@ -217,12 +217,15 @@ __global__ void __launch_bounds__(DC_NMAX + DC_HELP) dense_chain_kernel(const De
     if (TABLES && row) {
         int* s_fe = reinterpret_cast<int*>(ex);
         const unsigned free_rows = __ballot_sync(FULL, !live || (float)o < eps);
-        if (lane == 0) s_fe[warp] = free_rows ? warp * 32 + __ffs(free_rows) - 1 : BIGI;
+        const unsigned unbounded = __ballot_sync(FULL, live && !(o >= 0.0 && o <= 1.0));
+        if (lane == 0) { s_fe[warp] = free_rows ? warp * 32 + __ffs(free_rows) - 1 : BIGI; s_fe[8 + warp] = unbounded != 0u; }
     }
+    bool wild = false;               // a gate outside [0, 1] so far (tables: one that shows in the block's occupancies, or later)
     __syncthreads();
     if (TABLES && row) {
+        const int* s_fe = reinterpret_cast<const int*>(ex);
         fe = BIGI;
-        for (int w = 0; w < RW; w++) fe = min(fe, reinterpret_cast<int*>(ex)[w]);
+        for (int w = 0; w < RW; w++) { fe = min(fe, s_fe[w]); wild |= s_fe[8 + w] != 0; }
         fe = min(fe, N);
         if (tid == 0) A.lim[(size_t)lb * NB + jb0] = min(fe, N - 1);
     }
@@ -231,7 +234,6 @@ __global__ void __launch_bounds__(DC_NMAX + DC_HELP) dense_chain_kernel(const De
     if (row) dc_bar_rows(rows_t);
     if (!TABLES && !row) fetch_v(0, min(C, min(G, T)));
 
-    bool wild = false;                                       // a gate outside [0, 1] so far: occupancies are not bounded by 1
     int par = 0, c = 0, pt0 = 0, pcn = 0, pph = 0, pjb = 0;  // parity of the exchange, chunk, the chunk before
     for (int jb = jb0; jb < jb1; jb++) {
         const int tb = jb * G, bn = min(G, T - tb);
@@ -280,6 +282,7 @@ __global__ void __launch_bounds__(DC_NMAX + DC_HELP) dense_chain_kernel(const De
                         double* xs = ex + par * 64;          // [0..7] sums, [8..15] maxima, [16] e, [17] o of row fe
                         par ^= 1;
                         // the softmax's shift: a bound of every z where that cannot under- or overflow, the maximum else
+                        // (after a wild gate the occupancies are not bounded by 1)
                         double shift = fabs(temp) + fmax(0.0, -fr);
                         const bool bounded = 2.0 * fabs(temp) + fabs(fr) < 600.0 && (p.occ_bin || !wild);
                         if (!bounded) {

@@ -233,3 +233,31 @@ def test_hard_scan_isolates_rows_a_token_does_not_write():
     ref = O.scan_fwd(bad, inp["v"], inp["gate"], inp["fr"], N=N, temp=16.0, G=G, hard=True, q=inp["q"], occ_bin=True)
     assert np.array_equal(out[3].cpu().numpy(), ref["addr"])
     assert np.array_equal(np.isfinite(out[4].cpu().numpy().reshape(ref["kfin"].shape)), np.isfinite(ref["kfin"]))
+
+
+@pytest.mark.parametrize("N,fr", [(1, 400.0), (4, -500.0)])
+def test_soft_scan_gate_beyond_one_in_an_early_block(N, fr):
+    """One gate of 3 at the first token leaves an occupancy far above 1, and the penalty on o itself then puts the scores of
+    every later block where only a softmax about its maximum is finite: forward, and backward from the snapshots of blocks
+    whose own gates are ordinary."""
+    import slotscan_b200 as S
+    B, T, H, D, G = 1, 20, 2, 16, 4
+    gen = torch.Generator().manual_seed(2)
+    r = lambda *s: torch.randn(*s, generator=gen)
+    k, q, v, gate = r(B, T, H, D), r(B, T, H, D), r(B, T, H, D), torch.full((B, T, H), 0.05)
+    gate[:, 0] = 3.0
+    f = torch.tensor([fr])
+    kw = dict(N=N, temp=16.0, G=G, hard=False, q=q, occ_bin=False)
+    ref = O.scan_fwd(k, v, gate, f, **kw)
+    wk, wv = r(*ref["kbuf"].shape), r(*ref["vbuf"].shape)
+    gr = O.scan_bwd(k, v, gate, f, dkbuf=wk.numpy(), dvbuf=wv.numpy(), detach_addr=True, **kw)
+    x = [t.to(DEV).requires_grad_() for t in (k, q, v, gate, f)]
+    kb, vb = S.kv_scan_g(x[0], x[2], x[3], x[4], N, 16.0, G=G, hard=False, detach_addr=True, q=x[1], occ_bin=False)
+    for a, n in ((kb, "kbuf"), (vb, "vbuf")):
+        okc, worst = allclose_report(a.detach().cpu().numpy(), ref[n], 1e-5, 1e-5)
+        assert okc, (n, worst)
+    got = torch.autograd.grad([kb, vb], x, [wk.to(DEV), wv.to(DEV)])
+    for a, n in zip(got, ("dk", "dq", "dv", "dgate", "dfr")):
+        a = a.cpu().numpy().reshape(gr[n].shape)
+        assert np.isfinite(a).all(), n
+        assert rel_to_max(a, gr[n]) < 1e-4 or np.abs(gr[n]).max() < 1e-9, n
