@@ -156,13 +156,11 @@ int slotscan_hard_bwd_q(const slotscan_params* p, const void* k, const void* q, 
 /* The same backward for callers that cannot supply scratch memory.  [No counterpart in the reference: its host side
  * always allocates through torch.]  Meant for hosts whose device memory is already fully assigned (a server that
  * handed everything to its own arena, a binding with no device allocator) or that must not make a synchronising
- * allocation on this path.  The table D[t,n] and the partial sums live in ONE fixed array of
- * SLOTSCAN_NOALLOC_SCRATCH_BYTES inside the library (each GPU that loads the library holds that much until the process
- * exits).  Arguments and results are those of slotscan_hard_bwd without `scratch`; results are bit-identical to it.
- *   - Limit: the two D tables, the partial sums and a 32-row next-write table must fit the capacity, i.e. roughly
- *     B*H*T*N <= 1 M table entries; beyond that the call returns SLOTSCAN_E_TOO_LARGE and launches nothing.  (For the last
- *     2 % below the limit the next-write table of all rows has no room: sequences with more than 32 rows in use then take
- *     another kernel than slotscan_hard_bwd's, with the sums in another order.)
+ * allocation on this path.  The table D[t,n] and the partial sums live in ONE fixed array inside the library (1.5 times
+ * SLOTSCAN_NOALLOC_SCRATCH_BYTES; each GPU that loads the library holds that much until the process exits).  Arguments and results are those of slotscan_hard_bwd without `scratch`; results are bit-identical to it.
+ *   - Limit: the two D tables, the partial sums and a 32-row next-write table must fit SLOTSCAN_NOALLOC_SCRATCH_BYTES, i.e.
+ *     roughly B*H*T*N <= 1 M table entries; beyond that the call returns SLOTSCAN_E_TOO_LARGE and launches nothing.  (The
+ *     rest of the array holds the next-write table of all rows, which slotscan_hard_bwd_scratch_bytes counts too.)
  *   - The call itself allocates no device memory and frees none.
  *   - On EVERY call the current device (cudaGetDevice) must be the one that owns `stream` and all the pointers: the
  *     array used is the current device's copy.  Inputs found on another device are refused with SLOTSCAN_E_MODE.

@@ -459,7 +459,12 @@ extern "C" int slotscan_profile_read(slotscan_kernel_time* out, int cap) {
 //
 // The array's name is only a host-side handle for the symbol; the device address a kernel can use comes from
 // cudaGetSymbolAddress, asked once per device with that device current.
-static __device__ __align__(256) unsigned char g_fixed_scratch[SLOTSCAN_NOALLOC_SCRATCH_BYTES];
+//
+// SLOTSCAN_NOALLOC_SCRATCH_BYTES is what a problem's scratch may take without the next-write table of all rows.  That table
+// (an entry per 32 tokens and row) is at most half of the two D tables (an entry per token and row each, equal to it in size
+// where T = 1), so with half as much again every problem that is accepted runs the kernels of slotscan_hard_bwd.
+constexpr size_t FIXED_SCRATCH = (size_t)SLOTSCAN_NOALLOC_SCRATCH_BYTES * 3 / 2 + 256;
+static __device__ __align__(256) unsigned char g_fixed_scratch[FIXED_SCRATCH];
 static void* g_fixed_scratch_addr[MAX_DEVICES] = {nullptr};
 static std::mutex g_fixed_scratch_mu;
 
@@ -473,7 +478,7 @@ extern "C" int slotscan_hard_bwd_noalloc(const slotscan_params* p, const void* k
     if (rc) return rc;
     size_t off_part, off_vend, least, total;
     bwd_scratch_layout(p, &off_part, &off_vend, &least, &total);
-    if (least > (size_t)SLOTSCAN_NOALLOC_SCRATCH_BYTES) return SLOTSCAN_E_TOO_LARGE;
+    if (least > (size_t)SLOTSCAN_NOALLOC_SCRATCH_BYTES || total > FIXED_SCRATCH) return SLOTSCAN_E_TOO_LARGE;
     int dev = -1;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return (int)e;
@@ -499,7 +504,6 @@ extern "C" int slotscan_hard_bwd_noalloc(const slotscan_params* p, const void* k
     // The array keeps the previous call's contents.  Every D[t,n] and next-write entry that is read was written earlier
     // in the same call; the partial-sum table, whose unused slots must read as zero, is cleared by the call itself
     // (cudaMemsetAsync on the caller's stream, inside slotscan_hard_bwd).
-    return slotscan_hard_bwd(p, k, q, v, gate, fr, temp, log, dkbuf, dvbuf, scratch, (size_t)SLOTSCAN_NOALLOC_SCRATCH_BYTES,
-                             dk, dq, dv, dgate, dfr, dtemp, stream);
+    return slotscan_hard_bwd(p, k, q, v, gate, fr, temp, log, dkbuf, dvbuf, scratch, FIXED_SCRATCH, dk, dq, dv, dgate, dfr, dtemp, stream);
 }
 

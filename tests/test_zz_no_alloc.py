@@ -29,7 +29,7 @@ def _forward(inp, N, G):
     return (k, q, v, g, fr), lg
 
 
-def _both_backwards(tensors, lg, N, G, seed):
+def _both_backwards(tensors, lg, N, G, seed, near_limit=False):
     from slotscan_b200 import _lib
     L = _lib.lib()
     k, q, v, g, fr = tensors
@@ -47,7 +47,7 @@ def _both_backwards(tensors, lg, N, G, seed):
                 torch.full_like(g, float("nan")), torch.full_like(fr, float("nan")), torch.full((1,), float("nan"), device=DEV)]
 
     nbytes = L.slotscan_hard_bwd_scratch_bytes(ctypes.byref(p))
-    assert nbytes <= L.slotscan_hard_bwd_noalloc_capacity()
+    assert near_limit or nbytes <= L.slotscan_hard_bwd_noalloc_capacity()
     scratch = torch.empty(nbytes, dtype=torch.uint8, device=DEV)
     a = outputs()
     rc = L.slotscan_hard_bwd(ctypes.byref(p), _ptr(k), _ptr(q), _ptr(v), _ptr(g), _ptr(fr), _ptr(temp), ctypes.byref(log),
@@ -73,6 +73,19 @@ def test_noalloc_backward_matches_ordinary_backward_twice():
         for name, x, y in zip(("dk", "dq", "dv", "dgate", "dfr", "dtemp"), a, b):
             assert torch.isfinite(y).all(), (call, name)
             assert torch.equal(x, y), (call, name, (x - y).abs().max().item())
+
+
+def test_noalloc_backward_at_its_limit():
+    """The last problem sizes that are accepted (the tables of slotscan_hard_bwd_scratch_bytes are then larger than the
+    capacity), with more than 32 rows in use, where the next-write table of all rows decides which kernel runs."""
+    from slotscan_b200 import _lib
+    L, N, G = _lib.lib(), 192, 8
+    tensors, lg = _forward(make_inputs("fill", 17, 64, 5, 128, 128, seed=23), N, G)
+    p = _lib.Params(17, 64, 5, N, 128, 128, G, 0, 1, 1, _lib.F32, _lib.F32, 1e-4)
+    assert L.slotscan_hard_bwd_scratch_bytes(ctypes.byref(p)) > L.slotscan_hard_bwd_noalloc_capacity()
+    assert (lg["tfirst"][:, 33] < 64).any()
+    for x, y in zip(*_both_backwards(tensors, lg, N, G, seed=5, near_limit=True)):
+        assert torch.isfinite(y).all() and torch.equal(x, y)
 
 
 def test_noalloc_backward_refuses_what_does_not_fit():
