@@ -43,11 +43,17 @@ __device__ __forceinline__ int read_rows_in_use(const uint8_t* v, int N) {
     }
     return hv;
 }
-// Which snapshots a CTA of the two kernels below works on.  On its own: one, blockIdx.x.  Beside the tensor-core kernel
-// (SPARSE: the snapshots with at most `rows` rows in use) most are not its own, and a launch of a CTA per snapshot to
-// find that out took longer than the work (B = 32, T = 1024, every slot in use: 0.11 ms forward, 0.16 ms backward; now
-// 0.08, most of it the 4 % of snapshots that are its own, and 0.04): a grid that fits the machine looks the snapshots
-// over, one per warp at a time.
+// true if a row from `rows` on is valid; warp-collective, all loads in flight
+__device__ __forceinline__ bool read_row_beyond(const uint8_t* v, int N, int rows) {
+    bool any = false;
+#pragma unroll 8
+    for (int n = rows + (threadIdx.x & 31); n < N; n += 32) any |= v[n] != 0;
+    return __any_sync(FULL, any);
+}
+// Which snapshots a CTA of the backward works on.  On its own: one, blockIdx.x.  Beside the tensor-core kernel (SPARSE: the
+// snapshots without a row in use, at the start of a sequence) nearly all are not its own, and a launch of a CTA per snapshot
+// to find that out took longer than the work (B = 32, T = 1024, every slot in use: 0.16 ms; now 0.04): a grid that fits the
+// machine looks the snapshots over, one per warp at a time.
 template <bool SPARSE, typename F>
 __device__ __forceinline__ void read_each_snapshot(const uint8_t* valid, int N, long long total, int rows, F work) {
     if constexpr (!SPARSE) {
@@ -73,8 +79,12 @@ __device__ __forceinline__ void read_each_snapshot(const uint8_t* valid, int N, 
     }
 }
 
+// SPARSE: beside the tensor-core kernel, for the snapshots with at most RM_SPARSE_ROWS rows in use.  Those can be few (a memory
+// that has filled up) or all (few slots in use), so a CTA per snapshot it is, and a warp of another kernel's snapshot leaves
+// after one look at the rows beyond.  64 sequences of 144 tokens, 6 heads, ~55 rows in use, write and read: 511 us; 717 when CTAs
+// that fit the machine walked the snapshots, a few each, one after another.  B = 32, T = 1024, every slot in use: as fast as those.
 template <typename Tq, typename Tsn, bool SPARSE>
-__global__ void __launch_bounds__(RD_THREADS, SPARSE ? 8 : 0) read_fwd_kernel(const slotscan_read_params p, const Tq* __restrict__ qr,
+__global__ void __launch_bounds__(RD_THREADS) read_fwd_kernel(const slotscan_read_params p, const Tq* __restrict__ qr,
                                                              const float* __restrict__ sharp,
                                                              const Tsn* __restrict__ kbuf, const Tsn* __restrict__ vbuf,
                                                              const float* __restrict__ kinv,
@@ -86,7 +96,10 @@ __global__ void __launch_bounds__(RD_THREADS, SPARSE ? 8 : 0) read_fwd_kernel(co
     float* s_ki = rsm + N;                                     // [N] their kinv
     float* s_sc = rsm + ((2 * N + 3) & ~3);                    // [warps][N][4] logits, then attention weights (16-byte aligned)
     __shared__ int s_nv;
-    read_each_snapshot<SPARSE>(valid, N, (long long)p.B * NB * H, RM_SPARSE_ROWS, [&](const int so) {   // (b * NB + nb) * H + h
+    if (SPARSE && read_row_beyond(valid + (size_t)blockIdx.x * N, N, RM_SPARSE_ROWS)) return;
+    // a function of its own: written straight into the kernel it comes out with 56 registers in place of 64 and other loads, and a
+    // decode step over eight full float32 memories takes 210 us in place of 160
+    auto work = [&](const int so) {                            // (b * NB + nb) * H + h
     const int h = so % H, nb = (so / H) % NB, b = so / (H * NB);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
 
@@ -195,11 +208,12 @@ __global__ void __launch_bounds__(RD_THREADS, SPARSE ? 8 : 0) read_fwd_kernel(co
         }
         __syncwarp();
     }
-    });
+    };
+    work((int)blockIdx.x);
 }
 
-// a CTA per snapshot, or (sparse_only) what fits the machine beside `smem` bytes and 64 registers a thread each: one wave, or
-// the snapshots would be dealt to CTAs that start when the others have finished theirs
+// backward: a CTA per snapshot, or (sparse_only) what fits the machine beside `smem` bytes and 64 registers a thread each: one
+// wave, or the snapshots would be dealt to CTAs that start when the others have finished theirs
 static unsigned read_grid(int snapshots, size_t smem, int sparse_only) {
     if (!sparse_only) return (unsigned)snapshots;
     int dev = 0, sms = 148;
@@ -220,8 +234,7 @@ static cudaError_t launch_read(const slotscan_read_params& p, const void* qr, co
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
         if (e != cudaSuccess) return e;
     }
-    kern<<<read_grid(p.B * NB * p.H, sm, sparse_only), RD_THREADS, sm, st>>>(p, (const Tq*)qr, sharp, (const Tsn*)kbuf, (const Tsn*)vbuf,
-                                                                            kinv, valid, (Tq*)rd);
+    kern<<<p.B * NB * p.H, RD_THREADS, sm, st>>>(p, (const Tq*)qr, sharp, (const Tsn*)kbuf, (const Tsn*)vbuf, kinv, valid, (Tq*)rd);
     return cudaGetLastError();
 }
 
