@@ -114,16 +114,19 @@ def _scan_streams(k_, v_, q_, gate, fr, N, temp, G, hard_gate, eps, occ_bin, out
     return d
 
 
-# The storage quantiser inside the row replay saves the float32 snapshots and the passes over them, but lengthens the
-# replay's walk of a busy row.  With few snapshots the walk is what takes the time: 2.29 ms with the quantiser as a pass of
-# its own against 2.73 inside for 4 chunks of 6 sequences whose float32 snapshots are 71 MB each, 1.1 against 1.3 ms for a
-# training step with 62 MB; at 1.2 GB it is 6.7 against 3.3 and 4.8 against 2.0 ms.
-_QUANT_INSIDE_BYTES = 192 << 20
+# The storage quantiser inside the row replay saves the float32 snapshots and the passes over them, which cost time in
+# proportion to their bytes, but lengthens the replay's and the reverse scan's walk of a busy row, whatever the batch.  Both
+# grow with T, so what decides is the float32 snapshot bytes per token of the call.  Rows of 128 + 128, few slots in use,
+# T = 2048, 3 bits, forward and backward (ms, quantiser a pass of its own / inside):
+#   24 KB 1.70 / 2.56    96 KB 2.09 / 2.63    144 KB 2.36 / 2.65    192 KB 2.61 / 2.65    288 KB 3.13 / 2.66    576 KB 4.66 / 2.70
+# and the forward of e4m3 chunks of 2,048 tokens: 24 KB 2.31 / 2.76, 144 KB 2.71 / 2.86, 192 KB 2.90 / 2.87, 288 KB 3.21 / 2.89;
+# float32 rows, 204 KB, 8 bits, chunks of 536 tokens, forward: 1.78 / 1.86.
+_QUANT_INSIDE_BYTES = 256 << 10
 
 
 def _quant_inside(k_, v_, N, G, qbits):
     B, T, H, DK = k_.shape
-    return bool(qbits) and 4 * B * ((T + G - 1) // G) * H * N * (DK + v_.shape[-1]) >= _QUANT_INSIDE_BYTES
+    return bool(qbits) and 4 * B * H * N * (DK + v_.shape[-1]) >= _QUANT_INSIDE_BYTES * G
 
 
 def write_memory(k, v, gate, fr, N, temp, G=16, hard_gate=False, eps=1e-4, q=None, occ_bin=False,
@@ -134,7 +137,7 @@ def write_memory(k, v, gate, fr, N, temp, G=16, hard_gate=False, eps=1e-4, q=Non
     The scan kernels emit the snapshots in `out_dtype` and kinv / valid from the float32 state while each key row is in
     registers -- no pass over the snapshots at all; in the backward the kinv gradient enters the key rows inside the
     reverse row scan.  qbits in {2,3,4,8} or "e4m3": the rows go through the storage quantiser of `writer_epilogue` there,
-    and kinv / valid are the quantised rows' (with few snapshots: float32 snapshots, then that pass over them).
+    and kinv / valid are the quantised rows' (where a token has few snapshot bytes: float32 snapshots, then that pass).
     Differentiable in k, q, v, gate, fr, temp."""
     if not k.is_cuda:
         raise RuntimeError("slotscan_b200.write_memory: CUDA tensors only (no CPU path in this package)")
