@@ -50,7 +50,7 @@ __device__ __forceinline__ bool read_row_beyond(const uint8_t* v, int N, int row
     for (int n = rows + (threadIdx.x & 31); n < N; n += 32) any |= v[n] != 0;
     return __any_sync(FULL, any);
 }
-// Which snapshots a CTA of the backward works on.  On its own: one, blockIdx.x.  Beside the tensor-core kernel (SPARSE: the
+// Which snapshots a CTA works on.  One, blockIdx.x, but in the backward beside the tensor-core kernel (SPARSE: the
 // snapshots without a row in use, at the start of a sequence) nearly all are not its own, and a launch of a CTA per snapshot
 // to find that out took longer than the work (B = 32, T = 1024, every slot in use: 0.16 ms; now 0.04): a grid that fits the
 // machine looks the snapshots over, one per warp at a time.
@@ -97,9 +97,9 @@ __global__ void __launch_bounds__(RD_THREADS) read_fwd_kernel(const slotscan_rea
     float* s_sc = rsm + ((2 * N + 3) & ~3);                    // [warps][N][4] logits, then attention weights (16-byte aligned)
     __shared__ int s_nv;
     if (SPARSE && read_row_beyond(valid + (size_t)blockIdx.x * N, N, RM_SPARSE_ROWS)) return;
-    // a function of its own: written straight into the kernel it comes out with 56 registers in place of 64 and other loads, and a
+    // through the function above: called in place the body comes out with 56 registers in place of 64 and its loads later, and a
     // decode step over eight full float32 memories takes 210 us in place of 160
-    auto work = [&](const int so) {                            // (b * NB + nb) * H + h
+    read_each_snapshot<false>(valid, N, 0, 0, [&](const int so) {      // (b * NB + nb) * H + h
     const int h = so % H, nb = (so / H) % NB, b = so / (H * NB);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
 
@@ -208,8 +208,7 @@ __global__ void __launch_bounds__(RD_THREADS) read_fwd_kernel(const slotscan_rea
         }
         __syncwarp();
     }
-    };
-    work((int)blockIdx.x);
+    });
 }
 
 // backward: a CTA per snapshot, or (sparse_only) what fits the machine beside `smem` bytes and 64 registers a thread each: one
