@@ -47,6 +47,24 @@ static cudaError_t launch_wide(const slotscan_params& p, const void* q, const vo
     if (p.occ_bin) return carry ? go(addr_fwd_wide_kernel<DK, RPL, true, true, Tin>) : go(addr_fwd_wide_kernel<DK, RPL, true, false, Tin>);
     return carry ? go(addr_fwd_wide_kernel<DK, RPL, false, true, Tin>) : go(addr_fwd_wide_kernel<DK, RPL, false, false, Tin>);
 }
+// Which kernel takes the second pass.  The wide one fills an SM, so where more sequences may come than there are SMs and two or
+// more CTAs of the direct one fit beside each other, the direct one needs fewer rounds: 192 sequences, T = 256, all of 96 rows
+// x 128 in use, both passes 312 us against 396 wide, 296 sequences 429 against 517, rows of 64 (T = 512) 536 against 825.  With
+// at most a sequence per SM, or where the direct one fills an SM too (192 rows x 128), the wide one is ahead by how early the
+// sequences pass row 64: up to 128 rows always (T = 96 to 1024: 1.01 to 1.37 times as fast); past 128 rows, where it has six resolver
+// warps to wait for, from half of the tokens on (24 sequences, 192 rows x 128, T = 512, passed at 0.13 / 0.39 / 0.5 / 0.78 of
+// the tokens: 1.27 / 1.04 / 1.02 / 0.98).  A sequence passes row 64 after 64 tokens at the earliest, so below 192 tokens the
+// direct one takes it (T = 96: 0.94, T = 128: 0.97, T = 160: 0.98 to 1.06, T = 192: 0.96 to 1.12); with a state carried in
+// it may have passed already.
+template <int DK>
+static bool wide_second_pass(const slotscan_params& p, bool carry) {
+    int dev = 0, sms = 148;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const size_t direct = sizeof(float) * (size_t)addr_fwd_layout(p.N, DK, 6, (int)sizeof(Tin)).total + 1024;
+    if ((long long)p.B * p.H > sms && 2 * direct <= 228 * 1024) return false;
+    return p.N <= 128 || carry || p.T >= 192;
+}
 template <int DK>
 static cudaError_t launch_dk(const slotscan_params& p, const void* q, const void* k, const float* gate, const float* fr,
                              const float* temp, const slotscan_log& L, const AddrFwdState& S0, cudaStream_t st) {
@@ -54,9 +72,12 @@ static cudaError_t launch_dk(const slotscan_params& p, const void* q, const void
     cudaError_t e = launch_one<DK, 2>(p, q, k, gate, fr, temp, L, S0, AF_NCAP1, 0, st);
     if (e != cudaSuccess) return e;
     if constexpr (DK >= 64) {
-        if (p.N <= 128) return launch_wide<DK, 4>(p, q, k, gate, fr, temp, L, S0, st);
-        return launch_wide<DK, 6>(p, q, k, gate, fr, temp, L, S0, st);           // N <= 192
-    } else return launch_one<DK, 6>(p, q, k, gate, fr, temp, L, S0, p.N, 1, st);  // N <= 192
+        if (wide_second_pass<DK>(p, S0.K0 != nullptr)) {
+            if (p.N <= 128) return launch_wide<DK, 4>(p, q, k, gate, fr, temp, L, S0, st);
+            return launch_wide<DK, 6>(p, q, k, gate, fr, temp, L, S0, st);
+        }
+    }
+    return launch_one<DK, 6>(p, q, k, gate, fr, temp, L, S0, p.N, 1, st);         // N <= 192
 }
 
 cudaError_t SS_CAT(run_addr_fwd_, SLOTSCAN_SUFFIX)(const slotscan_params& p, const void* q, const void* k, const float* gate,

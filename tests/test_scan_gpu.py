@@ -320,6 +320,23 @@ def test_wide_address_scan_equals_direct_bitwise(N, D, dtype, occ_bin):
                 assert torch.equal(a[n][:, :t1 - t0], b[n]), (n, t1)
 
 
+@pytest.mark.parametrize("D,N,T,copies", [(128, 96, 200, 31), (64, 192, 200, 31), (128, 192, 150, 1)])
+def test_second_pass_rule(D, N, T, copies):
+    """The second pass by the kernel that the rule on sizes takes -- more sequences than SMs, or few tokens: the direct one --
+    against the wide one, which a longer call of few sequences takes: the log of the same tokens bit for bit."""
+    import slotscan_b200 as S
+    B, H, G, long = 1, 5, 8, 230
+    inp = make_inputs("fill", B, long, H, D, D, seed=19)
+    inp["fr"] = 2 * inp["fr"]                                  # a free row nearly always wins
+    x = [inp[n].cuda() for n in ("k", "v", "gate", "fr", "q")]
+    run = lambda y: S.scan_with_log(*y[:4], N, 16.0, G=G, q=y[4], occ_bin=True)
+    a = run(x)
+    assert (a["tfirst"][:, 64] < T - 20).all()
+    b = run([t[:, :T].repeat(copies, *[1] * (t.dim() - 1)).contiguous() for t in x])
+    for n in ("addr", "oold", "kiold", "kold"):
+        assert torch.equal(a[n][:, :T].expand_as(b[n]), b[n]), n
+
+
 @pytest.mark.parametrize("mode", ["hard", "soft", "keyless", "read"])
 def test_plain_calls_equal_registered_ops(mode, monkeypatch):
     """Ordinary eager calls go round the custom ops' wrapping; the same call through the ops gives the same bits, values and
