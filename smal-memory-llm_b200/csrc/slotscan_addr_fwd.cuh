@@ -152,7 +152,6 @@ __global__ void __launch_bounds__(AF_THREADS, (RPL <= 2 ? 3 : 1)) addr_fwd_direc
     const int c0 = cw * CW;                               // first column of this warp
     const bool wact = warp >= 1 && c0 < DK;
     const float temp = temp_p[0], eps = p.eps;
-    const float4 zero4 = make_float4(0.f, 0.f, 0.f, 0.f);
 
     if (second_pass && tfirst[(size_t)bh * N] != -1) return;          // finished in the first pass (uniform per CTA)
     __syncthreads();

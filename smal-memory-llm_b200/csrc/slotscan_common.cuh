@@ -53,6 +53,11 @@ __device__ __forceinline__ void st8(__nv_bfloat16* d, const float* s) {
     }
     *reinterpret_cast<uint4*>(d) = make_uint4(w[0], w[1], w[2], w[3]);
 }
+// one element, float32 or bfloat16
+__device__ __forceinline__ float ld1(const float* p) { return *p; }
+__device__ __forceinline__ float ld1(const __nv_bfloat16* p) { return __bfloat162float(*p); }
+__device__ __forceinline__ void st1(float* p, float v) { *p = v; }
+__device__ __forceinline__ void st1(__nv_bfloat16* p, float v) { *p = __float2bfloat16_rn(v); }
 
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll

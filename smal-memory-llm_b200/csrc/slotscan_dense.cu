@@ -37,8 +37,6 @@ namespace slotscan {
 
 constexpr int DN_THREADS = 256, DN_WARPS = DN_THREADS / 32;
 
-
-
 // The address of one token from the scores s[0..lim] and occupancies o[0..lim] (rows 0..lim are the candidates: the
 // occupied rows and the first empty one).  Writes afwd[n] (the address the forward uses) and asoft[n] (its softmax);
 // warp-collective, every lane returns the same am.  occ_out[n] (may be NULL) receives the penalty factor of row n.
@@ -172,8 +170,8 @@ __global__ void __launch_bounds__(DN_THREADS) dense_fwd_kernel(
             for (int i = tid; i < N * DV; i += DN_THREADS) vbuf[so * N * DV + i] = V[i];
             for (int i = tid; i < N; i += DN_THREADS) obuf[so * N + i] = (float)o[i];
         }
-        for (int d = tid; d < DK; d += DN_THREADS) { qv[d] = ldtok(q + ix * DK + d); kt[d] = ldtok(k + ix * DK + d); }
-        for (int d = tid; d < DV; d += DN_THREADS) vt[d] = ldtok(v + ix * DV + d);
+        for (int d = tid; d < DK; d += DN_THREADS) { qv[d] = ld1(q + ix * DK + d); kt[d] = ld1(k + ix * DK + d); }
+        for (int d = tid; d < DV; d += DN_THREADS) vt[d] = ld1(v + ix * DV + d);
         __syncthreads();
         const int lim = min(s_i[0], N - 1);                // candidates: rows 0 .. first empty row
         dense_scores(K, qv, DK, lim, temp, s, ki, nullptr);
@@ -283,8 +281,8 @@ __global__ void __launch_bounds__(DN_THREADS) dense_bwd_kernel(
             float* Kn = myseg + (size_t)(j + 1) * SS;
             float* Vn = Kn + SK;
             float* on = Vn + SV;
-            for (int d = tid; d < DK; d += DN_THREADS) { qv[d] = ldtok(q + ix * DK + d); kt[d] = ldtok(k + ix * DK + d); }
-            for (int d = tid; d < DV; d += DN_THREADS) vt[d] = ldtok(v + ix * DV + d);
+            for (int d = tid; d < DK; d += DN_THREADS) { qv[d] = ld1(q + ix * DK + d); kt[d] = ld1(k + ix * DK + d); }
+            for (int d = tid; d < DV; d += DN_THREADS) vt[d] = ld1(v + ix * DV + d);
             if (warp == 0) {
                 const int fe = first_empty(op, N, eps);
                 if (lane == 0) s_i[0] = min(fe, N - 1);
@@ -331,8 +329,8 @@ __global__ void __launch_bounds__(DN_THREADS) dense_bwd_kernel(
             const int t = t0 + j;
             const size_t ix = ((size_t)b * T + t) * H + h;
             const float *Kp = stK(j), *Vp = stV(j), *op = stO(j);
-            for (int d = tid; d < DK; d += DN_THREADS) { qv[d] = ldtok(q + ix * DK + d); kt[d] = ldtok(k + ix * DK + d); }
-            for (int d = tid; d < DV; d += DN_THREADS) vt[d] = ldtok(v + ix * DV + d);
+            for (int d = tid; d < DK; d += DN_THREADS) { qv[d] = ld1(q + ix * DK + d); kt[d] = ld1(k + ix * DK + d); }
+            for (int d = tid; d < DV; d += DN_THREADS) vt[d] = ld1(v + ix * DV + d);
             if (warp == 0) {
                 const int fe = first_empty(op, N, eps);
                 if (lane == 0) s_i[0] = min(fe, N - 1);
@@ -404,7 +402,7 @@ __global__ void __launch_bounds__(DN_THREADS) dense_bwd_kernel(
                         }
                     }
                 }
-                sttok(dk + ix * DK + d, acc);
+                st1(dk + ix * DK + d, acc);
                 my_dqn = qacc;
                 dqn[d] = qacc;
             }
@@ -413,7 +411,7 @@ __global__ void __launch_bounds__(DN_THREADS) dense_bwd_kernel(
                 float acc = 0.f;
                 for (int n = 0; n <= lim; n++)
                     if (a[n] != 0.f) acc = fmaf(g * a[n], dV[(size_t)n * DV + d], acc);
-                sttok(dv + ix * DV + d, acc);
+                st1(dv + ix * DV + d, acc);
             }
             {   // <dqn, qn> over the key columns, fixed order
                 float pr = (tid < DK) ? my_dqn * (qv[tid] * qinv) : 0.f;
@@ -426,7 +424,7 @@ __global__ void __launch_bounds__(DN_THREADS) dense_bwd_kernel(
                 for (int w = 0; w < DN_WARPS; w++) prq += s_f[8 + w];
                 const float qn = qv[tid] * qinv;
                 const float gq = (qnorm < 1e-6f) ? qinv * my_dqn : qinv * (my_dqn - qn * prq);
-                sttok(dq + ix * DK + tid, gq);
+                st1(dq + ix * DK + tid, gq);
             }
             // ---- carry the state adjoints to the pre-write side (slotkern_kvg.py:183-196) ----
             const bool emit = (j == 0);
@@ -495,7 +493,7 @@ __global__ void __launch_bounds__(256) dense_finish_kernel(const float* __restri
 template <typename Tin>
 __global__ void dense_add_into_kernel(Tin* __restrict__ dst, const Tin* __restrict__ src, size_t n) {
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
-        sttok(dst + i, ldtok(dst + i) + ldtok(src + i));
+        st1(dst + i, ld1(dst + i) + ld1(src + i));
 }
 
 constexpr size_t DENSE_SMEM_CAP = 227 * 1024;
@@ -566,7 +564,7 @@ cudaError_t run_dense_split_bwd(const slotscan_params& p, const void* k, const v
         if ((e = run_row_dsum(dp, tn, s.nsl, st)) != cudaSuccess) return e;
         const size_t warps = (size_t)nbh * NC;
         auto dz = [&](auto kern) {
-            kern<<<(unsigned)((warps + 3) / 4), 128, 0, st>>>(p, s.chunk, gate, fr, temp, as, sf, ki, ot, lim, dp, bh0, nbh, dgate,
+            kern<<<(unsigned)((warps + 3) / 4), 128, 0, st>>>(p, s.chunk, gate, fr, temp, as, sf, ki, ot, dp, bh0, nbh, dgate,
                                                             dfr, part, s.part_n);
             return cudaGetLastError();
         };

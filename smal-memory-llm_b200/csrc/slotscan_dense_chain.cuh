@@ -39,10 +39,6 @@ __device__ __forceinline__ double dc_rcp(double s) {         // hardware approxi
 }
 __device__ __forceinline__ void dc_bar_rows(int threads) { asm volatile("bar.sync 1, %0;" ::"r"(threads) : "memory"); }
 __device__ __forceinline__ void dc_bar_help() { asm volatile("bar.sync 2, %0;" ::"n"(DC_HELP) : "memory"); }
-__device__ __forceinline__ float ldtok(const float* p) { return *p; }
-__device__ __forceinline__ float ldtok(const __nv_bfloat16* p) { return __bfloat162float(*p); }
-__device__ __forceinline__ void sttok(float* p, float v) { *p = v; }
-__device__ __forceinline__ void sttok(__nv_bfloat16* p, float v) { *p = __float2bfloat16_rn(v); }
 __device__ __forceinline__ double warp_sum_d(double v) {
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(FULL, v, off);
@@ -122,7 +118,7 @@ __global__ void __launch_bounds__(DC_NMAX + DC_HELP) dense_chain_kernel(const De
             const int j = i / kp, d = i % kp;
             const bool in = j < cn && d < DK;
             const size_t at = (((size_t)b * T + t0 + j) * H + h) * DK + d;
-            const float qv = in ? ldtok(qg + at) : 0.f, kv = in ? ldtok(kg + at) : 0.f;
+            const float qv = in ? ld1(qg + at) : 0.f, kv = in ? ld1(kg + at) : 0.f;
             Q[j * QS + d] = (double)qv;
             Kd[j * QS + d] = (double)kv;
             Kf[j * kp + d] = kv;
@@ -156,7 +152,7 @@ __global__ void __launch_bounds__(DC_NMAX + DC_HELP) dense_chain_kernel(const De
     float xn[C];
     auto fetch_v = [&](int t0, int cn) {
 #pragma unroll
-        for (int j = 0; j < C; j++) xn[j] = j < cn ? ldtok(vg + (((size_t)b * T + t0 + j) * H + h) * DV + hd) : 0.f;
+        for (int j = 0; j < C; j++) xn[j] = j < cn ? ld1(vg + (((size_t)b * T + t0 + j) * H + h) * DV + hd) : 0.f;
     };
     // the values of a chunk whose tokens fetch_v has loaded, first token at place ph of block jb; and its addresses
     auto values = [&](int bf, int t0, int cn, int ph, int jb) {
@@ -415,7 +411,7 @@ __global__ void __launch_bounds__(128) dense_dz_kernel(const slotscan_params p, 
                                                        const float* __restrict__ fr, const float* __restrict__ temp_p,
                                                        const float* __restrict__ as, const float* __restrict__ sf,
                                                        const float* __restrict__ ki, const float* __restrict__ ot,
-                                                       const int* __restrict__ lim, float* __restrict__ D, int bh0, int nbh,
+                                                       float* __restrict__ D, int bh0, int nbh,
                                                        float* __restrict__ dgate, float* __restrict__ dfr,
                                                        float* __restrict__ part, size_t part_n) {
     const int N = p.N, T = p.T, H = p.H, NC = (T + chunk - 1) / chunk, lane = threadIdx.x & 31;
@@ -523,7 +519,7 @@ __global__ void __launch_bounds__(DQ_T) dense_dq_kernel(const slotscan_params p,
         }
         for (int i = tid; i < DQ_C * kp; i += DQ_T) {
             const int j = i / kp, d = i % kp;
-            kt[i] = (j < cn && d < DK) ? ldtok(k + (((size_t)b * T + t0 + j) * H + h) * DK + d) : 0.f;
+            kt[i] = (j < cn && d < DK) ? ld1(k + (((size_t)b * T + t0 + j) * H + h) * DK + d) : 0.f;
         }
         __syncthreads();
         float4 acc[DQ_C];
@@ -573,7 +569,7 @@ __global__ void __launch_bounds__(DQ_T) dense_dq_kernel(const slotscan_params p,
 #pragma unroll
             for (int c = 0; c < 4; c++) {
                 const int d = lane + 32 * c;
-                qv[c] = d < DK ? ldtok(q + ix * DK + d) : 0.f;
+                qv[c] = d < DK ? ld1(q + ix * DK + d) : 0.f;
                 qq = fma((double)qv[c], (double)qv[c], qq);
             }
             qq = warp_sum_d(qq);
@@ -587,7 +583,7 @@ __global__ void __launch_bounds__(DQ_T) dense_dq_kernel(const slotscan_params p,
                 const int d = lane + 32 * c;
                 if (d < DK) {
                     const float x = gq[j * kp + d];
-                    sttok(dq + ix * DK + d, (float)qn < 1e-6f ? qi * x : qi * (x - qv[c] * qi * pr));
+                    st1(dq + ix * DK + d, (float)qn < 1e-6f ? qi * x : qi * (x - qv[c] * qi * pr));
                 }
             }
         }

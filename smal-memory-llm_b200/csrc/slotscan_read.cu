@@ -28,10 +28,6 @@ namespace slotscan {
 
 constexpr int RD_THREADS = 128, RD_WARPS = 4, RD_QPW = 4, RD_MAXC = 4;     // columns per lane: up to 128 / 32
 
-__device__ __forceinline__ float ldf(const float* p) { return *p; }
-__device__ __forceinline__ float ldf(const __nv_bfloat16* p) { return __bfloat162float(*p); }
-__device__ __forceinline__ void stf(float* p, float v) { *p = v; }
-__device__ __forceinline__ void stf(__nv_bfloat16* p, float v) { *p = __float2bfloat16_rn(v); }
 
 // Highest valid row + 1 of a snapshot; warp-collective.
 __device__ __forceinline__ int read_rows_in_use(const uint8_t* v, int N) {
@@ -136,7 +132,7 @@ __global__ void __launch_bounds__(RD_THREADS) read_fwd_kernel(const slotscan_rea
 #pragma unroll
             for (int c = 0; c < RD_MAXC; c++) {
                 const int col = lane + 32 * c;
-                qv[u][c] = col < DK ? ldf(qr + qi[u] * DK + col) : 0.f;
+                qv[u][c] = col < DK ? ld1(qr + qi[u] * DK + col) : 0.f;
                 qq = fmaf(qv[u][c], qv[u][c], qq);
             }
             qq = warp_sum(qq);
@@ -147,7 +143,7 @@ __global__ void __launch_bounds__(RD_THREADS) read_fwd_kernel(const slotscan_rea
             const Tsn* row = Kb + (size_t)s_rows[j] * DK;
             float kx[RD_MAXC];
 #pragma unroll
-            for (int c = 0; c < RD_MAXC; c++) kx[c] = (lane + 32 * c) < DK ? ldf(row + lane + 32 * c) : 0.f;
+            for (int c = 0; c < RD_MAXC; c++) kx[c] = (lane + 32 * c) < DK ? ld1(row + lane + 32 * c) : 0.f;
             float d[RD_QPW];
 #pragma unroll
             for (int u = 0; u < RD_QPW; u++) {
@@ -193,7 +189,7 @@ __global__ void __launch_bounds__(RD_THREADS) read_fwd_kernel(const slotscan_rea
             const float a[4] = {a4.x, a4.y, a4.z, a4.w};
 #pragma unroll
             for (int c = 0; c < RD_MAXC; c++) {
-                const float vx = (lane + 32 * c) < DV ? ldf(row + lane + 32 * c) : 0.f;
+                const float vx = (lane + 32 * c) < DV ? ld1(row + lane + 32 * c) : 0.f;
 #pragma unroll
                 for (int u = 0; u < RD_QPW; u++) acc[u][c] = fmaf(a[u], vx, acc[u][c]);
             }
@@ -203,7 +199,7 @@ __global__ void __launch_bounds__(RD_THREADS) read_fwd_kernel(const slotscan_rea
             if (q0 + u < M) {
 #pragma unroll
                 for (int c = 0; c < RD_MAXC; c++)
-                    if (lane + 32 * c < DV) stf(rd + qi[u] * DV + lane + 32 * c, acc[u][c]);   // nv == 0: exactly zero
+                    if (lane + 32 * c < DV) st1(rd + qi[u] * DV + lane + 32 * c, acc[u][c]);   // nv == 0: exactly zero
             }
         }
         __syncwarp();
@@ -295,7 +291,7 @@ __device__ __forceinline__ void zero_fill(T* p, size_t n, int tid) {
         const uint4 z = make_uint4(0u, 0u, 0u, 0u);
         for (size_t i = tid; i < bytes / 16; i += RD_THREADS) p4[i] = z;
     } else {
-        for (size_t i = tid; i < n; i += RD_THREADS) stf(p + i, 0.f);
+        for (size_t i = tid; i < n; i += RD_THREADS) st1(p + i, 0.f);
     }
 }
 
@@ -376,8 +372,8 @@ __global__ void __launch_bounds__(RD_THREADS, SPARSE ? 4 : 0) read_bwd_kernel(
 #pragma unroll
             for (int c = 0; c < RD_MAXC; c++) {
                 const int col = lane + 32 * c;
-                qv[u][c] = col < DK ? ldf(qr + qi[u] * DK + col) : 0.f;
-                dr[u][c] = col < DV ? ldf(drd + qi[u] * DV + col) : 0.f;
+                qv[u][c] = col < DK ? ld1(qr + qi[u] * DK + col) : 0.f;
+                dr[u][c] = col < DV ? ld1(drd + qi[u] * DV + col) : 0.f;
                 qq = fmaf(qv[u][c], qv[u][c], qq);
             }
             qq = warp_sum(qq);
@@ -391,8 +387,8 @@ __global__ void __launch_bounds__(RD_THREADS, SPARSE ? 4 : 0) read_bwd_kernel(
             float kx[RD_MAXC], vx[RD_MAXC];
 #pragma unroll
             for (int c = 0; c < RD_MAXC; c++) {
-                kx[c] = (lane + 32 * c) < DK ? ldf(krow + lane + 32 * c) : 0.f;
-                vx[c] = (lane + 32 * c) < DV ? ldf(vrow + lane + 32 * c) : 0.f;
+                kx[c] = (lane + 32 * c) < DK ? ld1(krow + lane + 32 * c) : 0.f;
+                vx[c] = (lane + 32 * c) < DV ? ld1(vrow + lane + 32 * c) : 0.f;
             }
             float d[RD_QPW], da[RD_QPW];
 #pragma unroll
@@ -455,7 +451,7 @@ __global__ void __launch_bounds__(RD_THREADS, SPARSE ? 4 : 0) read_bwd_kernel(
             const float cfu[4] = {c4.x, c4.y, c4.z, c4.w};
 #pragma unroll
             for (int c = 0; c < RD_MAXC; c++) {
-                const float kx = (lane + 32 * c) < DK ? ldf(krow + lane + 32 * c) : 0.f;
+                const float kx = (lane + 32 * c) < DK ? ld1(krow + lane + 32 * c) : 0.f;
 #pragma unroll
                 for (int u = 0; u < RD_QPW; u++) acc[u][c] = fmaf(cfu[u], kx, acc[u][c]);
             }
@@ -472,7 +468,7 @@ __global__ void __launch_bounds__(RD_THREADS, SPARSE ? 4 : 0) read_bwd_kernel(
                     if (lane + 32 * c < DK) {
                         const float qn = qv[u][c] * qinv[u];
                         const float o = qinv[u] >= 1e6f ? qinv[u] * acc[u][c] : qinv[u] * (acc[u][c] - qn * pr);
-                        stf(dqr + qi[u] * DK + lane + 32 * c, o);
+                        st1(dqr + qi[u] * DK + lane + 32 * c, o);
                     }
                 }
             }
@@ -492,15 +488,15 @@ __global__ void __launch_bounds__(RD_THREADS, SPARSE ? 4 : 0) read_bwd_kernel(
 #pragma unroll
             for (int c = 0; c < RD_MAXC; c++) {
                 const int col = lane + 32 * c;
-                if (col < DV) aV[c] = fmaf(at, ldf(drd + qm * DV + col), aV[c]);
-                if (col < DK) aK[c] = fmaf(cq, ldf(qr + qm * DK + col), aK[c]);
+                if (col < DV) aV[c] = fmaf(at, ld1(drd + qm * DV + col), aV[c]);
+                if (col < DK) aK[c] = fmaf(cq, ld1(qr + qm * DK + col), aK[c]);
             }
         }
 #pragma unroll
         for (int c = 0; c < RD_MAXC; c++) {
             const int col = lane + 32 * c;
-            if (col < DK) stf(dkbuf + ((size_t)so * N + n) * DK + col, aK[c]);
-            if (col < DV) stf(dvbuf + ((size_t)so * N + n) * DV + col, aV[c]);
+            if (col < DK) st1(dkbuf + ((size_t)so * N + n) * DK + col, aK[c]);
+            if (col < DV) st1(dvbuf + ((size_t)so * N + n) * DV + col, aV[c]);
         }
         if (lane == 0) {
             float s = 0.f;

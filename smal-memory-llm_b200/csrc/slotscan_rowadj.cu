@@ -26,9 +26,6 @@
 
 namespace slotscan {
 
-__device__ __forceinline__ void ra_st(float* p, float v) { *p = v; }
-__device__ __forceinline__ void ra_st(__nv_bfloat16* p, float v) { *p = __float2bfloat16_rn(v); }
-
 __device__ __forceinline__ void ra_cp16(void* dst, const void* src) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
 }
@@ -230,7 +227,7 @@ __global__ void __maxnreg__(DS == 32 ? 168 : 255) row_adjoint_kernel(const RowAd
                 const int j = e / DS, d = e % DS;
                 float v = 0.f;
                 for (int q = 0; q < nw; q++) v += red[q * CT * DS + e];
-                if (d < dn) ra_st(dx + (size_t)(ts + j) * H * D + d, v);
+                if (d < dn) st1(dx + (size_t)(ts + j) * H * D + d, v);
             }
         }
         // to the post side of the block before: the block's factors, then the gradient of its snapshot

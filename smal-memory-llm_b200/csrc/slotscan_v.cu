@@ -35,10 +35,6 @@ namespace slotscan {
 
 constexpr int KV_THREADS = 128, KV_WARPS = KV_THREADS / 32;
 
-__device__ __forceinline__ float ldv(const float* p) { return *p; }
-__device__ __forceinline__ float ldv(const __nv_bfloat16* p) { return __bfloat162float(*p); }
-__device__ __forceinline__ void stv(float* p, float x) { *p = x; }
-__device__ __forceinline__ void stv(__nv_bfloat16* p, float x) { *p = __float2bfloat16_rn(x); }
 
 // One warp: address of a token from its logits and the occupancies.  z[n] (double scratch) is overwritten.
 // Returns the argmax (first maximum); asoft / afwd receive the softmax and the address the forward uses.
@@ -106,7 +102,7 @@ __global__ void __launch_bounds__(KV_THREADS) keyless_fwd_kernel(const slotscan_
             for (int i = tid; i < N; i += KV_THREADS) obuf[so * N + i] = (float)o[i];
         }
         for (int n = tid; n < N; n += KV_THREADS) wt[n] = wa[ix * N + n];
-        for (int d = tid; d < DV; d += KV_THREADS) vt[d] = ldv(v + ix * DV + d);
+        for (int d = tid; d < DV; d += KV_THREADS) vt[d] = ld1(v + ix * DV + d);
         __syncthreads();
         if (warp == 0) {
             const int am = keyless_address(wt, o, N, fr, p.hard, z, as, a);
@@ -177,7 +173,7 @@ __global__ void __launch_bounds__(KV_THREADS) keyless_bwd_kernel(const slotscan_
             float* Vn = myseg + (size_t)(j + 1) * SS;
             float* on = Vn + SV;
             for (int n = tid; n < N; n += KV_THREADS) wt[n] = wa[ix * N + n];
-            for (int d = tid; d < DV; d += KV_THREADS) vt[d] = ldv(v + ix * DV + d);
+            for (int d = tid; d < DV; d += KV_THREADS) vt[d] = ld1(v + ix * DV + d);
             __syncthreads();
             if (warp == 0) {
                 keyless_address(wt, op, N, fr, p.hard, z, as, a);
@@ -210,7 +206,7 @@ __global__ void __launch_bounds__(KV_THREADS) keyless_bwd_kernel(const slotscan_
             const size_t ix = ((size_t)b * T + t0 + j) * H + h;
             const float *Vp = stV(j), *op = stO(j);
             for (int n = tid; n < N; n += KV_THREADS) wt[n] = wa[ix * N + n];
-            for (int d = tid; d < DV; d += KV_THREADS) vt[d] = ldv(v + ix * DV + d);
+            for (int d = tid; d < DV; d += KV_THREADS) vt[d] = ld1(v + ix * DV + d);
             __syncthreads();
             for (int n = warp; n < N; n += KV_WARPS) {      // dw_n = <v - V_n, dV_n> + (1 - o_n) dO_n
                 float a1 = 0.f;
@@ -242,7 +238,7 @@ __global__ void __launch_bounds__(KV_THREADS) keyless_bwd_kernel(const slotscan_
                 float acc = 0.f;
                 for (int n = 0; n < N; n++)
                     if (a[n] != 0.f) acc = fmaf(g * a[n], dV[(size_t)n * DV + d], acc);
-                stv(dv + ix * DV + d, acc);
+                st1(dv + ix * DV + d, acc);
             }
             __syncthreads();
             const bool emit = (j == 0);
@@ -356,7 +352,7 @@ __global__ void __launch_bounds__(32 * (2 + KL_CW), MINB) keyless_fwd_chain_kern
     float xn[KL_CT];
     auto fetch_v = [&](int t0) {
 #pragma unroll
-        for (int j = 0; j < KL_CT; j++) xn[j] = t0 + j < T ? ldv(v + (((size_t)b * T + t0 + j) * H + h) * DV + dl) : 0.f;
+        for (int j = 0; j < KL_CT; j++) xn[j] = t0 + j < T ? ld1(v + (((size_t)b * T + t0 + j) * H + h) * DV + dl) : 0.f;
     };
     if (ct >= 0 && DV <= 32 * KL_CW) fetch_v(0);
     for (int c = -1; c <= NC; c++) {
@@ -466,7 +462,7 @@ __global__ void __launch_bounds__(32 * (2 + KL_CW), MINB) keyless_fwd_chain_kern
                 bool odd = p.hard != 0;                            // a row a token does not write must not see it: only an
 #pragma unroll
                 for (int j = 0; j < KL_CT; j++) {                  // infinite or NaN value would tell
-                    xv[j] = DV <= 32 * KL_CW ? xn[j] : (j < cn ? ldv(v + (((size_t)b * T + t0 + j) * H + h) * DV + d) : 0.f);
+                    xv[j] = DV <= 32 * KL_CW ? xn[j] : (j < cn ? ld1(v + (((size_t)b * T + t0 + j) * H + h) * DV + d) : 0.f);
                     odd |= !(fabsf(xv[j]) <= 3e38f);
                 }
                 if (DV <= 32 * KL_CW) fetch_v(t0 + KL_CT);
