@@ -31,12 +31,6 @@ __host__ __device__ inline size_t dc_smem(int C, int N, int DK, int DV, bool val
     return 2 * dc_tok_bytes(C, DK) + 8 * 128 + 8 * (size_t)2 * C * 8 + 4 * ((size_t)N * (kp + 4) + (values ? n4 * DV : 0) + 2 * C * n4 + 16);
 }
 
-__device__ __forceinline__ double dc_rcp(double s) {         // hardware approximation + one cubic Newton-Raphson step
-    double r;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(s));
-    const double t = fma(-s, r, 1.0);
-    return fma(r, fma(t, t, t), r);
-}
 __device__ __forceinline__ void dc_bar_rows(int threads) { asm volatile("bar.sync 1, %0;" ::"r"(threads) : "memory"); }
 __device__ __forceinline__ void dc_bar_help() { asm volatile("bar.sync 2, %0;" ::"n"(DC_HELP) : "memory"); }
 __device__ __forceinline__ double warp_sum_d(double v) {
@@ -300,7 +294,7 @@ __global__ void __launch_bounds__(DC_NMAX + DC_HELP) dense_chain_kernel(const De
                         const double2 e0 = *reinterpret_cast<const double2*>(xs), e1 = *reinterpret_cast<const double2*>(xs + 2);
                         const double2 e2 = *reinterpret_cast<const double2*>(xs + 4), e3 = *reinterpret_cast<const double2*>(xs + 6);
                         const double se = ((e0.x + e0.y) + (e1.x + e1.y)) + ((e2.x + e2.y) + (e3.x + e3.y));
-                        const double si = bounded ? dc_rcp(se) : 1.0 / se;
+                        const double si = bounded ? rcp_normal(se) : 1.0 / se;
                         const float a = cand ? (float)(E * si) : 0.f;        // also where the sum is not finite
                         if (TABLES) {
                             if (live) {

@@ -309,14 +309,6 @@ __device__ __forceinline__ double kl_softmax(const float (&wa)[R], const double 
     return se;
 }
 
-// 1 / s for a positive normal s: the hardware's approximation (about 20 bits) and one cubic Newton-Raphson step.
-__device__ __forceinline__ double kl_rcp(double s) {
-    double r;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(s));
-    const double t = fma(-s, r, 1.0);
-    return fma(r, fma(t, t, t), r);
-}
-
 // Warp 0: the chain.  Warp 1: what of a token's address does not depend on the occupancies -- exp(wa_n - max wa), a chunk
 // ahead -- so that the chain is exp(-fr o_n), one sum, one reciprocal and the blend.  Warps 2..9: the values, a chunk
 // behind.  The factors neither overflow nor vanish while |fr| <= 300 and the gates stay in [0, 1] (o in [0, 1]); anything
@@ -388,7 +380,7 @@ __global__ void __launch_bounds__(32 * (2 + KL_CW), MINB) keyless_fwd_chain_kern
                         }
 #pragma unroll
                         for (int off = 16; off > 0; off >>= 1) se += __shfl_xor_sync(FULL, se, off);
-                        si = kl_rcp(se);
+                        si = rcp_normal(se);
                     }
 #pragma unroll
                     for (int i = 0; i < R; i++) {
