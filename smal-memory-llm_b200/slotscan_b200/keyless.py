@@ -13,7 +13,7 @@ from typing import Optional, Tuple
 import torch
 
 from . import _lib
-from .ops import _Here, _ptr, _require_cuda, _stream, plain_call, wants_grad
+from .ops import _Here, _ptr, _require_cuda, _stream, plain_call, plain_grads, wants_grad
 
 _DT = {torch.float32: _lib.F32, torch.bfloat16: _lib.BF16}
 
@@ -111,7 +111,7 @@ class _Keyless(torch.autograd.Function):
     @staticmethod
     @torch.autograd.function.once_differentiable
     def backward(ctx, *grads):
-        return _backward(ctx, *grads, bwd=_keyless_bwd if plain_call(*grads) else None)
+        return _backward(ctx, *grads, bwd=_keyless_bwd if plain_grads(*grads) else None)
 
 
 def slot_scan_v(v, wa, gate, fr, N, C=256, G=1, buf_dtype=torch.float32, hard=False, hard_gate=False):

@@ -44,31 +44,41 @@ class _Here:
             self.guard.__exit__(*a)
 
 
+# looked up once: plain_call runs in every call
+_tracing, _dispatch_modes, _transforms = torch.jit.is_tracing, torch._C._len_torch_dispatch_stack, torch._C._functorch.peek_interpreter_stack
+_profiled, _function_modes = torch._C._autograd._profiler_enabled, torch._C._len_torch_function_stack
 _is_batched = torch._C._functorch.is_legacy_batchedtensor
+_Tensor, _Parameter = torch.Tensor, torch.nn.Parameter
 
 
-def _watched():
-    """A mode, tracer or profiler that has to see the call.  The mode of `torch.device` and `torch.set_default_device` concerns
-    factory functions alone."""
-    if torch.compiler.is_compiling() or torch.jit.is_tracing() or torch._C._len_torch_dispatch_stack() > 0 or \
-            torch._C._functorch.peek_interpreter_stack() is not None or torch._C._autograd._profiler_enabled():
-        return True
-    modes = torch._C._len_torch_function_stack()
-    return modes > 0 and any(type(torch._C._get_function_stack_at(i)) is not DeviceContext for i in range(modes))
+def _modes_watch(n):
+    """The mode of `torch.device` and `torch.set_default_device` concerns factory functions alone."""
+    return any(type(torch._C._get_function_stack_at(i)) is not DeviceContext for i in range(n))
 
 
 def plain_call(*ts):
-    """True when nothing looks over this call's shoulder (`_watched`) and its tensors are ordinary ones: of no other class, not
-    batched by the older vmap (`is_grads_batched`, `jacobian(vectorize=True)`), not a lazy negation.
+    """True when nothing looks over this call's shoulder and its tensors are ordinary ones: no tracing, compiling, fake or
+    functional mode, function mode or profiler; tensors of no other class and no lazy negation.
     The custom op's own wrapping costs about 80 us of host time per call and direction, as much as the kernels of a small
     call take; such a call goes to the same implementation without it, and through an autograd.Function with the same
     backward when a gradient is wanted.  Everything else takes the registered op."""
-    if _watched():
+    if torch.compiler.is_compiling() or _tracing() or _dispatch_modes() or _transforms() is not None or _profiled():
+        return False
+    modes = _function_modes()
+    if modes and _modes_watch(modes):
         return False
     for t in ts:
-        if t is not None and (type(t) is not torch.Tensor and type(t) is not torch.nn.Parameter or _is_batched(t) or t.is_neg()):
-            return False
+        if t is not None:
+            kind = type(t)
+            if kind is not _Tensor and kind is not _Parameter or t.is_neg():
+                return False
     return True
+
+
+def plain_grads(*ts):
+    """plain_call for the gradients that come into a backward: also not batched by the older vmap, whose tensors have the
+    ordinary class and no memory (`is_grads_batched`, `jacobian(vectorize=True)`)."""
+    return plain_call(*ts) and not any(t is not None and _is_batched(t) for t in ts)
 
 
 def wants_grad(*ts):
@@ -227,7 +237,7 @@ class _HardScan(torch.autograd.Function):
     @staticmethod
     @torch.autograd.function.once_differentiable
     def backward(ctx, *grads):
-        return _backward(ctx, *grads, bwd=_hard_bwd if plain_call(*grads) else None)
+        return _backward(ctx, *grads, bwd=_hard_bwd if plain_grads(*grads) else None)
 
 
 def run_hard_fwd(*args):
@@ -345,7 +355,7 @@ class _DenseScan(torch.autograd.Function):
     @staticmethod
     @torch.autograd.function.once_differentiable
     def backward(ctx, *grads):
-        return _dense_backward(ctx, *grads, bwd=_dense_bwd if plain_call(*grads) else None)
+        return _dense_backward(ctx, *grads, bwd=_dense_bwd if plain_grads(*grads) else None)
 
 
 def run_dense_fwd(*args):

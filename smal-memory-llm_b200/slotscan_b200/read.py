@@ -8,7 +8,7 @@ import ctypes
 import torch
 
 from . import _lib
-from .ops import _Here, _ptr, _require_cuda, _stream, as_flag_bytes, plain_call, wants_grad
+from .ops import _Here, _ptr, _require_cuda, _stream, as_flag_bytes, plain_call, plain_grads, wants_grad
 
 _CODE = {torch.float32: _lib.F32, torch.bfloat16: _lib.BF16}
 
@@ -108,7 +108,7 @@ class _Read(torch.autograd.Function):
     @staticmethod
     @torch.autograd.function.once_differentiable
     def backward(ctx, drd):
-        return _rd_backward(ctx, drd, bwd=_read_bwd if plain_call(drd) else None)
+        return _rd_backward(ctx, drd, bwd=_read_bwd if plain_grads(drd) else None)
 
 
 def read_snapshots(qr, sharp, kbuf, vbuf, kinv, valid, G):

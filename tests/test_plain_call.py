@@ -18,7 +18,7 @@ class Watch(TorchFunctionMode):
 
 
 def test_what_is_a_plain_call():
-    from slotscan_b200.ops import plain_call
+    from slotscan_b200.ops import plain_call, plain_grads
     x = torch.zeros(3, requires_grad=True)
     assert plain_call(x, None, torch.nn.Parameter(x.detach()))
     assert not plain_call(x, torch._neg_view(x))
@@ -31,7 +31,7 @@ def test_what_is_a_plain_call():
 
         @staticmethod
         def backward(ctx, g):
-            got.append(plain_call(g))
+            got.append(plain_grads(g))
             return g * 2
     torch.autograd.grad(Probe.apply(x), x, torch.ones(2, 3), is_grads_batched=True)
     torch.autograd.grad(Probe.apply(x), x, torch.ones(3))
