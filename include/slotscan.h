@@ -188,7 +188,7 @@ int slotscan_hard_bwd_noalloc(const slotscan_params* p, const void* k, const voi
  * slotscan_dense_fwd: addr (B,T,H) int32 = argmax of each token's address, kfin / vfin / ofin = the final state; each
  * of the four may be NULL.
  * slotscan_dense_bwd: needs the forward's kbuf, vbuf, obuf and scratch of slotscan_dense_bwd_scratch_bytes (soft,
- * detached, N <= 256: per-token tables of as many sequences as 2 GiB hold, more sequences go through in turns; else G
+ * detached, N <= 256: per-token tables of as many sequences as 2 GiB hold and at least one, more go through in turns; else G
  * states per (sequence, head)); dkbuf / dvbuf float32, either may be NULL.  Outputs as slotscan_hard_bwd. */
 typedef struct {
     slotscan_params base;
@@ -213,7 +213,9 @@ int slotscan_dense_bwd(const slotscan_dense_params* p, const void* k, const void
  *   buf (B,NB,H,N,DV) f32: the pre-write values at t = 0, G, 2G, ...; obuf (B,NB,H,N) f32: the occupancies at the same
  *   times (the backward's checkpoints); addr (B,T,H) int32 or NULL.
  * Backward: dv (in_dtype), dwa (B,T,H,N), dgate (B,T,H), dfr 1 float, from dbuf (f32, or NULL = zeros); scratch of
- * slotscan_v_bwd_scratch_bytes.  N * DV + 10 N floats must fit one CTA's shared memory. */
+ * slotscan_v_bwd_scratch_bytes (N <= 256: per-token tables, T * N * (2 + slices of 16 or 32 columns) floats per (sequence,
+ * head), of as many sequences as 2 GiB hold and at least one, more go through in turns; else G states per (sequence,
+ * head)).  N * DV + 10 N floats must fit one CTA's shared memory. */
 typedef struct {
     int32_t B, T, H, N, DV, G;
     int32_t hard, hard_gate;

@@ -14,7 +14,8 @@
 //                        the next-write table to a per-token table; then each warp takes 4 tokens: scores by 8 lanes
 //                        per row (4 rows at a time, 3 shuffle stages), softmax adjoint with lane = row, dq accumulated
 //                        with lane = 4 columns over the rows (no reduction).
-// A sequence that ever made row 32 a candidate is left to the chunked kernel.  [reference addr_bwd, slotkern_cuda.py:264-443]
+// A sequence that ever made row 32 a candidate is left to the tiles kernel (slotscan_addr_tiles.cuh), or, where the scratch
+// has no room for that kernel's next-write table, to the chunked one.  [reference addr_bwd, slotkern_cuda.py:264-443]
 #pragma once
 #include "slotscan_addr_fwd.cuh"
 #include "slotscan_async.cuh"

@@ -3,11 +3,18 @@
 //
 // Decomposition (the row a token writes is the only sequential decision):
 //   addr_fwd_direct_kernel (slotscan_addr_fwd.cuh)  one CTA per (sequence, head): keys resident in shared memory,
-//                      scores per chunk of 8 tokens in bulk, one warp resolves the addresses.   [addr_fwd, slotkern_cuda.py:72-174]
+//                      column warps and a resolver warp one token apart.                        [addr_fwd, slotkern_cuda.py:72-174]
+//   addr_fwd_wide_kernel (slotscan_addr_wide.cuh)   second pass, of sequences that use more than 64 rows: key rows in
+//                      registers, a resolver thread per row.
 //   replay_rows_kernel (slotscan_rows.cuh)  row-parallel: replays key / value rows from the log, emits the stride-G
 //                      snapshots, the undo log and the final state.                              [val_fwd :178-206]
-//   rows_bwd_kernel    (slotscan_rows.cuh)  row-parallel reverse scan: dK / dV recursion, dk / dv, the table D[t,n]. [rows_bwd :209-261]
-//   addr_bwd_chunked_kernel (slotscan_addr_bwd.cuh)  softmax adjoint per chunk: dgate, dfr, dtemp, dq.   [addr_bwd :264-443]
+//   rows_bwd3_kernel, rows_bwd2_kernel (slotscan_rows_bwd.cuh)  row-parallel reverse scan: dK / dV recursion, dk / dv, the
+//                      table D[t,n].                                                            [rows_bwd :209-261]
+//   softmax adjoint (dgate, dfr, dtemp, dq)                                                     [addr_bwd :264-443]
+//     addr_bwd_gather_kernel (slotscan_addr_gather.cuh)  token-parallel, sequences with at most 32 rows in use
+//     addr_bwd_tiles_kernel (slotscan_addr_tiles.cuh)    token-parallel, the others
+//     addr_bwd_chunked_kernel (slotscan_addr_bwd.cuh)    chunk by chunk with the key rows resident: the penalty on o itself,
+//                      widths below 32, scratch without room for the next-write table of all rows
 // Rows are taken in index order (only occupied rows and the lowest free row are candidates), so every row above
 // the highest row touched so far is exactly zero: all kernels skip those rows.
 #include <math.h>

@@ -16,8 +16,7 @@
 // Bound: the double-precision dots (N * DS * (G + 1) per block and slice) and, for few rows, the latency of one block's
 // phases -- hence 16-wide slices (half the dot's chain, twice the CTAs) up to 64 rows.  64 sequences, 64 x 64, 128 blocks of
 // 4 tokens: 0.29 ms (0.54 with loads that waited for one another before the weighted sum, 1.23 with 32-wide slices and 16
-// tokens a step); 48 sequences, 192 x (64 + 64), 32 blocks of 16: 0.42 ms
-// (0.60 with more than 168 registers a thread: 192 CTAs then run in two rounds).
+// tokens a step); 48 sequences, 192 x (64 + 64), 32 blocks of 16: 0.42 ms.
 #include <algorithm>
 
 #include "slotscan_common.cuh"
@@ -40,6 +39,10 @@ struct RowAdjShape {
     static size_t smem(int nt) { return 8 * (size_t)CT * DS + 4 * ((size_t)nt * (FS + 3 * SS) + (size_t)(nt / 32) * CT * DS + 2 * CT); }
 };
 
+// 168 registers for the 32-wide slices: 129 to 192 rows then run two CTAs to an SM where 255 would leave one, 65 to 96 three
+// instead of two (97 to 128: two either way, by shared memory; past 192 one).  What that spills (at most 0.5 KB a thread, at 16
+// tokens a step) costs less than the missing warps: 192 rows, 48 sequences x 4 slices, 0.60 -> 0.42 ms.  The 16-wide slices
+// (two warps at most) keep all they ask for.
 template <typename Tin, int CT, int DS, bool HARD>
 __global__ void __maxnreg__(DS == 32 ? 168 : 255) row_adjoint_kernel(const RowAdjArgs A) {
     constexpr int FS = RowAdjShape<CT, DS>::FS, SS = RowAdjShape<CT, DS>::SS;

@@ -69,10 +69,10 @@ struct ReplayArgs {
 };
 
 // NORM: kinv / valid may be asked for (checked per tensor at run time).  QUANT: the emitted copies go through the storage
-// quantiser while the float32 row is in registers, once per stretch between two writes of the row: no float32 snapshots,
-// no pass over them.  B = 16, T = 512, H = 6, 192 x (128 + 128), ~60 rows in use, 3 bits, bf16 hand-over, forward + backward:
-// 4.75 ms with the quantiser (and, backward, its copies and casts) as passes of their own, 2.9 ms so; the same write of
-// four 1024-token chunks of 8 sequences in e4m3, forward: 6.7 -> 3.3 ms.
+// quantiser while the float32 row is in registers, once per stretch between two writes of the row (a chunk of 32 tokens ends a
+// stretch too) that holds a snapshot: no float32 snapshots, no pass over them.  B = 16, T = 512, H = 6, 192 x (128 + 128), ~60
+// rows in use, 3 bits, bf16 hand-over, forward + backward: 4.32 ms with the quantiser (and, backward, its copies and casts) as
+// passes of their own, 1.92 ms so; the write of four 1024-token chunks of 8 sequences in e4m3, forward: 6.7 -> 3.2 ms.
 // EPL: elements per lane, 8 or 16.  With 16 a lane holds two pieces of 8 columns half a row apart (every load and store
 // of a row group stays one contiguous run of 16-byte pieces) and a CTA has half the threads: the busy tiles of a large
 // batch (one CTA per sequence, head and tensor) then all fit on the machine at once instead of in two waves.

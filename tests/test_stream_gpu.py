@@ -230,8 +230,8 @@ def test_config3_fp8_e4m3_storage_streamed():
 def test_quantised_write_equals_scan_then_quantiser(case, dtypes, monkeypatch):
     """write_memory with a quantiser against the float32 scan followed by writer_epilogue: the emitted rows come from the
     same float32 state through the same arithmetic, so they are bit-identical; kinv sums its squares in another order
-    (128 float32 terms: 1e-5 of itself is far above it), and the gradients differ by the order of two float32 additions,
-    the bound of the other gradient tests), with bf16 streams by their rounding (2^-8 of the largest) where that tips."""
+    (128 float32 terms: 1e-5 of itself is far above it), and the gradients differ by the order of two float32 additions (the
+    bound of the other gradient tests), with bf16 streams by their rounding (2^-8 of the largest) where that tips."""
     S = _S()
     monkeypatch.setattr("slotscan_b200.scan._QUANT_INSIDE_BYTES", 0)       # small shapes too
     DK, DV, G, bits, group, dist = case
