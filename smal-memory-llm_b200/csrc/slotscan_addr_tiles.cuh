@@ -61,10 +61,6 @@ static __global__ void __launch_bounds__(192) next_write_all_kernel(const slotsc
     }
 }
 
-// place of (slot, token) in St / C: quads of tokens swapped around by slot, so that 8 neighbouring slots of one token (step
-// 2) and 4 neighbouring tokens of one slot (step 3, one 16-byte load) both miss each other's banks
-__device__ __forceinline__ int tiles_at(int s, int j) { return s * 32 + ((((j >> 2) ^ (s & 7)) << 2) | (j & 3)); }
-
 // step 1 for NS groups of 32 slots: thread = rows rg + 32 i, tokens tq + 8 k
 template <int DK, int NS>
 __device__ __forceinline__ void tiles_scores(const float* rows, const float* sq, float* St) {
@@ -108,10 +104,12 @@ __device__ __forceinline__ void tiles_scores(const float* rows, const float* sq,
 #pragma unroll
         for (int k = 0; k < 4; k++) {
             const int s = rg + 32 * i, j = tq + 8 * k;
-            St[tiles_at(s, j)] = tot[i][k];
+            St[s * 32 + ((((j >> 2) ^ (s & 7)) << 2) | (j & 3))] = tot[i][k];
         }
 }
-
+// place of (slot, token) in St / C: quads of tokens swapped around by slot, so that 8 neighbouring slots of one token (step
+// 2) and 4 neighbouring tokens of one slot (step 3, one 16-byte load) both miss each other's banks
+__device__ __forceinline__ int tiles_at(int s, int j) { return s * 32 + ((((j >> 2) ^ (s & 7)) << 2) | (j & 3)); }
 
 template <int DK, typename Tin>
 __global__ void __launch_bounds__(TL_THREADS) addr_bwd_tiles_kernel(
