@@ -54,15 +54,17 @@ static cudaError_t launch_wide(const slotscan_params& p, const void* q, const vo
 // sequences pass row 64: up to 128 rows always (T = 96 to 1024: 1.01 to 1.37 times as fast); past 128 rows, where it has six resolver
 // warps to wait for, from half of the tokens on (24 sequences, 192 rows x 128, T = 512, passed at 0.13 / 0.39 / 0.5 / 0.78 of
 // the tokens: 1.27 / 1.04 / 1.02 / 0.98).  A sequence passes row 64 after 64 tokens at the earliest, so below 192 tokens the
-// direct one takes it (T = 96: 0.94, T = 128: 0.97, T = 160: 0.98 to 1.06, T = 192: 0.96 to 1.12); with a state carried in
-// it may have passed already.
+// direct one takes it (T = 96: 0.94, T = 128: 0.97, T = 160: 0.98 to 1.06, T = 192: 0.96 to 1.12).  With a state carried in it
+// has passed already and every row is scanned from the first token on: the wide one takes a short call of however many
+// sequences (8 tokens, 444 sequences, 96 rows x 128: 63 us against 77 direct; 192 rows x 64: 66 against 86; 192 sequences, 96
+// rows x 64: 34 against 32), while in a long one the rounds count again (256 tokens, 296 sequences, 96 rows x 128: 362 against 306).
 template <int DK>
 static bool wide_second_pass(const slotscan_params& p, bool carry) {
     int dev = 0, sms = 148;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const size_t direct = sizeof(float) * (size_t)addr_fwd_layout(p.N, DK, 6, (int)sizeof(Tin)).total + 1024;
-    if ((long long)p.B * p.H > sms && 2 * direct <= 228 * 1024) return false;
+    if ((long long)p.B * p.H > sms && 2 * direct <= 228 * 1024 && (!carry || p.T >= 192)) return false;
     return p.N <= 128 || carry || p.T >= 192;
 }
 template <int DK>
