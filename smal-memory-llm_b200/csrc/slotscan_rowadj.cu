@@ -40,8 +40,8 @@ struct RowAdjShape {
 };
 
 // 168 registers for the 32-wide slices: 129 to 192 rows then run two CTAs to an SM where 255 would leave one, 65 to 96 three
-// instead of two (97 to 128: two either way, by shared memory; past 192 one).  What that spills (at most 0.5 KB a thread, at 16
-// tokens a step) costs less than the missing warps: 192 rows, 48 sequences x 4 slices, 0.60 -> 0.42 ms.  The 16-wide slices
+// instead of two (97 to 128: two either way, by shared memory; past 192 one).  What that spills (at most 146 bytes a thread,
+// at 16 tokens a step) costs less than the missing warps: 192 rows, 48 sequences x 4 slices, 0.60 -> 0.42 ms.  The 16-wide slices
 // (two warps at most) keep all they ask for.
 template <typename Tin, int CT, int DS, bool HARD>
 __global__ void __maxnreg__(DS == 32 ? 168 : 255) row_adjoint_kernel(const RowAdjArgs A) {
