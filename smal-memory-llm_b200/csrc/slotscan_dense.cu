@@ -5,7 +5,7 @@
 //
 // Soft address, up to 256 rows: the forward and, where it is detached, the backward with the token chain reduced to scalars
 // (slotscan_dense_chain.cuh) and the row gradients block by block (slotscan_rowadj.cuh).  B = 4, T = 512, H = 12,
-// 192 x (64 + 64), G = 16, soft, detached, forward + backward: 35.2 ms token by token (5.9 + 29.9), 2.00 ms so (forward 0.92;
+// 192 x (64 + 64), G = 16, soft, detached, forward + backward: 35.2 ms token by token (5.9 + 29.9), 1.96 ms so (forward 0.90;
 // backward: tables 0.34, row gradients 0.42, query gradient 0.22, softmax adjoint 0.04).
 // The token-by-token kernels below take the rest: a hard address, whose backward has to find the forward's addresses again;
 // more rows than 256, or more shared memory than a CTA has beside the chain's token buffers; and the backward of an
