@@ -15,6 +15,8 @@
 // another with five barriers each.  B = 32, T = 1024, H = 6, 192 rows x 128 all in use, bf16: 2.07 ms chunked, 1.33 ms here
 // (1.44 with scalar multiply-adds);
 // B = 4, T = 1000, H = 12, ~60 rows x 64, float32 (48 sequences, so that the chunked kernel had 48 CTAs): 1.29 -> 0.27 ms.
+// Where all of many sequences use 33 to 96 rows and fill the chunked kernel's rounds of two to an SM, that one is ahead: T = 256,
+// 60 rows x 128, chunked / tiles us: 148 sequences 229 / 196, 240: 264 / 309, 300: 456 / 391, 444: 509 / 551, 800: 759 / 976.
 // Persistent: the CTAs share the items of the sequences that need this kernel, which they find from the forward's tfirst
 // table (a launch whose sequences all use few rows returns after that look).
 #pragma once
