@@ -326,7 +326,7 @@ __global__ void __launch_bounds__(RD_THREADS, SPARSE ? 4 : 0) read_bwd_kernel(
     float* s_att = rsm + L.att;
     float* s_cf = rsm + L.cf;
     __shared__ int s_nv;
-    read_each_snapshot<SPARSE>(valid, N, (long long)p.B * NB * H, RB_SPARSE_ROWS, [&](const int so) {
+    auto work = [&](const int so) {                            // (b * NB + nb) * H + h
     const int h = so % H, nb = (so / H) % NB, b = so / (H * NB);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
 
@@ -505,7 +505,10 @@ __global__ void __launch_bounds__(RD_THREADS, SPARSE ? 4 : 0) read_bwd_kernel(
             dkinv[(size_t)so * N + n] = s;
         }
     }
-    });
+    };
+    // on its own: in place, through the function above it takes 1 to 2 % longer (24 x 330 tokens, 4 queries each: 4.28 ms, 4.20 so)
+    if constexpr (SPARSE) read_each_snapshot<true>(valid, N, (long long)p.B * NB * H, RB_SPARSE_ROWS, work);
+    else work((int)blockIdx.x);
 }
 
 template <typename Tq, typename Tsn>
