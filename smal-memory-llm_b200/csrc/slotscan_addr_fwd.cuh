@@ -114,7 +114,7 @@ __global__ void __launch_bounds__(AF_THREADS, (RPL <= 2 ? 3 : 1)) addr_fwd_direc
     float* __restrict__ oold_out, float* __restrict__ kiold_out, float* __restrict__ ofin, int* __restrict__ tfirst,
     const float* __restrict__ K0, const float* __restrict__ o0, const double* __restrict__ nsq0,
     double* __restrict__ nsqfin, const int ncap, const int second_pass) {
-    // Two-pass protocol.  Most sequences touch few rows, and a CTA that holds only `ncap` rows is small enough for every
+    // Passes (slotscan_addr_fwd_inst.cuh: launch_dk; keys 64 or 128 wide have the narrow kernel before this one).  Most sequences touch few rows, and a CTA that holds only `ncap` rows is small enough for every
     // (sequence, head) of a large batch to be resident at once.  Pass 1 (ncap < N) runs every sequence; one that
     // needs row ncap gives up, marks itself by tfirst[bh][0] = -1 and leaves.  Pass 2 (ncap = N, second_pass = 1)
     // redoes exactly the marked sequences from the start and returns at once for the others.
@@ -426,6 +426,10 @@ __global__ void __launch_bounds__(AF_THREADS, (RPL <= 2 ? 3 : 1)) addr_fwd_direc
     __syncthreads();
 
     // The two roles run separate loops (their register states never mix) and meet at one named barrier per token.
+    // A pass with fewer rows than N leaves a sequence to the next one where it has no room, and ahead of that where nearly every
+    // token has taken a new row (40 rows in 80 tokens, if at that pace it runs out before its end).
+    const int lead = second_pass && ncap < N ? min(2, T / ncap) : 0;
+    auto full = [&](int l, int t) { return l >= ncap || (l >= lim0 + 40 && t < lead * (l - lim0)); };
 #define AF_PHASE_BARRIER() asm volatile("bar.sync 1, %0;" ::"n"(AF_THREADS) : "memory")
     if (warp == 0) {
         for (int t = 0; t < T; t++) {
@@ -450,7 +454,7 @@ __global__ void __launch_bounds__(AF_THREADS, (RPL <= 2 ? 3 : 1)) addr_fwd_direc
             am_prev = am; Rb_prev = Rb; pslot = sl;
             pc = cc; cc = nc;
             AF_PHASE_BARRIER();
-            if (lim >= ncap) {                             // the next token may address a row this CTA does not hold
+            if (full(lim, t + 1)) {                        // the next token may address a row this CTA does not hold
                 if (lane == 0) tfirst[(size_t)bh * N] = -1;
                 return;                                    // the column warps read the same limit and leave too
             }
@@ -493,7 +497,7 @@ __global__ void __launch_bounds__(AF_THREADS, (RPL <= 2 ? 3 : 1)) addr_fwd_direc
             }
             AF_PHASE_BARRIER();
             lim = s_cur[t & 1];
-            if (lim >= ncap) return;
+            if (full(lim, t + 1)) return;
         }
     }
 #undef AF_PHASE_BARRIER

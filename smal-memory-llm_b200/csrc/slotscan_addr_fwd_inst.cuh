@@ -3,6 +3,7 @@
 #include <stdio.h>
 
 #include "slotscan_addr_fwd.cuh"
+#include "slotscan_addr_narrow.cuh"
 #include "slotscan_addr_wide.cuh"
 #include "slotscan_launch.h"
 
@@ -67,17 +68,51 @@ static bool wide_second_pass(const slotscan_params& p, bool carry) {
     if ((long long)p.B * p.H > sms && 2 * direct <= 228 * 1024 && (!carry || p.T >= 192)) return false;
     return p.N <= 128 || carry || p.T >= 192;
 }
+template <int DK, int CTAS>
+static cudaError_t launch_narrow(const slotscan_params& p, const void* q, const void* k, const float* gate, const float* fr,
+                                 const float* temp, const slotscan_log& L, const AddrFwdState& S0, cudaStream_t st) {
+    const size_t sm = sizeof(float) * (size_t)addr_narrow_layout(DK).total;
+    cudaError_t e = cudaSuccess;
+    auto go = [&](auto kern) {
+        if ((e = opt_in_smem(kern, sm)) != cudaSuccess) return e;
+        kern<<<p.B * p.H, AN_THREADS, sm, st>>>(p, (const Tin*)q, (const Tin*)k, gate, fr, temp, L.addr, L.oold, L.kiold, L.ofin,
+                                                L.tfirst, S0.K0, S0.o0, S0.nsq0, S0.nsqfin);
+        return cudaGetLastError();
+    };
+    const bool carry = S0.K0 != nullptr;
+    if (p.occ_bin) return carry ? go(addr_fwd_narrow_kernel<DK, CTAS, true, true, Tin>) : go(addr_fwd_narrow_kernel<DK, CTAS, true, false, Tin>);
+    return carry ? go(addr_fwd_narrow_kernel<DK, CTAS, false, true, Tin>) : go(addr_fwd_narrow_kernel<DK, CTAS, false, false, Tin>);
+}
+// The passes: keys 64 or 128 wide start with the narrow kernel (32 rows), the others with the direct one.  The direct one with 64
+// rows, three CTAs to an SM, takes what the narrow one left, and the full-size one the rest.  With at most a sequence per SM and
+// 192 tokens or a carried-in state the wide kernel follows the narrow one at once: by then a sequence that takes new rows at all
+// often has passed row 64 and would be scanned a third time (48 sequences x 1000 tokens, 64 wide: 83 us; 96 x 512, 128 wide: 110;
+// 24 carried-in x 8: 12).  One that stays between 32 and 64 rows loses by it: 148 sequences x 1024 tokens, 43 rows x 128: 825 us
+// against 696, 24 x 512, 34 rows x 64: 253 against 280.
 template <int DK>
 static cudaError_t launch_dk(const slotscan_params& p, const void* q, const void* k, const float* gate, const float* fr,
                              const float* temp, const slotscan_log& L, const AddrFwdState& S0, cudaStream_t st) {
-    if (p.N <= AF_NCAP1) return launch_one<DK, 2>(p, q, k, gate, fr, temp, L, S0, p.N, 0, st);
-    cudaError_t e = launch_one<DK, 2>(p, q, k, gate, fr, temp, L, S0, AF_NCAP1, 0, st);
-    if (e != cudaSuccess) return e;
+    cudaError_t e;
     if constexpr (DK >= 64) {
-        if (wide_second_pass<DK>(p, S0.K0 != nullptr)) {
+        int dev = 0, sms = 148;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        const long long BH = (long long)p.B * p.H;
+        if (BH <= 2 * sms) e = launch_narrow<DK, 2>(p, q, k, gate, fr, temp, L, S0, st);
+        else e = launch_narrow<DK, 3>(p, q, k, gate, fr, temp, L, S0, st);
+        if (e != cudaSuccess || p.N <= AN_ROWS) return e;
+        const bool wide = p.N > AF_NCAP1 && wide_second_pass<DK>(p, S0.K0 != nullptr);
+        if (!wide || BH > sms || (p.T < 192 && S0.K0 == nullptr)) {
+            e = launch_one<DK, 2>(p, q, k, gate, fr, temp, L, S0, p.N <= AF_NCAP1 ? p.N : AF_NCAP1, 1, st);
+            if (e != cudaSuccess || p.N <= AF_NCAP1) return e;
+        }
+        if (wide) {
             if (p.N <= 128) return launch_wide<DK, 4>(p, q, k, gate, fr, temp, L, S0, st);
             return launch_wide<DK, 6>(p, q, k, gate, fr, temp, L, S0, st);
         }
+    } else {
+        e = launch_one<DK, 2>(p, q, k, gate, fr, temp, L, S0, p.N <= AF_NCAP1 ? p.N : AF_NCAP1, 0, st);
+        if (e != cudaSuccess || p.N <= AF_NCAP1) return e;
     }
     return launch_one<DK, 6>(p, q, k, gate, fr, temp, L, S0, p.N, 1, st);         // N <= 192
 }

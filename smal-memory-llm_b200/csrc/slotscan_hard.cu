@@ -2,10 +2,11 @@
 // (hard argmax address, address gradient detached from the stored keys).
 //
 // Decomposition (the row a token writes is the only sequential decision):
-//   addr_fwd_direct_kernel (slotscan_addr_fwd.cuh)  one CTA per (sequence, head): keys resident in shared memory,
-//                      column warps and a resolver warp one token apart.                        [addr_fwd, slotkern_cuda.py:72-174]
-//   addr_fwd_wide_kernel (slotscan_addr_wide.cuh)   second pass, of sequences that use more than 64 rows: key rows in
-//                      registers, a resolver thread per row.
+//   addr_fwd_narrow_kernel (slotscan_addr_narrow.cuh)  first pass of keys 64 or 128 wide: one CTA per (sequence, head), at most 32
+//                      rows, in registers of the column warps; resolver, norm and loader warps.  [addr_fwd, slotkern_cuda.py:72-174]
+//   addr_fwd_direct_kernel (slotscan_addr_fwd.cuh)  keys resident in shared memory, column warps and a resolver warp one
+//                      token apart: 33 to 64 rows, other widths, all rows where two CTAs fit an SM.
+//   addr_fwd_wide_kernel (slotscan_addr_wide.cuh)   sequences that use more rows: key rows in registers, a resolver thread per row.
 //   replay_rows_kernel (slotscan_rows.cuh)  row-parallel: replays key / value rows from the log, emits the stride-G
 //                      snapshots, the undo log and the final state.                              [val_fwd :178-206]
 //   rows_bwd3_kernel, rows_bwd2_kernel (slotscan_rows_bwd.cuh)  row-parallel reverse scan: dK / dV recursion, dk / dv, the

@@ -337,6 +337,44 @@ def test_second_pass_rule(D, N, T, copies):
         assert torch.equal(a[n][:, :T].expand_as(b[n]), b[n]), n
 
 
+@pytest.mark.parametrize("D,dtype,occ_bin,copies", [(128, torch.bfloat16, True, 1), (64, torch.float32, False, 1),
+                                                    (128, torch.float32, True, 75), (64, torch.bfloat16, True, 75)],
+                         ids=lambda x: str(x).split(".")[-1])
+def test_narrow_address_scan_equals_the_next_pass_bitwise(D, dtype, occ_bin, copies):
+    """The first pass (at most 32 rows, a row split over 4, 2, 1 lanes below 8, 16, 32 rows) against the passes for more rows: the
+    same tokens alone, and followed by a tail that always takes a free row, after which the whole sequence is scanned again.
+    Same sums in the same order: the log of the tokens is the same bit for bit, at lengths around the staging of 8 tokens, from the
+    empty memory and with the state carried in, with few sequences (two CTAs to an SM) and many (three)."""
+    import slotscan_b200 as S
+    B, H, N, G, T, tail = 2, 3, 96, 8, 150, 48
+    inp = make_inputs("bench", B, T + tail, H, D, D, seed=23)
+    k, q, v = (inp[n].to("cuda", dtype) for n in ("k", "q", "v"))
+    g, fr = inp["gate"].cuda(), inp["fr"].cuda()
+    fr[:, :T] += torch.tensor([0.0, 0.6, 1.2], device="cuda") * (128 / D)         # a head each for up to 8, 16 and 32 rows
+    fr[:, T:] = 40.0
+    g[:, T:] = 1.0
+    kw = dict(G=G, occ_bin=occ_bin)
+    rows = set()
+    for t0, ends in ((0, (1, 7, 8, 9, 33, T)), (8, (10, 16, 23, T))):
+        state = None
+        if t0:
+            lg = S.scan_with_log(k[:, :t0], v[:, :t0], g[:, :t0], fr[:, :t0], N, 16.0, q=q[:, :t0], **kw)
+            state = tuple(lg[n].repeat(copies, *[1] * (lg[n].dim() - 1)) for n in ("kfin", "vfin", "ofin", "nsqfin"))
+        cut = lambda x, a, b: x[:, a:b].repeat(copies, *[1] * (x.dim() - 1)).contiguous()
+        run = lambda a, b: S.scan_with_log(*(cut(x, a, b) for x in (k, v, g, fr)), N, 16.0, q=cut(q, a, b), state=state, **kw)
+        a = run(t0, T + tail)
+        assert (a["tfirst"][:, 32] < T + tail - t0).all()          # redone by the next pass
+        for t1 in ends:
+            b = run(t0, t1)
+            n = (b["tfirst"] < t1 - t0).sum(-1)
+            assert int(n.max()) <= 32
+            rows.update(n.tolist())
+            for name in ("addr", "oold", "kiold", "kold"):
+                assert torch.equal(a[name][:, :t1 - t0], b[name]), (name, t0, t1)
+    if occ_bin:
+        assert min(rows) < 8 and max(rows) > 16
+
+
 @pytest.mark.parametrize("mode", ["hard", "soft", "keyless", "read"])
 def test_plain_calls_equal_registered_ops(mode, monkeypatch):
     """Ordinary eager calls go round the custom ops' wrapping; the same call through the ops gives the same bits, values and
