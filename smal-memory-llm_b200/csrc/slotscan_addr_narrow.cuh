@@ -243,8 +243,10 @@ __global__ void __launch_bounds__(AN_THREADS, CTAS) addr_fwd_narrow_kernel(
             const bool more = (c + 2) * AN_L < T;
             if (more) fetch(c + 2);
             if ((c + 1) * AN_L < T) consts(c + 1);
-            if (c >= 1) {                                 // the log of 8 tokens that are finished
-                const int t = (c - 1) * AN_L - 1 + (lane & 7);
+            // the log of 8 tokens: the resolver came here in the phase of token 8 c - 1, which the norm warp may still be in, and
+            // there it writes the entries of token 8 c - 2
+            if (c >= 1) {
+                const int t = (c - 1) * AN_L - 2 + (lane & 7);
                 if (t >= 0 && lane < 24 && half == 0) {
                     const size_t ix = ((size_t)b * T + t) * H + h;
                     const int sl = t & (AN_RING - 1);
@@ -544,7 +546,7 @@ __global__ void __launch_bounds__(AN_THREADS, CTAS) addr_fwd_narrow_kernel(
         if (nsqfin != nullptr) nsqfin[(size_t)bh * N + i] = 0.0;
     }
     {   // log entries not written out yet
-        const int t = max((T - 1) / AN_L * AN_L - 1, 0) + tid;
+        const int t = max((T - 1) / AN_L * AN_L - 2, 0) + tid;
         if (t < T) {
             const size_t ix = ((size_t)b * T + t) * H + h;
             const int sl = t & (AN_RING - 1);
