@@ -6,9 +6,9 @@
 
 namespace slotscan {
 
-template <int D, typename Tin, typename Tsn>
-static cudaError_t replay_one(const slotscan_params& p, int ntensors, const ReplayPtrs& r0, const ReplayPtrs& r1,
-                              const float* gate, const int* am, const int* tfirst, int tile_lo, int tile_hi, cudaStream_t st) {
+template <int D, int EPL, typename Tin, typename Tsn>
+static cudaError_t replay_launch(const slotscan_params& p, int ntensors, const ReplayPtrs& r0, const ReplayPtrs& r1,
+                                 const float* gate, const int* am, const int* tfirst, int tile_lo, int tile_hi, cudaStream_t st) {
     constexpr int RPB = ROW_THREADS / (D / 8);
     const int ntiles = (p.N + RPB - 1) / RPB;
     if (tile_hi < 0 || tile_hi > ntiles) tile_hi = ntiles;
@@ -16,7 +16,6 @@ static cudaError_t replay_one(const slotscan_params& p, int ntensors, const Repl
     dim3 grid(p.B * p.H, tile_hi - tile_lo, ntensors);
     const ReplayArgs<Tin, Tsn> a0{(const Tin*)r0.x, r0.x0, (Tsn*)r0.xbuf, r0.xold, r0.xfin, r0.kinv, r0.valid, r0.zero_from, r0.bits, r0.group};
     const ReplayArgs<Tin, Tsn> a1{(const Tin*)r1.x, r1.x0, (Tsn*)r1.xbuf, r1.xold, r1.xfin, r1.kinv, r1.valid, r1.zero_from, r1.bits, r1.group};
-    constexpr int EPL = D >= 128 ? 16 : 8;                 // elements per lane: half-size CTAs for the widest rows
     constexpr int THREADS = ROW_THREADS * 8 / EPL;
     if (r0.bits)
         replay_rows_kernel<D, Tin, Tsn, true, true, EPL><<<grid, THREADS, 0, st>>>(p, a0, a1, gate, am, tfirst, tile_lo);
@@ -25,6 +24,20 @@ static cudaError_t replay_one(const slotscan_params& p, int ntensors, const Repl
     else
         replay_rows_kernel<D, Tin, Tsn, false, false, EPL><<<grid, THREADS, 0, st>>>(p, a0, a1, gate, am, tfirst, tile_lo);
     return cudaGetLastError();
+}
+// Columns per lane of rows 128 wide: 8 while the busy tiles (one per sequence, head and tensor where few rows are in use) leave
+// SMs idle, 16 beyond that.
+template <int D, typename Tin, typename Tsn>
+static cudaError_t replay_one(const slotscan_params& p, int ntensors, const ReplayPtrs& r0, const ReplayPtrs& r1,
+                              const float* gate, const int* am, const int* tfirst, int tile_lo, int tile_hi, cudaStream_t st) {
+    if constexpr (D >= 128) {
+        int dev = 0, sms = 148;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        if ((long long)p.B * p.H * 2 > sms)
+            return replay_launch<D, 16, Tin, Tsn>(p, ntensors, r0, r1, gate, am, tfirst, tile_lo, tile_hi, st);
+    }
+    return replay_launch<D, 8, Tin, Tsn>(p, ntensors, r0, r1, gate, am, tfirst, tile_lo, tile_hi, st);
 }
 
 #define ROWS_TYPES(CALL_F32_F32, CALL_F32_BF16, CALL_BF16_F32, CALL_BF16_BF16)            \

@@ -35,13 +35,21 @@ __device__ __forceinline__ bool tile_active(const int* tfirst_bh, int n, bool li
 // ======================================================================================================
 // kinv / valid of a row from its float32 state: rsqrt(max(|X|^2, 1e-12)) and [|X|^2 > 1e-12]  [memlm_sh.py:474-475]
 // The rows of one warp walk their events independently, so the sum runs over the row's own LPR lanes only (`gmask`).
+// 16 lanes of 8 columns add up as 8 lanes of two pieces of 8 do: the upper half goes on from the lower half's sums.
 template <int LPR, int EPL>
 __device__ __forceinline__ float row_nsq(const float* X, unsigned gmask) {
     float a = 0.f;
 #pragma unroll
     for (int j = 0; j < EPL; j++) a = fmaf(X[j], X[j], a);
+    if constexpr (LPR == 16) {
+        float b = __shfl_xor_sync(gmask, a, 8);
 #pragma unroll
-    for (int off = LPR / 2; off > 0; off >>= 1) a += __shfl_xor_sync(gmask, a, off);
+        for (int j = 0; j < EPL; j++) b = fmaf(X[j], X[j], b);
+        const float c = __shfl_xor_sync(gmask, b, 8);
+        a = (threadIdx.x & 8u) ? b : c;
+    }
+#pragma unroll
+    for (int off = LPR >= 8 ? 4 : LPR / 2; off > 0; off >>= 1) a += __shfl_xor_sync(gmask, a, off);
     return a;
 }
 template <int LPR>
@@ -75,7 +83,8 @@ struct ReplayArgs {
 // passes of their own, 1.92 ms so; the write of four 1024-token chunks of 8 sequences in e4m3, forward: 6.7 -> 3.2 ms.
 // EPL: elements per lane, 8 or 16.  With 16 a lane holds two pieces of 8 columns half a row apart (every load and store
 // of a row group stays one contiguous run of 16-byte pieces) and a CTA has half the threads: the busy tiles of a large
-// batch (one CTA per sequence, head and tensor) then all fit on the machine at once instead of in two waves.
+// batch (one CTA per sequence, head and tensor) then all fit on the machine at once instead of in two waves.  The rows of a warp
+// walk their events one after the other, so a batch that leaves SMs idle anyway is faster with 8 (slotscan_rows.cu: replay_one).
 template <int D, typename Tin, typename Tsn, bool NORM, bool QUANT, int EPL>
 __global__ void __launch_bounds__(ROW_THREADS * 8 / EPL, EPL == 16 ? (QUANT ? 4 : 6) : 1) replay_rows_kernel(
     const slotscan_params p, const ReplayArgs<Tin, Tsn> a0, const ReplayArgs<Tin, Tsn> a1,

@@ -261,3 +261,29 @@ def test_quantised_write_equals_scan_then_quantiser(case, dtypes, monkeypatch):
         assert (x.float() - y.float()).abs().max() <= band * y.float().abs().max(), n
     from slotscan_b200 import _lib
     assert _lib.device_status() == 0
+
+
+@pytest.mark.parametrize("D,bits,group", [(128, 0, 16), (128, 3, 128), (128, "e4m3", 16)])
+def test_replay_lane_split_is_bitwise(D, bits, group):
+    """The replay takes rows of 128 with 16 lanes each while two tiles per sequence leave SMs idle and with 8 beyond: the same rows,
+    norms and gradients bit for bit on both sides of the line, at a length that is no multiple of the staged chunk."""
+    S = _S()
+    H, N, G, T = 3, 40, 8, 75
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    B = sms // (2 * H) + 1                                              # 2 * B * H just past the SMs; one sequence less: not
+    inp = make_inputs("clustered", B, T, H, D, D, seed=8)
+    dev = [inp[n].to(DEV, torch.bfloat16 if n in ("k", "v", "q") else torch.float32) for n in ("k", "v", "gate", "fr", "q")]
+    gen = torch.Generator(device=DEV).manual_seed(3)
+    ups = [torch.randn(B, (T + G - 1) // G, H, N, *e, device=DEV, generator=gen).to(dt)
+           for e, dt in (((D,), torch.bfloat16), ((D,), torch.bfloat16), ((), torch.float32))]
+
+    def once(n):
+        x = [t[:n].contiguous().requires_grad_() for t in dev]
+        out = S.write_memory(x[0], x[1], x[2], x[3], N, 16.0, G=G, q=x[4], occ_bin=True, out_dtype=torch.bfloat16, qbits=bits,
+                             qgroup=group)
+        g = torch.autograd.grad(list(out[:3]), x, [u[:n].contiguous() for u in ups])
+        return [o.detach() for o in out] + list(g)
+    many, few = once(B), once(B - 1)
+    assert 2 * (B - 1) * H <= sms < 2 * B * H
+    for a, b in zip(many, few):
+        assert torch.equal(a[:B - 1], b)
