@@ -89,6 +89,16 @@ static cudaError_t launch_narrow(const slotscan_params& p, const void* q, const 
 // often has passed row 64 and would be scanned a third time (48 sequences x 1000 tokens, 64 wide: 83 us; 96 x 512, 128 wide: 110;
 // 24 carried-in x 8: 12).  One that stays between 32 and 64 rows loses by it: 148 sequences x 1024 tokens, 43 rows x 128: 825 us
 // against 696, 24 x 512, 34 rows x 64: 253 against 280.
+// The exception: the zero-fill of the snapshots runs beside the scan, and the replay behind the scan contends with it for the memory.
+// Where the fill is expected to outlast the direct kernel (its rate beside a scan, 4.66 MB per us, against 0.74 us per token and round
+// of three CTAs to an SM), a faster scan only brings that on earlier: 384 sequences x 1024 tokens, 192 rows x 128, bf16, forward and
+// backward 2.03 ms with the narrow pass first, 2.00 with the direct one.
+static bool behind_the_fill(const slotscan_params& p, int sms) {
+    const double snaps = (double)p.B * p.H * ((p.T + p.G - 1) / p.G), esz = p.snap_dtype == SLOTSCAN_F32 ? 4.0 : 2.0;
+    const double fill_us = snaps * (p.N - 16) * (p.DK + p.DV) * esz / 4.66e6;
+    const long long rounds = ((long long)p.B * p.H + 3 * sms - 1) / (3 * sms);
+    return fill_us > 0.74 * (double)p.T * (double)rounds;
+}
 template <int DK>
 static cudaError_t launch_dk(const slotscan_params& p, const void* q, const void* k, const float* gate, const float* fr,
                              const float* temp, const slotscan_log& L, const AddrFwdState& S0, cudaStream_t st) {
@@ -98,12 +108,16 @@ static cudaError_t launch_dk(const slotscan_params& p, const void* q, const void
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
         const long long BH = (long long)p.B * p.H;
-        if (BH <= 2 * sms) e = launch_narrow<DK, 2>(p, q, k, gate, fr, temp, L, S0, st);
-        else e = launch_narrow<DK, 3>(p, q, k, gate, fr, temp, L, S0, st);
-        if (e != cudaSuccess || p.N <= AN_ROWS) return e;
+        int second = 0;                                   // this pass takes the sequences that the one before it marked
+        if (BH <= 2 * sms || S0.K0 != nullptr || p.N <= AF_NCAP1 || !behind_the_fill(p, sms)) {
+            if (BH <= 2 * sms) e = launch_narrow<DK, 2>(p, q, k, gate, fr, temp, L, S0, st);
+            else e = launch_narrow<DK, 3>(p, q, k, gate, fr, temp, L, S0, st);
+            if (e != cudaSuccess || p.N <= AN_ROWS) return e;
+            second = 1;
+        }
         const bool wide = p.N > AF_NCAP1 && wide_second_pass<DK>(p, S0.K0 != nullptr);
         if (!wide || BH > sms || (p.T < 192 && S0.K0 == nullptr)) {
-            e = launch_one<DK, 2>(p, q, k, gate, fr, temp, L, S0, p.N <= AF_NCAP1 ? p.N : AF_NCAP1, 1, st);
+            e = launch_one<DK, 2>(p, q, k, gate, fr, temp, L, S0, p.N <= AF_NCAP1 ? p.N : AF_NCAP1, second, st);
             if (e != cudaSuccess || p.N <= AF_NCAP1) return e;
         }
         if (wide) {
