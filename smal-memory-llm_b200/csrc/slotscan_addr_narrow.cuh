@@ -483,7 +483,6 @@ __global__ void __launch_bounds__(AN_THREADS, CTAS) addr_fwd_narrow_kernel(
         __syncthreads();
         __syncthreads();
         float kinv = fminf(rsqrtf((float)nsq), 1e6f), g1 = 0.f, om1 = 0.f;
-        if (lane >= ncap) o = NAN;                        // a row not held is neither occupied nor free
         const unsigned below = (1u << lane) - 1u;
         int t = 0, a1 = -1;                               // the previous token's address
         bool left = false, none = false;
@@ -507,8 +506,8 @@ __global__ void __launch_bounds__(AN_THREADS, CTAS) addr_fwd_narrow_kernel(
                 // product, product, difference, each rounded: as the direct kernel's expression comes out
                 const float sc = __fmul_rn(c4.x, __fmul_rn(kinv, S));
                 const float z = OCCB ? __fsub_rn(sc, occ ? c4.y : 0.f) : __fmaf_rn(-c4.y, o, sc);
-                // candidates: occupied rows and the lowest free one
-                const float zc = occ || (isfree && !(fm & below)) ? z : -INFINITY;
+                // candidates: occupied rows and the lowest free one, of those up to row lim (with eps <= 0 every row is occupied)
+                const float zc = lane <= lim && (occ || (isfree && !(fm & below))) ? z : -INFINITY;
                 const float zm = redux_max(zc);
                 a1 = __ffs((int)__ballot_sync(FULL, zc == zm)) - 1;           // the lowest row of the largest score
                 none = !(zm > -INFINITY);                 // no candidate compares greater (NaN scores): row lim

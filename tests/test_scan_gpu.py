@@ -375,6 +375,29 @@ def test_narrow_address_scan_equals_the_next_pass_bitwise(D, dtype, occ_bin, cop
         assert min(rows) < 8 and max(rows) > 16
 
 
+@pytest.mark.parametrize("D,dist,N,eps,occ_bin", [(128, "clustered", 24, 0.0, True), (64, "clustered", 40, 0.0, False),
+                                                  (64, "bench", 17, -1.0, True), (128, "fill", 24, 1e-4, True)])
+def test_every_row_or_none_counts_as_occupied(D, dist, N, eps, occ_bin):
+    """A threshold of zero or less makes every row occupied, rows never written among them; and a memory of at most 32 rows that is
+    full.  The addresses are the oracle's and the final rows its rows (1e-5, as the other float32 cases), with few sequences and with
+    many, where the scan's kernels split a row over the lanes in other ways.  (Rows never written tie: the lowest is taken, so the
+    addresses are compared as they are; the oracle's own two precisions agree on them, so none is a near-tie.)"""
+    import slotscan_b200 as S
+    B, T, H, copies = 2, 100, 3, 75
+    inp = make_inputs(dist, B, T, H, D, D, seed=3)
+    kw = dict(N=N, temp=16.0, G=8, hard=True, q=inp["q"], occ_bin=occ_bin, eps=eps)
+    ref = O.scan_fwd(inp["k"], inp["v"], inp["gate"], inp["fr"], dtype=np.float64, **kw)
+    assert np.array_equal(ref["addr"], O.scan_fwd(inp["k"], inp["v"], inp["gate"], inp["fr"], dtype=np.float32, **kw)["addr"])
+    for n in (1, copies):
+        x = [inp[i].repeat(n, *[1] * (inp[i].dim() - 1)).cuda() for i in ("k", "v", "gate", "fr", "q")]
+        lg = S.scan_with_log(*x[:4], N, 16.0, G=8, q=x[4], occ_bin=occ_bin, eps=eps)
+        addr = lg["addr"].view(n, B, T, H).cpu().numpy()
+        assert (addr == ref["addr"]).all(), n
+        for name in ("kfin", "vfin", "ofin"):
+            got = lg[name].view(n, *ref[name].shape).cpu().numpy()
+            assert np.abs(got - ref[name]).max() < 1e-5, (name, n)
+
+
 @pytest.mark.parametrize("mode", ["hard", "soft", "keyless", "read"])
 def test_plain_calls_equal_registered_ops(mode, monkeypatch):
     """Ordinary eager calls go round the custom ops' wrapping; the same call through the ops gives the same bits, values and
