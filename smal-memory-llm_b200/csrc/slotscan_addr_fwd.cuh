@@ -328,7 +328,7 @@ __global__ void __launch_bounds__(AF_THREADS, (RPL <= 2 ? 3 : 1)) addr_fwd_direc
             }                                                                                                  \
         }                                                                                                      \
         o_new = __shfl_sync(FULL, o_new, am_prev & 31);                                                        \
-        if (am_prev == fe && o_new >= eps) {               /* the free row got taken: find the next one */     \
+        if (am_prev == fe && !(o_new < eps)) {             /* the free row got taken (or lost to a NaN): the next one */ \
             int m = BIGI;                                                                                      \
             _Pragma("unroll") for (int s = RPL - 1; s >= 0; s--) {                                             \
                 const int n = lane + 32 * s;                                                                   \

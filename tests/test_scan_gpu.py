@@ -398,6 +398,24 @@ def test_every_row_or_none_counts_as_occupied(D, dist, N, eps, occ_bin):
             assert np.abs(got - ref[name]).max() < 1e-5, (name, n)
 
 
+@pytest.mark.parametrize("D", [32, 128])
+def test_nan_gate_does_not_hold_the_free_row(D):
+    """A row whose occupancy a NaN gate destroyed is neither free nor occupied, as in the oracle: the tokens after it take the next
+    free row, with few sequences and with many, whichever kernel scans them first."""
+    import slotscan_b200 as S
+    B, T, H, N, copies = 2, 64, 3, 192, 75
+    inp = make_inputs("bench", B, T, H, D, D, seed=5)
+    inp["gate"][:, [2, 3, 17, 40]] = float("nan")
+    kw = dict(N=N, temp=16.0, G=8, hard=True, q=inp["q"], occ_bin=True)
+    ref = O.scan_fwd(inp["k"], inp["v"], inp["gate"], inp["fr"], dtype=np.float64, **kw)
+    assert np.array_equal(ref["addr"], O.scan_fwd(inp["k"], inp["v"], inp["gate"], inp["fr"], dtype=np.float32, **kw)["addr"])
+    for n in (1, copies):
+        x = [inp[i].repeat(n, *[1] * (inp[i].dim() - 1)).cuda() for i in ("k", "v", "gate", "fr", "q")]
+        lg = S.scan_with_log(*x[:4], N, 16.0, G=8, q=x[4], occ_bin=True)
+        assert (lg["addr"].view(n, B, T, H).cpu().numpy() == ref["addr"]).all(), n
+        assert np.array_equal(torch.isnan(lg["ofin"]).view(n, *ref["ofin"].shape)[-1].cpu().numpy(), np.isnan(ref["ofin"])), n
+
+
 @pytest.mark.parametrize("mode", ["hard", "soft", "keyless", "read"])
 def test_plain_calls_equal_registered_ops(mode, monkeypatch):
     """Ordinary eager calls go round the custom ops' wrapping; the same call through the ops gives the same bits, values and
