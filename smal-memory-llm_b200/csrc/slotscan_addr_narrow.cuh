@@ -505,7 +505,8 @@ __global__ void __launch_bounds__(AN_THREADS, CTAS) addr_fwd_narrow_kernel(
                 const unsigned fm = __ballot_sync(FULL, isfree);
                 // product, product, difference, each rounded: as the direct kernel's expression comes out
                 const float sc = __fmul_rn(c4.x, __fmul_rn(kinv, S));
-                const float z = OCCB ? __fsub_rn(sc, occ ? c4.y : 0.f) : __fmaf_rn(-c4.y, o, sc);
+                // (a penalty that is infinite or NaN is NaN on a row that is not occupied too: times zero, not left out)
+                const float z = OCCB ? __fsub_rn(sc, occ ? c4.y : __fmul_rn(c4.y, 0.f)) : __fmaf_rn(-c4.y, o, sc);
                 // candidates: occupied rows and the lowest free one, of those up to row lim (with eps <= 0 every row is occupied)
                 const float zc = lane <= lim && (occ || (isfree && !(fm & below))) ? z : -INFINITY;
                 const float zm = redux_max(zc);

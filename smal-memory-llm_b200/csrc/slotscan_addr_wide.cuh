@@ -294,7 +294,7 @@ __global__ void __launch_bounds__(aw_threads(RPL), 1) addr_fwd_wide_kernel(
             }
             // product, product, difference, each rounded: as the direct kernel's expression comes out
             const float sc = __fmul_rn(c4.x, __fmul_rn(kinv, S));
-            const float z = (OCCB ? __fsub_rn(sc, o >= eps ? c4.y : 0.f) : __fmaf_rn(-c4.y, o, sc)) + 0.f;
+            const float z = (OCCB ? __fsub_rn(sc, o >= eps ? c4.y : __fmul_rn(c4.y, 0.f)) : __fmaf_rn(-c4.y, o, sc)) + 0.f;
             const bool ok = n <= lim && (o >= eps || n == fe) && z > -INFINITY;
             const unsigned key = ok ? ord_key(z) : 0u;
             if (act) {

@@ -416,6 +416,29 @@ def test_nan_gate_does_not_hold_the_free_row(D):
         assert np.array_equal(torch.isnan(lg["ofin"]).view(n, *ref["ofin"].shape)[-1].cpu().numpy(), np.isnan(ref["ofin"])), n
 
 
+@pytest.mark.parametrize("dist,N,T", [("gates01", 192, 64), ("gates01:6", 96, 200)])
+def test_penalty_without_a_value(dist, N, T):
+    """An infinite or NaN penalty leaves no candidate that compares greater, whichever kernel scans the sequence (the direct one among
+    many sequences, the others among few): the token takes the first row never addressed, not a free one below it that a gate of
+    zero left, and the log is the same bit for bit."""
+    import slotscan_b200 as S
+    B, H, D, copies = 2, 3, 128, 75
+    inp = make_inputs(dist, B, T, H, D, D, seed=5)
+    bad = {5: float("inf"), 20: float("nan"), 21: float("nan"), 41: float("inf")}
+    for t, x in bad.items():
+        inp["fr"][:, t] = x
+    logs = []
+    for n in (1, copies):
+        x = [inp[i].repeat(n, *[1] * (inp[i].dim() - 1)).cuda() for i in ("k", "v", "gate", "fr", "q")]
+        lg = S.scan_with_log(*x[:4], N, 16.0, G=8, q=x[4], occ_bin=True)
+        logs.append({i: lg[i].view(n, B, T, H).cpu() for i in ("addr", "oold", "kiold")})
+    a = logs[0]["addr"][0]
+    for t in bad:
+        assert torch.equal(a[:, t], (a[:, :t].amax(1) + 1).clamp(max=N - 1)), t
+    for i in logs[0]:
+        assert torch.equal(logs[0][i].expand_as(logs[1][i]), logs[1][i]), i
+
+
 @pytest.mark.parametrize("mode", ["hard", "soft", "keyless", "read"])
 def test_plain_calls_equal_registered_ops(mode, monkeypatch):
     """Ordinary eager calls go round the custom ops' wrapping; the same call through the ops gives the same bits, values and
