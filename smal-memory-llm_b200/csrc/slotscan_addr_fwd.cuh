@@ -106,18 +106,32 @@ __device__ __forceinline__ void af_token_consts(const Ts* __restrict__ qrow, con
     }
 }
 
+// Passes.  Most sequences touch few rows, and a CTA that holds only `ncap` of them is smaller and faster, so a scan is a chain of
+// kernels that hold ever more rows (slotscan_addr_fwd_inst.cuh: launch_dk).  Each returns at once for a sequence that is finished
+// (tfirst[bh][0] = 0).  One whose next token t may address row ncap is marked by tfirst[bh][0] = af_mark(t) and left to the next kernel,
+// which goes on there.  Occupancies and squared norms are handed over in ofin and nsqfin as they are before token t, the log of the
+// tokens up to it is complete, and the key rows 0 to ncap - 1 lie in `hand` (the final key rows' place, written by the replay later)
+// without the write of token t - 1: the dots of token t have not seen that write in one kernel that scans it all either, so sums and
+// roundings are the same.  Mark 0: from the start (a carried-in state already needs more rows, or hand is NULL).
+__device__ __forceinline__ int af_mark(int t) { return -1 - t; }
+struct AfResume {
+    bool on;                                              // go on at token t0, the write of the token before it still open
+    int t0, am;                                           // am: the row it addressed, the highest in use
+    __device__ __forceinline__ AfResume(int mark, const int* am_out, size_t ix0, int H) {
+        t0 = -1 - mark;
+        on = t0 > 0;
+        am = on ? am_out[ix0 + (size_t)(t0 - 1) * H] : -1;
+    }
+};
+
 // RPL = row slots per lane (N <= 32 * RPL); CARRY: the scan starts from a state carried in from a preceding chunk
 template <int DK, int RPL, bool OCCB, bool CARRY, typename Tin>
-__global__ void __launch_bounds__(AF_THREADS, (RPL <= 2 ? 3 : 1)) addr_fwd_direct_kernel(
+__global__ void __launch_bounds__(AF_THREADS, (RPL <= 2 ? 3 : 2)) addr_fwd_direct_kernel(
     const slotscan_params p, const Tin* __restrict__ q, const Tin* __restrict__ k, const float* __restrict__ gate,
     const float* __restrict__ fr, const float* __restrict__ temp_p, int* __restrict__ am_out,
     float* __restrict__ oold_out, float* __restrict__ kiold_out, float* __restrict__ ofin, int* __restrict__ tfirst,
     const float* __restrict__ K0, const float* __restrict__ o0, const double* __restrict__ nsq0,
-    double* __restrict__ nsqfin, const int ncap, const int second_pass) {
-    // Passes (slotscan_addr_fwd_inst.cuh: launch_dk; keys 64 or 128 wide have the narrow kernel before this one).  Most sequences touch few rows, and a CTA that holds only `ncap` rows is small enough for every
-    // (sequence, head) of a large batch to be resident at once.  Pass 1 (ncap < N) runs every sequence; one that
-    // needs row ncap gives up, marks itself by tfirst[bh][0] = -1 and leaves.  Pass 2 (ncap = N, second_pass = 1)
-    // redoes exactly the marked sequences from the start and returns at once for the others.
+    double* __restrict__ nsqfin, const int ncap, const int second_pass, float* __restrict__ hand) {
     extern __shared__ __align__(16) float smem[];
     constexpr int C = af_ch(RPL);                         // tokens per staged chunk
     constexpr int RING = 2 * C;                           // token t lives in slot t % RING of every per-token array
@@ -130,7 +144,7 @@ __global__ void __launch_bounds__(AF_THREADS, (RPL <= 2 ? 3 : 1)) addr_fwd_direc
     // per token, so unpacking bf16 there costs as many instructions as the dots themselves: the small variant converts
     // once per chunk instead.  The full-size variant keeps the input dtype to save shared memory.
     typedef typename std::conditional<(RPL <= 2), float, Tin>::type Ts;
-    const int N = p.N, T = p.T, H = p.H;
+    const int N = p.N, H = p.H;
     const AddrFwdSmem L = addr_fwd_layout(ncap, DK, RPL, (int)sizeof(Tin));
     const int KS = L.kstride;
     float* K = smem + L.K;
@@ -153,15 +167,32 @@ __global__ void __launch_bounds__(AF_THREADS, (RPL <= 2 ? 3 : 1)) addr_fwd_direc
     const bool wact = warp >= 1 && c0 < DK;
     const float temp = temp_p[0], eps = p.eps;
 
-    if (second_pass && tfirst[(size_t)bh * N] != -1) return;          // finished in the first pass (uniform per CTA)
+    const int mark = second_pass ? tfirst[(size_t)bh * N] : af_mark(0);
+    if (mark >= 0) return;                                            // finished in an earlier pass (uniform per CTA)
+    const AfResume rs(mark, am_out, (size_t)b * p.T * H + h, H);
+    const int T = p.T - rs.t0;                                        // tokens are counted from rs.t0 on
+    const size_t bT = (size_t)b * p.T + rs.t0;
     __syncthreads();
     for (int i = tid; i < ncap * KS; i += AF_THREADS) K[i] = 0.f;
-    for (int i = tid; i < DK; i += AF_THREADS) Ks[(RING - 1) * DK + i] = (Ts)0.f;    // "the key before token 0"
+    for (int i = tid; i < DK; i += AF_THREADS)                        // "the key before token 0"
+        Ks[(RING - 1) * DK + i] = rs.on ? (Ts)(float)k[((bT - 1) * H + h) * DK + i] : (Ts)0.f;
+    if (rs.on && tid == 0) {                                          // that token's row and gate
+        s_am[RING - 1] = rs.am;
+        s_tok[4 * (RING - 1) + 2] = gate_eff(gate[(bT - 1) * H + h], p.hard_gate);
+    }
     // State carried in from a preceding chunk (K0 / o0, optionally the squared key norms as that scan carried them).
     // hw0 = the highest row it has touched: rows above it are exactly zero, as in a scan from the empty memory.
-    int hw0 = -1;
+    int hw0 = rs.am;
     double* s_nsq = reinterpret_cast<double*>(smem + L.part);         // N doubles, before `part` is first written
-    if (CARRY) {
+    if (rs.on) {
+        __syncthreads();
+        for (int i = tid; i <= rs.am; i += AF_THREADS) s_nsq[i] = nsqfin[(size_t)bh * N + i];
+        for (int i = tid; i < (rs.am + 1) * (DK / 4); i += AF_THREADS) {
+            const int n = i / (DK / 4), c = 4 * (i - n * (DK / 4));
+            st4(K + (size_t)n * KS + c, ld4(hand + ((size_t)bh * N + n) * DK + c));
+        }
+        __syncthreads();
+    } else if (CARRY) {
         for (int n = warp; n < N; n += AF_WARPS) {
             double a = 0.0;
             if (nsq0 != nullptr) {
@@ -184,10 +215,14 @@ __global__ void __launch_bounds__(AF_THREADS, (RPL <= 2 ? 3 : 1)) addr_fwd_direc
             K[(size_t)n * KS + c] = K0[((size_t)bh * N + n) * DK + c];
         }
     }
-    const int lim0 = CARRY ? min(hw0 + 1, N - 1) : 0;                 // candidate limit of token 0
-    for (int i = tid; i < N; i += AF_THREADS) tfirst[(size_t)bh * N + i] = (i <= hw0 + 1) ? 0 : T;
-    if (CARRY && lim0 >= ncap) {                                      // the carried-in state already needs more rows
-        if (tid == 0) tfirst[(size_t)bh * N] = -1;
+    const int lim0 = CARRY || rs.on ? min(hw0 + 1, N - 1) : 0;        // candidate limit of the first token to be resolved
+    if (rs.on) {
+        if (tid == 0) tfirst[(size_t)bh * N] = 0;                     // the others stand as the pass before left them
+    } else {
+        for (int i = tid; i < N; i += AF_THREADS) tfirst[(size_t)bh * N + i] = (i <= hw0 + 1) ? 0 : T;
+    }
+    if (CARRY && !rs.on && lim0 >= ncap) {                            // the carried-in state already needs more rows
+        if (tid == 0) tfirst[(size_t)bh * N] = af_mark(0);
         return;
     }
 
@@ -200,13 +235,13 @@ __global__ void __launch_bounds__(AF_THREADS, (RPL <= 2 ? 3 : 1)) addr_fwd_direc
             const int id_ = ltid + r_ * LT;                                                                \
             if (id_ < 2 * IPS) {                                                                           \
                 const int s_ = id_ / IPS, rr_ = id_ % IPS, j_ = rr_ / (DK / 8), c_ = (rr_ % (DK / 8)) * 8; \
-                if ((T0) + j_ < T) pre[r_].load((s_ ? k : q) + (((size_t)b * T + (T0) + j_) * H + h) * DK + c_); \
+                if ((T0) + j_ < T) pre[r_].load((s_ ? k : q) + ((bT + (T0) + j_) * H + h) * DK + c_); \
                 else pre[r_].zero();                                                                       \
             }                                                                                              \
         }                                                                                                  \
         if (ltid < 2 * C) {                                                                                \
             const int tt_ = (T0) + (ltid & (C - 1));                                                       \
-            const size_t ix_ = ((size_t)b * T + tt_) * H + h;                                              \
+            const size_t ix_ = (bT + tt_) * H + h;                                              \
             if (ltid < C) pre_s = (tt_ < T) ? gate[ix_] : 0.f;   /* no arithmetic: the load stays in flight */ \
             else pre_s = (tt_ < T) ? (p.fr_per_token ? fr[ix_] : fr[0]) : 0.f;                             \
         }                                                                                                  \
@@ -313,7 +348,7 @@ __global__ void __launch_bounds__(AF_THREADS, (RPL <= 2 ? 3 : 1)) addr_fwd_direc
     // warp 0: the bookkeeping of the token resolved in the previous phase (am_prev, its constants in pc, the owner
     // lane's <K_am, k> in Rb_prev).  The owner lane is the one that holds row am_prev.
 #define AF_FINISH_PREV(NS)                                                                                     \
-    if (am_prev >= 0) {                                                                                        \
+    {                                                                                                          \
         const bool owner_ = (am_prev & 31) == lane;                                                            \
         const int ai_ = am_prev >> 5;                                                                          \
         float o_new = 0.f;                                                                                     \
@@ -346,7 +381,7 @@ __global__ void __launch_bounds__(AF_THREADS, (RPL <= 2 ? 3 : 1)) addr_fwd_direc
         _Pragma("unroll") for (int s = 0; s < (NS); s++)                                                       \
             _Pragma("unroll") for (int w = 0; w < AF_CWARPS; w++)                                              \
                 if (w * CW < DK) pr[s][w] = part[(((BUF) * RPL + s) * AF_CWARPS + w) * 32 + lane];             \
-        AF_FINISH_PREV(NS)                                                                                     \
+        if (t > 0) AF_FINISH_PREV(NS)                                                                          \
         float bz = -INFINITY;                                                                                  \
         int bi = BIGI;                                                                                         \
         Rb = 0.f;                                                                                              \
@@ -387,22 +422,24 @@ __global__ void __launch_bounds__(AF_THREADS, (RPL <= 2 ? 3 : 1)) addr_fwd_direc
 #pragma unroll
     for (int s = 0; s < RPL; s++) { nsq_r[s] = 0.0; kinv_r[s] = 1e6f; o_r[s] = 0.f; }
     int hw = hw0, fe = 0, lim = lim0;                     // highest row touched; lowest free row (N if none)
-    if (CARRY && warp == 0) {
+    if ((CARRY || rs.on) && warp == 0) {
         int m = BIGI;
 #pragma unroll
         for (int s = RPL - 1; s >= 0; s--) {
             const int n = lane + 32 * s;
             if (n < N) {
-                nsq_r[s] = s_nsq[n];
-                kinv_r[s] = fminf(rsqrtf((float)nsq_r[s]), 1e6f);
-                o_r[s] = o0[(size_t)bh * N + n];
+                if (!rs.on || n <= rs.am) {
+                    nsq_r[s] = s_nsq[n];
+                    kinv_r[s] = fminf(rsqrtf((float)nsq_r[s]), 1e6f);
+                    o_r[s] = (rs.on ? ofin : o0)[(size_t)bh * N + n];
+                }
                 if (o_r[s] < eps) m = n;
             }
         }
         m = (int)__reduce_min_sync(FULL, (unsigned)m);
         fe = (m == BIGI) ? N : m;
     }
-    int am_prev = -1, pslot = 0;                          // the token whose bookkeeping is still open
+    int am_prev = rs.am, pslot = 0;                       // the token whose bookkeeping is still open (from token 1 on)
     float Rb_prev = 0.f;
     TokC cc = {}, pc = {}, nc = {};                       // constants of the current, previous and next token
 
@@ -419,21 +456,20 @@ __global__ void __launch_bounds__(AF_THREADS, (RPL <= 2 ? 3 : 1)) addr_fwd_direc
     }
     __syncthreads();
     if (wact) {
-        if (CARRY) { AF_DOTS_DISPATCH(lim0, 0, 0) }
+        if (CARRY || rs.on) { AF_DOTS_DISPATCH(lim0, 0, 0) }
         else { AF_DOTS_SPLIT(4, 0, 0) }
     }
-    if (warp == 0) AF_LOAD_CONSTS(cc, 0);
+    if (warp == 0) {
+        AF_LOAD_CONSTS(cc, 0);
+        pc.g = s_tok[4 * (RING - 1) + 2];                 // token 0 repairs the open write's row, if there is one
+    }
     __syncthreads();
 
     // The two roles run separate loops (their register states never mix) and meet at one named barrier per token.
-    // A pass with fewer rows than N leaves a sequence to the next one where it has no room, and ahead of that where nearly every
-    // token has taken a new row (40 rows in 80 tokens, if at that pace it runs out before its end).
-    const int lead = second_pass && ncap < N ? min(2, T / ncap) : 0;
-    auto full = [&](int l, int t) { return l >= ncap || (l >= lim0 + 40 && t < lead * (l - lim0)); };
 #define AF_PHASE_BARRIER() asm volatile("bar.sync 1, %0;" ::"n"(AF_THREADS) : "memory")
     if (warp == 0) {
         for (int t = 0; t < T; t++) {
-            const int sl = t & (RING - 1);
+            const int sl = t & (RING - 1), jj = t & (C - 1);
             if (t + 1 < T) AF_LOAD_CONSTS(nc, (t + 1) & (RING - 1));
             int am = 0;
             float Rb = 0.f;
@@ -444,7 +480,7 @@ __global__ void __launch_bounds__(AF_THREADS, (RPL <= 2 ? 3 : 1)) addr_fwd_direc
             else AF_RESOLVE(RPL, t & 1)
             if (am > hw) {
                 hw = am;
-                if (lane == 0 && am + 1 < N) tfirst[(size_t)bh * N + am + 1] = t + 1;
+                if (lane == 0 && am + 1 < N) tfirst[(size_t)bh * N + am + 1] = rs.t0 + t + 1;
             }
             lim = min(hw + 1, N - 1);                      // the next token's candidate limit
             if (lane == 0) {
@@ -454,8 +490,25 @@ __global__ void __launch_bounds__(AF_THREADS, (RPL <= 2 ? 3 : 1)) addr_fwd_direc
             am_prev = am; Rb_prev = Rb; pslot = sl;
             pc = cc; cc = nc;
             AF_PHASE_BARRIER();
-            if (full(lim, t + 1)) {                        // the next token may address a row this CTA does not hold
-                if (lane == 0) tfirst[(size_t)bh * N] = -1;
+            if (RPL <= 2 && lim >= ncap && t + 1 < T) {    // the next token may address a row this CTA does not hold
+                if (hand != nullptr) {
+                    AF_FINISH_PREV(RPL)
+#pragma unroll
+                    for (int s = 0; s < RPL; s++) {
+                        ofin[(size_t)bh * N + lane + 32 * s] = o_r[s];
+                        nsqfin[(size_t)bh * N + lane + 32 * s] = nsq_r[s];
+                    }
+                    __syncwarp();
+                    const int tp = max(t - jj - (jj >= 1 ? 0 : C), 0) + lane;     // the log up to this token: 17 entries at most
+                    if (tp <= t) {
+                        const int sp = tp & (RING - 1);
+                        const size_t ix = (bT + tp) * H + h;
+                        am_out[ix] = s_am[sp];
+                        oold_out[ix] = s_oold[sp];
+                        kiold_out[ix] = s_kiold[sp];
+                    }
+                }
+                if (lane == 0) tfirst[(size_t)bh * N] = af_mark(hand != nullptr ? rs.t0 + t + 1 : 0);
                 return;                                    // the column warps read the same limit and leave too
             }
         }
@@ -469,6 +522,7 @@ __global__ void __launch_bounds__(AF_THREADS, (RPL <= 2 ? 3 : 1)) addr_fwd_direc
             }
         }
     } else {
+        if (wact && rs.on) { AF_WRITE_ROW(RING - 1) }     // the open one
         for (int t = 0; t < T; t++) {
             const int jj = t & (C - 1);
             if (wact) {
@@ -483,7 +537,7 @@ __global__ void __launch_bounds__(AF_THREADS, (RPL <= 2 ? 3 : 1)) addr_fwd_direc
             if (jj == 1) {
                 if (t - jj >= C && ltid < C) {             // the previous chunk's log goes out
                     const int tp = t - jj - C + ltid, sp = tp & (RING - 1);
-                    const size_t ix = ((size_t)b * T + tp) * H + h;
+                    const size_t ix = (bT + tp) * H + h;
                     am_out[ix] = s_am[sp];
                     oold_out[ix] = s_oold[sp];
                     kiold_out[ix] = s_kiold[sp];
@@ -497,7 +551,13 @@ __global__ void __launch_bounds__(AF_THREADS, (RPL <= 2 ? 3 : 1)) addr_fwd_direc
             }
             AF_PHASE_BARRIER();
             lim = s_cur[t & 1];
-            if (full(lim, t + 1)) return;
+            if (RPL <= 2 && lim >= ncap && t + 1 < T) {
+                for (int i = ltid; hand != nullptr && i < ncap * (DK / 4); i += LT) {
+                    const int n = i / (DK / 4), c = 4 * (i - n * (DK / 4));
+                    st4(hand + ((size_t)bh * N + n) * DK + c, ld4(K + (size_t)n * KS + c));
+                }
+                return;
+            }
         }
     }
 #undef AF_PHASE_BARRIER
@@ -511,7 +571,7 @@ __global__ void __launch_bounds__(AF_THREADS, (RPL <= 2 ? 3 : 1)) addr_fwd_direc
         const int f0 = (((T - 1) & (C - 1)) >= 1 ? cl : max(cl - 1, 0)) * C;
         for (int tp = f0 + tid; tp < T; tp += AF_THREADS) {
             const int sp = tp & (RING - 1);
-            const size_t ix = ((size_t)b * T + tp) * H + h;
+            const size_t ix = (bT + tp) * H + h;
             am_out[ix] = s_am[sp];
             oold_out[ix] = s_oold[sp];
             kiold_out[ix] = s_kiold[sp];

@@ -1,5 +1,6 @@
 // Instantiation body of the forward address scan for one input dtype: included by slotscan_addr_fwd_{f32,bf16}.cu
 // with SLOTSCAN_TIN and SLOTSCAN_SUFFIX defined.
+#include <stdint.h>
 #include <stdio.h>
 
 #include "slotscan_addr_fwd.cuh"
@@ -15,7 +16,7 @@ typedef SLOTSCAN_TIN Tin;
 
 template <int DK, int RPL>
 static cudaError_t launch_one(const slotscan_params& p, const void* q, const void* k, const float* gate, const float* fr,
-                              const float* temp, const slotscan_log& L, const AddrFwdState& S0, int ncap, int second,
+                              const float* temp, const slotscan_log& L, const AddrFwdState& S0, int ncap, int second, float* hand,
                               cudaStream_t st) {
     const size_t sm = sizeof(float) * (size_t)addr_fwd_layout(ncap, DK, RPL, (int)sizeof(Tin)).total;
     cudaError_t e = cudaSuccess;
@@ -24,7 +25,7 @@ static cudaError_t launch_one(const slotscan_params& p, const void* q, const voi
         auto kern = addr_fwd_direct_kernel<DK, RPL, OCCB_, CARRY_, Tin>;                                                  \
         if ((e = opt_in_smem(kern, sm)) != cudaSuccess) return e;                                                         \
         kern<<<p.B * p.H, AF_THREADS, sm, st>>>(p, (const Tin*)q, (const Tin*)k, gate, fr, temp, L.addr, L.oold, L.kiold, \
-                                                L.ofin, L.tfirst, S0.K0, S0.o0, S0.nsq0, S0.nsqfin, ncap, second);        \
+                                                L.ofin, L.tfirst, S0.K0, S0.o0, S0.nsq0, S0.nsqfin, ncap, second, hand);  \
     }
     const bool carry = S0.K0 != nullptr;
     if (p.occ_bin) { if (carry) AF_LAUNCH(true, true) else AF_LAUNCH(true, false) }
@@ -35,13 +36,13 @@ static cudaError_t launch_one(const slotscan_params& p, const void* q, const voi
 
 template <int DK, int RPL>
 static cudaError_t launch_wide(const slotscan_params& p, const void* q, const void* k, const float* gate, const float* fr,
-                               const float* temp, const slotscan_log& L, const AddrFwdState& S0, cudaStream_t st) {
+                               const float* temp, const slotscan_log& L, const AddrFwdState& S0, const float* hand, cudaStream_t st) {
     const size_t sm = sizeof(float) * (size_t)addr_wide_layout(RPL, DK).total;
     cudaError_t e = cudaSuccess;
     auto go = [&](auto kern) {
         if ((e = opt_in_smem(kern, sm)) != cudaSuccess) return e;
         kern<<<p.B * p.H, aw_threads(RPL), sm, st>>>(p, (const Tin*)q, (const Tin*)k, gate, fr, temp, L.addr, L.oold, L.kiold, L.ofin,
-                                                     L.tfirst, S0.K0, S0.o0, S0.nsq0, S0.nsqfin);
+                                                     L.tfirst, S0.K0, S0.o0, S0.nsq0, S0.nsqfin, hand);
         return cudaGetLastError();
     };
     const bool carry = S0.K0 != nullptr;
@@ -70,13 +71,13 @@ static bool wide_second_pass(const slotscan_params& p, bool carry) {
 }
 template <int DK, int CTAS>
 static cudaError_t launch_narrow(const slotscan_params& p, const void* q, const void* k, const float* gate, const float* fr,
-                                 const float* temp, const slotscan_log& L, const AddrFwdState& S0, cudaStream_t st) {
+                                 const float* temp, const slotscan_log& L, const AddrFwdState& S0, float* hand, cudaStream_t st) {
     const size_t sm = sizeof(float) * (size_t)addr_narrow_layout(DK).total;
     cudaError_t e = cudaSuccess;
     auto go = [&](auto kern) {
         if ((e = opt_in_smem(kern, sm)) != cudaSuccess) return e;
         kern<<<p.B * p.H, AN_THREADS, sm, st>>>(p, (const Tin*)q, (const Tin*)k, gate, fr, temp, L.addr, L.oold, L.kiold, L.ofin,
-                                                L.tfirst, S0.K0, S0.o0, S0.nsq0, S0.nsqfin);
+                                                L.tfirst, S0.K0, S0.o0, S0.nsq0, S0.nsqfin, hand);
         return cudaGetLastError();
     };
     const bool carry = S0.K0 != nullptr;
@@ -84,11 +85,14 @@ static cudaError_t launch_narrow(const slotscan_params& p, const void* q, const 
     return carry ? go(addr_fwd_narrow_kernel<DK, CTAS, false, true, Tin>) : go(addr_fwd_narrow_kernel<DK, CTAS, false, false, Tin>);
 }
 // The passes: keys 64 or 128 wide start with the narrow kernel (32 rows), the others with the direct one.  The direct one with 64
-// rows, three CTAs to an SM, takes what the narrow one left, and the full-size one the rest.  With at most a sequence per SM and
-// 192 tokens or a carried-in state the wide kernel follows the narrow one at once: by then a sequence that takes new rows at all
-// often has passed row 64 and would be scanned a third time (48 sequences x 1000 tokens, 64 wide: 83 us; 96 x 512, 128 wide: 110;
-// 24 carried-in x 8: 12).  One that stays between 32 and 64 rows loses by it: 148 sequences x 1024 tokens, 43 rows x 128: 825 us
-// against 696, 24 x 512, 34 rows x 64: 253 against 280.
+// rows, three CTAs to an SM, goes on with what the narrow one left, and the full-size one with the rest (slotscan_addr_fwd.cuh:
+// AfResume).  With at most a sequence per SM and 192 tokens or a carried-in state the wide kernel follows the narrow one at once: the
+// direct one between them costs a launch that does nothing where no sequence needs it (12 sequences x 256 tokens, 9 rows x 128: 71 us
+// against 76; 48 x 1024, 11 rows: 255 against 259), and the wide one is as fast from row 32 on or nearly (us, narrow to wide / with the
+// direct one between / direct to wide, no narrow one): 148 x 1024, 42 rows x 128 of 192: 820 / 745 / 626; of 96: 625 / 745 / 627;
+// 148 x 1024, 39 rows x 64: 559 / 609 / 513; 148 x 1024, 32 rows x 128: 607 / 584 / 571; 24 x 512, all of 192 rows x 128: 401 / - / 449.
+// Sequences that end between 32 and 64 rows are where a chain of passes is behind: each pass waits for the last sequence of the one
+// before.  Up to 32 rows it is ahead by nearly half: 24 x 1024, 22 rows x 128: 305 against 535 without the narrow kernel.
 // The exception: the zero-fill of the snapshots runs beside the scan, and the replay behind the scan contends with it for the memory.
 // Where the fill is expected to outlast the direct kernel (its rate beside a scan, 4.66 MB per us, against 0.74 us per token and round
 // of three CTAs to an SM), a faster scan only brings that on earlier: 384 sequences x 1024 tokens, 192 rows x 128, bf16, forward and
@@ -99,10 +103,23 @@ static bool behind_the_fill(const slotscan_params& p, int sms) {
     const long long rounds = ((long long)p.B * p.H + 3 * sms - 1) / (3 * sms);
     return fill_us > 0.74 * (double)p.T * (double)rounds;
 }
+// Where a pass leaves key rows for the next one: the final rows' place, which the replay writes later.  NULL, so that the next pass
+// starts again, where the caller gave no room for the norms or where it carries the state in place.
+static float* hand_over_rows(const slotscan_params& p, const slotscan_log& L, const AddrFwdState& S0) {
+    const size_t rows = (size_t)p.B * p.H * p.N;
+    auto apart = [](const void* a, const void* b, size_t bytes) {
+        const uintptr_t x = (uintptr_t)a, y = (uintptr_t)b;
+        return a == nullptr || x + bytes <= y || y + bytes <= x;
+    };
+    const bool ok = S0.nsqfin != nullptr && apart(S0.K0, L.kfin, rows * p.DK * sizeof(float)) && apart(S0.o0, L.ofin, rows * sizeof(float)) &&
+                    apart(S0.nsq0, S0.nsqfin, rows * sizeof(double));
+    return ok ? L.kfin : nullptr;
+}
 template <int DK>
 static cudaError_t launch_dk(const slotscan_params& p, const void* q, const void* k, const float* gate, const float* fr,
                              const float* temp, const slotscan_log& L, const AddrFwdState& S0, cudaStream_t st) {
     cudaError_t e;
+    float* hand = hand_over_rows(p, L, S0);
     if constexpr (DK >= 64) {
         int dev = 0, sms = 148;
         cudaGetDevice(&dev);
@@ -110,25 +127,25 @@ static cudaError_t launch_dk(const slotscan_params& p, const void* q, const void
         const long long BH = (long long)p.B * p.H;
         int second = 0;                                   // this pass takes the sequences that the one before it marked
         if (BH <= 2 * sms || S0.K0 != nullptr || p.N <= AF_NCAP1 || !behind_the_fill(p, sms)) {
-            if (BH <= 2 * sms) e = launch_narrow<DK, 2>(p, q, k, gate, fr, temp, L, S0, st);
-            else e = launch_narrow<DK, 3>(p, q, k, gate, fr, temp, L, S0, st);
+            if (BH <= 2 * sms) e = launch_narrow<DK, 2>(p, q, k, gate, fr, temp, L, S0, hand, st);
+            else e = launch_narrow<DK, 3>(p, q, k, gate, fr, temp, L, S0, hand, st);
             if (e != cudaSuccess || p.N <= AN_ROWS) return e;
             second = 1;
         }
         const bool wide = p.N > AF_NCAP1 && wide_second_pass<DK>(p, S0.K0 != nullptr);
         if (!wide || BH > sms || (p.T < 192 && S0.K0 == nullptr)) {
-            e = launch_one<DK, 2>(p, q, k, gate, fr, temp, L, S0, p.N <= AF_NCAP1 ? p.N : AF_NCAP1, second, st);
+            e = launch_one<DK, 2>(p, q, k, gate, fr, temp, L, S0, p.N <= AF_NCAP1 ? p.N : AF_NCAP1, second, hand, st);
             if (e != cudaSuccess || p.N <= AF_NCAP1) return e;
         }
         if (wide) {
-            if (p.N <= 128) return launch_wide<DK, 4>(p, q, k, gate, fr, temp, L, S0, st);
-            return launch_wide<DK, 6>(p, q, k, gate, fr, temp, L, S0, st);
+            if (p.N <= 128) return launch_wide<DK, 4>(p, q, k, gate, fr, temp, L, S0, hand, st);
+            return launch_wide<DK, 6>(p, q, k, gate, fr, temp, L, S0, hand, st);
         }
     } else {
-        e = launch_one<DK, 2>(p, q, k, gate, fr, temp, L, S0, p.N <= AF_NCAP1 ? p.N : AF_NCAP1, 0, st);
+        e = launch_one<DK, 2>(p, q, k, gate, fr, temp, L, S0, p.N <= AF_NCAP1 ? p.N : AF_NCAP1, 0, hand, st);
         if (e != cudaSuccess || p.N <= AF_NCAP1) return e;
     }
-    return launch_one<DK, 6>(p, q, k, gate, fr, temp, L, S0, p.N, 1, st);         // N <= 192
+    return launch_one<DK, 6>(p, q, k, gate, fr, temp, L, S0, p.N, 1, hand, st);         // N <= 192
 }
 
 cudaError_t SS_CAT(run_addr_fwd_, SLOTSCAN_SUFFIX)(const slotscan_params& p, const void* q, const void* k, const float* gate,

@@ -88,8 +88,8 @@ __global__ void __launch_bounds__(AN_THREADS, CTAS) addr_fwd_narrow_kernel(
     const float* __restrict__ fr, const float* __restrict__ temp_p, int* __restrict__ am_out,
     float* __restrict__ oold_out, float* __restrict__ kiold_out, float* __restrict__ ofin, int* __restrict__ tfirst,
     const float* __restrict__ K0, const float* __restrict__ o0, const double* __restrict__ nsq0,
-    double* __restrict__ nsqfin) {
-    // A sequence that needs a row above the 32 is marked by tfirst[bh][0] = -1 and left to the next pass, which starts again.
+    double* __restrict__ nsqfin, float* __restrict__ hand) {
+    // A sequence that needs a row above the 32 is left to the next pass (slotscan_addr_fwd.cuh: AfResume).
     extern __shared__ __align__(16) float smem[];
     constexpr int CW = DK / 4, NF = CW / 4;               // columns and float4 per quarter
     const int N = p.N, T = p.T, H = p.H, ncap = min(N, AN_ROWS);
@@ -137,7 +137,7 @@ __global__ void __launch_bounds__(AN_THREADS, CTAS) addr_fwd_narrow_kernel(
         }
         lim = min(hw0 + 1, N - 1);
         if (lim >= ncap) {                                // uniform over the CTA
-            if (tid == 0) tfirst[(size_t)bh * N] = -1;
+            if (tid == 0) tfirst[(size_t)bh * N] = af_mark(0);
             return;
         }
         __syncthreads();
@@ -145,11 +145,6 @@ __global__ void __launch_bounds__(AN_THREADS, CTAS) addr_fwd_narrow_kernel(
     const int lim0 = lim;
     // lanes that share a row, by the last row that a token's dots visit
     auto mode_of = [](int limd) { return limd < 8 ? 4 : (limd < 16 ? 2 : 1); };
-    // Whether token t, with candidate rows up to l, is left to the next pass: at the latest where it has no room, and as soon as
-    // this call has taken 12 rows at less than 8 tokens each, if at that pace it runs out before its end (the rows of random
-    // keys come ever more slowly, about one per doubling of the tokens; where every write wants a new row this pass is a waste).
-    const int lead = N > AN_ROWS ? min(8, T / AN_ROWS) : 0;
-    auto full = [&](int l, int t) { return l >= ncap || (l >= lim0 + 12 && t < lead * (l - lim0)); };
     for (int i = tid; i < N; i += AN_THREADS) tfirst[(size_t)bh * N + i] = i <= lim0 ? 0 : T;
     for (int i = tid; i < DK; i += AN_THREADS) Ks[(AN_RING - 1) * DK + i] = 0.f;           // "the key before token 0"
     for (int i = tid; i < 2 * 2 * AN_PART; i += AN_THREADS) s_part[i] = 0.f;
@@ -317,7 +312,7 @@ __global__ void __launch_bounds__(AN_THREADS, CTAS) addr_fwd_narrow_kernel(
                     bool more = false;
                     if ((unsigned)a >= 0x40000000u) {
                         if (a < 0) {                      // a row not written before: one more candidate
-                            if (full(++lim, t)) { left = true; return true; }
+                            if (++lim >= ncap) { left = true; return true; }
                             more = F > 1 && min(lim + 1, N - 1) >= R;
                         }
                         a &= 0x3fffffff;
@@ -405,6 +400,11 @@ __global__ void __launch_bounds__(AN_THREADS, CTAS) addr_fwd_narrow_kernel(
             }
             run(std::integral_constant<int, 1>(), K1);
         }
+        if (left && hand != nullptr) {                    // lane = row, as in every token since row 16 (the write of token t - 1 is open)
+            float* d = hand + ((size_t)bh * N + lane) * DK + cw * CW;
+#pragma unroll
+            for (int i = 0; i < NF; i++) *reinterpret_cast<f32x4*>(d + 4 * i) = K1[i];
+        }
     } else if (warp == 1) {
         // ------------------------------------------------------------------ norm warp
         __syncthreads();
@@ -434,9 +434,9 @@ __global__ void __launch_bounds__(AN_THREADS, CTAS) addr_fwd_narrow_kernel(
             kinv = mine ? hy.x : kinv;
             o = mine ? hy.y : o;
         };
-        auto none = [&]() {                               // no score compared greater: token t - 1 again, as if the dot were zero
+        auto none = [&](bool meet) {                      // no score compared greater: token t - 1 again, as if the dot were zero
             would(t - 1, 0.0, g1, om1);
-            AN_BAR(3, 64);
+            if (meet) AN_BAR(3, 64);
         };
         auto run = [&](auto fc) {                         // while the token's dots come in F parts
             constexpr int F = decltype(fc)::value;
@@ -450,9 +450,9 @@ __global__ void __launch_bounds__(AN_THREADS, CTAS) addr_fwd_narrow_kernel(
                 if ((unsigned)a1 >= 0x40000000u && t > 0) {
                     if (a1 < 0) {
                         more = true;
-                        if (full(++lim, t)) { left = true; return; }          // before the meeting below: the resolver has left too
+                        if (++lim >= ncap) { left = true; return; }           // before the meeting below: the resolver has left too
                     }
-                    if (a1 & 0x40000000) none();
+                    if (a1 & 0x40000000) none(true);
                     a1 &= 0x3fffffff;
                 }
                 const bool mine = lane == a1;
@@ -469,20 +469,19 @@ __global__ void __launch_bounds__(AN_THREADS, CTAS) addr_fwd_narrow_kernel(
         if (mode_of(lim0) == 4) run(std::integral_constant<int, 4>());
         if (!left && t < T && mode_of(t ? min(lim + 1, N - 1) : lim0) == 2) run(std::integral_constant<int, 2>());
         if (!left && t < T) run(std::integral_constant<int, 1>());
-        if (!left) {
-            const int a1 = s_am[(T - 1) & (AN_RING - 1)];
-            if (a1 & 0x40000000) none();
-            settle(lane == (a1 & 0x3fffffff));
-            if (lane < ncap) {
-                ofin[(size_t)bh * N + lane] = o;
-                if (nsqfin != nullptr) nsqfin[(size_t)bh * N + lane] = nsq;
-            }
+        const int a1 = s_am[(t - 1) & (AN_RING - 1)];     // the last token, or the one before it leaves
+        if (a1 & 0x40000000) none(!left);
+        settle(lane == (a1 & 0x3fffffff));
+        if (lane < ncap && (!left || hand != nullptr)) {
+            ofin[(size_t)bh * N + lane] = o;
+            if (nsqfin != nullptr) nsqfin[(size_t)bh * N + lane] = nsq;
         }
     } else {
         // ------------------------------------------------------------------ resolver warp
         __syncthreads();
         __syncthreads();
         float kinv = fminf(rsqrtf((float)nsq), 1e6f), g1 = 0.f, om1 = 0.f;
+        if (lane > lim) o = NAN;                          // a row above lim is neither occupied (which eps <= 0 makes every row) nor free
         const unsigned below = (1u << lane) - 1u;
         int t = 0, a1 = -1;                               // the previous token's address
         bool left = false, none = false;
@@ -506,9 +505,9 @@ __global__ void __launch_bounds__(AN_THREADS, CTAS) addr_fwd_narrow_kernel(
                 // product, product, difference, each rounded: as the direct kernel's expression comes out
                 const float sc = __fmul_rn(c4.x, __fmul_rn(kinv, S));
                 // (a penalty that is infinite or NaN is NaN on a row that is not occupied too: times zero, not left out)
-                const float z = OCCB ? __fsub_rn(sc, occ ? c4.y : __fmul_rn(c4.y, 0.f)) : __fmaf_rn(-c4.y, o, sc);
-                // candidates: occupied rows and the lowest free one, of those up to row lim (with eps <= 0 every row is occupied)
-                const float zc = lane <= lim && (occ || (isfree && !(fm & below))) ? z : -INFINITY;
+                const float z = __fmaf_rn(-c4.y, OCCB ? (occ ? 1.f : 0.f) : o, sc);
+                // candidates: occupied rows and the lowest free one
+                const float zc = occ || (isfree && !(fm & below)) ? z : -INFINITY;
                 const float zm = redux_max(zc);
                 a1 = __ffs((int)__ballot_sync(FULL, zc == zm)) - 1;           // the lowest row of the largest score
                 none = !(zm > -INFINITY);                 // no candidate compares greater (NaN scores): row lim
@@ -522,9 +521,10 @@ __global__ void __launch_bounds__(AN_THREADS, CTAS) addr_fwd_narrow_kernel(
                 const bool more = F > 1 && min(lim + 1, N - 1) >= 32 / F;     // token t's dots, taken before this address was known
                 if (fresh) {
                     lim++;
+                    if (lane == lim) o = 0.f;             // never written: from here on a candidate
                     if (lane == 0) tfirst[(size_t)bh * N + lim] = t;
-                    if (t < T && full(lim, t)) {          // the next token may address a row this CTA does not hold
-                        if (lane == 0) { tfirst[(size_t)bh * N] = -1; *s_leave = t; }
+                    if (t < T && lim >= ncap) {           // the next token may address a row this CTA does not hold
+                        if (lane == 0) { tfirst[(size_t)bh * N] = af_mark(hand != nullptr ? t : 0); *s_leave = t; }
                         __syncwarp();
                         if ((t | 7) < T) AN_BAR(2, 96);   // the loaders come to it
                         left = true;
@@ -540,14 +540,14 @@ __global__ void __launch_bounds__(AN_THREADS, CTAS) addr_fwd_narrow_kernel(
         if (!left && none) AN_BAR(3, 64);
     }
     __syncthreads();
-    if (*s_leave) return;
-    for (int i = ncap + tid; i < N; i += AN_THREADS) {                // rows this pass never held
+    const int Tn = *s_leave ? *s_leave : T;               // tokens whose log is complete
+    if (Tn == T) for (int i = ncap + tid; i < N; i += AN_THREADS) {                // rows this pass never held
         ofin[(size_t)bh * N + i] = 0.f;
         if (nsqfin != nullptr) nsqfin[(size_t)bh * N + i] = 0.0;
     }
-    {   // log entries not written out yet
-        const int t = max((T - 1) / AN_L * AN_L - 2, 0) + tid;
-        if (t < T) {
+    {   // log entries not written out yet (the loaders' last turn was in the chunk of the token in work)
+        const int t = max((*s_leave ? Tn : T - 1) / AN_L * AN_L - 2, 0) + tid;
+        if (t < Tn) {
             const size_t ix = ((size_t)b * T + t) * H + h;
             const int sl = t & (AN_RING - 1);
             am_out[ix] = s_am[sl] & 0x3fffffff;

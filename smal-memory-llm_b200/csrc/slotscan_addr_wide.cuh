@@ -59,13 +59,13 @@ __global__ void __launch_bounds__(aw_threads(RPL), 1) addr_fwd_wide_kernel(
     const float* __restrict__ fr, const float* __restrict__ temp_p, int* __restrict__ am_out,
     float* __restrict__ oold_out, float* __restrict__ kiold_out, float* __restrict__ ofin, int* __restrict__ tfirst,
     const float* __restrict__ K0, const float* __restrict__ o0, const double* __restrict__ nsq0,
-    double* __restrict__ nsqfin) {
+    double* __restrict__ nsqfin, const float* __restrict__ hand) {
     extern __shared__ __align__(16) float smem[];
     constexpr int CW = DK / 4, NF = CW / 4, SPG = AW_SPG;              // columns and float4 per quarter, slots per column warp
     constexpr int AW_COL = aw_col(RPL);
     constexpr int F8 = NF >= 4 ? 4 : 1, F16 = NF >= 2 ? 2 : 1;        // the direct kernel's splits below 8 and 16 rows
     constexpr int NT = aw_threads(RPL);
-    const int N = p.N, T = p.T, H = p.H;
+    const int N = p.N, H = p.H;
     const AddrWideSmem L = addr_wide_layout(RPL, DK);
     float2* part = reinterpret_cast<float2*>(smem + L.part);
     float* s_tok = smem + L.tok;
@@ -79,12 +79,16 @@ __global__ void __launch_bounds__(aw_threads(RPL), 1) addr_fwd_wide_kernel(
     const int bh = blockIdx.x, b = bh / H, h = bh % H;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const float temp = temp_p[0], eps = p.eps;
-    if (tfirst[(size_t)bh * N] != -1) return;                         // finished in the first pass (uniform per CTA)
+    const int mark = tfirst[(size_t)bh * N];
+    if (mark >= 0) return;                                            // finished in an earlier pass (uniform per CTA)
+    const AfResume rs(mark, am_out, (size_t)b * p.T * H + h, H);
+    const int T = p.T - rs.t0;                                        // tokens are counted from rs.t0 on
+    const size_t bT = (size_t)b * p.T + rs.t0;
     __syncthreads();
     // a carried-in state: squared norms as the direct kernel takes or sums them, the highest row it has touched
-    int hw0 = -1;
+    int hw0 = rs.am;
     double* s_nsq = reinterpret_cast<double*>(smem + L.part);         // [N] before `part` is first written
-    if (CARRY) {
+    if (CARRY && !rs.on) {
         for (int n = warp; n < N; n += NT / 32) {
             double a = 0.0;
             if (nsq0 != nullptr) {
@@ -106,8 +110,12 @@ __global__ void __launch_bounds__(aw_threads(RPL), 1) addr_fwd_wide_kernel(
             if (used) hw0 = n0 + 31 - __clz(used);
         }
     }
-    const int lim0 = CARRY ? min(hw0 + 1, N - 1) : 0;                 // candidate limit of token 0
-    for (int i = tid; i < N; i += NT) tfirst[(size_t)bh * N + i] = (i <= hw0 + 1) ? 0 : T;
+    const int lim0 = CARRY || rs.on ? min(hw0 + 1, N - 1) : 0;        // candidate limit of token 0
+    if (rs.on) {
+        if (tid == 0) tfirst[(size_t)bh * N] = 0;                     // the others stand as the pass before left them
+    } else {
+        for (int i = tid; i < N; i += NT) tfirst[(size_t)bh * N + i] = (i <= hw0 + 1) ? 0 : T;
+    }
     if (tid < 16) s_cmb[tid] = make_int4(0, 0, 0, 0);
 #define AW_BARRIER() asm volatile("bar.sync 1, %0;" ::"n"(NT) : "memory")
     // the address of the token whose entries lie in buffer `buf` (lim: its last candidate row): the largest score, in the lowest
@@ -135,7 +143,8 @@ __global__ void __launch_bounds__(aw_threads(RPL), 1) addr_fwd_wide_kernel(
 #pragma unroll
             for (int i = 0; i < NF; i++) {
                 K[s][i] = {0ull, 0ull};
-                if (CARRY && n < N) K[s][i] = ld4x2(K0 + ((size_t)bh * N + n) * DK + c0 + 4 * i);
+                if (rs.on) { if (n <= rs.am) K[s][i] = ld4x2(hand + ((size_t)bh * N + n) * DK + c0 + 4 * i); }
+                else if (CARRY && n < N) K[s][i] = ld4x2(K0 + ((size_t)bh * N + n) * DK + c0 + 4 * i);
             }
         }
         auto dots = [&](int limd, int sl, int buf) {
@@ -193,31 +202,32 @@ __global__ void __launch_bounds__(aw_threads(RPL), 1) addr_fwd_wide_kernel(
             else many(std::integral_constant<int, SPG>());
         };
         __syncthreads();                                              // the prologue's tokens are staged (and s_nsq is read)
-        dots(CARRY ? lim0 : 0, 0, 0);
+        dots(lim0, 0, 0);
         AW_BARRIER();
-        int lim = lim0;
+        int lim = lim0, a = rs.am;
         for (int t = 0; t < T; t++) {
-            if (t >= 1) {                                             // the write of token t - 1
-                const int a = resolved((t - 1) & 1, lim).am, sa = (a >> 5) - s_base;
+            if (t >= 1) {
+                a = resolved((t - 1) & 1, lim).am;
                 lim = max(lim, min(a + 1, N - 1));
-                if (sa >= 0 && sa < SPG) {
-                    const int sl = (t - 1) & (AW_RING - 1);
-                    const float g = s_tok[AW_TOK * sl + 2];
-                    const f32x2 g2 = pack2(g, g), om2 = pack2(1.f - g, 1.f - g);
-                    const float* kr = Ks + sl * DK + c0;
+            }
+            const int sa = a < 0 ? -1 : (a >> 5) - s_base;            // the write of token t - 1
+            if (sa >= 0 && sa < SPG) {
+                const int sl = (t - 1) & (AW_RING - 1);
+                const float g = s_tok[AW_TOK * sl + 2];
+                const f32x2 g2 = pack2(g, g), om2 = pack2(1.f - g, 1.f - g);
+                const float* kr = Ks + sl * DK + c0;
 #pragma unroll
-                    for (int s = 0; s < SPG; s++) {
-                        if (s == sa && lane == (a & 31)) {
+                for (int s = 0; s < SPG; s++) {
+                    if (s == sa && lane == (a & 31)) {
 #pragma unroll
-                            for (int i = 0; i < NF; i++) {
-                                const f32x4 k4 = ld4x2(kr + 4 * i);
-                                K[s][i].a = fma2(g2, k4.a, mul2(om2, K[s][i].a));      // blend, two columns at a time
-                                K[s][i].b = fma2(g2, k4.b, mul2(om2, K[s][i].b));
-                            }
+                        for (int i = 0; i < NF; i++) {
+                            const f32x4 k4 = ld4x2(kr + 4 * i);
+                            K[s][i].a = fma2(g2, k4.a, mul2(om2, K[s][i].a));      // blend, two columns at a time
+                            K[s][i].b = fma2(g2, k4.b, mul2(om2, K[s][i].b));
                         }
                     }
-                    __syncwarp();
                 }
+                __syncwarp();
             }
             if (t + 1 < T) dots(min(lim + 1, N - 1), (t + 1) & (AW_RING - 1), (t + 1) & 1);
             AW_BARRIER();
@@ -228,10 +238,10 @@ __global__ void __launch_bounds__(aw_threads(RPL), 1) addr_fwd_wide_kernel(
         const bool live = n < N;
         double nsq = 0.0;
         float kinv = 1e6f, o = 0.f;
-        if (CARRY && live) {
-            nsq = s_nsq[n];
+        if (rs.on ? n <= rs.am : CARRY && live) {
+            nsq = rs.on ? nsqfin[(size_t)bh * N + n] : s_nsq[n];
             kinv = fminf(rsqrtf((float)nsq), 1e6f);
-            o = o0[(size_t)bh * N + n];
+            o = (rs.on ? ofin : o0)[(size_t)bh * N + n];
         }
         // lowest free row (N if none): every resolver warp knows it.  After a change: one mask per warp, in shared memory.
         auto publish = [&](bool is_free) {
@@ -255,7 +265,7 @@ __global__ void __launch_bounds__(aw_threads(RPL), 1) addr_fwd_wide_kernel(
             if (tid == AW_COL * 32) s_am[ps] = a.am;
             if (a.am >= lim && lim < N - 1) {                         // a row not written before: one more candidate
                 lim++;
-                if (tid == AW_COL * 32) tfirst[(size_t)bh * N + lim] = t;
+                if (tid == AW_COL * 32) tfirst[(size_t)bh * N + lim] = rs.t0 + t;
             }
             mine = n == a.am;
             if (mine) {
@@ -272,6 +282,7 @@ __global__ void __launch_bounds__(aw_threads(RPL), 1) addr_fwd_wide_kernel(
             else if (is_free && a.am < fe) fe = a.am;
         };
         __syncthreads();
+        if (rs.on) { mine = n == rs.am; g_prev = s_tok[AW_TOK * (AW_RING - 1) + 2]; }
         fe = publish(live && o < eps);
         AW_BARRIER();
         for (int t = 0; t < T; t++) {
@@ -318,7 +329,7 @@ __global__ void __launch_bounds__(aw_threads(RPL), 1) addr_fwd_wide_kernel(
         struct alignas(EPL * sizeof(Tin)) Vec { Tin v[EPL]; };
         struct Tok { Vec q, k; float g, f; };
         auto fetch = [&](Tok& d, int u) {                             // loads only: they stay in flight
-            const size_t ix = ((size_t)b * T + min(u, T - 1)) * H + h;
+            const size_t ix = (bT + min(u, T - 1)) * H + h;
             d.q = *reinterpret_cast<const Vec*>(q + ix * DK + lane * EPL);
             d.k = *reinterpret_cast<const Vec*>(k + ix * DK + lane * EPL);
             d.g = gate[ix];
@@ -346,15 +357,21 @@ __global__ void __launch_bounds__(aw_threads(RPL), 1) addr_fwd_wide_kernel(
             const int t = t0 + lane;
             if (t < t1) {
                 const int sl = t & (AW_RING - 1);
-                const size_t ix = ((size_t)b * T + t) * H + h;
+                const size_t ix = (bT + t) * H + h;
                 am_out[ix] = s_am[sl];
                 oold_out[ix] = s_oold[sl];
                 kiold_out[ix] = s_kiold[sl];
             }
         };
-        if (hp == 0) {
+        if (hp == 0) {                                                // "the key before token 0"
+            if (rs.on) {
+                Tok e;
+                fetch(e, -1);
+                commit(e, -1);
+            } else {
 #pragma unroll
-            for (int i = 0; i < EPL; i++) Ks[(AW_RING - 1) * DK + lane * EPL + i] = 0.f;      // "the key before token 0"
+                for (int i = 0; i < EPL; i++) Ks[(AW_RING - 1) * DK + lane * EPL + i] = 0.f;
+            }
         }
         Tok d[AW_PRE];
         for (int u0 = hp; u0 < AW_LEAD; u0 += 2 * AW_HELP) {          // the first tokens, two in flight
@@ -401,7 +418,7 @@ __global__ void __launch_bounds__(aw_threads(RPL), 1) addr_fwd_wide_kernel(
             const int t = t0 + lane;
             if (t < T) {
                 const int sl = t & (AW_RING - 1);
-                const size_t ix = ((size_t)b * T + t) * H + h;
+                const size_t ix = (bT + t) * H + h;
                 am_out[ix] = s_am[sl];
                 oold_out[ix] = s_oold[sl];
                 kiold_out[ix] = s_kiold[sl];

@@ -439,6 +439,43 @@ def test_penalty_without_a_value(dist, N, T):
         assert torch.equal(logs[0][i].expand_as(logs[1][i]), logs[1][i]), i
 
 
+@pytest.mark.parametrize("D,dtype,N,T,copies", [(128, torch.bfloat16, 192, 200, 1), (64, torch.float32, 96, 150, 1),
+                                                (128, torch.float32, 96, 203, 40), (64, torch.bfloat16, 192, 180, 80),
+                                                (32, torch.bfloat16, 96, 200, 1), (128, torch.bfloat16, 40, 150, 1)],
+                         ids=lambda x: str(x).split(".")[-1])
+def test_passes_go_on_where_the_one_before_stopped(D, dtype, N, T, copies, monkeypatch):
+    """A sequence that runs out of a kernel's rows goes on in the next kernel at the token where it stopped.  Without room for the
+    squared norms (the C interface allows it) the next kernel starts again at token 0: the same log and the same final rows, bit for
+    bit, for sequences that need one, two and three kernels, from the empty memory and from a state."""
+    import slotscan_b200 as S
+    from slotscan_b200 import _lib
+    B, H, t0 = 2, 3, 24
+    few, many = (make_inputs(d, B, t0 + T, H, D, D, seed=29) for d in ("bench", "fill"))
+    x = {n: few[n].clone() for n in ("k", "v", "gate", "fr", "q")}
+    for n in x:
+        x[n][:, :, 2] = many[n][:, :, 2]                       # the last head takes a row with nearly every token
+    x["fr"][:, :, 1] += 1.9 * (128 / D) ** 0.5                 # the one before it with every fourth
+    x["fr"][:, :, 2] *= 2
+    dev = {n: x[n].cuda().to(dtype if n in ("k", "v", "q") else torch.float32) for n in x}
+    extra = _lib.FwdExtra
+    rows = []
+    for a, b, state in ((0, T, None), (t0, t0 + T, "carry")):
+        if state is not None:
+            lg = S.scan_with_log(*(dev[n][:, :a].contiguous() for n in ("k", "v", "gate", "fr")), N, 16.0, G=8, q=dev["q"][:, :a].contiguous(),
+                                 occ_bin=True)
+            state = tuple(lg[n].repeat(copies, *[1] * (lg[n].dim() - 1)) for n in ("kfin", "vfin", "ofin", "nsqfin"))
+        y = {n: t[:, a:b].repeat(copies, *[1] * (t.dim() - 1)).contiguous() for n, t in dev.items()}
+        run = lambda: S.scan_with_log(y["k"], y["v"], y["gate"], y["fr"], N, 16.0, G=8, q=y["q"], occ_bin=True, state=state)
+        on = run()
+        monkeypatch.setattr(_lib, "FwdExtra", lambda *p: extra(*p[:4], 0, *p[5:]))
+        again = run()
+        monkeypatch.undo()
+        for n in ("addr", "oold", "kiold", "kold", "kfin", "vfin", "ofin", "tfirst", "kbuf"):
+            assert torch.equal(on[n], again[n]), (n, a)
+        rows += (on["tfirst"] < T).sum(-1).tolist()
+    assert min(rows) <= 32 < max(rows) and (N <= 64 or max(rows) > 64 and any(32 < r <= 64 for r in rows)), sorted(set(rows))
+
+
 @pytest.mark.parametrize("mode", ["hard", "soft", "keyless", "read"])
 def test_plain_calls_equal_registered_ops(mode, monkeypatch):
     """Ordinary eager calls go round the custom ops' wrapping; the same call through the ops gives the same bits, values and
