@@ -113,7 +113,22 @@ __global__ void __launch_bounds__(AN_THREADS, CTAS) addr_fwd_narrow_kernel(
     int lim = 0;                                          // the current token's last candidate row
     if (CARRY) {
         double* s_nsq = reinterpret_cast<double*>(s_part);            // [N], where none came with the state: the direct kernel's sums
-        if (nsq0 == nullptr) {
+        for (bool sums = nsq0 != nullptr;; sums = true) {             // (first without them: a row in use most often shows in its occupancy)
+            int hw0 = -1;                                 // highest row that the state has touched
+            for (int n0 = 0; n0 < N; n0 += 32) {
+                const int n = n0 + lane;
+                const double a = n >= N || !sums ? 0.0 : (nsq0 != nullptr ? nsq0[(size_t)bh * N + n] : s_nsq[n]);
+                const float on = n < N ? o0[(size_t)bh * N + n] : 0.f;
+                const unsigned used = __ballot_sync(FULL, a > 0.0 || on != 0.f);
+                if (used) hw0 = n0 + 31 - __clz(used);
+                if (n0 == 0) { nsq = a; o = on; }
+            }
+            lim = min(hw0 + 1, N - 1);
+            if (lim >= ncap) {                            // uniform over the CTA
+                if (tid == 0) tfirst[(size_t)bh * N] = af_mark(0);
+                return;
+            }
+            if (sums) break;
             for (int n = warp; n < N; n += AN_THREADS / 32) {
                 double a = 0.0;
                 for (int c = lane; c < DK; c += 32) {
@@ -125,20 +140,6 @@ __global__ void __launch_bounds__(AN_THREADS, CTAS) addr_fwd_narrow_kernel(
                 if (lane == 0) s_nsq[n] = a;
             }
             __syncthreads();
-        }
-        int hw0 = -1;                                     // highest row that the state has touched
-        for (int n0 = 0; n0 < N; n0 += 32) {
-            const int n = n0 + lane;
-            const double a = n >= N ? 0.0 : (nsq0 != nullptr ? nsq0[(size_t)bh * N + n] : s_nsq[n]);
-            const float on = n < N ? o0[(size_t)bh * N + n] : 0.f;
-            const unsigned used = __ballot_sync(FULL, a > 0.0 || on != 0.f);
-            if (used) hw0 = n0 + 31 - __clz(used);
-            if (n0 == 0) { nsq = a; o = on; }
-        }
-        lim = min(hw0 + 1, N - 1);
-        if (lim >= ncap) {                                // uniform over the CTA
-            if (tid == 0) tfirst[(size_t)bh * N] = af_mark(0);
-            return;
         }
         __syncthreads();
     }

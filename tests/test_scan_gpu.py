@@ -476,6 +476,28 @@ def test_passes_go_on_where_the_one_before_stopped(D, dtype, N, T, copies, monke
     assert min(rows) <= 32 < max(rows) and (N <= 64 or max(rows) > 64 and any(32 < r <= 64 for r in rows)), sorted(set(rows))
 
 
+@pytest.mark.parametrize("used,occupied", [(8, 8), (31, 31), (32, 32), (70, 70), (40, 8), (32, 5)])
+def test_state_without_norms(used, occupied):
+    """A carried-in state may come without its squared norms: they are summed from the key rows, and rows in use that a kernel has no
+    room for show in their occupancies or, where those are zero, in the sums.  Keys whose squares add up exactly: bit for bit the
+    scan with the norms given."""
+    import slotscan_b200 as S
+    B, T, H, N, D = 2, 40, 3, 96, 64
+    inp = make_inputs("bench", B, T, H, D, D, seed=31)
+    x = [inp[n].cuda() for n in ("k", "v", "gate", "fr", "q")]
+    gen = torch.Generator().manual_seed(2)
+    K0, V0 = torch.zeros(B * H, N, D), torch.zeros(B * H, N, D)
+    K0[:, :used] = torch.randint(-4, 5, (B * H, used, D), generator=gen) / 16.0
+    V0[:, :used] = torch.randn(B * H, used, D, generator=gen)
+    o0 = torch.zeros(B * H, N)
+    o0[:, :occupied] = 0.25 + 0.5 * torch.rand(B * H, occupied, generator=gen)
+    state = tuple(t.cuda() for t in (K0, V0, o0, K0.double().square().sum(-1)))
+    a, b = (S.scan_with_log(*x[:4], N, 16.0, G=8, q=x[4], occ_bin=True, state=st) for st in (state[:3], state))
+    assert ((a["tfirst"] == 0).sum(-1) == used + 1).all()
+    for n in ("addr", "oold", "kiold", "kfin", "vfin", "ofin", "tfirst", "nsqfin"):
+        assert torch.equal(a[n], b[n]), n
+
+
 @pytest.mark.parametrize("mode", ["hard", "soft", "keyless", "read"])
 def test_plain_calls_equal_registered_ops(mode, monkeypatch):
     """Ordinary eager calls go round the custom ops' wrapping; the same call through the ops gives the same bits, values and
