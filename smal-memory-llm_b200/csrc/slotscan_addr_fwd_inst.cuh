@@ -93,15 +93,20 @@ static cudaError_t launch_narrow(const slotscan_params& p, const void* q, const 
 // 148 x 1024, 39 rows x 64: 559 / 609 / 513; 148 x 1024, 32 rows x 128: 607 / 584 / 571; 24 x 512, all of 192 rows x 128: 401 / - / 449.
 // Sequences that end between 32 and 64 rows are where a chain of passes is behind: each pass waits for the last sequence of the one
 // before.  Up to 32 rows it is ahead by nearly half: 24 x 1024, 22 rows x 128: 305 against 535 without the narrow kernel.
-// The exception: the zero-fill of the snapshots runs beside the scan, and the replay behind the scan contends with it for the memory.
-// Where the fill is expected to outlast the direct kernel (its rate beside a scan, 4.66 MB per us, against 0.74 us per token and round
-// of three CTAs to an SM), a faster scan only brings that on earlier: 384 sequences x 1024 tokens, 192 rows x 128, bf16, forward and
-// backward 2.03 ms with the narrow pass first, 2.00 with the direct one.
+// The exception, more than two sequences per SM from the empty memory: the zero-fill of the snapshots runs beside the scan (rows past
+// the first replay tile), and the replay behind the scan contends with it for the memory.  Where the fill (4.66 MB per us beside a scan)
+// outlasts the direct kernel (0.74 us per token and round of three CTAs to an SM) by a fifth, a faster scan only brings that on
+// earlier.  Narrow first / direct first, us, forward and then forward and backward, few rows in use, fill over scan in front:
+//   0.98  300 x 1024, 192 rows x 128, bf16      898 / 995     1732 / 1823     0.98  300 x 512, float32, stride 16   520 / 597    1000 / 1077
+//   1.14  384 x 512, 96 x 128, float32          657 / 680     1250 / 1275     1.14  384 x 1024, 192 x 64, float32  1000 / 1051   1969 / 2077
+//   1.25  384 x 1024, 192 x 128, bf16          1133 / 1112    2076 / 2055     1.96  300 x 512, 192 x 128, float32   865 / 845    1389 / 1381
+// Short calls are ahead with it past the line too (1.25, 384 x 128: 214 / 233, 430 / 434); sequences that take a new row every second
+// token are behind on both sides of it (0.98, 300 x 512: 1679 / 1626, 3832 / 3802).
 static bool behind_the_fill(const slotscan_params& p, int sms) {
     const double snaps = (double)p.B * p.H * ((p.T + p.G - 1) / p.G), esz = p.snap_dtype == SLOTSCAN_F32 ? 4.0 : 2.0;
-    const double fill_us = snaps * (p.N - 16) * (p.DK + p.DV) * esz / 4.66e6;
+    const double cols = (double)(p.N - replay_tile_rows(p.DK)) * p.DK + (double)(p.N - replay_tile_rows(p.DV)) * p.DV;
     const long long rounds = ((long long)p.B * p.H + 3 * sms - 1) / (3 * sms);
-    return fill_us > 0.74 * (double)p.T * (double)rounds;
+    return snaps * cols * esz / 4.66e6 > 1.2 * 0.74 * (double)p.T * (double)rounds;
 }
 // Where a pass leaves key rows for the next one: the final rows' place, which the replay writes later.  NULL, so that the next pass
 // starts again, where the caller gave no room for the norms or where it carries the state in place.
