@@ -498,6 +498,41 @@ def test_state_without_norms(used, occupied):
         assert torch.equal(a[n], b[n]), n
 
 
+@pytest.mark.parametrize("D,dtype,N,lengths,used,first_few,first_many", [
+    (128, torch.float32, 192, (1, 9, 64, 100), 0, "narrow<2>", "direct"), (128, torch.float32, 40, (1, 7, 8, 9, 33, 96), 0, "narrow<2>", "narrow<3>"),
+    (64, torch.bfloat16, 32, (1, 8, 17, 96), 0, "narrow<2>", "narrow<3>"), (64, torch.bfloat16, 32, (1, 8, 17), 9, "narrow<2>", "narrow<3>"),
+    (128, torch.bfloat16, 96, (1, 9, 200), 40, "wide", "direct")], ids=lambda x: str(x).split(".")[-1])
+def test_log_does_not_depend_on_the_kernel(D, dtype, N, lengths, used, first_few, first_many):
+    """The same sequences alone and among many, where other kernels scan them: the log, the last state and the rows' first tokens are
+    the same bit for bit.  Which kernel does the work is read from a profile: the first one that launches, or with a state that has
+    more rows in use than the narrow one holds (it only looks at such a sequence) the one behind it."""
+    import re
+    import slotscan_b200 as S
+    B, H, copies = 2, 3, 75
+    inp = make_inputs("gates01:3", B, max(lengths), H, D, D, seed=41)
+    gen = torch.Generator().manual_seed(3)
+    K0, V0, o0 = torch.zeros(B * H, N, D), torch.zeros(B * H, N, D), torch.zeros(B * H, N)
+    K0[:, :used], V0[:, :used] = (torch.randn(B * H, used, D, generator=gen) for _ in range(2))
+    o0[:, :used] = torch.rand(B * H, used, generator=gen)
+    def scan(n, T):
+        x = [inp[i][:, :T].repeat(n, 1, 1, *[1] * (inp[i].dim() - 3)).cuda() for i in ("k", "v", "gate", "fr", "q")]
+        x = [t.to(dtype) if t.dim() == 4 else t for t in x]
+        st = tuple(t.repeat(n, *[1] * (t.dim() - 1)).cuda() for t in (K0, V0, o0, K0.double().square().sum(-1))) if used else None
+        with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
+            lg = S.scan_with_log(*x[:4], N, 16.0, G=8, q=x[4], occ_bin=True, state=st)
+            torch.cuda.synchronize()
+        names = [e.name for e in sorted(prof.events(), key=lambda e: e.time_range.start) if "addr_fwd_" in e.name]
+        names = [re.search(r"addr_fwd_(\w+?)_kernel<\d+, (\d+)", n).groups() for n in names]
+        order = ["narrow<%s>" % c if k == "narrow" else k for k, c in names]
+        return lg, order[1 if used > 32 else 0]
+    for T in lengths:
+        few, k1 = scan(1, T)
+        many, k2 = scan(copies, T)
+        assert (k1, k2) == (first_few, first_many), T
+        for i in ("addr", "oold", "kiold", "kold", "tfirst", "ofin", "nsqfin", "kfin"):
+            assert torch.equal(few[i].repeat(copies, *[1] * (few[i].dim() - 1)), many[i]), (T, i)
+
+
 @pytest.mark.parametrize("mode", ["hard", "soft", "keyless", "read"])
 def test_plain_calls_equal_registered_ops(mode, monkeypatch):
     """Ordinary eager calls go round the custom ops' wrapping; the same call through the ops gives the same bits, values and
