@@ -162,6 +162,8 @@ cudaError_t SS_CAT(run_addr_fwd_, SLOTSCAN_SUFFIX)(const slotscan_params& p, con
 }
 
 void SS_CAT(attrs_addr_fwd_, SLOTSCAN_SUFFIX)(slotscan_kernel_attr* out, int cap, int& n) {
+    fill_attr(out, cap, n, "addr_fwd_narrow<128,rows<=32,2 CTAs>", addr_fwd_narrow_kernel<128, 2, true, false, Tin>);
+    fill_attr(out, cap, n, "addr_fwd_narrow<128,rows<=32,3 CTAs>", addr_fwd_narrow_kernel<128, 3, true, false, Tin>);
     fill_attr(out, cap, n, "addr_fwd<128,rows<=64>", addr_fwd_direct_kernel<128, 2, true, false, Tin>);
     fill_attr(out, cap, n, "addr_fwd_wide<128,rows<=192>", addr_fwd_wide_kernel<128, 6, true, false, Tin>);
 }

@@ -115,6 +115,8 @@ void attrs_rows(slotscan_kernel_attr* out, int cap, int& n) {
     fill_attr(out, cap, n, "replay_rows<128,bf16,bf16>", replay_rows_kernel<128, __nv_bfloat16, __nv_bfloat16, false, false, 16>);
     fill_attr(out, cap, n, "replay_rows<128,bf16,bf16,kinv>", replay_rows_kernel<128, __nv_bfloat16, __nv_bfloat16, true, false, 16>);
     fill_attr(out, cap, n, "replay_rows<128,f32,f32>", replay_rows_kernel<128, float, float, false, false, 16>);
+    fill_attr(out, cap, n, "replay_rows<128,bf16,bf16,16 lanes>", replay_rows_kernel<128, __nv_bfloat16, __nv_bfloat16, false, false, 8>);
+    fill_attr(out, cap, n, "replay_rows<128,f32,f32,16 lanes>", replay_rows_kernel<128, float, float, false, false, 8>);
 }
 
 }  // namespace slotscan

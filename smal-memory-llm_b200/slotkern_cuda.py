@@ -8,10 +8,10 @@ def kernel_attrs(N=None, D=None, occb=True, frt=True, eps=1e-4):
     """Signature of the reference's kernel_attrs(N, D, occb, frt, eps) (slotkern_cuda.py:467-479), which compiles for
     that shape and returns {addr_fwd, val_fwd, rows_bwd, addr_bwd: (registers, local bytes)}.  The kernels here are
     compiled ahead of time for every shape, so the arguments only pick the D = 128 entries that correspond to the
-    reference's four kernels; the full table (every instantiation, with shared memory and thread limits) is
-    slotscan_b200.kernel_attrs()."""
+    reference's four kernels (the address scan by the one that most calls start with); the table of all kernels at 128
+    columns, with shared memory and thread limits, is slotscan_b200.kernel_attrs()."""
     full = _kernel_attrs()
-    pick = {"addr_fwd": "addr_fwd<128,rows<=64>", "val_fwd": "replay_rows<128,f32,f32>",
-            "rows_bwd": "rows_bwd<128,f32,f32>", "addr_bwd": "addr_bwd_gather<128>"}
+    pick = {"addr_fwd": "addr_fwd_narrow<128,rows<=32,2 CTAs>", "val_fwd": "replay_rows<128,f32,f32>",
+            "rows_bwd": "rows_bwd<128,snap=in>", "addr_bwd": "addr_bwd_gather<128>"}
     return {ref: tuple(full[mine][:2]) for ref, mine in pick.items() if mine in full}
 

@@ -533,6 +533,19 @@ def test_log_does_not_depend_on_the_kernel(D, dtype, N, lengths, used, first_few
             assert torch.equal(few[i].repeat(copies, *[1] * (few[i].dim() - 1)), many[i]), (T, i)
 
 
+def test_kernel_attributes():
+    """The drop-in's table has an entry for each of the reference's four kernels, and the address scan's is the kernel that a call
+    starts with; the full table knows the kernels of the scan and of the replay by their variants."""
+    import slotkern_cuda
+    import slotscan_b200 as S
+    full, four = S.kernel_attrs(), slotkern_cuda.kernel_attrs(192, 128)
+    assert set(four) == {"addr_fwd", "val_fwd", "rows_bwd", "addr_bwd"}
+    assert four["addr_fwd"] == full["addr_fwd_narrow<128,rows<=32,2 CTAs>"][:2]
+    for n in ("addr_fwd_narrow<128,rows<=32,3 CTAs>", "addr_fwd<128,rows<=64>", "addr_fwd_wide<128,rows<=192>", "replay_rows<128,bf16,bf16>",
+              "replay_rows<128,bf16,bf16,16 lanes>"):
+        assert full[n][0] > 0, n
+
+
 @pytest.mark.parametrize("mode", ["hard", "soft", "keyless", "read"])
 def test_plain_calls_equal_registered_ops(mode, monkeypatch):
     """Ordinary eager calls go round the custom ops' wrapping; the same call through the ops gives the same bits, values and
