@@ -546,6 +546,31 @@ def test_kernel_attributes():
         assert full[n][0] > 0, n
 
 
+@pytest.mark.parametrize("N", [40, 192])
+def test_scores_without_a_value(N):
+    """NaN queries and infinite keys: a token none of whose scores compares greater takes the first row never addressed; alone and among
+    many sequences, where other kernels scan them, the log is the same bit for bit."""
+    import slotscan_b200 as S
+    B, T, H, D, copies = 2, 64, 3, 128, 75
+    inp = make_inputs("gates01:3", B, T, H, D, D, seed=43)
+    nan = [0, 5, 6, 18, 40, 41]
+    inp["q"][:, nan, :, 17] = float("nan")
+    inp["k"][:, 9::13, 1:, 70] = float("inf")
+    inp["k"][:, 12::17, 1:, 3] = -float("inf")
+    logs = []
+    for n in (1, copies):
+        x = [inp[i].repeat(n, *[1] * (inp[i].dim() - 1)).cuda() for i in ("k", "v", "gate", "fr", "q")]
+        lg = S.scan_with_log(*x[:4], N, 16.0, G=8, q=x[4], occ_bin=True)
+        logs.append({i: lg[i].view(n, B, T, H).cpu() for i in ("addr", "oold", "kiold")})
+    a = logs[0]["addr"][0]
+    assert (a[:, 0] == 0).all()
+    for t in nan[1:]:
+        assert torch.equal(a[:, t], (a[:, :t].amax(1) + 1).clamp(max=N - 1)), t
+    for i in logs[0]:
+        few, many = logs[0][i].expand_as(logs[1][i]), logs[1][i]
+        assert ((few == many) | (few != few) & (many != many)).all(), i
+
+
 @pytest.mark.parametrize("mode", ["hard", "soft", "keyless", "read"])
 def test_plain_calls_equal_registered_ops(mode, monkeypatch):
     """Ordinary eager calls go round the custom ops' wrapping; the same call through the ops gives the same bits, values and
