@@ -183,6 +183,36 @@ static cudaError_t fwd_run(const slotscan_params& p, const void* k, const void* 
     } else {
         e = scan_on(st);
         if (e != cudaSuccess) return e;
+        // Without a fill beside the scan (a carried-in state) the first row tile and the others run side by side too, where the chunk is
+        // long enough for the two events.  Two chunks of 512 tokens of 72 sequences, 192 rows x 128, the whole pass, one launch / two: all
+        // rows in use 1,233 / 1,142 us, few 447 / 431.  Not with the quantiser (e4m3): all rows 1,464 / 1,318, but few rows, four chunks of
+        // 1024 tokens of 48 sequences, 1,833 / 1,852: beside its walk the others' zeros cost more than they do behind one another.
+        if (qs.bits == 0 && p.T >= 256 && p.DK == p.DV && replay_first_tile_apart(p, p.DK) && (side = side_stream(st)) != nullptr) {
+            if (cudaEventCreateWithFlags(&fork, cudaEventDisableTiming) == cudaSuccess &&
+                cudaEventCreateWithFlags(&joined, cudaEventDisableTiming) == cudaSuccess) {
+                e = cudaEventRecord(fork, st);
+                if (e == cudaSuccess) {
+                    ProfScope ps(K_REPLAY_K, st);
+                    e = run_replay(p, p.DK, 2, rk, rv, gate, L.addr, L.tfirst, 0, 1, st);
+                }
+                if (e == cudaSuccess) e = cudaStreamWaitEvent(side, fork, 0);
+                if (e == cudaSuccess) {
+                    {
+                        ProfScope ps(K_REPLAY_V, side);
+                        e = run_replay(p, p.DK, 2, rk, rv, gate, L.addr, L.tfirst, 1, -1, side);
+                    }
+                    // whatever became of the launch: the second stream has joined before this call returns
+                    const cudaError_t ej = cudaEventRecord(joined, side);
+                    const cudaError_t ew = ej == cudaSuccess ? cudaStreamWaitEvent(st, joined, 0) : ej;
+                    if (e == cudaSuccess) e = ew;
+                }
+                cudaEventDestroy(fork);
+                cudaEventDestroy(joined);
+                return e;
+            }
+            if (fork != nullptr) cudaEventDestroy(fork);
+            fork = joined = nullptr;
+        }
         if (p.DK == p.DV) {
             ProfScope ps(K_REPLAY_K, st);
             return run_replay(p, p.DK, 2, rk, rv, gate, L.addr, L.tfirst, 0, -1, st);

@@ -49,6 +49,8 @@ struct ReplayPtrs { const void* x; const float* x0; void* xbuf; float* xold; flo
 cudaError_t run_replay(const slotscan_params& p, int D, int ntensors, const ReplayPtrs& r0, const ReplayPtrs& r1,
                        const float* gate, const int* am, const int* tfirst, int tile_lo, int tile_hi, cudaStream_t st);
 int replay_tile_rows(int D);
+// whether the first row tile is better replayed by a launch of its own, beside the others (few sequences; keys and values together)
+bool replay_first_tile_apart(const slotscan_params& p, int D);
 int replay_status();
 // zero-fill of rows [zk, N) of every key snapshot (+ kinv = 1e6, valid = 0 when given) and [zv, N) of every value snapshot
 cudaError_t run_zero_rows(const slotscan_params& p, void* kbuf, int zk, void* vbuf, int zv, float* kinv, uint8_t* valid,

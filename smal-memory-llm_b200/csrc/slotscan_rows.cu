@@ -25,16 +25,26 @@ static cudaError_t replay_launch(const slotscan_params& p, int ntensors, const R
         replay_rows_kernel<D, Tin, Tsn, false, false, EPL><<<grid, THREADS, 0, st>>>(p, a0, a1, gate, am, tfirst, tile_lo);
     return cudaGetLastError();
 }
-// Columns per lane of rows 128 wide: 8 while the busy tiles (one per sequence, head and tensor where few rows are in use) leave
-// SMs idle, 16 beyond that.
+// Columns per lane of rows 128 wide: 8 while the tiles that are expected to be busy leave SMs idle, 16 beyond that.  The first tile is
+// busy in every sequence, the ones after it together or not at all; a launch of all tiles goes by the first.  (us, all of 192 rows in
+// use, 8 for every tile / 16 / 8 for the first alone: 48 sequences x 909 tokens 262 / 223 / 219; 72 x 512, 3 bits 218 / 199 / 209; few rows
+// in use: 48 x 1024 97 / 112 / 95; four carried chunks of 48 x 1024 in e4m3, one launch each, 771 / 1093.)
+static int sm_count() {
+    int dev = 0, sms = 148;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    return sms;
+}
+bool replay_first_tile_apart(const slotscan_params& p, int D) {
+    return D >= 128 && p.N > replay_tile_rows(D) && (long long)p.B * p.H * 2 <= sm_count();
+}
 template <int D, typename Tin, typename Tsn>
 static cudaError_t replay_one(const slotscan_params& p, int ntensors, const ReplayPtrs& r0, const ReplayPtrs& r1,
                               const float* gate, const int* am, const int* tfirst, int tile_lo, int tile_hi, cudaStream_t st) {
     if constexpr (D >= 128) {
-        int dev = 0, sms = 148;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        if ((long long)p.B * p.H * 2 > sms)
+        const int ntiles = (p.N + ROW_THREADS / (D / 8) - 1) / (ROW_THREADS / (D / 8));
+        const int busy = tile_lo > 0 ? (tile_hi < 0 || tile_hi > ntiles ? ntiles : tile_hi) - tile_lo : 1;
+        if ((long long)p.B * p.H * 2 * busy > sm_count())
             return replay_launch<D, 16, Tin, Tsn>(p, ntensors, r0, r1, gate, am, tfirst, tile_lo, tile_hi, st);
     }
     return replay_launch<D, 8, Tin, Tsn>(p, ntensors, r0, r1, gate, am, tfirst, tile_lo, tile_hi, st);

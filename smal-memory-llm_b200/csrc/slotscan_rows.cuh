@@ -84,7 +84,8 @@ struct ReplayArgs {
 // EPL: elements per lane, 8 or 16.  With 16 a lane holds two pieces of 8 columns half a row apart (every load and store
 // of a row group stays one contiguous run of 16-byte pieces) and a CTA has half the threads: the busy tiles of a large
 // batch (one CTA per sequence, head and tensor) then all fit on the machine at once instead of in two waves.  The rows of a warp
-// walk their events one after the other, so a batch that leaves SMs idle anyway is faster with 8 (slotscan_rows.cu: replay_one).
+// walk their events one after the other, so a batch that leaves SMs idle anyway is faster with 8 (slotscan_rows.cu: replay_one); held
+// to 64 registers, for a fourth CTA to an SM, that one costs a training step of 48 sequences x 1024 tokens 9 of 700 us.
 template <int D, typename Tin, typename Tsn, bool NORM, bool QUANT, int EPL>
 __global__ void __launch_bounds__(ROW_THREADS * 8 / EPL, EPL == 16 ? (QUANT ? 4 : 6) : 1) replay_rows_kernel(
     const slotscan_params p, const ReplayArgs<Tin, Tsn> a0, const ReplayArgs<Tin, Tsn> a1,

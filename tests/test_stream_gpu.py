@@ -287,3 +287,43 @@ def test_replay_lane_split_is_bitwise(D, bits, group):
     assert 2 * (B - 1) * H <= sms < 2 * B * H
     for a, b in zip(many, few):
         assert torch.equal(a[:B - 1], b)
+
+
+@pytest.mark.parametrize("bits", [0, "e4m3"])
+def test_replay_of_a_carried_chunk_does_not_depend_on_its_launches(bits):
+    """A long chunk of few sequences has its first row tile replayed beside the others, on a second stream, one of more sequences all
+    tiles in one launch: the same snapshots, norms and final rows bit for bit, with few and with all rows in use; and a captured graph
+    of such a call gives what the call gives."""
+    S = _S()
+    D, H, N, G, T = 128, 3, 40, 8, 261
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    B = sms // (2 * H) + 1                                              # 2 * B * H just past the SMs; one sequence less: not
+    few, all_rows = (make_inputs(d, B, 2 * 264, H, D, D, seed=12) for d in ("bench", "fill"))
+    dev = {n: torch.cat([few[n][::2], all_rows[n][1::2]]).to(DEV, torch.bfloat16 if n in ("k", "v", "q") else torch.float32)
+           for n in ("k", "v", "gate", "fr", "q")}
+
+    def chunks(n):
+        sc = S.StreamingScan(N, 16.0, G=G, occ_bin=True, out_dtype=torch.bfloat16, qbits=bits, qgroup=16)
+        out = []
+        for a, b in ((0, 264), (264, 264 + T)):
+            x = {i: t[:n, a:b].contiguous() for i, t in dev.items()}
+            out += list(sc.push(x["k"], x["v"], x["gate"], x["fr"], q=x["q"]))
+        return out + [t.view(n, H, *t.shape[1:]) for t in sc.state]
+    # the order of the sequences: the few come first in both, so a shorter batch is a prefix of the longer one
+    many, less = chunks(B), chunks(B - 1)
+    assert 2 * (B - 1) * H <= sms < 2 * B * H
+    for a, b in zip(many, less):
+        assert torch.equal(a[:B - 1], b)
+    x = {i: t[:2, :T].contiguous() for i, t in dev.items()}
+    state = tuple(t[:2].flatten(0, 1).contiguous() for t in less[-4:])
+    call = lambda: S.scan_with_log(x["k"], x["v"], x["gate"], x["fr"], N, temp, G=G, q=x["q"], occ_bin=True, state=state, want_norm=True)
+    temp = torch.full((1,), 16.0, device=DEV)
+    eager = call()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        got = call()
+    graph.replay()
+    torch.cuda.synchronize()
+    for n in eager:
+        assert torch.equal(eager[n], got[n]), n
