@@ -49,24 +49,25 @@ static cudaError_t launch_wide(const slotscan_params& p, const void* q, const vo
     if (p.occ_bin) return carry ? go(addr_fwd_wide_kernel<DK, RPL, true, true, Tin>) : go(addr_fwd_wide_kernel<DK, RPL, true, false, Tin>);
     return carry ? go(addr_fwd_wide_kernel<DK, RPL, false, true, Tin>) : go(addr_fwd_wide_kernel<DK, RPL, false, false, Tin>);
 }
-// Which kernel takes the second pass.  The wide one fills an SM, so where more sequences may come than there are SMs and two or
-// more CTAs of the direct one fit beside each other, the direct one needs fewer rounds: 192 sequences, T = 256, all of 96 rows
-// x 128 in use, both passes 312 us against 396 wide, 296 sequences 429 against 517, rows of 64 (T = 512) 536 against 825.  With
-// at most a sequence per SM, or where the direct one fills an SM too (192 rows x 128), the wide one is ahead by how early the
-// sequences pass row 64: up to 128 rows always (T = 96 to 1024: 1.01 to 1.37 times as fast); past 128 rows, where it has six resolver
-// warps to wait for, from half of the tokens on (24 sequences, 192 rows x 128, T = 512, passed at 0.13 / 0.39 / 0.5 / 0.78 of
-// the tokens: 1.27 / 1.04 / 1.02 / 0.98).  A sequence passes row 64 after 64 tokens at the earliest, so below 192 tokens the
-// direct one takes it (T = 96: 0.94, T = 128: 0.97, T = 160: 0.98 to 1.06, T = 192: 0.96 to 1.12).  With a state carried in it
-// has passed already and every row is scanned from the first token on: the wide one takes a short call of however many
-// sequences (8 tokens, 444 sequences, 96 rows x 128: 63 us against 77 direct; 192 rows x 64: 66 against 86; 192 sequences, 96
-// rows x 64: 34 against 32), while in a long one the rounds count again (256 tokens, 296 sequences, 96 rows x 128: 362 against 306).
+// Which kernel takes the last pass.  The wide one fills an SM, so where more sequences may come than there are SMs and two or more
+// CTAs of the direct one fit beside each other, the direct one needs fewer rounds (each kernel starting at token 0: 192 sequences,
+// T = 256, all of 96 rows x 128 in use, 312 us against 396 wide, 296 sequences 429 against 517, rows of 64 (T = 512) 536 against 825).
+// With at most a sequence per SM the wide one is ahead at every length, the direct kernel of 64 rows left out as well (us, narrow to
+// wide / direct of 64 rows and wide / direct of 64 rows and of all; 192 rows x 128): 24 sequences x 96 tokens, all rows in use 70 / 79 /
+// 84, x 128 93 / 105 / 113; 144 x 160, clustered, 125 / 141 / 147; x 64: 144 x 160 95 / 119 / 121.  Past 128 rows, where it has six
+// resolver warps to wait for, more sequences than SMs take it from 192 tokens on (a sequence passes row 64 after 64 tokens at the
+// earliest).  With a state carried in that has more rows in use every row is scanned from the first token on: the wide one takes a short
+// call of however many sequences (8 tokens, 444 sequences, 96 rows x 128: 63 us against 77 direct; 192 rows x 64: 66 against 86; 192
+// sequences, 96 rows x 64: 34 against 32), while in a long one the rounds count again (256 tokens, 296 sequences, 96 rows x 128: 362
+// against 306).
 template <int DK>
 static bool wide_second_pass(const slotscan_params& p, bool carry) {
     int dev = 0, sms = 148;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const size_t direct = sizeof(float) * (size_t)addr_fwd_layout(p.N, DK, 6, (int)sizeof(Tin)).total + 1024;
-    if ((long long)p.B * p.H > sms && 2 * direct <= 228 * 1024 && (!carry || p.T >= 192)) return false;
+    if ((long long)p.B * p.H <= sms) return true;
+    if (2 * direct <= 228 * 1024 && (!carry || p.T >= 192)) return false;
     return p.N <= 128 || carry || p.T >= 192;
 }
 template <int DK, int CTAS>
@@ -86,7 +87,7 @@ static cudaError_t launch_narrow(const slotscan_params& p, const void* q, const 
 }
 // The passes: keys 64 or 128 wide start with the narrow kernel (32 rows), the others with the direct one.  The direct one with 64
 // rows, three CTAs to an SM, goes on with what the narrow one left, and the full-size one with the rest (slotscan_addr_fwd.cuh:
-// AfResume).  With at most a sequence per SM and 192 tokens or a carried-in state the wide kernel follows the narrow one at once: the
+// AfResume).  With at most a sequence per SM the wide kernel follows the narrow one at once: the
 // direct one between them costs a launch that does nothing where no sequence needs it (12 sequences x 256 tokens, 9 rows x 128: 71 us
 // against 76; 48 x 1024, 11 rows: 255 against 259), and the wide one is as fast from row 32 on or nearly (us, narrow to wide / with the
 // direct one between / direct to wide, no narrow one): 148 x 1024, 42 rows x 128 of 192: 820 / 745 / 626; of 96: 625 / 745 / 627;
@@ -138,7 +139,7 @@ static cudaError_t launch_dk(const slotscan_params& p, const void* q, const void
             second = 1;
         }
         const bool wide = p.N > AF_NCAP1 && wide_second_pass<DK>(p, S0.K0 != nullptr);
-        if (!wide || BH > sms || (p.T < 192 && S0.K0 == nullptr)) {
+        if (!wide || BH > sms) {
             e = launch_one<DK, 2>(p, q, k, gate, fr, temp, L, S0, p.N <= AF_NCAP1 ? p.N : AF_NCAP1, second, hand, st);
             if (e != cudaSuccess || p.N <= AF_NCAP1) return e;
         }
