@@ -12,10 +12,12 @@
 //   loader warps    2: everything that is not per token: rows of the chunk after next, token constants, log.
 // Resolver, norm and column warps run one token apart and meet at one barrier per token, as in the direct kernel; the loaders meet
 // the resolver once per chunk of 8.
-// B200, about 11 of 192 rows x 128 in use, this kernel against the direct one alone: 48 sequences x 1024 tokens, bf16: 497 -> 273 us;
-// 12 x 256, float32: 126 -> 66; 3072 x 128 (96 rows), three CTAs to an SM: 632 -> 433.
+// B200, about 11 of 192 rows x 128 in use, this kernel against the direct one, each on its own: 48 sequences x 1024 tokens, bf16: 497 ->
+// 251 us (487 cycles per token; 271 us beside the zero-fill); 12 x 256, float32: 126 -> 67; 3072 x 128 (96 rows), three CTAs to an SM:
+// 632 -> 433 (80 registers; at 128 columns 32 bytes are spilled, where the pieces of the rows change lanes).
 #pragma once
 #include "slotscan_addr_fwd.cuh"
+#include "slotscan_async.cuh"
 
 namespace slotscan {
 
@@ -41,10 +43,6 @@ __host__ __device__ inline AddrNarrowSmem addr_narrow_layout(int DK) {
     L.total = L.K + AN_RING * DK;
     return L;
 }
-__device__ __forceinline__ void cp_async16(void* dst, const void* src) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 __device__ __forceinline__ float redux_max(float v) {
     float r;
     asm volatile("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));

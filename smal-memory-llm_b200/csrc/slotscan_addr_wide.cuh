@@ -10,12 +10,12 @@
 //                   warp of the CTA takes the largest of the entries for itself;
 //   helper warps    2, every other token each: loads in registers three of its tokens ahead, then into a ring in shared
 //                   memory with the token's constants; the log out.
-// The roles run one token apart as in the direct kernel (see its schedule comment), one barrier per token.  Every warp issues an instruction about every five cycles, so what counts is the longest role's
-// instructions per token.  One CTA fills an SM, as the direct kernel's 192 rows did; it is the second pass, of sequences that
-// use more than AF_NCAP1 rows, where that pays (wide_second_pass): with few rows the direct kernel's split of a row over lanes is
-// shorter.  B200, second
-// pass alone: 192 sequences x 1024 tokens, 192 rows x 128 all in use, bf16: 2.27 -> 1.74 ms (two CTAs' worth of rounds on 148 SMs;
-// column warps of three slots: 2.02); 48 x 1000, ~60 rows x 64, float32: 0.81 -> 0.56; 24 x 8 carried-in tokens: 31 -> 17 us.
+// The roles run one token apart as in the direct kernel (see its schedule comment), one barrier per token.  Every warp issues an
+// instruction about every five cycles, so what counts is the longest role's instructions per token.  One CTA fills an SM, as the direct
+// kernel's 192 rows did; it is the last pass where that pays (slotscan_addr_fwd_inst.cuh: wide_second_pass), with at most a sequence per
+// SM right behind the narrow kernel.  B200, against the full-size direct kernel, each on its own: 192 sequences x 1024 tokens, 192 rows
+// x 128 all in use, bf16: 2.27 -> 1.60 ms (two CTAs' worth of rounds on 148 SMs; column warps of three slots: 2.02); 48 x 1000, ~60 rows
+// x 64, float32: 0.81 -> 0.53; 24 x 8 carried-in tokens: 31 -> 17 us.
 #pragma once
 #include "slotscan_addr_fwd.cuh"
 

@@ -1,5 +1,5 @@
-// Bulk asynchronous copies into shared memory and the mbarrier that counts their bytes (sm_90 and later): the staging
-// path of the kernels that stream token chunks or snapshot tiles.  Every wait is bounded.
+// Asynchronous copies into shared memory: the staging path of the kernels that stream token chunks or snapshot tiles.  Bulk copies with
+// the mbarrier that counts their bytes (sm_90 and later; every wait is bounded), and 16 bytes per thread.
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -46,6 +46,12 @@ template <int PENDING>
 __device__ __forceinline__ void bulk_wait_read() { asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(PENDING) : "memory"); }
 template <int PENDING>
 __device__ __forceinline__ void bulk_wait() { asm volatile("cp.async.bulk.wait_group %0;" ::"n"(PENDING) : "memory"); }
+
+// ---- 16 bytes global -> shared per thread, both addresses 16-byte aligned; wait_all: for this thread's own copies ----
+__device__ __forceinline__ void cp_async16(void* dst, const void* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
 // Bounded wait: a copy that never lands must not hang the GPU.  Returns false after ~0.2 s of polling.
 __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, unsigned parity) {

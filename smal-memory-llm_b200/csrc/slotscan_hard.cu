@@ -78,8 +78,8 @@ struct ProfScope {
 
 constexpr size_t SMEM_CAP = 227 * 1024;
 
-// Extra streams so that the sequential address scan and the zero-fill of the snapshot rows its first pass cannot touch
-// run side by side: one per (device, caller stream), created on first use and kept until the process exits, so that
+// Extra streams so that the sequential address scan and the zero-fill of the snapshot rows past the first replay tile, or two parts of
+// the replay, run side by side: one per (device, caller stream), created on first use and kept until the process exits, so that
 // callers that work on several streams of a device at once (a pipeline over batch chunks) keep their scans independent
 // of one another.  Beyond SIDE_STREAMS_MAX caller streams per device the extra streams are shared round-robin.
 constexpr int MAX_DEVICES = 64;

@@ -9,7 +9,8 @@
 
 namespace slotscan {
 
-// rows a first-pass CTA of the address kernels holds in shared memory (sequences that need more rerun at full size)
+// rows that the smaller direct address scan and the smaller address backward hold in shared memory, three CTAs to an SM (a sequence that
+// needs more goes on, or in the backward is taken, by a kernel that holds all)
 constexpr int AF_NCAP1 = 64;
 
 template <typename F>

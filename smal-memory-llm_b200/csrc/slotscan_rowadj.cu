@@ -19,15 +19,13 @@
 // tokens a step); 48 sequences, 192 x (64 + 64), 32 blocks of 16: 0.42 ms.
 #include <algorithm>
 
+#include "slotscan_async.cuh"
 #include "slotscan_common.cuh"
 #include "slotscan_launch.h"
 #include "slotscan_rowadj.cuh"
 
 namespace slotscan {
 
-__device__ __forceinline__ void ra_cp16(void* dst, const void* src) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
-}
 __device__ __forceinline__ void ra_cp4(void* dst, const void* src) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
 }
@@ -81,7 +79,7 @@ __global__ void __maxnreg__(DS == 32 ? 168 : 255) row_adjoint_kernel(const RowAd
         const float* base = src + (((size_t)b * NB + jb) * H + h) * N * D + d0;
         if (vec) {
             const int q = dn >> 2;
-            for (int i = tid; i < N * q; i += NT) { const int r = i / q, c = (i % q) * 4; ra_cp16(dst + r * SS + c, base + (size_t)r * D + c); }
+            for (int i = tid; i < N * q; i += NT) { const int r = i / q, c = (i % q) * 4; cp_async16(dst + r * SS + c, base + (size_t)r * D + c); }
         } else {
             for (int i = tid; i < N * dn; i += NT) { const int r = i / dn, c = i % dn; ra_cp4(dst + r * SS + c, base + (size_t)r * D + c); }
         }

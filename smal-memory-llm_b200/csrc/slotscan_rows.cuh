@@ -259,10 +259,9 @@ __global__ void __launch_bounds__(ROW_THREADS * 8 / EPL, EPL == 16 ? (QUANT ? 4 
 
 // ======================================================================================================
 // Zero-fill of the rows [zero_from, N) of every snapshot (and their kinv = 1e6 / valid = 0), launched on a second
-// stream while the sequential address scan runs: the scan needs almost no memory bandwidth, and its first pass holds
-// only the first AF_NCAP1 rows, so every sequence that finishes in that pass leaves the rows above untouched -- they
-// are zero in every snapshot.  Sequences that do need them (second pass) rewrite those tiles afterwards in the replay,
-// which is ordered after this kernel.  Small CTAs (2 warps, few registers) so that they fit beside the scan's CTAs.
+// stream while the sequential address scan runs: the scan needs almost no memory bandwidth, rows are taken in index order, and most
+// sequences never take one past the first replay tile -- those rows are zero in every snapshot.  Sequences that do take them rewrite
+// their tiles afterwards in the replay, which is ordered after this kernel.  Small CTAs (2 warps, few registers) so that they fit beside the scan's CTAs.
 constexpr int ZR_THREADS = 64;
 template <typename Tsn>
 __global__ void __launch_bounds__(ZR_THREADS) zero_rows_kernel(Tsn* __restrict__ xbuf, float* __restrict__ kinv,
