@@ -14,7 +14,7 @@
 // instruction about every five cycles, so what counts is the longest role's instructions per token.  One CTA fills an SM, as the direct
 // kernel's 192 rows did; it is the last pass where that pays (slotscan_addr_fwd_inst.cuh: wide_second_pass), with at most a sequence per
 // SM right behind the narrow kernel.  B200, against the full-size direct kernel, each on its own: 192 sequences x 1024 tokens, 192 rows
-// x 128 all in use, bf16: 2.27 -> 1.60 ms (two CTAs' worth of rounds on 148 SMs; column warps of three slots: 2.02); 48 x 1000, ~60 rows
+// x 128 all in use, bf16: 2.27 -> 1.62 ms (two CTAs' worth of rounds on 148 SMs; column warps of three slots: 2.02); 48 x 1000, ~60 rows
 // x 64, float32: 0.81 -> 0.53; 24 x 8 carried-in tokens: 31 -> 17 us.
 #pragma once
 #include "slotscan_addr_fwd.cuh"
