@@ -91,7 +91,10 @@ int slotscan_hard_fwd(const slotscan_params* p, const void* k, const void* q, co
  *                state.  A long context is streamed chunk by chunk this way with memory constant in T.
  *   nsq0         (B*H,N) f64: squared key norms carried with the state (nsqfin of the preceding call).  NULL: they are
  *                summed again from K0, which may move a score by one float32 ulp against the unchunked scan.
- *   nsqfin       (B*H,N) f64 out: squared key norms of the final state as the scan carried them.
+ *   nsqfin       (B*H,N) f64 out: squared key norms of the final state as the scan carried them.  With it a sequence that takes
+ *                more rows than the kernel in work holds goes on in the next one (kfin, ofin, nsqfin, addr hold its state in
+ *                between); without it, or where the state is carried in place (K0 = kfin, o0 = ofin, nsq0 = nsqfin), such a
+ *                sequence is scanned again from its first token: the same results, later.
  *   kinv, valid  (B,NB,H,N) f32 / bytes out, both or neither: rsqrt(max(|K_n|^2, 1e-12)) and [|K_n|^2 > 1e-12] of every
  *                emitted key row, taken from the float32 state while the row is in registers (what memlm_sh.py:474-475
  *                computes from the float32 kbuf before casting it): no separate pass over the snapshots.
